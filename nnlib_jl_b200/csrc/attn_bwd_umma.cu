@@ -61,7 +61,13 @@ static_assert(BwCfg<128, true>::kSmemBytes <= 232448 && BwCfg<128, false>::kSmem
 
 struct BwBarriers {
   uint64_t fix_full, a_full[3], a_empty[3], b_full[2], b_empty[2];
-  uint64_t s_full, dp_full, s_read, ds_ready, acc_full, col_ready;
+  uint64_t s_full, dp_full, s_read, acc_full, col_ready;
+  // dS of step it is handed over on ds_ready[it & 1].  The dq half issues S and dP of step it + 1 before the dS of
+  // step it is complete, so a warp with little to do (rows past the end of the sequence) can be through step it + 1
+  // while another still works on step it: on one barrier its second arrival stood in for the slow warp's first, and
+  // the products read a dS that was not there yet.  (It cannot be two steps ahead: step it + 2 waits until the
+  // products of step it have read its dS buffer.)
+  uint64_t ds_ready[2];
   uint64_t dp_read;    // dq half: dP is in registers
   uint64_t pt_ready;   // dk/dv half: P^T is in shared memory
   uint32_t tmem_base;
@@ -214,7 +220,8 @@ attn_bwd_umma_kernel(const __grid_constant__ CUtensorMap tm_fa, const __grid_con
     mbar_init(&bars->s_full, 1);
     mbar_init(&bars->dp_full, 1);
     mbar_init(&bars->s_read, 8);
-    mbar_init(&bars->ds_ready, 8);
+    mbar_init(&bars->ds_ready[0], 8);
+    mbar_init(&bars->ds_ready[1], 8);
     mbar_init(&bars->acc_full, 1);
     mbar_init(&bars->col_ready, 8);
     mbar_init(&bars->dp_read, 8);
@@ -368,12 +375,12 @@ attn_bwd_umma_kernel(const __grid_constant__ CUtensorMap tm_fa, const __grid_con
             tc_fence_after();
             issue_dp(it + 1);
           }
-          ok = mbar_wait(&bars->ds_ready, par, abort_flag);
+          ok = mbar_wait(&bars->ds_ready[it & 1], (it >> 1) & 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
           issue_ds_acc(it);
         } else {
-          ok = mbar_wait(&bars->ds_ready, par, abort_flag);
+          ok = mbar_wait(&bars->ds_ready[it & 1], (it >> 1) & 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
           issue_ds_acc(it);
@@ -681,7 +688,7 @@ attn_bwd_umma_kernel(const __grid_constant__ CUtensorMap tm_fa, const __grid_con
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->ds_ready);
+      if (lane == 0) mbar_arrive(&bars->ds_ready[par]);
 
       if (BIAS && !DKV && dbias_p) {
         // gradient of the bias = dS in fp32 (masked and dropped-out positions included: they are zero /

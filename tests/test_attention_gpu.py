@@ -1633,3 +1633,18 @@ def test_random_configurations_with_an_opaque_fdrop(seed):
     yo, ao = O.dot_product_attention(qn, kn, vn, mask=mask_np, nheads=H, fdrop=lambda al: al * keep_np / np.float32(0.7))
     _close(an, ao, dtype, "alpha', " + what)
     _close(nb.jl_to_numpy(y), yo, dtype, "x, " + what)
+
+
+def test_query_gradient_of_a_ragged_tile_is_the_same_every_time():
+    """A query tile whose last warps have no rows: those warps run ahead of the others by almost a step, and their
+    arrivals must not stand in for a slow warp's.  dq is computed without atomics, so 400 runs give the same bits."""
+    rng = np.random.default_rng(24)
+    d, H, Lq, Lkv, B = 48, 3, 333, 295, 2
+    q, k, v, dy = (_dev(_round_to(rng.standard_normal((d * H, n, B)), torch.bfloat16), torch.bfloat16)
+                   for n in (Lq, Lkv, Lkv, Lq))
+    bias = _dev(_round_to(0.5 * rng.standard_normal((Lkv, 1, 1, B)), torch.bfloat16), torch.bfloat16)
+    mask = nb.jl_from_numpy(np.arange(Lkv)[:, None, None, None] < np.array([226, 168])[None, None, None, :], device=DEV)
+    x, _, back = nb.dot_product_attention_pullback(q, k, v, bias, mask=mask, nheads=H, fdrop=nb.PhiloxDropout(0.25, seed=7))
+    first = back(dy)[0].clone()
+    assert back.path == nb._lib.PATH_UMMA
+    assert all(torch.equal(back(dy)[0], first) for _ in range(400))
