@@ -219,6 +219,11 @@ int attention_both(const nnlib_b200_attn_params* p, void* stream) {
     log_call("attention", p, a, "tcgen05 (x and alpha in one pass)", nullptr);
     return finish(short_attention(a, p->dtype, (cudaStream_t)stream));
   }
+  // (the tensor-core paths of the two halves are asked first: Float32 in fast math mode takes those)
+  if (a.Lq > 0 && a.B > 0 && !force_simt() && !use_tile(a, p->dtype, true) && fma_row_supports(a, p->dtype)) {
+    log_call("attention", p, a, "cuda-core (x and alpha in one pass)", simt_reason(a, p->dtype, true));
+    return finish(fma_row(a, p->dtype, (cudaStream_t)stream));
+  }
   rc = nnlib_b200_attn_fwd(p, stream);
   if (rc) return rc;
   return nnlib_b200_attn_scores(p, stream);
@@ -246,7 +251,7 @@ int nnlib_b200_attn_fwd(const nnlib_b200_attn_params* p, void* stream) {
   }
   if (!simt_supports(a.d, a.dv)) return NNLIB_B200_UNSUPPORTED_SHAPE;
   log_call("attn_fwd", p, a, "cuda-core", simt_reason(a, p->dtype, true));
-  return finish(simt_fwd(a, p->dtype, st));
+  return finish(!force_simt() && fma_supports(a.d, a.dv) ? fma_fwd(a, p->dtype, st) : simt_fwd(a, p->dtype, st));
 }
 
 // does the split-key forward apply to this call, and is it worth it (a long key sequence, too few units to
@@ -298,7 +303,7 @@ int nnlib_b200_attn_stats(const nnlib_b200_attn_params* p, void* stream) {
   }
   if (!simt_supports(a.d, 1)) return NNLIB_B200_UNSUPPORTED_SHAPE;
   log_call("attn_stats", p, a, "cuda-core", simt_reason(a, p->dtype, false));
-  return finish(simt_stats(a, p->dtype, st));
+  return finish(!force_simt() && fma_supports(a.d, 1) ? fma_stats(a, p->dtype, st) : simt_stats(a, p->dtype, st));
 }
 
 int nnlib_b200_attn_scores(const nnlib_b200_attn_params* p, void* stream) {
@@ -317,7 +322,7 @@ int nnlib_b200_attn_scores(const nnlib_b200_attn_params* p, void* stream) {
   }
   if (!simt_supports(a.d, 1)) return NNLIB_B200_UNSUPPORTED_SHAPE;
   log_call("attn_scores", p, a, "cuda-core", simt_reason(a, p->dtype, false));
-  return finish(simt_scores(a, p->dtype, st));
+  return finish(!force_simt() && fma_supports(a.d, 1) ? fma_scores(a, p->dtype, st) : simt_scores(a, p->dtype, st));
 }
 
 int nnlib_b200_attn_apply(const nnlib_b200_attn_params* p, void* stream) {
@@ -333,7 +338,8 @@ int nnlib_b200_attn_apply(const nnlib_b200_attn_params* p, void* stream) {
   log_call("attn_apply", p, a, "cuda-core", force_simt() ? "NNLIB_B200_FORCE_SIMT is set"
                                                          : "16-bit arrays with dv a multiple of 8 up to 128, Lkv % 8 == 0 and "
                                                            "16-byte aligned rows only");
-  return finish(simt_apply(a, p->dtype, (cudaStream_t)stream));
+  return finish(!force_simt() && fma_supports(1, a.dv) ? fma_apply(a, p->dtype, (cudaStream_t)stream)
+                                      : simt_apply(a, p->dtype, (cudaStream_t)stream));
 }
 
 // shared front half of attn_bwd / attn_bwd_path: validates and resolves both argument blocks

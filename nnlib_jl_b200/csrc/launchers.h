@@ -19,6 +19,16 @@ cudaError_t simt_apply(const AttnArgs& a, int dtype, cudaStream_t st);
 cudaError_t causal_fill(unsigned char* m, long long L, cudaStream_t st);
 cudaError_t causal_check(const unsigned char* m, long long L, int* flag, cudaStream_t st);
 
+// tiled CUDA-core kernels, head sizes up to 128 (attn_fma.cu, attn_bwd_fma.cu)
+bool fma_supports(int d, int dv);
+cudaError_t fma_fwd(const AttnArgs& a, int dtype, cudaStream_t st);
+cudaError_t fma_stats(const AttnArgs& a, int dtype, cudaStream_t st);
+cudaError_t fma_scores(const AttnArgs& a, int dtype, cudaStream_t st);
+cudaError_t fma_apply(const AttnArgs& a, int dtype, cudaStream_t st);
+bool fma_row_supports(const AttnArgs& a, int dtype);     // x, alpha and lse in one pass (short key sequences)
+cudaError_t fma_row(const AttnArgs& a, int dtype, cudaStream_t st);
+cudaError_t fma_bwd(const AttnArgs& a, const BwdArgs& g, int dtype, cudaStream_t st);
+
 // backward on CUDA cores (attn_bwd_simt.cu)
 bool simt_bwd_supports(int d, int dv);
 cudaError_t simt_bwd(const AttnArgs& a, const BwdArgs& g, int dtype, cudaStream_t st);
@@ -52,7 +62,8 @@ bool umma_bwd_supports(const AttnArgs& a, const BwdArgs& g, int dtype);
 cudaError_t umma_bwd(const AttnArgs& a, const BwdArgs& g, int dtype, cudaStream_t st);
 cudaError_t umma_bwd_take_abort(int* out, cudaStream_t st);
 
-// strided-batched matrix product (gemm_umma.cu): tcgen05 kernel for 16-bit arrays, CUDA-core kernel for the rest
+// strided-batched matrix product: tcgen05 kernel for 16-bit arrays (gemm_umma.cu), CUDA-core kernel for the rest
+// (gemm_fma.cu)
 const char* gemm_umma_reject_reason(const GemmArgs& g, int dtype);
 cudaError_t gemm_umma(const GemmArgs& g, int dtype, cudaStream_t st);
 cudaError_t gemm_simt(const GemmArgs& g, int dtype, cudaStream_t st);

@@ -1648,3 +1648,97 @@ def test_query_gradient_of_a_ragged_tile_is_the_same_every_time():
     first = back(dy)[0].clone()
     assert back.path == nb._lib.PATH_UMMA
     assert all(torch.equal(back(dy)[0], first) for _ in range(400))
+
+
+# --------------------------------------------------------------------------
+# tiled CUDA-core kernels (exact Float32)
+# --------------------------------------------------------------------------
+
+@pytest.mark.parametrize("d,dv,H,Lq,Lkv,B,kind,drop", [
+    (64, 64, 2, 1, 65, 1, "none", 0.0),         # one query (blocks of 8), one key past a tile
+    (64, 64, 2, 8, 300, 2, "offset", 0.0),      # a full block of 8
+    (128, 128, 1, 33, 64, 1, "pad", 0.2),       # one query past a block of 32, one exact key tile
+    (32, 32, 4, 129, 63, 5, "none", 0.1),       # one key short of a tile
+    (40, 40, 4, 127, 127, 40, "causal", 0.0),   # enough units for blocks of 64
+    (80, 96, 8, 200, 333, 10, "window", 0.1),   # dv != d; blocks of 64, ragged in both directions
+    (33, 7, 2, 50, 70, 2, "pad", 0.0),          # rows that are not 16-byte aligned: element-wise copies
+    (64, 64, 2, 96, 640, 1, "causal0", 0.0),    # Lkv too long for the one-pass x + alpha kernel
+    (128, 64, 2, 40, 260, 1, "offset-", 0.0),   # the first queries see no key at all
+])
+def test_float32_tiles_match_the_oracle(d, dv, H, Lq, Lkv, B, kind, drop):
+    """Exact Float32 on the tiled CUDA-core kernels at the edges of their tiles, x, alpha (lazy and eager: two
+    kernels each way), and all gradients, against the oracle."""
+    dtype = torch.float32
+    rng = np.random.default_rng(1000 + d + Lq + Lkv)
+    qn, kn = (rng.standard_normal((d * H, L, B), dtype=np.float32) for L in (Lq, Lkv))
+    vn = rng.standard_normal((dv * H, Lkv, B), dtype=np.float32)
+    dyn = rng.standard_normal((dv * H, Lq, B), dtype=np.float32)
+    bn = (0.5 * rng.standard_normal((Lkv, Lq, H, 1))).astype(np.float32) if kind in ("window", "pad") else None
+    mask_np, mask = None, None
+    if kind in ("causal", "causal0", "offset", "offset-"):
+        off = {"offset": Lkv - Lq, "offset-": -7}.get(kind, 0)
+        mask_np, mask = _offset_mask(Lkv, Lq, off), nb.CausalMask(off)
+    elif kind == "pad":
+        lens = rng.integers((Lkv + 1) // 2, Lkv + 1, size=B)
+        mask_np = np.arange(Lkv)[:, None, None, None] < lens[None, None, None, :]
+    elif kind == "window":
+        back = np.arange(Lq)[None, :] - np.arange(Lkv)[:, None]
+        mask_np = (back >= -40) & (back < 60)
+    if mask_np is not None and mask is None:
+        mask = nb.jl_from_numpy(mask_np, device=DEV)
+    q, k, v, dy = (_dev(t, dtype) for t in (qn, kn, vn, dyn))
+    bias = None if bn is None else _dev(bn, dtype)
+    assert _path(q, k, v, H) == _lib.PATH_SIMT
+    fdrop = lambda: nb.PhiloxDropout(drop, seed=9, offset=3) if drop else nb.identity
+    keep = P.keep_mask((Lkv, Lq, H, B), drop, 9, 3) if drop else None
+    with np.errstate(invalid="ignore"):
+        yo, ao = O.dot_product_attention(qn, kn, vn, bn, mask=mask_np, nheads=H,
+                                         fdrop=(lambda al: al * keep / np.float32(1 - drop)) if drop else (lambda al: al))
+    live = np.ones(Lq, bool) if mask_np is None else np.broadcast_to(
+        O._bcast_to_scores(mask_np), (Lkv, Lq, H, B)).any(axis=(0, 2, 3))
+    y, a = nb.dot_product_attention(q, k, v, bias, mask=mask, nheads=H, fdrop=fdrop())
+    nb.set_scores_mode("eager")
+    try:
+        y2, a2 = nb.dot_product_attention(q, k, v, bias, mask=mask, nheads=H, fdrop=fdrop())
+    finally:
+        nb.set_scores_mode("lazy")
+    for what, yt, at in (("lazy", y, np.asarray(a)), ("eager", y2, nb.jl_to_numpy(a2))):
+        yn = nb.jl_to_numpy(yt)
+        _close(yn[:, live], yo[:, live], dtype, "x, " + what)
+        _close(at[:, live], ao[:, live], dtype, "alpha, " + what)
+        assert np.isnan(yn[:, ~live]).all() and np.isnan(at[:, ~live]).all()
+    xt, _, back = nb.dot_product_attention_pullback(q, k, v, bias, mask=mask, nheads=H, fdrop=fdrop())
+    if live.all():
+        grads = back(dy)
+        want = O.dot_product_attention_grad(qn, kn, vn, dyn, bn, mask=mask_np, nheads=H, keep=keep, p=drop)
+        for name, got, w in zip(("dq", "dk", "dv", "dbias"), grads, want):
+            if got is not None:
+                _grad_close(nb.jl_to_numpy(got), w, dtype, name)
+
+
+def test_float32_masked_keys_may_hold_anything():
+    """A key that the mask takes out contributes nothing, whatever its rows of k and v hold: x, alpha and the
+    gradients of the kept ones are those of the same arrays with zeros there (the tiled kernels leave a zero
+    weight's row out when a tile holds a value that is not finite)."""
+    rng = np.random.default_rng(77)
+    d, H, Lq, Lkv, B = 64, 2, 70, 200, 2
+    E = d * H
+    qn, kn, vn, dyn = (rng.standard_normal((E, L, B), dtype=np.float32) for L in (Lq, Lkv, Lkv, Lq))
+    keep = np.arange(Lkv) < 150
+    kb, vb = kn.copy(), vn.copy()
+    kb[:, ~keep], vb[:, ~keep] = np.nan, np.inf
+    kn[:, ~keep], vn[:, ~keep] = 0, 0
+    mask = nb.jl_from_numpy(keep.reshape(Lkv, 1, 1, 1), device=DEV)
+    out = []
+    for kk, vv in ((kn, vn), (kb, vb)):
+        q, k, v, dy = (_dev(t, torch.float32) for t in (qn, kk, vv, dyn))
+        x, a, back = nb.dot_product_attention_pullback(q, k, v, mask=mask, nheads=H)
+        dq, dk, dv, _ = back(dy)
+        nb.set_scores_mode("eager")
+        try:
+            x2, a2 = nb.dot_product_attention(q, k, v, mask=mask, nheads=H)
+        finally:
+            nb.set_scores_mode("lazy")
+        out.append([nb.jl_to_numpy(t) for t in (x, a.materialize(), dq, dk, dv, x2, a2)])
+    for want, got in zip(*out):
+        np.testing.assert_array_equal(got, want)
