@@ -266,26 +266,6 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tm_n, const __grid_constant
   }
 }
 
-// ---- any shape, stride and element type on the CUDA cores: one thread per element of C ---------------
-template <typename T>
-__global__ void __launch_bounds__(256) gemm_simt_kernel(const GemmArgs g) {
-  const int m = blockIdx.x * 32 + (threadIdx.x & 31);
-  const int n = blockIdx.y * 8 + (threadIdx.x >> 5);
-  const int b = blockIdx.z;
-  if (m >= g.M || n >= g.N) return;
-  const T* A = reinterpret_cast<const T*>(g.A) + (g.a_bcast ? 0 : (long long)b * g.strideA);
-  const T* B = reinterpret_cast<const T*>(g.B) + (g.b_bcast ? 0 : (long long)b * g.strideB);
-  const long long a_m = g.transA ? g.lda : 1, a_k = g.transA ? 1 : g.lda;
-  const long long b_k = g.transB ? g.ldb : 1, b_n = g.transB ? 1 : g.ldb;
-  float acc = 0.f;
-  for (int k = 0; k < g.K; ++k)
-    acc = fmaf(Elem<T>::to_f(A[m * a_m + k * a_k]), Elem<T>::to_f(B[k * b_k + n * b_n]), acc);
-  T* c = reinterpret_cast<T*>(g.C) + (long long)b * g.strideC + (long long)n * g.ldc + m;
-  float out = g.alpha * acc;
-  if (g.beta != 0.f) out = fmaf(g.beta, Elem<T>::to_f(*c), out);
-  *c = Elem<T>::from_f(out);
-}
-
 // (contiguous extent, rows, batch) view of one operand with the box its layout needs:
 // K-major: contiguous = K, box 64 x 128; MN-major: contiguous = M or N, box 64 x 64
 bool make_operand_map(CUtensorMap* m, const void* base, int dtype, long long contiguous, long long rows, long long batch,
@@ -379,20 +359,6 @@ cudaError_t gemm_umma(const GemmArgs& g0, int dtype, cudaStream_t st) {
 #undef NB_G3
 #undef NB_G4
   return cudaErrorInvalidValue;
-}
-
-cudaError_t gemm_simt(const GemmArgs& g, int dtype, cudaStream_t st) {
-  if (g.M < 1 || g.N < 1 || g.batch < 1) return cudaSuccess;
-  const long long gx = (g.M + 31) / 32, gy = (g.N + 7) / 8;
-  if (gx > 0x7fffffffLL || gy > 65535 || g.batch > 65535) return cudaErrorInvalidConfiguration;
-  const dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)g.batch);
-  switch (dtype) {
-    case NNLIB_B200_F16:  gemm_simt_kernel<__half><<<grid, 256, 0, st>>>(g); break;
-    case NNLIB_B200_BF16: gemm_simt_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(g); break;
-    default:              gemm_simt_kernel<float><<<grid, 256, 0, st>>>(g); break;
-  }
-  count_launch();
-  return cudaGetLastError();
 }
 
 // Reads and clears the sticky "a bounded wait ran out" flag of the product kernels on the current device.

@@ -189,3 +189,23 @@ def test_random_products_match_the_oracle(seed):
     nb.batched_mul_(Cd, opA, opB, alpha, beta)
     want = BO.batched_gemm(ta, tb, np.float32(alpha), An, Bn, np.float32(beta), Cn)
     _close(nb.jl_to_numpy(Cd), want, dtype, what)
+
+
+@pytest.mark.parametrize("ta,tb", [("N", "N"), ("T", "N"), ("N", "T"), ("T", "T")])
+@pytest.mark.parametrize("M,N,K,nbatch", [
+    (1, 1, 1, 1),             # smallest
+    (33, 31, 17, 2),          # 32 x 32 tiles, one K element past a stage
+    (65, 130, 16, 50),        # 64 x 64 tiles, exactly one stage
+    (257, 127, 33, 60),       # 128 x 128 tiles, ragged in every dimension
+])
+def test_float32_product_tiles(ta, tb, M, N, K, nbatch):
+    rng = np.random.default_rng(M + N + K)
+    An = rng.standard_normal((M, K, nbatch) if ta == "N" else (K, M, nbatch)).astype(np.float32)
+    Bn = rng.standard_normal((K, N, nbatch) if tb == "N" else (N, K, nbatch)).astype(np.float32)
+    A, B = _dev(An, torch.float32), _dev(Bn, torch.float32)
+    got = nb.jl_to_numpy(nb.batched_mul(A if ta == "N" else nb.batched_transpose(A), B if tb == "N" else nb.batched_transpose(B)))
+    a64, b64 = (An if ta == "N" else An.transpose(1, 0, 2)).astype(np.float64), (Bn if tb == "N" else Bn.transpose(1, 0, 2)).astype(np.float64)
+    want = np.einsum("mkb,knb->mnb", a64, b64)
+    # each of K fused multiply-adds rounds once: |error| <= K 2^-24 sum_k |a b|
+    bound = K * 2.0 ** -24 * np.einsum("mkb,knb->mnb", np.abs(a64), np.abs(b64)) + 1e-30
+    assert (np.abs(got - want) <= bound).all()
