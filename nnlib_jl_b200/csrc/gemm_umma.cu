@@ -19,7 +19,11 @@
 //   warp 0      TMA producer: a ring of stages, each holding the n-side rows
 //               and the m-side rows of one K block (128-byte swizzle)
 //   warp 1      allocates tensor memory, issues every tcgen05.mma
-//   warps 2-9   epilogue: TMEM -> registers -> alpha / beta -> C
+//   warps 2-9   epilogue: TMEM -> registers -> alpha / beta -> C.  Without beta and with 16-byte aligned columns a
+//               warp stages 32 columns n x 64 rows m in shared memory and sends them off as one TMA store: a
+//               thread's own 16-byte stores touch 32 different columns per instruction, which the load / store
+//               unit takes one by one (2048 x 2048 x 64, batch 64: the 537 MB of C took 207 us = 2.8 TB/s that way,
+//               106 us = 5.4 TB/s so)
 // Whether an operand is K-major or MN-major in shared memory follows from the
 // transpose flags: op(A) = A ('N') has m contiguous (MN-major), A^T ('T') has k
 // contiguous (K-major); B ('N') has k contiguous (K-major), B^T has n contiguous.
@@ -47,15 +51,20 @@ struct GCfg {
   static constexpr int kNBytes = NH * kHalfBytes;
   static constexpr int kMBytes = (MT / 128) * kHalfBytes;
   static constexpr int kStage = kNBytes + kMBytes;
-  static constexpr int kStages = (200 * 1024) / kStage;          // 3 (64 KB), 4 (48 KB), 6 (32 KB)
+  // epilogue staging: per warp one (NH = 2, whose ring needs the room) or two boxes of 32 columns x 128 bytes
+  static constexpr int kOutBufs = (NH == 2) ? 1 : 2;
+  static constexpr int kOutBytes = 8 * kOutBufs * 4096;
+  static constexpr int kStages = (226 * 1024 - kOutBytes) / kStage;   // 3 (64 KB), 3 (48 KB), 5 (32 KB)
   static constexpr int kAccCols = NH * MT;                       // fp32 columns of one tile
   static constexpr int kAccBufs = (kAccCols <= 256) ? 2 : 1;
   static constexpr int kTmemCols = (kAccCols * kAccBufs <= 256) ? 256 : 512;
-  static constexpr int kBarOff = kStages * kStage;
+  static constexpr int kOutOff = kStages * kStage;
+  static constexpr int kBarOff = kOutOff + kOutBytes;
   static constexpr int kSmemBytes = kBarOff + 256 + 1024;
 };
-static_assert(GCfg<2, 256>::kStages == 3 && GCfg<1, 256>::kStages == 4 && GCfg<1, 128>::kStages == 6, "ring depth");
-static_assert(GCfg<2, 256>::kSmemBytes <= 232448, "shared memory budget");
+static_assert(GCfg<2, 256>::kStages == 3 && GCfg<1, 256>::kStages == 3 && GCfg<1, 128>::kStages == 5, "ring depth");
+static_assert(GCfg<2, 256>::kSmemBytes <= 232448 && GCfg<1, 256>::kSmemBytes <= 232448 && GCfg<1, 128>::kSmemBytes <= 232448,
+              "shared memory budget");
 
 struct GBarriers {
   uint64_t full[8], empty[8];
@@ -67,7 +76,8 @@ static_assert(sizeof(GBarriers) <= 256, "barrier block");
 
 template <bool BF16, int NH, int MT, bool N_KMAJ, bool M_KMAJ>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_umma_kernel(const __grid_constant__ CUtensorMap tm_n, const __grid_constant__ CUtensorMap tm_m, const GemmArgs g) {
+gemm_umma_kernel(const __grid_constant__ CUtensorMap tm_n, const __grid_constant__ CUtensorMap tm_m,
+                 const __grid_constant__ CUtensorMap tm_c, const GemmArgs g) {
   using C = GCfg<NH, MT>;
   using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
   extern __shared__ uint8_t smem_raw[];
@@ -192,6 +202,8 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tm_n, const __grid_constant
     constexpr int kCols = (NH == 2) ? MT : MT / 2;
     const int col0 = (NH == 2) ? 0 : part * kCols;
     const float alpha = g.alpha, beta = g.beta;
+    uint8_t* out = smem + C::kOutOff + (warp - 2) * (C::kOutBufs * 4096);
+    int n_out = 0;                           // boxes this warp has sent
     bool ok = true;
     int ti = 0;
     for (long long t = blockIdx.x; t < g.tiles && ok; t += gridDim.x, ++ti) {
@@ -204,6 +216,41 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tm_n, const __grid_constant
       tc_fence_after();
       const int n = n0 + half * 128 + wq * 32 + lane;
       const uint32_t taddr = tmem + (static_cast<uint32_t>(wq * 32) << 16) + ab * C::kAccCols + half * MT + col0;
+      if (g.c_tma) {
+#pragma unroll 1
+        for (int c = 0; c < kCols / 64; ++c, ++n_out) {
+          uint32_t acc[2][32];
+          tmem_ld32(taddr + c * 64, acc[0]);
+          tmem_ld32(taddr + c * 64 + 32, acc[1]);
+          tmem_wait_ld();
+          if (c == kCols / 64 - 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->acc_empty[ab]);
+          }
+          uint8_t* box = out + (n_out % C::kOutBufs) * 4096;
+          if (lane == 0 && n_out >= C::kOutBufs) tma_store_wait_read<C::kOutBufs - 1>();   // its last store has left
+          __syncwarp();
+#pragma unroll
+          for (int p = 0; p < 8; ++p) {
+            const uint32_t* f = &acc[p >> 2][(p & 3) * 8];
+            uint4 v;
+            v.x = pack2<BF16>(alpha * __uint_as_float(f[0]), alpha * __uint_as_float(f[1]));
+            v.y = pack2<BF16>(alpha * __uint_as_float(f[2]), alpha * __uint_as_float(f[3]));
+            v.z = pack2<BF16>(alpha * __uint_as_float(f[4]), alpha * __uint_as_float(f[5]));
+            v.w = pack2<BF16>(alpha * __uint_as_float(f[6]), alpha * __uint_as_float(f[7]));
+            *reinterpret_cast<uint4*>(box + lane * 128 + ((p ^ (lane & 7)) << 4)) = v;
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          const int m = m0 + col0 + c * 64, nw = n0 + half * 128 + wq * 32;
+          if (lane == 0) {
+            if (m < g.M && nw < g.N) tma_store_3d(&tm_c, box, m, nw, b);   // clipped at the edges of C
+            tma_store_commit();
+          }
+        }
+        continue;
+      }
       T* ccol = reinterpret_cast<T*>(g.C) + (long long)b * g.strideC + (long long)n * g.ldc;
 #pragma unroll 1
       for (int c = 0; c < kCols / 32; ++c) {
@@ -251,6 +298,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tm_n, const __grid_constant
         }
       }
     }
+    if (lane == 0) tma_store_wait_read<0>();   // shared memory stays until the last box has been read
   }
 
   // ---------------------------------------------------------------- teardown
@@ -283,6 +331,20 @@ bool make_operand_map(CUtensorMap* m, const void* base, int dtype, long long con
   return r == CUDA_SUCCESS;
 }
 
+// (m, n, batch) view of C with the boxes a warp of the epilogue stores
+bool make_out_map(CUtensorMap* m, const GemmArgs& g, int dtype) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return false;
+  const cuuint64_t dims[3] = {(cuuint64_t)g.M, (cuuint64_t)g.N, (cuuint64_t)g.batch};
+  const cuuint64_t strides[2] = {(cuuint64_t)g.ldc * 2, (cuuint64_t)(g.batch > 1 ? g.strideC : g.ldc * g.N) * 2};
+  const cuuint32_t box[3] = {64, 32, 1};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = fn(m, dtype == NNLIB_B200_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
+                        3, g.C, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS;
+}
+
 int sm_count() {
   int dev = 0, n = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
@@ -292,7 +354,7 @@ int sm_count() {
 }
 
 template <bool BF16, int NH, int MT, bool N_KMAJ, bool M_KMAJ>
-cudaError_t launch_gemm(const CUtensorMap& mn, const CUtensorMap& mm, GemmArgs g, cudaStream_t st) {
+cudaError_t launch_gemm(const CUtensorMap& mn, const CUtensorMap& mm, const CUtensorMap& mc, GemmArgs g, cudaStream_t st) {
   using C = GCfg<NH, MT>;
   auto kern = gemm_umma_kernel<BF16, NH, MT, N_KMAJ, M_KMAJ>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
@@ -301,7 +363,7 @@ cudaError_t launch_gemm(const CUtensorMap& mn, const CUtensorMap& mm, GemmArgs g
   g.tiles_n = (g.N + NH * 128 - 1) / (NH * 128);
   g.tiles = (long long)g.tiles_m * g.tiles_n * g.batch;
   const long long grid = g.tiles < sm_count() ? g.tiles : sm_count();
-  kern<<<(unsigned)grid, kGemmThreads, C::kSmemBytes, st>>>(mn, mm, g);
+  kern<<<(unsigned)grid, kGemmThreads, C::kSmemBytes, st>>>(mn, mm, mc, g);
   count_launch();
   return cudaGetLastError();
 }
@@ -333,6 +395,9 @@ cudaError_t gemm_umma(const GemmArgs& g0, int dtype, cudaStream_t st) {
                : make_operand_map(&mm, g.A, dtype, g.M, g.K, bm, g.lda, g.strideA, false)))
     return cudaErrorInvalidValue;
   g.c_vec = (aligned16(g.C) && g.ldc % 8 == 0 && (g.batch == 1 || g.strideC % 8 == 0)) ? 1 : 0;
+  // (a tensor map addresses strides below 2^40 bytes and extents below 2^32; the direct stores know no such limit)
+  CUtensorMap mc = mn;
+  g.c_tma = (g.c_vec && g.beta == 0.f && make_out_map(&mc, g, dtype)) ? 1 : 0;
   const bool bf16 = dtype == NNLIB_B200_BF16;
   // tile: 256 x 256 for large products, 128 n-rows for narrow ones, 128 m-columns for short ones
   // (a short K leaves the 256 x 256 tile, whose accumulator fills all of tensor memory, with nothing to overlap
@@ -342,11 +407,11 @@ cudaError_t gemm_umma(const GemmArgs& g0, int dtype, cudaStream_t st) {
 #define NB_G4(BF, NHH, MTT)                                                               \
   do {                                                                                    \
     if (n_kmaj) {                                                                         \
-      if (m_kmaj) return launch_gemm<BF, NHH, MTT, true, true>(mn, mm, g, st);            \
-      return launch_gemm<BF, NHH, MTT, true, false>(mn, mm, g, st);                       \
+      if (m_kmaj) return launch_gemm<BF, NHH, MTT, true, true>(mn, mm, mc, g, st);            \
+      return launch_gemm<BF, NHH, MTT, true, false>(mn, mm, mc, g, st);                       \
     }                                                                                     \
-    if (m_kmaj) return launch_gemm<BF, NHH, MTT, false, true>(mn, mm, g, st);             \
-    return launch_gemm<BF, NHH, MTT, false, false>(mn, mm, g, st);                        \
+    if (m_kmaj) return launch_gemm<BF, NHH, MTT, false, true>(mn, mm, mc, g, st);             \
+    return launch_gemm<BF, NHH, MTT, false, false>(mn, mm, mc, g, st);                        \
   } while (0)
 #define NB_G3(BF)                                            \
   do {                                                       \
