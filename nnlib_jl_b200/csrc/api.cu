@@ -149,6 +149,8 @@ int resolve(const nnlib_b200_attn_params* p, unsigned need, AttnArgs* out, bool 
   {
     const double th = std::floor((double)p->dropout_p * 65536.0);
     a.drop_thresh = (unsigned int)(th > 65535.0 ? 65535.0 : th);
+    a.drop_add = (0x8000u - (a.drop_thresh & 0x7fffu)) * 0x00010001u;
+    a.drop_maj = a.drop_thresh < 0x8000u ? 0xffffffffu : 0u;
   }
   a.key0 = (unsigned int)(p->philox_seed & 0xffffffffull);
   a.key1 = (unsigned int)(p->philox_seed >> 32);

@@ -513,7 +513,7 @@ attn_bwd_umma_kernel(const __grid_constant__ CUtensorMap tm_fa, const __grid_con
           kb[1] = dropout_keep32(a, srow, (unsigned int)(c0 >> 5) + 1u);
         } else {
           // a column of scores (one key, 64 queries): lane L draws the call of (query L%8 of an 8-query
-          // block, key group L/8 of this warp's 32 keys) and the lanes trade the 8-bit results
+          // block, key group L/8 of this warp's 32 keys) and the lanes trade the results by votes
           const unsigned int j8 = (unsigned int)(t0 + wq * 32) / 8u + (unsigned int)(lane >> 3);
           kb[0] = kb[1] = 0u;
 #pragma unroll 2
@@ -521,18 +521,18 @@ attn_bwd_umma_kernel(const __grid_constant__ CUtensorMap tm_fa, const __grid_con
             const int qi = c0 + cb * 8 + (lane & 7);
             unsigned int w[4];
             dropout_words(a, score_row(a, qi, h, b), j8, w);
-            unsigned int byte = 0;
+            // vote e: bit L says whether (query L % 8, key 8 (L / 8) + e) survives; the lane of key (lane % 8) of its
+            // group keeps that vote, whose byte of its group holds its eight queries
+            unsigned int vote = 0u;
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              byte |= ((w[e] & 0xffffu) >= a.drop_thresh ? 1u : 0u) << (2 * e);
-              byte |= ((w[e] >> 16) >= a.drop_thresh ? 1u : 0u) << (2 * e + 1);
+              const unsigned int k = keep_lanes(a, w[e]);
+              const unsigned int v0 = __ballot_sync(0xffffffffu, (k & 0x8000u) != 0u);
+              const unsigned int v1 = __ballot_sync(0xffffffffu, (int)k < 0);
+              if ((lane & 7) == 2 * e) vote = v0;
+              if ((lane & 7) == 2 * e + 1) vote = v1;
             }
-            unsigned int bits8 = 0;
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              const unsigned int other = __shfl_sync(0xffffffffu, byte, q + (lane & 24));
-              bits8 |= ((other >> (lane & 7)) & 1u) << q;
-            }
+            const unsigned int bits8 = (vote >> (lane & 24)) & 0xffu;
             kb[cb >> 2] |= bits8 << ((cb & 3) * 8);
           }
         }
@@ -635,7 +635,7 @@ attn_bwd_umma_kernel(const __grid_constant__ CUtensorMap tm_fa, const __grid_con
       // dS of score e of the dq half: P (keep/(1-p) dP - D)
       auto ds_of = [&](int e) -> float {
         float gval = __uint_as_float(dpq[e >> 5][e & 31]);
-        if (DROP) gval = ((kb[e >> 5] >> (e & 31)) & 1u) ? gval * a.inv_keep : 0.f;
+        if (DROP) gval = ((kb[e >> 5] >> keep_pos(e & 31)) & 1u) ? gval * a.inv_keep : 0.f;
         return (gval - dl_row) * NB_SR(e);
       };
       if (!DKV) {

@@ -490,7 +490,7 @@ attn_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
               add2(sum2[(e >> 1) & 1], p0, p1);
             }
             pk[e >> 1] = pack2<BF16>(p0, p1);
-            if (DROP) pk[e >> 1] &= (((kb >> e) & 1u) ? 0x0000ffffu : 0u) | (((kb >> (e + 1)) & 1u) ? 0xffff0000u : 0u);
+            if (DROP) pk[e >> 1] &= keep_pair_mask(kb, e >> 1);
           }
           l += XBIAS ? sum0 + sum1 : pair_sum(sum2[0]) + pair_sum(sum2[1]);
           tmem_st16(lane_base + (g >> 2) * kBN + (g & 3) * 16, pk);   // chunk c of tile t -> [128 t + 16 c, +16)

@@ -398,7 +398,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             float al = ex2_approx(fmaf(__uint_as_float(sr[c][e]), cs, -lse2));   // -inf (masked) gives 0
             if (rinf) al = (sr[c][e] == 0x7f800000u) ? inf_share : 0.f;
             if (row_const) al = const_val;
-            if (drop) al = ((kb[c] >> e) & 1u) ? al * a.inv_keep : 0.f;
+            if (drop) al = ((kb[c] >> keep_pos(e)) & 1u) ? al * a.inv_keep : 0.f;
             sr[c][e] = __float_as_uint(al);
           }
         if (row_ok) {
@@ -477,7 +477,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           if (SIDE && row_inf) p = (sr[c][e] == 0x7f800000u) ? 1.f : 0.f;
           sum += p;
           // dropout follows the softmax: the row sum keeps the dropped scores
-          sr[c][e] = ((kb[c] >> e) & 1u) ? (TF32 ? to_tf32(p) : __float_as_uint(p)) : 0u;
+          sr[c][e] = ((kb[c] >> keep_pos(e)) & 1u) ? (TF32 ? to_tf32(p) : __float_as_uint(p)) : 0u;
         }
       l += sum;
       if (PV) {

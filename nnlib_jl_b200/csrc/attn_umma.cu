@@ -521,9 +521,7 @@ attn_fwd_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 #pragma unroll
                 for (int e = 0; e < 16; ++e) {
                   // pk[cc*16 + e] holds keys 2e (low half) and 2e+1 (high half) of this 32-key chunk
-                  const unsigned int m = (((kbc >> (2 * e)) & 1u) ? 0x0000ffffu : 0u) |
-                                         (((kbc >> (2 * e + 1)) & 1u) ? 0xffff0000u : 0u);
-                  pk[cc * 16 + e] &= m;
+                  pk[cc * 16 + e] &= keep_pair_mask(kbc, e);
                 }
               }
             }
@@ -874,7 +872,7 @@ attn_scores_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
 #pragma unroll
             for (int e = 0; e < 32; ++e) {
               const float al = __uint_as_float(sr[c & 1][e]);
-              sr[c & 1][e] = __float_as_uint(((kb >> e) & 1u) ? al * a.inv_keep : 0.f);
+              sr[c & 1][e] = __float_as_uint(((kb >> keep_pos(e)) & 1u) ? al * a.inv_keep : 0.f);
             }
           }
 #pragma unroll

@@ -34,6 +34,7 @@ struct AttnArgs {
   unsigned int key0, key1, off_lo, off_hi;
   unsigned int rkey[20];   // the ten round keys of Philox4x32-10 (key0 + r*W0, key1 + r*W1), bumped once on the host
   unsigned int drop_thresh;  // floor(p * 2^16): a score is dropped iff its 16-bit lane is below it
+  unsigned int drop_add, drop_maj;   // the same test for two packed lanes at once (dropout_keep32)
   float inv_keep;            // 1/(1-p)
   float dropout_p;
   float scale;               // multiplies q·k (natural units)
@@ -146,23 +147,37 @@ __device__ __forceinline__ bool dropout_keep1(const AttnArgs& a, unsigned long l
   return ((word >> (16u * (e & 1u))) & 0xffffu) >= a.drop_thresh;
 }
 
-// Keep-bits of 32 consecutive keys (bit e: key 32*c32 + e of score row r survives).  Two calls at a time:
-// their ten rounds interleave (each round waits on the previous one's multiplies), more would cost registers.
+// Keep bits of 32 consecutive keys of score row r (keys 32*c32 ..): bit keep_pos(e) says whether key e survives.
+// The even keys' bits sit in the low half, the odd ones' in the high half, the way the 16-bit lanes of the random
+// words and the packed 16-bit probabilities are paired up, so that neither the test nor the use takes a pair apart:
+// per pair of lanes five integer instructions here and three in keep_pair_mask, against eleven and five for one
+// bit per key in ascending order.
+// bits 15 and 31: the low / high 16-bit lane of a random word is kept.  A lane x is kept iff x >= t = drop_thresh.
+// Bit 15 of s: the low 15 bits of x are >= those of t; with that, x >= t iff (bit 15 of x or s) for t < 2^15, (bit 15
+// of x and s) for larger t: a majority with a constant.
+__device__ __forceinline__ unsigned int keep_lanes(const AttnArgs& a, unsigned int w) {
+  const unsigned int s = (w & 0x7fff7fffu) + a.drop_add;
+  return ((s & w) | (a.drop_maj & (s | w))) & 0x80008000u;
+}
+__host__ __device__ constexpr int keep_pos(int e) { return (e >> 1) + ((e & 1) << 4); }
 __device__ __forceinline__ unsigned int dropout_keep32(const AttnArgs& a, unsigned long long r, unsigned int c32) {
   unsigned int bits = 0;
 #pragma unroll 2
   for (int g = 0; g < 4; ++g) {
     unsigned int w[4];
     dropout_words(a, r, c32 * 4 + g, w);
-    unsigned int byte = 0;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      byte |= ((w[e] & 0xffffu) >= a.drop_thresh ? 1u : 0u) << (2 * e);
-      byte |= ((w[e] >> 16) >= a.drop_thresh ? 1u : 0u) << (2 * e + 1);
+      bits = (bits >> 1) | keep_lanes(a, w[e]);
     }
-    bits |= byte << (8 * g);
   }
   return bits;
+}
+// all-ones halves for the surviving keys of pair e (keys 2e and 2e+1 of the 32)
+__device__ __forceinline__ unsigned int keep_pair_mask(unsigned int bits, int e) {
+  unsigned int m;
+  asm("prmt.b32 %0, %1, 0, 0xBB99;" : "=r"(m) : "r"(bits << (15 - e)));   // the sign of each half in all its bits
+  return m;
 }
 
 // global score-row number of query i, head h, batch b (see nnlib_b200.h, dropout)
