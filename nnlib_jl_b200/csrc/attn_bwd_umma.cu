@@ -18,9 +18,11 @@
 //   warps 0-3   compute, columns 0-63 of the step (thread r owns row r of the resident tile)
 //   warps 4-7   compute, columns 64-127
 //   warp 8      TMA producer of the resident pair and of ring A'; TMEM allocation
-//   warp 9      MMA issuer
+//   warp 9      MMA issuer of S and, in the dq half, dP, in the dk/dv half, dV
 //   warp 10     TMA producer of ring B'
-//   warp 11     idle (completes the warpgroup of warps 8-10)
+//   warp 11     MMA issuer of the product with dS (dQ or dK) and, in the dk/dv half, of dP
+// Two issuers, because one was what bounded a step: 24 (dq) or 32 (dk/dv) instructions at about 75 cycles each and some
+// 1000 cycles of barrier waits and commits per step in a row, against 1536 / 2048 cycles of tensor work.
 // TMEM columns: S [0,128)  dP [128,256)  accumulator 0 [256,256+D)  accumulator 1 [384,384+D).
 // dS (half precision): the dq half double-buffers it in columns [384,512) (its second accumulator is
 // unused), the dk/dv half writes it over dP: columns [128,160) for ring rows 0-63, [192,224) for rows 64-127.
@@ -38,8 +40,7 @@ __device__ int g_bwd_abort = 0;  // sticky: a bounded wait of a backward kernel 
 
 namespace {
 
-// 12 warps = three whole warpgroups: setmaxnreg is a warpgroup-wide instruction, so the copy / issue
-// warps 8-10 need their (idle) fourth warp 11
+// 12 warps = three whole warpgroups (setmaxnreg is a warpgroup-wide instruction)
 constexpr int kBwThreads = 384;
 
 template <int D, bool DKV>
@@ -222,7 +223,7 @@ attn_bwd_umma_kernel(const __grid_constant__ CUtensorMap tm_fa, const __grid_con
     mbar_init(&bars->s_read, 8);
     mbar_init(&bars->ds_ready[0], 8);
     mbar_init(&bars->ds_ready[1], 8);
-    mbar_init(&bars->acc_full, 1);
+    mbar_init(&bars->acc_full, DKV ? 2 : 1);   // one per issuer with an accumulator
     mbar_init(&bars->col_ready, 8);
     mbar_init(&bars->dp_read, 8);
     mbar_init(&bars->pt_ready, 8);
@@ -293,8 +294,8 @@ attn_bwd_umma_kernel(const __grid_constant__ CUtensorMap tm_fa, const __grid_con
         for (int jj = max(0, it - C::kStagesB); jj < it; ++jj)
           mbar_wait_drain(&bars->b_full[jj % C::kStagesB], (jj / C::kStagesB) & 1, kDrainNs);
     }
-  } else if (start_ok && warp == 9) {
-    // -------------------------------------------------------------- MMA issuer
+  } else if (start_ok && (warp == 9 || warp == 11)) {
+    // ------------------------------------------------------------- MMA issuers
     if (lane == 0 && n > 0) {
       constexpr uint32_t idesc_nt = make_idesc_f16(BF16, 128, 128, false, false);  // both operands K-major
       constexpr uint32_t idesc_acc = make_idesc_f16(BF16, 128, D, false, true);    // B MN-major
@@ -350,51 +351,61 @@ attn_bwd_umma_kernel(const __grid_constant__ CUtensorMap tm_fa, const __grid_con
         umma_commit(&bars->b_empty[it % C::kStagesB]);   // also tells that P^T has been consumed
       };
 
-      // S and dP of the next step are issued as early as the compute warps allow (they have the
-      // previous S / dP in registers), the accumulating products when dS (and P^T) are ready.
+      // S and dP of the next step are issued as early as the compute warps allow (they have the previous S / dP in
+      // registers), the accumulating products when dS (and P^T) are ready.  In the dk/dv half dP overwrites dS, so it
+      // follows the product with dS in the same thread.  A ring stage is given back by the thread whose product
+      // reads it last: that product's other operand was made from the results of the stage's first product.
       bool ok = mbar_wait(&bars->fix_full, 0, abort_flag);
-      if (ok) ok = mbar_wait(&bars->a_full[0], 0, abort_flag);
-      if (ok) issue_s(0);
-      if (ok) ok = mbar_wait(&bars->b_full[0], 0, abort_flag);
-      if (ok) issue_dp(0);
-      for (int it = 0; it < n && ok; ++it) {
-        const uint32_t par = it & 1;
-        const bool more = it + 1 < n;
-        if (more) {
-          ok = mbar_wait(&bars->a_full[(it + 1) % C::kStagesA], ((it + 1) / C::kStagesA) & 1, abort_flag);
-          if (ok) ok = mbar_wait(&bars->s_read, par, abort_flag);
-          if (!ok) break;
-          tc_fence_after();
-          issue_s(it + 1);
-        }
-        if (!DKV) {
+      if (warp == 9) {
+        if (ok) ok = mbar_wait(&bars->a_full[0], 0, abort_flag);
+        if (ok) issue_s(0);
+        if (ok) ok = mbar_wait(&bars->b_full[0], 0, abort_flag);
+        if (ok && !DKV) issue_dp(0);
+        for (int it = 0; it < n && ok; ++it) {
+          const uint32_t par = it & 1;
+          const bool more = it + 1 < n;
           if (more) {
-            ok = mbar_wait(&bars->b_full[(it + 1) % C::kStagesB], ((it + 1) / C::kStagesB) & 1, abort_flag);
-            if (ok) ok = mbar_wait(&bars->dp_read, par, abort_flag);
+            ok = mbar_wait(&bars->a_full[(it + 1) % C::kStagesA], ((it + 1) / C::kStagesA) & 1, abort_flag);
+            if (ok) ok = mbar_wait(&bars->s_read, par, abort_flag);
             if (!ok) break;
             tc_fence_after();
-            issue_dp(it + 1);
+            issue_s(it + 1);
           }
-          ok = mbar_wait(&bars->ds_ready[it & 1], (it >> 1) & 1, abort_flag);
+          if (!DKV) {
+            if (more) {
+              ok = mbar_wait(&bars->b_full[(it + 1) % C::kStagesB], ((it + 1) / C::kStagesB) & 1, abort_flag);
+              if (ok) ok = mbar_wait(&bars->dp_read, par, abort_flag);
+              if (!ok) break;
+              tc_fence_after();
+              issue_dp(it + 1);
+            }
+          } else {
+            ok = mbar_wait(&bars->b_full[it % C::kStagesB], (it / C::kStagesB) & 1, abort_flag);
+            if (ok) ok = mbar_wait(&bars->pt_ready, par, abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+            issue_dv(it);
+          }
+        }
+        if (ok && DKV) umma_commit(&bars->acc_full);
+      } else {
+        // (in the dq half ring B' belongs to the other issuer: its barriers may be phases ahead of this thread)
+        if (DKV && ok) ok = mbar_wait(&bars->b_full[0], 0, abort_flag);
+        if (DKV && ok) issue_dp(0);
+        for (int it = 0; it < n && ok; ++it) {
+          ok = mbar_wait(&bars->a_full[it % C::kStagesA], (it / C::kStagesA) & 1, abort_flag);
+          if (ok) ok = mbar_wait(&bars->ds_ready[it & 1], (it >> 1) & 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
           issue_ds_acc(it);
-        } else {
-          ok = mbar_wait(&bars->ds_ready[it & 1], (it >> 1) & 1, abort_flag);
-          if (!ok) break;
-          tc_fence_after();
-          issue_ds_acc(it);
-          if (more) {
+          if (DKV && it + 1 < n) {
             ok = mbar_wait(&bars->b_full[(it + 1) % C::kStagesB], ((it + 1) / C::kStagesB) & 1, abort_flag);
             if (!ok) break;
             issue_dp(it + 1);   // overwrites dS: ordered behind the dK products above
           }
-          ok = mbar_wait(&bars->pt_ready, par, abort_flag);
-          if (!ok) break;
-          issue_dv(it);
         }
+        if (ok) umma_commit(&bars->acc_full);
       }
-      if (ok) umma_commit(&bars->acc_full);
     }
   }
   } else {
