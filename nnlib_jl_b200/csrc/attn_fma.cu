@@ -78,8 +78,9 @@ __host__ __device__ constexpr int fma_smem() {
 
 __host__ __device__ constexpr bool fm_with_v(int mode) { return mode == FM_FWD || mode == FM_APPLY; }
 
+// (d = 64, 8 rows a thread: three blocks on an SM with a few spilled words are faster than two without)
 template <typename T, int DP, int MI, int NTHR, int MODE>
-__global__ void __launch_bounds__(NTHR) attn_fma_kernel(const AttnArgs a, const int n_tiles, const int vec) {
+__global__ void __launch_bounds__(NTHR, MODE == FM_FWD && MI == 8 && DP == 64 ? 3 : 1) attn_fma_kernel(const AttnArgs a, const int n_tiles, const int vec) {
   constexpr int BM = NTHR / 16 * MI, LD = DP + 4, CN = DP / 16;
   extern __shared__ __align__(16) float sm[];
   float* qs = sm;
