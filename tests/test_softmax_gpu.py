@@ -144,3 +144,40 @@ def test_random_shapes_and_dims_match_the_oracle(seed):
     dy2 = _as_cm(_dev(dyn, dtype), dtype)
     SM.softmax_pullback(dy2, y, dims=dims, out=dy2)
     assert torch.equal(dy2, dx), what
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("inner,n,outer", [
+    (2, 1, 1),            # smallest
+    (7, 65, 3),           # fewer columns than a sector
+    (33, 300, 2),         # one column past a block of 32; eight loads in flight and a remainder
+    (40, 1500, 1),        # long reduction: 1024 threads
+    (70, 63, 400),        # enough columns for blocks of 32
+])
+@pytest.mark.parametrize("log", [False, True])
+def test_strided_reduction_blocks(dtype, inner, n, outer, log):
+    rng = np.random.default_rng(inner + n)
+    xn = 3 * rng.standard_normal((inner, n, outer)).astype(np.float32)
+    dn = rng.standard_normal((inner, n, outer)).astype(np.float32)
+    if n > 10:
+        xn[0, 3, 0] = np.inf                   # equal shares on the +Inf entries
+        xn[1, :, 0] = -np.inf                  # nothing but -Inf: NaN
+        xn[-1, 5, -1] = np.nan
+    x, dy = (nb.jl_from_numpy(a, dtype=dtype, device="cuda:0") for a in (xn, dn))
+    x64, d64 = (t.to(torch.float64) for t in (x, dy))
+    fwd, back = (nb.softmax.logsoftmax, nb.softmax.logsoftmax_pullback) if log else (nb.softmax.softmax, nb.softmax.softmax_pullback)
+    y = fwd(x, dims=2)
+    ok = torch.isfinite(x64).all(dim=1, keepdim=True).expand_as(x64)
+    want = torch.log_softmax(x64, 1) if log else torch.softmax(x64, 1)
+    # the fast exponential and logarithm: a few 2^-22 of |x| <= 16; one rounding to the element type
+    rel = 2.0 ** -8 if dtype == torch.bfloat16 else 5e-6
+    scale = want.abs().clamp_min(1.0 if log else 0.0)
+    assert ((y.double() - want).abs() <= rel * scale + 1e-12)[ok].all()
+    if n > 10:
+        assert y[0, 3, 0].item() == (0.0 if log else 1.0) and torch.isnan(y[1, :, 0]).all() and torch.isnan(y[-1, :, -1]).all()
+    dx = back(dy, y, dims=2)
+    y64 = y.double()
+    s = (d64 if log else d64 * y64).sum(1, keepdim=True)
+    wantd = d64 - torch.exp(y64) * s if log else y64 * (d64 - s)
+    size = d64.abs() + (torch.exp(y64) if log else y64) * (d64 if log else d64 * y64).abs().sum(1, keepdim=True) + y64.abs() * d64.abs()
+    assert ((dx.double() - wantd).abs() <= 2 * rel * size + 1e-12)[ok].all()
