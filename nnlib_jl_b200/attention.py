@@ -483,9 +483,31 @@ def _fused(q, k, v, bias, mask, nheads, dropout):
     return x, LazyAttnScores(pr, (pr.Lkv, pr.Lq, pr.H, pr.B))
 
 
-def _fused_into(q, k, v, mask, nheads, x_out, lse_out):
-    """The fused call writing into caller-owned buffers (no allocation): ``x_out`` is a column-major
-    ``(Ev, Lq, B)`` array of the inputs' element type, ``lse_out`` a Float32 array of ``Lq*H*B`` elements."""
+def _launch_unit_exact(pr, piece: bool = False):
+    """x of a part of a larger call (a shard's heads and batches, a chunk of the batch), the same bits the whole call
+    gives.  The split-key forwards for a handful of queries without side inputs and for exact Float32 split by the
+    number of keys alone, so a part takes them like the whole does; the one-tile kernels split by the number of units
+    as well, and a part does not take those.  ``piece``: a range of a longer call's queries, which the whole call
+    handled in the ordinary forward."""
+    if pr.Lq == 0 or pr.B == 0:
+        return
+    lib, p = _lib.load(), pr.p
+    reach = max(0, min(pr.Lkv, pr.Lq + p.causal_offset)) if p.causal else pr.Lkv
+    by_keys = not piece and reach > 1024 and pr.Lq <= 32 and not p.dropout_p > 0 and not p.allow_tf32 and pr.d <= 128 and \
+        pr.dv <= 128 and (pr.dtype == torch.float32 or (pr.Lq <= 16 and not p.bias and not p.mask))
+    with torch.cuda.device(pr.dev):
+        need = lib.nnlib_b200_attn_decode_workspace_bytes(C.byref(p)) if by_keys else 0
+        if need:
+            ws = torch.empty(need, dtype=torch.uint8, device=pr.dev)
+            _check(lib.nnlib_b200_attn_decode(C.byref(p), ws.data_ptr(), need, _stream()), "attn_decode")
+        else:
+            _check(lib.nnlib_b200_attn_fwd(C.byref(p), _stream()), "attn_fwd")
+
+
+def _fused_into(q, k, v, mask, nheads, x_out, lse_out, piece: bool = False):
+    """The fused call writing into caller-owned buffers (at most a split-key workspace is allocated): ``x_out`` is a
+    column-major ``(Ev, Lq, B)`` array of the inputs' element type, ``lse_out`` a Float32 array of ``Lq*H*B``
+    elements.  ``piece``: see :func:`_launch_unit_exact`."""
     pr = _Problem(q, k, v, None, mask, nheads, None, need_v=True)
     if tuple(x_out.shape) != (pr.Ev, pr.Lq, pr.B) or x_out.dtype != pr.dtype or not is_column_major(x_out):
         raise ArgumentError("x_out must be a dense column-major (Ev, Lq, B) array of the inputs' element type")
@@ -495,9 +517,7 @@ def _fused_into(q, k, v, mask, nheads, x_out, lse_out):
     pr.p.x = x_out.data_ptr()
     pr.lse = lse_out
     pr.p.lse = lse_out.data_ptr()
-    if pr.Lq > 0 and pr.B > 0:
-        with torch.cuda.device(pr.dev):
-            _check(_lib.load().nnlib_b200_attn_fwd(C.byref(pr.p), _stream()), "attn_fwd")
+    _launch_unit_exact(pr, piece)
     return x_out
 
 
@@ -508,9 +528,7 @@ def _fused_with_origin(q, k, v, bias, mask, nheads, dropout, rng_origin):
     pr = _Problem(q, k, v, bias, mask, nheads, dropout, need_v=True, rng_origin=rng_origin)
     x = pr.alloc_x()
     pr.alloc_lse()
-    if pr.Lq > 0 and pr.B > 0:
-        with torch.cuda.device(pr.dev):
-            _check(_lib.load().nnlib_b200_attn_fwd(C.byref(pr.p), _stream()), "attn_fwd")
+    _launch_unit_exact(pr)
     return x
 
 

@@ -192,6 +192,9 @@ bool use_tile(const AttnArgs& a, int dtype, bool need_v) {
   return !force_simt() && tile_reject_reason(a, dtype, need_v, a.allow_tf32 != 0) == nullptr;
 }
 
+// at most 16 queries without side inputs, through attn_decode
+bool use_decode(const AttnArgs& a, int dtype) { return !force_simt() && decode_supports(a, dtype); }
+
 // why a call does not run on the tensor-core kernels (for the log)
 const char* simt_reason(const AttnArgs& a, int dtype, bool need_v) {
   return force_simt() ? "NNLIB_B200_FORCE_SIMT is set" : tile_reject_reason(a, dtype, need_v, a.allow_tf32 != 0);
@@ -256,19 +259,28 @@ int nnlib_b200_attn_fwd(const nnlib_b200_attn_params* p, void* stream) {
   return finish(!force_simt() && fma_supports(a.d, a.dv) ? fma_fwd(a, p->dtype, st) : simt_fwd(a, p->dtype, st));
 }
 
-// does the split-key forward apply to this call, and is it worth it (a long key sequence, too few units to
-// fill the GPU otherwise)?
-static bool use_split(const AttnArgs& a, int dtype) {
-  if (a.Lq > 128 || force_simt()) return false;
-  if (tile_reject_reason(a, dtype, true, a.allow_tf32 != 0) != nullptr) return false;
-  return tile_split_count(a) > 1;
+// Which split-key forward takes the call: long key sequences whose units alone would not fill the GPU.
+enum SplitPath { SPLIT_NONE, SPLIT_DECODE, SPLIT_TILE, SPLIT_FMA };
+static SplitPath split_path(const AttnArgs& a, int dtype) {
+  if (a.Lq < 1 || a.Lq > 128 || a.B < 1 || a.Lkv < 1 || force_simt()) return SPLIT_NONE;
+  if (use_decode(a, dtype) && decode_split_count(a) > 1) return SPLIT_DECODE;
+  if (tile_reject_reason(a, dtype, true, a.allow_tf32 != 0) == nullptr) return tile_split_count(a) > 1 ? SPLIT_TILE : SPLIT_NONE;
+  return fma_split_count(a, dtype) > 1 ? SPLIT_FMA : SPLIT_NONE;
+}
+static size_t split_workspace(const AttnArgs& a, int dtype, SplitPath path) {
+  switch (path) {
+    case SPLIT_DECODE: return decode_workspace_bytes(a);
+    case SPLIT_TILE:   return tile_split_workspace_bytes(a);
+    case SPLIT_FMA:    return fma_split_workspace_bytes(a, dtype);
+    default:           return 0;
+  }
 }
 
 size_t nnlib_b200_attn_decode_workspace_bytes(const nnlib_b200_attn_params* p) {
   AttnArgs a;
   if (resolve(p, NEED_QK | NEED_V, &a, false) != NNLIB_B200_OK) return 0;
-  if (a.Lq == 0 || a.B == 0 || !use_split(a, p->dtype)) return 0;
-  return tile_split_workspace_bytes(a);
+  if (a.Lq == 0 || a.B == 0) return 0;
+  return split_workspace(a, p->dtype, split_path(a, p->dtype));
 }
 
 int nnlib_b200_attn_decode(const nnlib_b200_attn_params* p, void* workspace, size_t workspace_bytes, void* stream) {
@@ -276,17 +288,23 @@ int nnlib_b200_attn_decode(const nnlib_b200_attn_params* p, void* workspace, siz
   const int rc = resolve(p, NEED_QK | NEED_V, &a);
   if (rc) return rc;
   if (a.Lq == 0 || a.B == 0) return NNLIB_B200_OK;
-  if (!use_split(a, p->dtype)) return nnlib_b200_attn_fwd(p, stream);
-  const size_t need = tile_split_workspace_bytes(a);
+  const SplitPath path = split_path(a, p->dtype);
+  if (path == SPLIT_NONE) return nnlib_b200_attn_fwd(p, stream);
+  const size_t need = split_workspace(a, p->dtype, path);
   if (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 15u) != 0)
     return NNLIB_B200_WORKSPACE_TOO_SMALL;
   a.ws = static_cast<float*>(workspace);
+  const int n = path == SPLIT_DECODE ? decode_split_count(a) : path == SPLIT_TILE ? tile_split_count(a) : fma_split_count(a, p->dtype);
   if (log_calls()) {
     char what[96];
-    std::snprintf(what, sizeof(what), "tcgen05 (keys split over %d CTAs per unit)", tile_split_count(a));
+    std::snprintf(what, sizeof(what), "%s (keys split over %d CTAs per unit)",
+                  path == SPLIT_DECODE ? "streamed keys" : path == SPLIT_TILE ? "tcgen05" : "cuda-core", n);
     log_call("attn_decode", p, a, what, nullptr);
   }
-  return finish(tile_split(a, p->dtype, (cudaStream_t)stream));
+  cudaStream_t st = (cudaStream_t)stream;
+  if (path == SPLIT_DECODE) return finish(decode_fwd(a, p->dtype, n, st));
+  if (path == SPLIT_TILE) return finish(tile_split(a, p->dtype, st));
+  return finish(fma_split(a, p->dtype, st));
 }
 
 int nnlib_b200_attn_stats(const nnlib_b200_attn_params* p, void* stream) {

@@ -10,6 +10,8 @@
 //     FM_STATS   the log-sum-exp only
 //     FM_SCORES  alpha from a given log-sum-exp; the key tiles of a block row may be dealt to several blocks
 //     FM_APPLY   x = V alpha for scores the caller holds
+//     FM_SPLIT   FM_FWD for few queries against many keys: the key tiles of a unit are dealt to gridDim.y blocks,
+//                each leaving its maximum, sum and unnormalised O in a workspace (split_reduce.cuh merges them)
 // A warp per query that walked the keys one lane per key (attn_simt.cu, still there for larger heads) re-read every
 // key row through L1 for each query, uncoalesced: 441 us for x and alpha at d = 64, 8 heads, 128 x 128, batch 4,
 // where one pass of the row kernel takes 32 us including 25 us of host time between calls.
@@ -21,13 +23,14 @@
 #include "common.cuh"
 #include "fma_tile.cuh"
 #include "launchers.h"
+#include "split_reduce.cuh"
 
 namespace nb200 {
 namespace {
 
 using namespace fma_tile;
 
-enum : int { FM_FWD = 0, FM_STATS = 1, FM_SCORES = 2, FM_APPLY = 3 };
+enum : int { FM_FWD = 0, FM_STATS = 1, FM_SCORES = 2, FM_APPLY = 3, FM_SPLIT = 4 };
 constexpr int kRowBM = 32;                       // queries of a block of the row kernel
 constexpr int kVecQ = 1, kVecK = 2, kVecV = 4;   // 16-byte copies of that array's rows are possible
 
@@ -76,7 +79,7 @@ __host__ __device__ constexpr int fma_smem() {
               (MODE != FM_STATS && MODE != FM_SCORES ? kBN * (DP + 4) : 0)) + BM * 8;
 }
 
-__host__ __device__ constexpr bool fm_with_v(int mode) { return mode == FM_FWD || mode == FM_APPLY; }
+__host__ __device__ constexpr bool fm_with_v(int mode) { return mode == FM_FWD || mode == FM_APPLY || mode == FM_SPLIT; }
 
 // (d = 64, 8 rows a thread: three blocks on an SM with a few spilled words are faster than two without)
 template <typename T, int DP, int MI, int NTHR, int MODE>
@@ -117,9 +120,16 @@ __global__ void __launch_bounds__(NTHR, MODE == FM_FWD && MI == 8 && DP == 64 ? 
 
   const int kend = key_end(a, min(q0 + BM, a.Lq) - 1);
   // every score is written in FM_SCORES and read in FM_APPLY, the others end at the last key in reach
-  const int kstop = (MODE == FM_SCORES || MODE == FM_APPLY) ? a.Lkv : kend;
+  int kstart = blockIdx.y * kBN, kstep = kBN * gridDim.y;
+  int kstop = (MODE == FM_SCORES || MODE == FM_APPLY) ? a.Lkv : kend;
+  if (MODE == FM_SPLIT) {                                  // a contiguous share
+    const int per = ((kstop + kBN - 1) / kBN + gridDim.y - 1) / gridDim.y * kBN;
+    kstart = blockIdx.y * per;
+    kstop = min(kstop, kstart + per);
+    kstep = kBN;
+  }
   const int d4 = (a.d + 3) >> 2;
-  for (int k0 = blockIdx.y * kBN; k0 < kstop; k0 += kBN * gridDim.y) {
+  for (int k0 = kstart; k0 < kstop; k0 += kstep) {
     const bool live = MODE == FM_APPLY || k0 < kend;       // false: all above the causal diagonal
     if (MODE != FM_APPLY && live) {
       load_tile<T, kBN, DP, LD, NTHR>(kp, kbase + (long long)k0 * a.k_sl, a.k_sl, a.Lkv - k0, a.d, (vec & kVecK) != 0);
@@ -212,6 +222,18 @@ __global__ void __launch_bounds__(NTHR, MODE == FM_FWD && MI == 8 && DP == 64 ? 
     if (MODE != FM_APPLY) {
       const float ls = sum16(l[i]);                        // all 16 lanes of a row take part
       if (gi >= a.Lq) continue;                            // whole half-warps
+      if (MODE == FM_SPLIT) {                              // the merge works in base 2
+        const long long slot = ((long long)unit * gridDim.y + blockIdx.y) * a.Lq + gi;
+        if (tx == 0) {
+          a.ws[slot * 2] = m[i] * 1.4426950408889634f;
+          a.ws[slot * 2 + 1] = ls;
+        }
+        float* ow = a.ws + split_ml_floats(a, gridDim.y) + slot * a.dv;
+#pragma unroll
+        for (int c = 0; c < CN; ++c)
+          if (colmap<DP>(tx, c) < a.dv) ow[colmap<DP>(tx, c)] = o[i][c];
+        continue;
+      }
       if (a.lse && tx == 0) a.lse[gi + (long long)a.Lq * h + a.lse_sb * b] = make_lse(m[i], ls);
       if (MODE == FM_STATS) continue;
       scale = a.inv_keep / ls;
@@ -371,7 +393,7 @@ __global__ void __launch_bounds__(NTHR) attn_fma_row_kernel(const AttnArgs a, co
 // the GPU twice over; 32 when they do not, 8 for a handful of queries (a decode step), where most of a larger
 // block would be padding.
 template <typename T, int DP, int MI, int MODE>
-cudaError_t launch_fma_mi(const AttnArgs& a, int vec, cudaStream_t st) {
+cudaError_t launch_fma_mi(const AttnArgs& a, int vec, cudaStream_t st, int n_splits = 1) {
   constexpr int NTHR = 128, BM = NTHR / 16 * MI;
   constexpr int smem = fma_smem<DP, BM, MODE>();
   auto kern = attn_fma_kernel<T, DP, MI, NTHR, MODE>;
@@ -384,8 +406,15 @@ cudaError_t launch_fma_mi(const AttnArgs& a, int vec, cudaStream_t st) {
     const long long nkt = ((long long)a.Lkv + kBN - 1) / kBN;
     ky = (int)std::max<long long>(1, std::min<long long>({nkt, (4 * 148 + blocks - 1) / blocks, 65535}));
   }
+  if (MODE == FM_SPLIT) ky = n_splits;
   kern<<<dim3((unsigned)blocks, (unsigned)ky), NTHR, smem, st>>>(a, (int)n_tiles, vec);
   count_launch();
+  if (MODE == FM_SPLIT) {
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    attn_split_reduce_kernel<T><<<(unsigned)(a.H * a.B * a.Lq), 128, 0, st>>>(a, n_splits);
+    count_launch();
+  }
   return cudaGetLastError();
 }
 
@@ -440,6 +469,30 @@ cudaError_t launch_row(const AttnArgs& a, int vec, cudaStream_t st) {
 }
 
 }  // namespace
+
+// Split-key forward, Float32, at most 32 queries: 256 keys (four tiles) per block once there are more than 1024
+// (below that one launch is quicker than two).
+// A function of the number of keys alone, so that a (head, batch) unit gives the same bits in whatever company it is
+// computed.  (Without dropout: the merge does not know whether a row without attended keys kept one.)
+int fma_split_count(const AttnArgs& a, int dtype) {
+  if (dtype != NNLIB_B200_F32 || a.Lq < 1 || a.Lq > 32 || a.H < 1 || a.B < 1 || !fma_supports(a.d, a.dv) || a.dropout_p > 0.f)
+    return 1;
+  const long long last = a.causal ? std::min<long long>(a.Lkv, std::max<long long>(0, (long long)a.Lq + a.coff)) : a.Lkv;
+  if (last <= 1024 || (long long)a.H * a.B * a.Lq > 0x7fffffffLL) return 1;
+  return (int)std::min<long long>((last + 255) / 256, 65535);
+}
+size_t fma_split_workspace_bytes(const AttnArgs& a, int dtype) {
+  const int n = fma_split_count(a, dtype);
+  return n > 1 ? (size_t)split_ws_floats(a, n) * sizeof(float) : 0;
+}
+cudaError_t fma_split(const AttnArgs& a, int dtype, cudaStream_t st) {
+  const int n = fma_split_count(a, dtype), dm = std::max(a.d, a.dv);
+  const int vec = (rows_vec(a.q, a.q_sl, a.q_sb, a.d, dtype) ? kVecQ : 0) |
+                  (rows_vec(a.k, a.k_sl, a.k_sb, a.d, dtype) ? kVecK : 0) |
+                  (rows_vec(a.v, a.v_sl, a.v_sb, a.dv, dtype) ? kVecV : 0);
+  if (dm <= 64) return a.Lq <= 8 ? launch_fma_mi<float, 64, 1, FM_SPLIT>(a, vec, st, n) : launch_fma_mi<float, 64, 4, FM_SPLIT>(a, vec, st, n);
+  return a.Lq <= 8 ? launch_fma_mi<float, 128, 1, FM_SPLIT>(a, vec, st, n) : launch_fma_mi<float, 128, 4, FM_SPLIT>(a, vec, st, n);
+}
 
 bool fma_supports(int d, int dv) { return d >= 1 && d <= 128 && dv >= 1 && dv <= 128; }
 

@@ -25,6 +25,9 @@ cudaError_t fma_fwd(const AttnArgs& a, int dtype, cudaStream_t st);
 cudaError_t fma_stats(const AttnArgs& a, int dtype, cudaStream_t st);
 cudaError_t fma_scores(const AttnArgs& a, int dtype, cudaStream_t st);
 cudaError_t fma_apply(const AttnArgs& a, int dtype, cudaStream_t st);
+int fma_split_count(const AttnArgs& a, int dtype);       // blocks per unit of the split-key forward (1: not split)
+size_t fma_split_workspace_bytes(const AttnArgs& a, int dtype);
+cudaError_t fma_split(const AttnArgs& a, int dtype, cudaStream_t st);   // a.ws holds the workspace
 bool fma_row_supports(const AttnArgs& a, int dtype);     // x, alpha and lse in one pass (short key sequences)
 cudaError_t fma_row(const AttnArgs& a, int dtype, cudaStream_t st);
 cudaError_t fma_bwd(const AttnArgs& a, const BwdArgs& g, int dtype, cudaStream_t st);
@@ -51,6 +54,12 @@ cudaError_t tile_take_abort(int* out, cudaStream_t st);
 int tile_split_count(const AttnArgs& a);                 // 0: the split-key forward does not apply (Lq > 128)
 size_t tile_split_workspace_bytes(const AttnArgs& a);
 cudaError_t tile_split(const AttnArgs& a, int dtype, cudaStream_t st);   // a.ws holds the workspace
+
+// at most 16 queries, 16-bit arrays, no side input: keys streamed through warp-level products (attn_decode.cu)
+bool decode_supports(const AttnArgs& a, int dtype);
+int decode_split_count(const AttnArgs& a);
+size_t decode_workspace_bytes(const AttnArgs& a);        // 0: too few keys to split
+cudaError_t decode_fwd(const AttnArgs& a, int dtype, int n_splits, cudaStream_t st);   // a.ws holds the workspace
 
 // x and alpha in one pass when a query's whole score row fits in tensor memory (attn_short.cu)
 bool short_supports(const AttnArgs& a, int dtype);

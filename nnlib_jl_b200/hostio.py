@@ -145,7 +145,7 @@ class HostPipelinedAttention:
                         else:
                             m = self.mask[:, l0:l1]
                         _fused_into(q[:, l0:l1, e:e + 1], k[:, :, e:e + 1], v[:, :, e:e + 1], m, self.nheads,
-                                    x[:, l0:l1, e:e + 1], self.lse[s][lse_off + l0 * self.nheads:])
+                                    x[:, l0:l1, e:e + 1], self.lse[s][lse_off + l0 * self.nheads:], piece=True)
                         self.piece_computed[pz].record(comp)
                         self.out_stream.wait_event(self.piece_computed[pz])
                         with torch.cuda.stream(self.out_stream):

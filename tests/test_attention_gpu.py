@@ -1742,3 +1742,34 @@ def test_float32_masked_keys_may_hold_anything():
         out.append([nb.jl_to_numpy(t) for t in (x, a.materialize(), dq, dk, dv, x2, a2)])
     for want, got in zip(*out):
         np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("dtype,d,dv,H,B,Lq,Lkv,off", [
+    (torch.bfloat16, 128, 128, 2, 1, 1, 1, 0),          # one key
+    (torch.bfloat16, 64, 64, 3, 2, 8, 17, 9),           # one key past a step of 16; all 8 rows of the small form
+    (torch.float16, 128, 128, 4, 120, 9, 130, 121),     # 9 queries: the 16-row form; one CTA per unit
+    (torch.bfloat16, 80, 40, 2, 3, 16, 999, 983),       # heads narrower than the padded sizes, dv != d
+    (torch.float16, 8, 128, 2, 1, 1, 5000, 4999),       # split, d = 8
+    (torch.bfloat16, 128, 64, 1, 1, 16, 4097, 4000),    # split, the last keys out of every query's reach
+    (torch.bfloat16, 64, 64, 2, 2, 5, 700, -2),         # the first two queries see no key
+    (torch.float16, 64, 64, 2, 2, 7, 300, None),        # no mask
+    (torch.float32, 64, 64, 2, 1, 1, 3000, 2999),       # exact Float32, keys split over blocks of 8 queries
+    (torch.float32, 128, 96, 1, 2, 40, 1500, 1460),     # ... and of 32
+    (torch.float32, 32, 32, 2, 1, 4, 2000, -1),         # ... the first query sees no key
+])
+def test_decode_steps_match_the_oracle(dtype, d, dv, H, B, Lq, Lkv, off):
+    """A handful of queries against a key / value history: x and (through the lazy alpha) the log-sum-exp."""
+    rng = np.random.default_rng(500 + Lq + Lkv)
+    qn = _round_to(rng.standard_normal((d * H, Lq, B)), dtype)
+    kn = _round_to(rng.standard_normal((d * H, Lkv, B)), dtype)
+    vn = _round_to(rng.standard_normal((dv * H, Lkv, B)), dtype)
+    mask = None if off is None else _offset_mask(Lkv, Lq, off)
+    y, a = nb.dot_product_attention(_dev(qn, dtype), _dev(kn, dtype), _dev(vn, dtype),
+                                    mask=None if off is None else nb.CausalMask(off), nheads=H)
+    with np.errstate(invalid="ignore"):
+        yo, ao = O.dot_product_attention(qn, kn, vn, mask=mask, nheads=H)
+    live = np.ones(Lq, bool) if mask is None else mask.any(axis=0)
+    yn, an = nb.jl_to_numpy(y), np.asarray(a)
+    _close(yn[:, live], yo[:, live], dtype, "x")
+    _close(an[:, live], ao[:, live], dtype, "alpha")
+    assert np.isnan(yn[:, ~live]).all() and np.isnan(an[:, ~live]).all()
