@@ -513,6 +513,7 @@ int nnlib_b200_batched_gemm(const nnlib_b200_gemm_params* p, void* stream) {
                  (double)g.beta, why ? "cuda-core" : "tcgen05", why ? ": " : "", why ? why : "");
   }
   if (!why) return finish(gemm_umma(g, p->dtype, (cudaStream_t)stream));
+  if (!force_simt() && gemm_mma_supports(g, p->dtype)) return finish(gemm_mma(g, p->dtype, (cudaStream_t)stream));
   return finish(gemm_simt(g, p->dtype, (cudaStream_t)stream));
 }
 

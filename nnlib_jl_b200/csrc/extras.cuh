@@ -43,6 +43,21 @@ __device__ __forceinline__ RowSide make_row_side(const AttnArgs& a, int i, int h
   return rs;
 }
 
+// 4 N bytes from p, at any alignment, as words; bytes at and beyond `end` are whatever shares a word with a byte in
+// front of it, else 0.  Aligned words are read and shifted into place, all loads under way together (a word that
+// holds a byte of the array lies within the array's allocation, whose granularity is far coarser).
+template <int N>
+__device__ __forceinline__ void load_shifted(const unsigned char* p, const unsigned char* end, unsigned int (&w)[N]) {
+  const unsigned int mis = (unsigned int)(reinterpret_cast<unsigned long long>(p) & 3ull);
+  const unsigned char* q = p - mis;
+  unsigned int x[N + 1];
+#pragma unroll
+  for (int i = 0; i <= N; ++i)
+    x[i] = (q + 4 * i < end && (i < N || mis != 0u)) ? __ldg(reinterpret_cast<const unsigned int*>(q + 4 * i)) : 0u;
+#pragma unroll
+  for (int i = 0; i < N; ++i) w[i] = __funnelshift_r(x[i], x[i + 1], 8u * mis);
+}
+
 // Start the 16-byte loads of keys jj0 .. jj0+31 (only when the whole chunk lies inside the array).
 template <bool WITH_BIAS>
 __device__ __forceinline__ void side_issue(const RowSide& rs, int jj0, int Lkv, uint4 (&bq)[4], uint4 (&mq)[2]) {

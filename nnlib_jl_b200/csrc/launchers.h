@@ -76,6 +76,8 @@ cudaError_t umma_bwd_take_abort(int* out, cudaStream_t st);
 const char* gemm_umma_reject_reason(const GemmArgs& g, int dtype);
 cudaError_t gemm_umma(const GemmArgs& g, int dtype, cudaStream_t st);
 cudaError_t gemm_simt(const GemmArgs& g, int dtype, cudaStream_t st);
+bool gemm_mma_supports(const GemmArgs& g, int dtype);    // 16-bit, any alignment: warp-level products (gemm_mma.cu)
+cudaError_t gemm_mma(const GemmArgs& g, int dtype, cudaStream_t st);
 cudaError_t gemm_take_abort(int* out, cudaStream_t st);
 
 // softmax / logsoftmax over one dimension (softmax.cu)

@@ -209,3 +209,28 @@ def test_float32_product_tiles(ta, tb, M, N, K, nbatch):
     # each of K fused multiply-adds rounds once: |error| <= K 2^-24 sum_k |a b|
     bound = K * 2.0 ** -24 * np.einsum("mkb,knb->mnb", np.abs(a64), np.abs(b64)) + 1e-30
     assert (np.abs(got - want) <= bound).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("ta,tb", [("N", "N"), ("T", "N"), ("N", "T"), ("T", "T")])
+@pytest.mark.parametrize("M,N,K,nbatch", [
+    (33, 47, 17, 2),          # smallest tiles, one K element past a fragment
+    (129, 127, 95, 2),        # one row past a tile, K one short of whole stages
+    (257, 131, 33, 3),        # several tiles, one K element past a stage
+])
+def test_products_the_copy_engine_cannot_address(dtype, ta, tb, M, N, K, nbatch):
+    """16-bit arrays with odd leading dimensions (every 2-byte alignment in turn), with an addend as well."""
+    rng = np.random.default_rng(M * 3 + N + K)
+    An = _round_to(rng.standard_normal((M, K, nbatch) if ta == "N" else (K, M, nbatch)), dtype)
+    Bn = _round_to(rng.standard_normal((K, N, nbatch) if tb == "N" else (N, K, nbatch)), dtype)
+    Cn = _round_to(rng.standard_normal((M, N, nbatch)), dtype)
+    A, B = _dev(An, dtype), _dev(Bn, dtype)
+    opA = A if ta == "N" else nb.batched_transpose(A)
+    opB = B if tb == "N" else nb.batched_transpose(B)
+    C = _dev(Cn, dtype)
+    assert BM.batched_mul_path(C, opA, opB) == _lib.PATH_SIMT
+    got = nb.jl_to_numpy(nb.batched_mul(opA, opB))
+    zero = np.zeros((M, N, nbatch), np.float32)
+    _close(got, BO.batched_gemm(ta, tb, np.float32(1), An, Bn, np.float32(0), zero), dtype, f"{ta}{tb}")
+    nb.batched_mul_(C, opA, opB, 0.5, 2.0)
+    _close(nb.jl_to_numpy(C), BO.batched_gemm(ta, tb, np.float32(0.5), An, Bn, np.float32(2), Cn), dtype, f"{ta}{tb} with an addend")
