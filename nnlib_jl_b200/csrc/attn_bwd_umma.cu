@@ -29,6 +29,7 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "extras.cuh"
 #include "launchers.h"
 #include "umma.cuh"
 #include "umma_shared.cuh"
@@ -106,6 +107,8 @@ __device__ __forceinline__ void load_mask64(const unsigned char* p, long long st
       const uint4 q = __ldg(reinterpret_cast<const uint4*>(p) + v);
       mw[4 * v + 0] = q.x; mw[4 * v + 1] = q.y; mw[4 * v + 2] = q.z; mw[4 * v + 3] = q.w;
     }
+  } else if (stride == 1 && n_valid >= 64) {
+    load_shifted<16>(p, p + 64, mw);     // rows of any other alignment: aligned words, shifted into place
   } else {
 #pragma unroll
     for (int w = 0; w < 16; ++w) {
@@ -130,6 +133,8 @@ __device__ __forceinline__ void load_bias16x64(const unsigned char* p, long long
       const uint4 q = __ldg(reinterpret_cast<const uint4*>(p) + v);
       bw[4 * v + 0] = q.x; bw[4 * v + 1] = q.y; bw[4 * v + 2] = q.z; bw[4 * v + 3] = q.w;
     }
+  } else if (stride == 1 && n_valid >= 64) {
+    load_shifted<32>(p, p + 128, bw);    // (2-byte elements)
   } else {
 #pragma unroll
     for (int w = 0; w < 32; ++w) {

@@ -87,7 +87,8 @@ static_assert(sizeof(Barriers) <= 512, "barrier block");
 // BSM: the bias tiles arrive in shared memory by TMA (a whole round ahead, issued by the otherwise
 // idle warp 2) instead of through per-thread loads; needs a 16-bit bias with key stride 1 whose rows
 // the tensor map can address (the host decides).
-template <int D, bool BF16, int XM, bool STATS, bool BSM>
+// SHIFT: bias / mask rows of any alignment (extras.cuh); without it they are all aligned and whole.
+template <int D, bool BF16, int XM, bool STATS, bool BSM, bool SHIFT>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_fwd_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_b,
@@ -357,8 +358,8 @@ attn_fwd_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         // bias / mask of the first 64 keys of this tile: in flight while the scores are awaited
         uint4 bq[2][4], mq[2][2];
         if (EXTRAS) {
-          side_issue<XBIAS && !BSM>(rs, j * kBN, a.Lkv, bq[0], mq[0]);
-          side_issue<XBIAS && !BSM>(rs, j * kBN + 32, a.Lkv, bq[1], mq[1]);
+          side_issue<XBIAS && !BSM, SHIFT>(rs, j * kBN, a.Lkv, bq[0], mq[0]);
+          side_issue<XBIAS && !BSM, SHIFT>(rs, j * kBN + 32, a.Lkv, bq[1], mq[1]);
         }
         // which of this tile's 128 scores survive dropout depends on their position only: drawn while
         // the tensor core still works on the scores
@@ -406,8 +407,8 @@ attn_fwd_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 if (lane == 0) mbar_arrive(&bars->bias_empty[t][hf]);
               }
             }
-            side_apply<XBIAS, BSM>(rs, sr[c], bq[c & 1], mq[c & 1], j0 + c * 32, a.Lkv, lim, row_ok, c2);
-            if (c + 2 < 4) side_issue<XBIAS && !BSM>(rs, j0 + (c + 2) * 32, a.Lkv, bq[c & 1], mq[c & 1]);
+            side_apply<XBIAS, BSM, SHIFT>(rs, sr[c], bq[c & 1], mq[c & 1], j0 + c * 32, a.Lkv, lim, row_ok, c2);
+            if (c + 2 < 4) side_issue<XBIAS && !BSM, SHIFT>(rs, j0 + (c + 2) * 32, a.Lkv, bq[c & 1], mq[c & 1]);
           }
           if (!ok) break;
         } else if (j0 + kBN - 1 > lim) {
@@ -1075,10 +1076,10 @@ int fwd_sm_count() {
   return n;
 }
 
-template <int D, bool BF16, int XM, bool STATS, bool BSM>
+template <int D, bool BF16, int XM, bool STATS, bool BSM, bool SHIFT>
 cudaError_t launch_fwd_impl(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mb,
                             const AttnArgs& a, cudaStream_t st) {
-  auto kern = attn_fwd_umma_kernel<D, BF16, XM, STATS, BSM>;
+  auto kern = attn_fwd_umma_kernel<D, BF16, XM, STATS, BSM, SHIFT>;
   constexpr int smem = BSM ? Cfg<D>::kSmemBytesStaged : Cfg<D>::kSmemBytes;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
@@ -1094,14 +1095,29 @@ cudaError_t launch_fwd_impl(const CUtensorMap& mq, const CUtensorMap& mk, const 
   return cudaGetLastError();
 }
 
+// every row of the mask (of the bias) starts on a 16-byte boundary and holds whole chunks of 32 keys
+bool mask_rows_aligned(const AttnArgs& a) {
+  return !a.mask || (a.mask_s[0] == 1 && aligned16(a.mask) && a.mask_s[1] % 16 == 0 && a.mask_s[2] % 16 == 0 &&
+                     a.mask_s[3] % 16 == 0 && a.Lkv % 32 == 0);
+}
+bool bias_rows_aligned(const AttnArgs& a) {
+  return !a.bias || (a.bias_dtype != NNLIB_B200_F32 && a.bias_s[0] == 1 && aligned16(a.bias) && a.bias_s[1] % 8 == 0 &&
+                     a.bias_s[2] % 8 == 0 && a.bias_s[3] % 8 == 0 && a.Lkv % 32 == 0);
+}
+
 // `mb` != nullptr: the bias can be staged through shared memory by TMA (d = 64 forward with bias)
 template <int D, bool BF16, int XM, bool STATS>
 cudaError_t launch_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap* mb,
                        const AttnArgs& a, cudaStream_t st) {
-  if constexpr (D == 64 && (XM % 3) == 2 && !STATS) {
-    if (mb) return launch_fwd_impl<D, BF16, XM, STATS, true>(mq, mk, mv, *mb, a, st);
+  if constexpr ((XM % 3) != 0 && !STATS) {
+    const bool mask_al = mask_rows_aligned(a);
+    if constexpr (D == 64 && (XM % 3) == 2) {
+      if (mb && mask_al) return launch_fwd_impl<D, BF16, XM, STATS, true, false>(mq, mk, mv, *mb, a, st);
+      if (mb) return launch_fwd_impl<D, BF16, XM, STATS, true, true>(mq, mk, mv, *mb, a, st);
+    }
+    if (mask_al && bias_rows_aligned(a)) return launch_fwd_impl<D, BF16, XM, STATS, false, false>(mq, mk, mv, mq, a, st);
   }
-  return launch_fwd_impl<D, BF16, XM, STATS, false>(mq, mk, mv, mq, a, st);
+  return launch_fwd_impl<D, BF16, XM, STATS, false, true>(mq, mk, mv, mq, a, st);
 }
 
 template <int D, bool BF16, int XM, bool TST>

@@ -2,9 +2,9 @@
 //
 // A softmax / epilogue thread owns one query row and walks over its keys in
 // chunks of 32.  bias (NNlib.jl src/attention.jl:129-131) and mask (:133-138)
-// may have any strides; when the key stride is 1 and the row starts on a
-// 16-byte boundary, a chunk is fetched with 16-byte loads that are issued one
-// chunk ahead of their use, otherwise element by element.
+// may have any strides; when the key stride is 1, a chunk is fetched with
+// 16-byte loads (the row starts on a 16-byte boundary) or aligned words that are
+// issued one chunk ahead of their use, otherwise element by element.
 #pragma once
 
 #include "common.cuh"
@@ -18,6 +18,7 @@ struct RowSide {
   int bias_dtype;
   bool bias_vec;                  // 2-byte elements, key stride 1, 16-byte aligned row
   bool mask_vec;                  // key stride 1, 16-byte aligned row
+  bool bias_s1, mask_s1;          // key stride 1 whatever the alignment (bias: 2-byte elements)
 };
 
 __device__ __forceinline__ RowSide make_row_side(const AttnArgs& a, int i, int h, int b, bool row_ok) {
@@ -27,18 +28,20 @@ __device__ __forceinline__ RowSide make_row_side(const AttnArgs& a, int i, int h
   rs.bias_s0 = a.bias_s[0];
   rs.mask_s0 = a.mask_s[0];
   rs.bias_dtype = a.bias_dtype;
-  rs.bias_vec = false;
-  rs.mask_vec = false;
+  rs.bias_vec = rs.bias_s1 = false;
+  rs.mask_vec = rs.mask_s1 = false;
   if (row_ok && a.bias) {
     const long long off = (long long)i * a.bias_s[1] + (long long)h * a.bias_s[2] + (long long)b * a.bias_s[3];
     const int esz = (a.bias_dtype == NNLIB_B200_F32) ? 4 : 2;
     rs.bias_row = reinterpret_cast<const unsigned char*>(a.bias) + off * esz;
-    rs.bias_vec = (esz == 2) && (a.bias_s[0] == 1) && ((reinterpret_cast<unsigned long long>(rs.bias_row) & 15ull) == 0);
+    rs.bias_s1 = (esz == 2) && (a.bias_s[0] == 1);
+    rs.bias_vec = rs.bias_s1 && ((reinterpret_cast<unsigned long long>(rs.bias_row) & 15ull) == 0);
   }
   if (row_ok && a.mask) {
     const long long off = (long long)i * a.mask_s[1] + (long long)h * a.mask_s[2] + (long long)b * a.mask_s[3];
     rs.mask_row = a.mask + off;
-    rs.mask_vec = (a.mask_s[0] == 1) && ((reinterpret_cast<unsigned long long>(rs.mask_row) & 15ull) == 0);
+    rs.mask_s1 = (a.mask_s[0] == 1);
+    rs.mask_vec = rs.mask_s1 && ((reinterpret_cast<unsigned long long>(rs.mask_row) & 15ull) == 0);
   }
   return rs;
 }
@@ -58,19 +61,38 @@ __device__ __forceinline__ void load_shifted(const unsigned char* p, const unsig
   for (int i = 0; i < N; ++i) w[i] = __funnelshift_r(x[i], x[i + 1], 8u * mis);
 }
 
-// Start the 16-byte loads of keys jj0 .. jj0+31 (only when the whole chunk lies inside the array).
-template <bool WITH_BIAS>
+// Start the loads of keys jj0 .. jj0+31: 16 bytes each where the row is aligned and the chunk whole, else aligned
+// words.  (Rows of an odd number of keys are aligned once in eight; read one element after the other, as other strides
+// still are in groups of eight, they cost 32 load latencies per chunk: x and alpha of 5356 keys with bias and mask
+// took 10.1 ms, 4.1 so.)
+// SHIFT = false: a kernel compiled for calls whose rows are all aligned and whole (the host decides); it holds no trace
+// of the other form, which costs the aligned calls 5 - 10 %.
+template <bool WITH_BIAS, bool SHIFT = true>
 __device__ __forceinline__ void side_issue(const RowSide& rs, int jj0, int Lkv, uint4 (&bq)[4], uint4 (&mq)[2]) {
   const bool inside = jj0 + 32 <= Lkv;
-  if (WITH_BIAS && rs.bias_vec && inside) {
-    const uint4* p = reinterpret_cast<const uint4*>(rs.bias_row + (long long)jj0 * 2);
+  if (WITH_BIAS && (SHIFT ? rs.bias_s1 : rs.bias_vec && inside)) {
+    const unsigned char* p = rs.bias_row + (long long)jj0 * 2;
+    if (!SHIFT || (rs.bias_vec && inside)) {
 #pragma unroll
-    for (int v = 0; v < 4; ++v) bq[v] = __ldg(p + v);
+      for (int v = 0; v < 4; ++v) bq[v] = __ldg(reinterpret_cast<const uint4*>(p) + v);
+    } else {
+      unsigned int w[16];
+      load_shifted<16>(p, rs.bias_row + (long long)Lkv * 2, w);
+#pragma unroll
+      for (int v = 0; v < 4; ++v) bq[v] = make_uint4(w[4 * v], w[4 * v + 1], w[4 * v + 2], w[4 * v + 3]);
+    }
   }
-  if (rs.mask_vec && inside) {
-    const uint4* p = reinterpret_cast<const uint4*>(rs.mask_row + jj0);
+  if (SHIFT ? rs.mask_s1 : rs.mask_vec && inside) {
+    const unsigned char* p = rs.mask_row + jj0;
+    if (!SHIFT || (rs.mask_vec && inside)) {
 #pragma unroll
-    for (int v = 0; v < 2; ++v) mq[v] = __ldg(p + v);
+      for (int v = 0; v < 2; ++v) mq[v] = __ldg(reinterpret_cast<const uint4*>(p) + v);
+    } else {
+      unsigned int w[8];
+      load_shifted<8>(p, rs.mask_row + Lkv, w);
+#pragma unroll
+      for (int v = 0; v < 2; ++v) mq[v] = make_uint4(w[4 * v], w[4 * v + 1], w[4 * v + 2], w[4 * v + 3]);
+    }
   }
 }
 
@@ -114,14 +136,14 @@ __device__ __forceinline__ unsigned int mask_keep_bits_bytes(const RowSide& rs, 
 // masked, beyond `lim` (causal / end of the keys) or the row is out of range.  Works in place.
 // BIAS_STAGED: bq was filled from a shared-memory copy of the bias tile (zero beyond the array), so the
 // vector form applies to every chunk.
-template <bool WITH_BIAS, bool BIAS_STAGED = false>
+template <bool WITH_BIAS, bool BIAS_STAGED = false, bool SHIFT = true>
 __device__ __forceinline__ void side_apply(const RowSide& rs, unsigned int (&s)[32], const uint4 (&bq)[4],
                                            const uint4 (&mq)[2], int jj0, int Lkv, int lim, bool row_ok, float c2) {
   constexpr float kLog2eF = 1.4426950408889634f;
   const bool inside = jj0 + 32 <= Lkv;
   const int lim_e = row_ok ? lim - jj0 : -1;   // element e of the chunk is in range iff e <= lim_e
   // ---- scale (+ bias)
-  if (WITH_BIAS && rs.bias_row && (BIAS_STAGED || (rs.bias_vec && inside))) {
+  if (WITH_BIAS && rs.bias_row && (BIAS_STAGED || (SHIFT ? rs.bias_s1 : rs.bias_vec && inside))) {
     if (rs.bias_dtype == NNLIB_B200_BF16) {
 #pragma unroll
       for (int e = 0; e < 32; e += 2) {
@@ -146,14 +168,14 @@ __device__ __forceinline__ void side_apply(const RowSide& rs, unsigned int (&s)[
       float bv = 0.f;
       if (e <= lim_e) bv = load_bias(rs.bias_row, (jj0 + e) * rs.bias_s0, rs.bias_dtype) * kLog2eF;
       s[e] = __float_as_uint(fmaf(__uint_as_float(s[e]), c2, bv));
-      asm volatile("" ::: "memory");   // one load at a time: this path must not cost registers
+      if (!SHIFT || (e & 7) == 7) asm volatile("" ::: "memory");   // few loads at a time: this path must not cost registers
     }
   } else {
 #pragma unroll
     for (int e = 0; e < 32; ++e) s[e] = __float_as_uint(__uint_as_float(s[e]) * c2);
   }
   // ---- range and mask
-  if (rs.mask_row && rs.mask_vec && inside) {
+  if (rs.mask_row && (SHIFT ? rs.mask_s1 : rs.mask_vec && inside)) {
     // most chunks of a padding-style mask are all true: one test instead of 32 byte extractions
     const unsigned int nz = nonzero_bytes(mq[0].x) & nonzero_bytes(mq[0].y) & nonzero_bytes(mq[0].z) &
                             nonzero_bytes(mq[0].w) & nonzero_bytes(mq[1].x) & nonzero_bytes(mq[1].y) &
@@ -171,7 +193,7 @@ __device__ __forceinline__ void side_apply(const RowSide& rs, unsigned int (&s)[
       bool keep = e <= lim_e;
       if (keep) keep = rs.mask_row[(jj0 + e) * rs.mask_s0] != 0;
       if (!keep) s[e] = 0xff800000u;
-      asm volatile("" ::: "memory");     // one load at a time: this path must not cost registers
+      if (!SHIFT || (e & 7) == 7) asm volatile("" ::: "memory");   // few loads at a time: this path must not cost registers
     }
   } else if (lim_e < 31) {
 #pragma unroll

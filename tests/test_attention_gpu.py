@@ -1773,3 +1773,45 @@ def test_decode_steps_match_the_oracle(dtype, d, dv, H, B, Lq, Lkv, off):
     _close(yn[:, live], yo[:, live], dtype, "x")
     _close(an[:, live], ao[:, live], dtype, "alpha")
     assert np.isnan(yn[:, ~live]).all() and np.isnan(an[:, ~live]).all()
+
+
+@pytest.mark.parametrize("dtype,d,dv,Lq,Lkv,shift", [
+    (torch.bfloat16, 64, 64, 70, 203, 0),       # rows of odd length: every alignment of bias and mask in turn
+    (torch.float16, 128, 128, 130, 257, 0),     # one key past a whole tile
+    (torch.bfloat16, 96, 40, 33, 333, 0),       # the one-tile kernels
+    (torch.float16, 64, 64, 40, 640, 1),        # rows of whole 16 bytes, shifted off their boundary by one element
+    (torch.bfloat16, 128, 128, 40, 200, 3),
+])
+def test_bias_and_mask_rows_of_any_alignment(dtype, d, dv, Lq, Lkv, shift):
+    """Bias and Bool mask with key stride 1 whose rows start anywhere: x, alpha (lazy and eager) and the gradients."""
+    rng = np.random.default_rng(700 + Lkv)
+    H, B = 2, 2
+    qn, kn = (_round_to(rng.standard_normal((d * H, L, B)), dtype) for L in (Lq, Lkv))
+    vn = _round_to(rng.standard_normal((dv * H, Lkv, B)), dtype)
+    bn = _round_to(0.5 * rng.standard_normal((Lkv, Lq, H, B)), dtype)
+    mask = rng.random((Lkv, Lq, H, B)) > 0.3
+    mask[0] = True
+
+    def dev(a, dt):   # column-major copy that starts `shift` elements behind an aligned address
+        flat = torch.zeros(a.size + shift + 64, dtype=dt, device=DEV)
+        flat[shift:shift + a.size] = torch.from_numpy(np.ascontiguousarray(a.transpose(3, 2, 1, 0))).reshape(-1).to(DEV).to(dt)
+        return flat[shift:shift + a.size].view(a.shape[::-1]).permute(3, 2, 1, 0)
+
+    q, k, v, b, m = _dev(qn, dtype), _dev(kn, dtype), _dev(vn, dtype), dev(bn, dtype), dev(mask, torch.bool)
+    yo, ao = O.dot_product_attention(qn, kn, vn, bn, mask=mask, nheads=H)
+    y, a = nb.dot_product_attention(q, k, v, b, mask=m, nheads=H)
+    nb.set_scores_mode("eager")
+    try:
+        y2, a2 = nb.dot_product_attention(q, k, v, b, mask=m, nheads=H)
+    finally:
+        nb.set_scores_mode("lazy")
+    for what, yt, at in (("lazy", nb.jl_to_numpy(y), np.asarray(a)), ("eager", nb.jl_to_numpy(y2), nb.jl_to_numpy(a2))):
+        _close(yt, yo, dtype, "x, " + what)
+        _close(at, ao, dtype, "alpha, " + what)
+        assert (at[~mask] == 0).all()
+    dyn = _round_to(rng.standard_normal((dv * H, Lq, B)), dtype)
+    _, _, back = nb.dot_product_attention_pullback(q, k, v, b, mask=m, nheads=H)
+    got = back(_dev(dyn, dtype))
+    want = O.dot_product_attention_grad(qn, kn, vn, dyn, bn, mask=mask, nheads=H)
+    for name, g, w in zip(("dq", "dk", "dv", "dbias"), got, want):
+        _grad_close(nb.jl_to_numpy(g), w, dtype, name)
