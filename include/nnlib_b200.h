@@ -296,8 +296,8 @@ NNLIB_B200_API int nnlib_b200_softmax_bwd(const nnlib_b200_softmax_params* p, vo
    (i, j) of a stored matrix sits at X[i + ld*j + stride*b]; a batch stride of 0 for A or B uses one matrix for
    every batch (size(A, 3) == 1 in the reference, src/gemm.jl:116-117).  beta = 0 never reads C.  Accumulation
    is fp32.  16-bit element types with 16-byte aligned A and B and leading dimensions / batch strides that are
-   multiples of 8 elements run on the tensor cores (tcgen05), everything else (Float32 included) on a plain
-   CUDA-core kernel. */
+   multiples of 8 elements run on the tensor cores (tcgen05), other 16-bit arrays on warp-level products and
+   Float32 on a tiled CUDA-core kernel (both NNLIB_B200_PATH_SIMT). */
 typedef struct nnlib_b200_gemm_params {
   size_t struct_size;        /* = sizeof(nnlib_b200_gemm_params) */
   int32_t dtype;             /* NNLIB_B200_F16 / BF16 / F32: element type of A, B and C */
