@@ -493,8 +493,9 @@ def _launch_unit_exact(pr, piece: bool = False):
         return
     lib, p = _lib.load(), pr.p
     reach = max(0, min(pr.Lkv, pr.Lq + p.causal_offset)) if p.causal else pr.Lkv
-    by_keys = not piece and reach > 1024 and pr.Lq <= 32 and not p.dropout_p > 0 and not p.allow_tf32 and pr.d <= 128 and \
-        pr.dv <= 128 and (pr.dtype == torch.float32 or (pr.Lq <= 16 and not p.bias and not p.mask))
+    few = 1024 if pr.Lq <= 8 or pr.dtype == torch.float32 else 2048      # up to so many keys nothing is split by keys
+    by_keys = not piece and reach > few and pr.Lq <= 32 and not p.dropout_p > 0 and not p.allow_tf32 and \
+        pr.d <= 128 and pr.dv <= 128 and (pr.dtype == torch.float32 or (pr.Lq <= 16 and not p.bias and not p.mask))
     with torch.cuda.device(pr.dev):
         need = lib.nnlib_b200_attn_decode_workspace_bytes(C.byref(p)) if by_keys else 0
         if need:
