@@ -128,7 +128,8 @@ attn_decode_kernel(const AttnArgs a, const int n_splits, const int steps_per_spl
       qf[r][G] = (i < a.Lq && f < a.d) ? *reinterpret_cast<const uint4*>(qp + f) : zero4;
     }
   }
-  // keys of step s; past the end the last attended key is read again (its weight is zero)
+  // keys of step s; past the end the last attended key of K is read again (its score is not used) and V is zero (the
+  // weight there is zero, but 0 * Inf would be a NaN; zeroing V where it is used instead costs every step 2 %)
   uint4 kf[2][GQ], vf[4][GV];
   auto load_k = [&](int s) {
 #pragma unroll
@@ -144,11 +145,12 @@ attn_decode_kernel(const AttnArgs a, const int n_splits, const int steps_per_spl
   auto load_v = [&](int s) {
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const T* vp = vbase + (long long)min(s * kDecKeys + 2 * c + (u & 1) + (u >> 1) * 8, kend - 1) * a.v_sl;
+      const int j = s * kDecKeys + 2 * c + (u & 1) + (u >> 1) * 8;
+      const T* vp = vbase + (long long)j * a.v_sl;
 #pragma unroll
       for (int F = 0; F < GV; ++F) {
         const int f = 64 * F + 8 * g;
-        vf[u][F] = (f < a.dv) ? load_stream(vp + f) : zero4;
+        vf[u][F] = (f < a.dv && j < kend) ? load_stream(vp + f) : zero4;
       }
     }
   };

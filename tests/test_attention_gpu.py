@@ -1815,3 +1815,21 @@ def test_bias_and_mask_rows_of_any_alignment(dtype, d, dv, Lq, Lkv, shift):
     want = O.dot_product_attention_grad(qn, kn, vn, dyn, bn, mask=mask, nheads=H)
     for name, g, w in zip(("dq", "dk", "dv", "dbias"), got, want):
         _grad_close(nb.jl_to_numpy(g), w, dtype, name)
+
+
+@pytest.mark.parametrize("dtype,d,Lq", [(torch.bfloat16, 128, 1), (torch.float16, 64, 3), (torch.bfloat16, 64, 12)])
+def test_decode_with_an_infinite_value_in_the_last_key(dtype, d, Lq):
+    """The number of keys is not a multiple of the 16 a warp takes at a time: what fills up the last step must not
+    bring the infinite value in once more with weight zero (0 * Inf = NaN)."""
+    rng = np.random.default_rng(d + Lq)
+    H, Lkv = 2, 2053
+    qn = _round_to(rng.standard_normal((d * H, Lq, 1)), dtype)
+    kn = _round_to(rng.standard_normal((d * H, Lkv, 1)), dtype)
+    vn = _round_to(rng.standard_normal((d * H, Lkv, 1)), dtype)
+    vn[5, -1, 0], vn[d + 7, -1, 0] = np.inf, -np.inf
+    y, _ = nb.dot_product_attention(_dev(qn, dtype), _dev(kn, dtype), _dev(vn, dtype), nheads=H)
+    yn = nb.jl_to_numpy(y)
+    assert (yn[5] == np.inf).all() and (yn[d + 7] == -np.inf).all()
+    rest = np.setdiff1d(np.arange(d * H), [5, d + 7])
+    yo, _ = O.dot_product_attention(qn, kn, np.where(np.isfinite(vn), vn, 0), nheads=H)
+    _close(yn[rest], yo[rest], dtype, "x")
