@@ -1756,6 +1756,8 @@ def test_float32_masked_keys_may_hold_anything():
     (torch.float32, 64, 64, 2, 1, 1, 3000, 2999),       # exact Float32, keys split over blocks of 8 queries
     (torch.float32, 128, 96, 1, 2, 40, 1500, 1460),     # ... and of 32
     (torch.float32, 32, 32, 2, 1, 4, 2000, -1),         # ... the first query sees no key
+    (torch.bfloat16, 128, 40, 1, 1, 2, 40000, 39998),   # 40 shares: more than the lanes of the warp that merges them
+    (torch.float32, 64, 64, 1, 1, 1, 8300, 8299),       # 33 shares
 ])
 def test_decode_steps_match_the_oracle(dtype, d, dv, H, B, Lq, Lkv, off):
     """A handful of queries against a key / value history: x and (through the lazy alpha) the log-sum-exp."""
