@@ -304,7 +304,7 @@ cudaError_t launch_decode(const AttnArgs& a, int n_splits, cudaStream_t st) {
   count_launch();
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  attn_split_reduce_kernel<T><<<(unsigned)(a.H * a.B * a.Lq), 128, 0, st>>>(a, n_splits);
+  attn_split_reduce_kernel<T, false><<<(unsigned)(a.H * a.B * a.Lq), 128, 0, st>>>(a, n_splits);
   count_launch();
   return cudaGetLastError();
 }

@@ -11,7 +11,7 @@
 //     FM_SCORES  alpha from a given log-sum-exp; the key tiles of a block row may be dealt to several blocks
 //     FM_APPLY   x = V alpha for scores the caller holds
 //     FM_SPLIT   FM_FWD for few queries against many keys: the key tiles of a unit are dealt to gridDim.y blocks,
-//                each leaving its maximum, sum and unnormalised O in a workspace (split_reduce.cuh merges them)
+//                each leaving its maximum, sum and O in a workspace (split_reduce.cuh merges them)
 // A warp per query that walked the keys one lane per key (attn_simt.cu, still there for larger heads) re-read every
 // key row through L1 for each query, uncoalesced: 441 us for x and alpha at d = 64, 8 heads, 128 x 128, batch 4,
 // where one pass of the row kernel takes 32 us including 25 us of host time between calls.
@@ -129,6 +129,11 @@ __global__ void __launch_bounds__(NTHR, MODE == FM_FWD && MI == 8 && DP == 64 ? 
     kstep = kBN;
   }
   const int d4 = (a.d + 3) >> 2;
+  // O is summed with weights up to 1 a key and divided by their sum at the end: the weights of the sum are taken 2^e
+  // times smaller, 2^e > Lkv, so that values near the end of the type's range do not overflow on the way to their mean
+  const int e_keys = 32 - __clz(a.Lkv);
+  const float p_scale = MODE == FM_APPLY ? 1.f : __int_as_float((127 - e_keys) << 23);
+  const float o_scale = MODE == FM_APPLY ? 1.f : __int_as_float((127 + e_keys) << 23);
   for (int k0 = kstart; k0 < kstop; k0 += kstep) {
     const bool live = MODE == FM_APPLY || k0 < kend;       // false: all above the causal diagonal
     if (MODE != FM_APPLY && live) {
@@ -192,7 +197,7 @@ __global__ void __launch_bounds__(NTHR, MODE == FM_FWD && MI == 8 && DP == 64 ? 
             sum += p;
             if (fm_with_v(MODE)) {
               if (drop && !((keep[r * 8 + (k >> 3)] >> (k & 7)) & 1)) p = 0.f;
-              kp[r * kLDP + k] = p;
+              kp[r * kLDP + k] = p * p_scale;
             }
           }
           l[i] = fmaf(l[i], f, sum);
@@ -229,9 +234,10 @@ __global__ void __launch_bounds__(NTHR, MODE == FM_FWD && MI == 8 && DP == 64 ? 
           a.ws[slot * 2 + 1] = ls;
         }
         float* ow = a.ws + split_ml_floats(a, gridDim.y) + slot * a.dv;
+        const float inv = ls > 0.f ? 1.f / ls : 0.f;
 #pragma unroll
         for (int c = 0; c < CN; ++c)
-          if (colmap<DP>(tx, c) < a.dv) ow[colmap<DP>(tx, c)] = o[i][c];
+          if (colmap<DP>(tx, c) < a.dv) ow[colmap<DP>(tx, c)] = o[i][c] * inv * o_scale;
         continue;
       }
       if (a.lse && tx == 0) a.lse[gi + (long long)a.Lq * h + a.lse_sb * b] = make_lse(m[i], ls);
@@ -247,7 +253,7 @@ __global__ void __launch_bounds__(NTHR, MODE == FM_FWD && MI == 8 && DP == 64 ? 
 #pragma unroll
       for (int c = 0; c < CN; ++c) {
         const int e = colmap<DP>(tx, c);
-        if (e < a.dv) xr[e] = Elem<T>::from_f(special ? fixed : o[i][c] * scale);
+        if (e < a.dv) xr[e] = Elem<T>::from_f(special ? fixed : o[i][c] * scale * o_scale);
       }
     }
   }
@@ -412,7 +418,7 @@ cudaError_t launch_fma_mi(const AttnArgs& a, int vec, cudaStream_t st, int n_spl
   if (MODE == FM_SPLIT) {
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    attn_split_reduce_kernel<T><<<(unsigned)(a.H * a.B * a.Lq), 128, 0, st>>>(a, n_splits);
+    attn_split_reduce_kernel<T, true><<<(unsigned)(a.H * a.B * a.Lq), 128, 0, st>>>(a, n_splits);
     count_launch();
   }
   return cudaGetLastError();

@@ -594,7 +594,7 @@ cudaError_t launch_tile_side(const CUtensorMap& mq, const CUtensorMap& mk, const
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const long long rows = (long long)a.Lq * a.H * a.B;
-    attn_split_reduce_kernel<T><<<(unsigned)rows, 128, 0, st>>>(a, n_splits);
+    attn_split_reduce_kernel<T, false><<<(unsigned)rows, 128, 0, st>>>(a, n_splits);
     count_launch();
   }
   return cudaGetLastError();

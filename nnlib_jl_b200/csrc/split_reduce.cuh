@@ -11,7 +11,7 @@ namespace nb200 {
 namespace {
 
 // Workspace of the split-key forward, in floats: (maximum, sum) per (unit, split, query), rounded up so that
-// the O rows behind them start on a 16-byte boundary, then dv floats of unnormalised O per (unit, split, query).
+// the O rows behind them start on a 16-byte boundary, then dv floats of O per (unit, split, query).
 __host__ __device__ inline long long split_ml_floats(const AttnArgs& a, int n_splits) {
   return (((long long)a.H * a.B * n_splits * a.Lq * 2) + 3) & ~3LL;
 }
@@ -25,7 +25,9 @@ __host__ __device__ inline long long split_ws_floats(const AttnArgs& a, int n_sp
 // sum and weight, and hand these round while the O rows of up to 32 shares are under way; both sums run over the shares
 // in order.  (One query of one unit against 1M keys, 1024 shares: the whole call 493 us with the shares walked one load after
 // the other, 129 so; 8 units, 131072 keys: 154 and 106 us.)
-template <typename T>
+// NORM: O_s is already divided by l_s (attn_fma.cu).  The weights of the sum are taken 2^e times smaller, 2^e > Lkv, so
+// that nothing overflows that the result does not, and a share whose weight vanishes takes no part, whatever its O holds.
+template <typename T, bool NORM>
 __global__ void __launch_bounds__(128) attn_split_reduce_kernel(const AttnArgs a, const int n_splits) {
   const long long row = blockIdx.x;              // unit * Lq + i
   const int i = (int)(row % a.Lq);
@@ -46,6 +48,8 @@ __global__ void __launch_bounds__(128) attn_split_reduce_kernel(const AttnArgs a
   for (int off = 16; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
   any_nan = __any_sync(0xffffffffu, any_nan);
   const bool inf_row = (M == pinf);
+  const int e_keys = 32 - __clz(a.Lkv);
+  const float p_scale = __int_as_float((127 - e_keys) << 23), o_scale = __int_as_float((127 + e_keys) << 23);
   T* xrow = reinterpret_cast<T*>(a.x) + (long long)i * a.x_sl + (long long)b * a.x_sb + (long long)h * a.dv;
   for (int e0 = threadIdx.x - lane; e0 < a.dv; e0 += 128) {
     const int e = min(e0 + lane, a.dv - 1);      // (lanes past the end keep their warp company)
@@ -55,6 +59,7 @@ __global__ void __launch_bounds__(128) attn_split_reduce_kernel(const AttnArgs a
       const int s = s0 + min(lane, cnt - 1);
       const float m = ml[s * sstride * 2], l = ml[s * sstride * 2 + 1];
       const float w = inf_row ? (m == M ? 1.f : 0.f) : exp2f(m - M);
+      const float wo = NORM ? w * (l * p_scale) : w;   // the weight of the share's O
       const unsigned int live = __ballot_sync(0xffffffffu, l > 0.f);
       auto merge = [&](auto group, int j0) {
         constexpr int G = decltype(group)::value;
@@ -64,9 +69,10 @@ __global__ void __launch_bounds__(128) attn_split_reduce_kernel(const AttnArgs a
 #pragma unroll
         for (int j = 0; j < G; ++j) {
           const float wj = __shfl_sync(0xffffffffu, w, j0 + j), lj = __shfl_sync(0xffffffffu, l, j0 + j);
+          const float oj = NORM ? __shfl_sync(0xffffffffu, wo, j0 + j) : wj;
           if (j0 + j < cnt && ((live >> (j0 + j)) & 1u)) {
             L = fmaf(wj, lj, L);
-            acc = fmaf(wj, ov[j], acc);
+            if (!NORM || oj != 0.f) acc = fmaf(oj, ov[j], acc);
           }
         }
       };
@@ -75,6 +81,7 @@ __global__ void __launch_bounds__(128) attn_split_reduce_kernel(const AttnArgs a
     }
     const bool dead = !(L > 0.f) && !any_nan;
     float out = acc * (a.inv_keep / L);
+    if (NORM) out *= o_scale;
     if (dead) out = a.nan_fm ? nanv : 0.f;
     if (any_nan) out = nanv;
     if (e0 + lane < a.dv) xrow[e] = Elem<T>::from_f(out);

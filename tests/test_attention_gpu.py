@@ -1835,3 +1835,28 @@ def test_decode_with_an_infinite_value_in_the_last_key(dtype, d, Lq):
     rest = np.setdiff1d(np.arange(d * H), [5, d + 7])
     yo, _ = O.dot_product_attention(qn, kn, np.where(np.isfinite(vn), vn, 0), nheads=H)
     _close(yn[rest], yo[rest], dtype, "x")
+
+
+@pytest.mark.parametrize("Lq,Lkv", [(3, 700), (40, 700), (70, 100), (2, 3000), (20, 3000)])   # one pass; keys split
+def test_float32_values_near_the_end_of_the_range(Lq, Lkv):
+    """The weighted mean of values of 3e38 is 3e38: the sum before the division must not overflow.  The other features
+    keep their precision, and keys whose weight vanishes may hold infinities."""
+    rng = np.random.default_rng(Lkv)
+    d, H, B = 64, 2, 1
+    qn, kn = (rng.standard_normal((d * H, L, B), dtype=np.float32) for L in (Lq, Lkv))
+    vn = rng.standard_normal((d * H, Lkv, B), dtype=np.float32)
+    qn[0], kn[0], kn[0, :min(260, Lkv // 2)] = 8.0, 0.0, -200.0     # head 0: the first keys have logits of about -200
+    vn[3, 17] = np.inf
+    vn[d + 9] = 3e38
+    vn[d + 10, Lkv // 2] = -2e38                     # one huge value among ordinary ones
+    y, _ = nb.dot_product_attention(*(_dev(t, torch.float32) for t in (qn, kn, vn)), nheads=H)
+    yn = nb.jl_to_numpy(y).astype(np.float64)
+    v64 = np.where(np.isfinite(vn), vn, 0).astype(np.float64)
+    for h in range(H):
+        s = slice(h * d, h * d + d)
+        logit = np.einsum("dj,di->ij", kn[s, :, 0].astype(np.float64), qn[s, :, 0].astype(np.float64)) / np.sqrt(d)
+        al = np.exp(logit - logit.max(1, keepdims=True))
+        al /= al.sum(1, keepdims=True)
+        want, size = v64[s, :, 0] @ al.T, np.abs(v64[s, :, 0]) @ al.T
+        # logits of |q k| <= 60 rounded in fp32 (64 products), the weights carry that and a sum over the keys
+        assert (np.abs(yn[s, :, 0] - want) <= 2e-5 * size).all(), f"head {h}"
