@@ -227,10 +227,10 @@ __global__ void __launch_bounds__(NTHR, MODE == FM_FWD && MI == 8 && DP == 64 ? 
     if (MODE != FM_APPLY) {
       const float ls = sum16(l[i]);                        // all 16 lanes of a row take part
       if (gi >= a.Lq) continue;                            // whole half-warps
-      if (MODE == FM_SPLIT) {                              // the merge works in base 2
+      if (MODE == FM_SPLIT) {
         const long long slot = ((long long)unit * gridDim.y + blockIdx.y) * a.Lq + gi;
         if (tx == 0) {
-          a.ws[slot * 2] = m[i] * 1.4426950408889634f;
+          a.ws[slot * 2] = m[i];
           a.ws[slot * 2 + 1] = ls;
         }
         float* ow = a.ws + split_ml_floats(a, gridDim.y) + slot * a.dv;

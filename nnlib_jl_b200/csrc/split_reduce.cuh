@@ -25,9 +25,10 @@ __host__ __device__ inline long long split_ws_floats(const AttnArgs& a, int n_sp
 // sum and weight, and hand these round while the O rows of up to 32 shares are under way; both sums run over the shares
 // in order.  (One query of one unit against 1M keys, 1024 shares: the whole call 493 us with the shares walked one load after
 // the other, 129 so; 8 units, 131072 keys: 154 and 106 us.)
-// NORM: O_s is already divided by l_s (attn_fma.cu).  The weights of the sum are taken 2^e times smaller, 2^e > Lkv, so
+// EXACT (attn_fma.cu): the maxima are natural logarithms, not base 2, whose conversion would be one rounding more, and
+// O_s is already divided by l_s.  The weights of the sum are taken 2^e times smaller, 2^e > Lkv, so
 // that nothing overflows that the result does not, and a share whose weight vanishes takes no part, whatever its O holds.
-template <typename T, bool NORM>
+template <typename T, bool EXACT>
 __global__ void __launch_bounds__(128) attn_split_reduce_kernel(const AttnArgs a, const int n_splits) {
   const long long row = blockIdx.x;              // unit * Lq + i
   const int i = (int)(row % a.Lq);
@@ -58,8 +59,8 @@ __global__ void __launch_bounds__(128) attn_split_reduce_kernel(const AttnArgs a
       const int cnt = min(32, n_splits - s0);
       const int s = s0 + min(lane, cnt - 1);
       const float m = ml[s * sstride * 2], l = ml[s * sstride * 2 + 1];
-      const float w = inf_row ? (m == M ? 1.f : 0.f) : exp2f(m - M);
-      const float wo = NORM ? w * (l * p_scale) : w;   // the weight of the share's O
+      const float w = inf_row ? (m == M ? 1.f : 0.f) : (EXACT ? expf(m - M) : exp2f(m - M));
+      const float wo = EXACT ? w * (l * p_scale) : w;   // the weight of the share's O
       const unsigned int live = __ballot_sync(0xffffffffu, l > 0.f);
       auto merge = [&](auto group, int j0) {
         constexpr int G = decltype(group)::value;
@@ -69,10 +70,10 @@ __global__ void __launch_bounds__(128) attn_split_reduce_kernel(const AttnArgs a
 #pragma unroll
         for (int j = 0; j < G; ++j) {
           const float wj = __shfl_sync(0xffffffffu, w, j0 + j), lj = __shfl_sync(0xffffffffu, l, j0 + j);
-          const float oj = NORM ? __shfl_sync(0xffffffffu, wo, j0 + j) : wj;
+          const float oj = EXACT ? __shfl_sync(0xffffffffu, wo, j0 + j) : wj;
           if (j0 + j < cnt && ((live >> (j0 + j)) & 1u)) {
             L = fmaf(wj, lj, L);
-            if (!NORM || oj != 0.f) acc = fmaf(oj, ov[j], acc);
+            if (!EXACT || oj != 0.f) acc = fmaf(oj, ov[j], acc);
           }
         }
       };
@@ -81,12 +82,12 @@ __global__ void __launch_bounds__(128) attn_split_reduce_kernel(const AttnArgs a
     }
     const bool dead = !(L > 0.f) && !any_nan;
     float out = acc * (a.inv_keep / L);
-    if (NORM) out *= o_scale;
+    if (EXACT) out *= o_scale;
     if (dead) out = a.nan_fm ? nanv : 0.f;
     if (any_nan) out = nanv;
     if (e0 + lane < a.dv) xrow[e] = Elem<T>::from_f(out);
     if (threadIdx.x == 0 && e0 == 0 && a.lse) {
-      float lse = dead ? ninf : (M + log2f(L)) * 0.6931471805599453f;
+      float lse = dead ? ninf : (EXACT ? M + logf(L) : fmaf(M, 0.6931471805599453f, logf(L)));
       if (inf_row && !dead) lse = lse_inf_rows(L);
       if (any_nan) lse = nanv;
       a.lse[i + (long long)a.Lq * h + a.lse_sb * b] = lse;

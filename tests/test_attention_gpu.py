@@ -6,6 +6,7 @@ Tolerances (max-abs, mean-rel = mean|y-ŷ| / mean|ŷ|) against the Float32 oracl
 evaluated on the upcast inputs:
     bf16 : 2e-2 , 5e-3        f16 : 3e-3 , 1e-3        f32 : 1e-5 (atol, like the reference's GPU tests)
 """
+import ctypes
 import math
 import time
 
@@ -1860,3 +1861,18 @@ def test_float32_values_near_the_end_of_the_range(Lq, Lkv):
         want, size = v64[s, :, 0] @ al.T, np.abs(v64[s, :, 0]) @ al.T
         # logits of |q k| <= 60 rounded in fp32 (64 products), the weights carry that and a sum over the keys
         assert (np.abs(yn[s, :, 0] - want) <= 2e-5 * size).all(), f"head {h}"
+
+
+def test_float32_split_log_sum_exp_is_rounded_once():
+    """Every logit of a query is the same t, exactly: its log-sum-exp is t + log(keys), to be rounded once (and once in
+    the logarithm)."""
+    d, Lq, Lkv = 64, 32, 4096
+    t = np.random.default_rng(8).uniform(-90, 90, Lq).astype(np.float32)
+    qn, kn = np.zeros((d, Lq, 1), np.float32), np.zeros((d, Lkv, 1), np.float32)
+    qn[0, :, 0], kn[0] = 8 * t, 1.0                         # the scale is 1/8
+    q, k, v = (_dev(a, torch.float32) for a in (qn, kn, np.ones((d, Lkv, 1), np.float32)))
+    x, alpha = nb.dot_product_attention(q, k, v)
+    assert _lib.load().nnlib_b200_attn_decode_workspace_bytes(ctypes.byref(alpha._problem.p)) > 0   # keys are split
+    got, log_n = alpha._problem.lse.cpu().numpy().reshape(-1), np.log(Lkv)
+    bound = 0.5 * np.spacing(np.abs(t) + np.float32(log_n)) + np.spacing(np.float32(log_n))
+    assert (np.abs(got - (t.astype(np.float64) + log_n)) <= bound).all()
