@@ -178,15 +178,27 @@ NNLIB_B200_API int nnlib_b200_attn_fwd(const nnlib_b200_attn_params* p, void* st
 
 /* The same result as nnlib_b200_attn_fwd for a call with few queries against many keys (Lq <= 128; typically
    one new token, or a handful, against a long key / value history, with causal_offset = Lkv - Lq).  attn_fwd
-   gives such a call one CTA per (head, batch) unit, which leaves most of the GPU idle when H*B is small; here
-   the key tiles of a unit are dealt to several CTAs and a second kernel merges their running maxima, sums and
-   partial outputs.  The partial results live in `workspace` (device memory, 16-byte aligned, at least
-   nnlib_b200_attn_decode_workspace_bytes(p)); when that function returns 0 the call gains nothing from
-   splitting (or its shape is outside the tensor-core kernels) and is simply forwarded to attn_fwd.
+   gives such a call one CTA per (head, batch) unit; here the keys of a unit are cut into shares that run side
+   by side, and a second kernel merges their running maxima, sums and partial outputs.  16-bit arrays with at
+   most 16 queries and no side input stream their keys (csrc/attn_decode.cu), Float32 arrays with at most 32
+   queries and no dropout are split on the CUDA cores (csrc/attn_fma.cu), other calls of few units on the
+   one-tile tensor-core kernels (csrc/attn_tile.cu).  The partial results live in `workspace` (device memory,
+   16-byte aligned, at least nnlib_b200_attn_decode_workspace_bytes(p)); when that function returns 0 the call
+   gains nothing from splitting and is simply forwarded to attn_fwd.
    The reference has no counterpart: make_causal_mask is square only (src/attention.jl:149-153). */
 NNLIB_B200_API size_t nnlib_b200_attn_decode_workspace_bytes(const nnlib_b200_attn_params* p);
 NNLIB_B200_API int nnlib_b200_attn_decode(const nnlib_b200_attn_params* p, void* workspace, size_t workspace_bytes,
                                           void* stream);
+
+/* x (and lse) of some heads and batch elements of a larger call of `units` (head, batch) units, for drivers that
+   cut a call into parts: whatever way nnlib_b200_attn_decode takes for the whole call, the part takes too where
+   that way cuts a unit by its number of keys alone (the first two of the three above), and gives the bits of
+   the whole call; everything else goes through attn_fwd, whose bits do not depend on the other units.  (A whole
+   call that is split on the one-tile kernels is cut by its number of units; its parts agree with it to rounding
+   only.)  Workspace as above, from nnlib_b200_attn_part_workspace_bytes. */
+NNLIB_B200_API size_t nnlib_b200_attn_part_workspace_bytes(const nnlib_b200_attn_params* p, int64_t units);
+NNLIB_B200_API int nnlib_b200_attn_part(const nnlib_b200_attn_params* p, int64_t units, void* workspace,
+                                        size_t workspace_bytes, void* stream);
 
 /* lse only: the first half of dot_product_attention_scores
    (src/attention.jl:117-125) reduced to one float per query. */

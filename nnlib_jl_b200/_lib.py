@@ -35,6 +35,8 @@ EXPORTS = (
     "nnlib_b200_attn_fwd",
     "nnlib_b200_attn_decode",
     "nnlib_b200_attn_decode_workspace_bytes",
+    "nnlib_b200_attn_part",
+    "nnlib_b200_attn_part_workspace_bytes",
     "nnlib_b200_attn_stats",
     "nnlib_b200_attn_scores",
     "nnlib_b200_attn_apply",
@@ -174,6 +176,10 @@ def load() -> C.CDLL:
     lib.nnlib_b200_attn_decode.restype = C.c_int
     lib.nnlib_b200_attn_decode_workspace_bytes.argtypes = [P]
     lib.nnlib_b200_attn_decode_workspace_bytes.restype = C.c_size_t
+    lib.nnlib_b200_attn_part.argtypes = [P, C.c_int64, C.c_void_p, C.c_size_t, C.c_void_p]
+    lib.nnlib_b200_attn_part.restype = C.c_int
+    lib.nnlib_b200_attn_part_workspace_bytes.argtypes = [P, C.c_int64]
+    lib.nnlib_b200_attn_part_workspace_bytes.restype = C.c_size_t
     lib.nnlib_b200_attention.argtypes = [P, C.c_void_p, C.c_size_t, C.c_void_p]
     lib.nnlib_b200_attention.restype = C.c_int
     lib.nnlib_b200_attention_static.argtypes = [P, C.c_void_p]

@@ -483,32 +483,27 @@ def _fused(q, k, v, bias, mask, nheads, dropout):
     return x, LazyAttnScores(pr, (pr.Lkv, pr.Lq, pr.H, pr.B))
 
 
-def _launch_unit_exact(pr, piece: bool = False):
-    """x of a part of a larger call (a shard's heads and batches, a chunk of the batch), the same bits the whole call
-    gives.  The split-key forwards for a handful of queries without side inputs and for exact Float32 split by the
-    number of keys alone, so a part takes them like the whole does; the one-tile kernels split by the number of units
-    as well, and a part does not take those.  ``piece``: a range of a longer call's queries, which the whole call
-    handled in the ordinary forward."""
+def _launch_part(pr, units: int, piece: bool = False):
+    """x of a part of a larger call of ``units`` (head, batch) units: a shard's heads and batches, a chunk of the
+    batch.  The library takes the way it takes for the whole call wherever that way cuts a unit by its number of keys
+    alone, and the part then has the bits of the whole (nnlib_b200_attn_part says what is left).  ``piece``: a range
+    of a longer call's queries, which the whole call handled in the ordinary forward."""
     if pr.Lq == 0 or pr.B == 0:
         return
     lib, p = _lib.load(), pr.p
-    reach = max(0, min(pr.Lkv, pr.Lq + p.causal_offset)) if p.causal else pr.Lkv
-    few = 1024 if pr.Lq <= 8 or pr.dtype == torch.float32 else 2048      # up to so many keys nothing is split by keys
-    by_keys = not piece and reach > few and pr.Lq <= 32 and not p.dropout_p > 0 and not p.allow_tf32 and \
-        pr.d <= 128 and pr.dv <= 128 and (pr.dtype == torch.float32 or (pr.Lq <= 16 and not p.bias and not p.mask))
     with torch.cuda.device(pr.dev):
-        need = lib.nnlib_b200_attn_decode_workspace_bytes(C.byref(p)) if by_keys else 0
-        if need:
-            ws = torch.empty(need, dtype=torch.uint8, device=pr.dev)
-            _check(lib.nnlib_b200_attn_decode(C.byref(p), ws.data_ptr(), need, _stream()), "attn_decode")
-        else:
+        if piece:
             _check(lib.nnlib_b200_attn_fwd(C.byref(p), _stream()), "attn_fwd")
+            return
+        need = lib.nnlib_b200_attn_part_workspace_bytes(C.byref(p), units) if pr.Lq <= 128 else 0
+        ws = torch.empty(need, dtype=torch.uint8, device=pr.dev) if need else None
+        _check(lib.nnlib_b200_attn_part(C.byref(p), units, ws.data_ptr() if need else None, need, _stream()), "attn_part")
 
 
-def _fused_into(q, k, v, mask, nheads, x_out, lse_out, piece: bool = False):
+def _fused_into(q, k, v, mask, nheads, x_out, lse_out, units: int, piece: bool = False):
     """The fused call writing into caller-owned buffers (at most a split-key workspace is allocated): ``x_out`` is a
     column-major ``(Ev, Lq, B)`` array of the inputs' element type, ``lse_out`` a Float32 array of ``Lq*H*B``
-    elements.  ``piece``: see :func:`_launch_unit_exact`."""
+    elements.  ``units``, ``piece``: see :func:`_launch_part`."""
     pr = _Problem(q, k, v, None, mask, nheads, None, need_v=True)
     if tuple(x_out.shape) != (pr.Ev, pr.Lq, pr.B) or x_out.dtype != pr.dtype or not is_column_major(x_out):
         raise ArgumentError("x_out must be a dense column-major (Ev, Lq, B) array of the inputs' element type")
@@ -518,18 +513,19 @@ def _fused_into(q, k, v, mask, nheads, x_out, lse_out, piece: bool = False):
     pr.p.x = x_out.data_ptr()
     pr.lse = lse_out
     pr.p.lse = lse_out.data_ptr()
-    _launch_unit_exact(pr, piece)
+    _launch_part(pr, units, piece)
     return x_out
 
 
 def _fused_with_origin(q, k, v, bias, mask, nheads, dropout, rng_origin):
     """The fused call for a shard of a larger problem (see ``shard.py``):
     ``rng_origin`` places the shard's heads and batches in the whole problem so
-    that dropout draws the whole problem's mask.  Returns x only."""
+    that dropout draws the whole problem's mask; its ``units`` is the number of
+    units of that problem.  Returns x only."""
     pr = _Problem(q, k, v, bias, mask, nheads, dropout, need_v=True, rng_origin=rng_origin)
     x = pr.alloc_x()
     pr.alloc_lse()
-    _launch_unit_exact(pr)
+    _launch_part(pr, getattr(rng_origin, "units", pr.H * pr.B))
     return x
 
 

@@ -276,19 +276,14 @@ static size_t split_workspace(const AttnArgs& a, int dtype, SplitPath path) {
   }
 }
 
-size_t nnlib_b200_attn_decode_workspace_bytes(const nnlib_b200_attn_params* p) {
-  AttnArgs a;
-  if (resolve(p, NEED_QK | NEED_V, &a, false) != NNLIB_B200_OK) return 0;
-  if (a.Lq == 0 || a.B == 0) return 0;
-  return split_workspace(a, p->dtype, split_path(a, p->dtype));
+// the call's own way, or for a part of a call the way of the whole (nnlib_b200.h)
+static SplitPath part_path(const AttnArgs& a, int dtype) {
+  const SplitPath path = split_path(a, dtype);
+  return path == SPLIT_TILE ? SPLIT_NONE : path;
 }
 
-int nnlib_b200_attn_decode(const nnlib_b200_attn_params* p, void* workspace, size_t workspace_bytes, void* stream) {
-  AttnArgs a;
-  const int rc = resolve(p, NEED_QK | NEED_V, &a);
-  if (rc) return rc;
-  if (a.Lq == 0 || a.B == 0) return NNLIB_B200_OK;
-  const SplitPath path = split_path(a, p->dtype);
+static int run_split(const nnlib_b200_attn_params* p, AttnArgs& a, SplitPath path, void* workspace, size_t workspace_bytes,
+                     void* stream) {
   if (path == SPLIT_NONE) return nnlib_b200_attn_fwd(p, stream);
   const size_t need = split_workspace(a, p->dtype, path);
   if (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 15u) != 0)
@@ -305,6 +300,37 @@ int nnlib_b200_attn_decode(const nnlib_b200_attn_params* p, void* workspace, siz
   if (path == SPLIT_DECODE) return finish(decode_fwd(a, p->dtype, n, st));
   if (path == SPLIT_TILE) return finish(tile_split(a, p->dtype, st));
   return finish(fma_split(a, p->dtype, st));
+}
+
+size_t nnlib_b200_attn_decode_workspace_bytes(const nnlib_b200_attn_params* p) {
+  AttnArgs a;
+  if (resolve(p, NEED_QK | NEED_V, &a, false) != NNLIB_B200_OK || a.Lq == 0 || a.B == 0) return 0;
+  return split_workspace(a, p->dtype, split_path(a, p->dtype));
+}
+
+int nnlib_b200_attn_decode(const nnlib_b200_attn_params* p, void* workspace, size_t workspace_bytes, void* stream) {
+  AttnArgs a;
+  const int rc = resolve(p, NEED_QK | NEED_V, &a);
+  if (rc) return rc;
+  if (a.Lq == 0 || a.B == 0) return NNLIB_B200_OK;
+  return run_split(p, a, split_path(a, p->dtype), workspace, workspace_bytes, stream);
+}
+
+size_t nnlib_b200_attn_part_workspace_bytes(const nnlib_b200_attn_params* p, int64_t units) {
+  AttnArgs a;
+  if (resolve(p, NEED_QK | NEED_V, &a, false) != NNLIB_B200_OK || a.Lq == 0 || a.B == 0) return 0;
+  if (units < (int64_t)a.H * a.B) return 0;
+  return split_workspace(a, p->dtype, part_path(a, p->dtype));
+}
+
+int nnlib_b200_attn_part(const nnlib_b200_attn_params* p, int64_t units, void* workspace, size_t workspace_bytes,
+                         void* stream) {
+  AttnArgs a;
+  const int rc = resolve(p, NEED_QK | NEED_V, &a);
+  if (rc) return rc;
+  if (a.Lq == 0 || a.B == 0) return NNLIB_B200_OK;
+  if (units < (int64_t)a.H * a.B) return NNLIB_B200_INVALID_ARG;
+  return run_split(p, a, part_path(a, p->dtype), workspace, workspace_bytes, stream);
 }
 
 int nnlib_b200_attn_stats(const nnlib_b200_attn_params* p, void* stream) {

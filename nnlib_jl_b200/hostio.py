@@ -36,10 +36,13 @@ class HostPipelinedAttention:
     and of x, and needs nothing but its own rows of q beside the element's k and v): its kernels and copies
     back run while the rest of its q is still arriving, and only a ``tail_split``-th of a result follows the
     last input byte.
+
+    ``units``: the (head, batch) units of the call that these arrays are a part of (default: they are the whole).
     """
 
     def __init__(self, E: int, Ev: int, Lq: int, Lkv: int, B: int, dtype: torch.dtype, *, nheads: int,
-                 mask=None, chunk: int = 1, device=None, tail_split: int = 4):
+                 mask=None, chunk: int = 1, device=None, tail_split: int = 4,
+                 units: int | None = None):
         if mask is not None and not isinstance(mask, CausalMask):
             # a Bool array on the device that does not depend on the batch (what make_causal_mask returns, or
             # any (Lkv, Lq[, H]) mask): every chunk uses it as it is
@@ -52,6 +55,7 @@ class HostPipelinedAttention:
         self.dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
         self.E, self.Ev, self.Lq, self.Lkv, self.B = int(E), int(Ev), int(Lq), int(Lkv), int(B)
         self.dtype, self.nheads, self.mask = dtype, int(nheads), mask
+        self.units = self.nheads * self.B if units is None else int(units)
         self.chunk = min(int(chunk), self.B)
         self.tail_split = max(1, min(int(tail_split), self.Lq // 256)) if self.Lq >= 512 else 1
         c = self.chunk
@@ -117,7 +121,7 @@ class HostPipelinedAttention:
                 wf = w - 1 if tail else w                              # batch elements handled whole
                 if wf > 0:
                     qf, kf, vf, xf = (q, k, v, x) if wf == c else (q[:, :, :wf], k[:, :, :wf], v[:, :, :wf], x[:, :, :wf])
-                    _fused_into(qf, kf, vf, self.mask, self.nheads, xf, self.lse[s])
+                    _fused_into(qf, kf, vf, self.mask, self.nheads, xf, self.lse[s], self.units)
                     self.computed[s].record(comp)
                     self.out_stream.wait_event(self.computed[s])
                     with torch.cuda.stream(self.out_stream):
@@ -145,7 +149,8 @@ class HostPipelinedAttention:
                         else:
                             m = self.mask[:, l0:l1]
                         _fused_into(q[:, l0:l1, e:e + 1], k[:, :, e:e + 1], v[:, :, e:e + 1], m, self.nheads,
-                                    x[:, l0:l1, e:e + 1], self.lse[s][lse_off + l0 * self.nheads:], piece=True)
+                                    x[:, l0:l1, e:e + 1], self.lse[s][lse_off + l0 * self.nheads:], self.units,
+                                    piece=True)
                         self.piece_computed[pz].record(comp)
                         self.out_stream.wait_event(self.piece_computed[pz])
                         with torch.cuda.stream(self.out_stream):

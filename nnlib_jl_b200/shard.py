@@ -109,6 +109,16 @@ def _slice_bcast(t: Optional[torch.Tensor], rect: Rect, H: int, B: int):
     return t[tuple(idx)]
 
 
+class ShardOrigin(tuple):
+    """(first head, first batch element, heads of the whole call) of a shard; ``units``: the (head, batch) units of the
+    whole call, by which the library chooses how it is computed."""
+
+    def __new__(cls, h0: int, b0: int, H: int, B: int):
+        self = super().__new__(cls, (h0, b0, H))
+        self.units = H * B
+        return self
+
+
 def _cuda_compute(dev, q, k, v, bias, mask, nheads, dropout, rng_origin):
     """Default per-rectangle computation: the single-GPU library call."""
     from . import attention as A
@@ -142,7 +152,7 @@ class ShardedAttention:
         self.out_device = out_device
         self._pipes = {}      # per-device pipelines for shards whose arrays cross the bus (see _pipelined)
 
-    def _pipelined(self, slot, dev, rect, q, k, v, x, bias, mask, dropout, H) -> bool:
+    def _pipelined(self, slot, dev, rect, q, k, v, x, bias, mask, dropout, H, B) -> bool:
         """A rectangle of whole batch elements whose inputs and output sit in pinned host memory goes through
         a per-device :class:`HostPipelinedAttention` (one batch element at a time, so that the copy of the
         next element, the kernels of this one and the copy back of the previous one overlap).  Returns False
@@ -161,10 +171,10 @@ class ShardedAttention:
         E, Lq, _ = q.shape
         Ev, Lkv = v.shape[0], k.shape[1]
         # one pipeline per worker thread (`slot`): two shards may share a device, never staging buffers
-        key = (slot, str(dev), E, Ev, Lq, Lkv, rect.nb, q.dtype, H, repr(mask))
+        key = (slot, str(dev), E, Ev, Lq, Lkv, rect.nb, q.dtype, H, B, repr(mask))
         pipe = self._pipes.get(key)
         if pipe is None:
-            pipe = HostPipelinedAttention(E, Ev, Lq, Lkv, rect.nb, q.dtype, nheads=H, mask=mask, chunk=1, device=dev)
+            pipe = HostPipelinedAttention(E, Ev, Lq, Lkv, rect.nb, q.dtype, nheads=H, mask=mask, chunk=1, device=dev, units=H * B)
             self._pipes[key] = pipe
         bs = slice(rect.b0, rect.b0 + rect.nb)
         with torch.cuda.device(dev):
@@ -202,7 +212,7 @@ class ShardedAttention:
             try:
                 for rect in res.rects:
                     bs = slice(rect.b0, rect.b0 + rect.nb)
-                    if self._pipelined(results.index(res), res.device, rect, q, k, v, x, bias, mask, dropout, H):
+                    if self._pipelined(results.index(res), res.device, rect, q, k, v, x, bias, mask, dropout, H, B):
                         continue
                     qs = q[rect.h0 * d:(rect.h0 + rect.nh) * d, :, bs]
                     ks = k[rect.h0 * d:(rect.h0 + rect.nh) * d, :, bs]
@@ -220,7 +230,7 @@ class ShardedAttention:
                     if isinstance(mask_d, torch.Tensor):
                         mask_d = mask_d.to(dev, non_blocking=True)
                     drop = None if dropout is None else PhiloxDropout(dropout.p, dropout.seed, dropout.offset)
-                    y = self.compute(dev, *on_dev, bias_d, mask_d, rect.nh, drop, (rect.h0, rect.b0, H))
+                    y = self.compute(dev, *on_dev, bias_d, mask_d, rect.nh, drop, ShardOrigin(rect.h0, rect.b0, H, B))
                     x[rect.h0 * dv:(rect.h0 + rect.nh) * dv, :, bs].copy_(y, non_blocking=True)
                 if str(res.device).startswith("cuda"):
                     torch.cuda.synchronize(res.device)

@@ -221,6 +221,16 @@ def test_decode_entry_and_new_fields_without_a_gpu(lib):
     # more than one query tile never splits; neither does a short key sequence
     assert lib.nnlib_b200_attn_decode_workspace_bytes(C.byref(_params(Lq=129, Lkv=100000))) == 0
     assert lib.nnlib_b200_attn_decode_workspace_bytes(C.byref(_params(Lq=1, Lkv=128))) == 0
+    # a part of a call: never more units than the whole; what the whole splits by keys alone its parts split too
+    assert lib.nnlib_b200_attn_part(None, 1, None, 0, None) == _lib.INVALID_ARG
+    assert lib.nnlib_b200_attn_part(C.byref(_params(Lq=0)), 0, None, 0, None) == _lib.OK
+    assert lib.nnlib_b200_attn_part_workspace_bytes(None, 1) == 0
+    few = _params(Lq=1, Lkv=5000)
+    units = few.H * few.B
+    assert lib.nnlib_b200_attn_part_workspace_bytes(C.byref(few), units - 1) == 0
+    assert lib.nnlib_b200_attn_part_workspace_bytes(C.byref(few), units) == lib.nnlib_b200_attn_decode_workspace_bytes(C.byref(few)) > 0
+    masked = _params(Lq=1, Lkv=5000, mask=0x9000, mask_stride=(C.c_int64 * 4)(1, 0, 0, 0))   # split by the number of units
+    assert lib.nnlib_b200_attn_part_workspace_bytes(C.byref(masked), units) == 0
     # Float32 takes the tensor cores only when the caller allows TF32
     assert lib.nnlib_b200_attn_path(C.byref(_params(dtype=_lib.F32))) == _lib.PATH_SIMT
     assert lib.nnlib_b200_attn_path(C.byref(_params(dtype=_lib.F32, allow_tf32=1))) in (_lib.PATH_TILE, _lib.PATH_SIMT)

@@ -1876,3 +1876,24 @@ def test_float32_split_log_sum_exp_is_rounded_once():
     got, log_n = alpha._problem.lse.cpu().numpy().reshape(-1), np.log(Lkv)
     bound = 0.5 * np.spacing(np.abs(t) + np.float32(log_n)) + np.spacing(np.float32(log_n))
     assert (np.abs(got - (t.astype(np.float64) + log_n)) <= bound).all()
+
+
+@pytest.mark.parametrize("dtype,d,H,B,Lq,Lkv", [
+    (torch.bfloat16, 128, 4, 2, 1, 3000),
+    (torch.float16, 64, 3, 3, 12, 2500),
+    (torch.float32, 64, 4, 2, 5, 2100),
+])
+@pytest.mark.parametrize("pinned", [False, True])
+def test_shards_of_a_call_with_split_keys(dtype, d, H, B, Lq, Lkv, pinned):
+    """Shards (plain and, from pinned memory, pipelined) of a call whose keys are split give the bits of the call."""
+    from nnlib_jl_b200.shard import ShardedAttention
+    g = torch.Generator().manual_seed(Lkv)
+    q, k, v = (torch.randn(B, L, d * H, generator=g).to(dtype).permute(2, 1, 0) for L in (Lq, Lkv, Lkv))
+    mask = nb.CausalMask(Lkv - Lq)
+    x, a = nb.dot_product_attention(*(_dev(nb.jl_to_numpy(t), dtype) for t in (q, k, v)), mask=mask, nheads=H)
+    assert _lib.load().nnlib_b200_attn_decode_workspace_bytes(ctypes.byref(a._problem.p)) > 0   # keys are split
+    if pinned:
+        q, k, v = (t.permute(2, 1, 0).contiguous().pin_memory().permute(2, 1, 0) for t in (q, k, v))
+    for n in (1, 3):
+        y = ShardedAttention([f"cuda:{i % torch.cuda.device_count()}" for i in range(n)])(q, k, v, mask=mask, nheads=H)
+        assert torch.equal(y.to(DEV), x)
