@@ -259,11 +259,13 @@ int nnlib_b200_attn_fwd(const nnlib_b200_attn_params* p, void* stream) {
   return finish(!force_simt() && fma_supports(a.d, a.dv) ? fma_fwd(a, p->dtype, st) : simt_fwd(a, p->dtype, st));
 }
 
-// Which split-key forward takes the call: long key sequences whose units alone would not fill the GPU.
+// Which split-key forward takes a call of `units` units, of which `a` is the whole or a part: long key sequences whose
+// units alone would not fill the GPU.
 enum SplitPath { SPLIT_NONE, SPLIT_DECODE, SPLIT_TILE, SPLIT_FMA };
-static SplitPath split_path(const AttnArgs& a, int dtype) {
+static SplitPath split_path(const AttnArgs& a, int dtype, long long units) {
   if (a.Lq < 1 || a.Lq > 128 || a.B < 1 || a.Lkv < 1 || force_simt()) return SPLIT_NONE;
-  if (use_decode(a, dtype) && decode_split_count(a) > 1) return SPLIT_DECODE;
+  if (use_decode(a, dtype) && decode_split_count(a) > 1 && !(use_umma_fwd(a, dtype, true) && decode_leaves(a, units)))
+    return SPLIT_DECODE;
   if (tile_reject_reason(a, dtype, true, a.allow_tf32 != 0) == nullptr) return tile_split_count(a) > 1 ? SPLIT_TILE : SPLIT_NONE;
   return fma_split_count(a, dtype) > 1 ? SPLIT_FMA : SPLIT_NONE;
 }
@@ -277,8 +279,8 @@ static size_t split_workspace(const AttnArgs& a, int dtype, SplitPath path) {
 }
 
 // the call's own way, or for a part of a call the way of the whole (nnlib_b200.h)
-static SplitPath part_path(const AttnArgs& a, int dtype) {
-  const SplitPath path = split_path(a, dtype);
+static SplitPath part_path(const AttnArgs& a, int dtype, long long units) {
+  const SplitPath path = split_path(a, dtype, units);
   return path == SPLIT_TILE ? SPLIT_NONE : path;
 }
 
@@ -305,7 +307,7 @@ static int run_split(const nnlib_b200_attn_params* p, AttnArgs& a, SplitPath pat
 size_t nnlib_b200_attn_decode_workspace_bytes(const nnlib_b200_attn_params* p) {
   AttnArgs a;
   if (resolve(p, NEED_QK | NEED_V, &a, false) != NNLIB_B200_OK || a.Lq == 0 || a.B == 0) return 0;
-  return split_workspace(a, p->dtype, split_path(a, p->dtype));
+  return split_workspace(a, p->dtype, split_path(a, p->dtype, (long long)a.H * a.B));
 }
 
 int nnlib_b200_attn_decode(const nnlib_b200_attn_params* p, void* workspace, size_t workspace_bytes, void* stream) {
@@ -313,14 +315,14 @@ int nnlib_b200_attn_decode(const nnlib_b200_attn_params* p, void* workspace, siz
   const int rc = resolve(p, NEED_QK | NEED_V, &a);
   if (rc) return rc;
   if (a.Lq == 0 || a.B == 0) return NNLIB_B200_OK;
-  return run_split(p, a, split_path(a, p->dtype), workspace, workspace_bytes, stream);
+  return run_split(p, a, split_path(a, p->dtype, (long long)a.H * a.B), workspace, workspace_bytes, stream);
 }
 
 size_t nnlib_b200_attn_part_workspace_bytes(const nnlib_b200_attn_params* p, int64_t units) {
   AttnArgs a;
   if (resolve(p, NEED_QK | NEED_V, &a, false) != NNLIB_B200_OK || a.Lq == 0 || a.B == 0) return 0;
   if (units < (int64_t)a.H * a.B) return 0;
-  return split_workspace(a, p->dtype, part_path(a, p->dtype));
+  return split_workspace(a, p->dtype, part_path(a, p->dtype, units));
 }
 
 int nnlib_b200_attn_part(const nnlib_b200_attn_params* p, int64_t units, void* workspace, size_t workspace_bytes,
@@ -330,7 +332,7 @@ int nnlib_b200_attn_part(const nnlib_b200_attn_params* p, int64_t units, void* w
   if (rc) return rc;
   if (a.Lq == 0 || a.B == 0) return NNLIB_B200_OK;
   if (units < (int64_t)a.H * a.B) return NNLIB_B200_INVALID_ARG;
-  return run_split(p, a, part_path(a, p->dtype), workspace, workspace_bytes, stream);
+  return run_split(p, a, part_path(a, p->dtype, units), workspace, workspace_bytes, stream);
 }
 
 int nnlib_b200_attn_stats(const nnlib_b200_attn_params* p, void* stream) {

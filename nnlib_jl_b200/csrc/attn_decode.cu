@@ -346,6 +346,23 @@ int decode_split_count(const AttnArgs& a) {
   const int kend = dec_key_end(a), per = kend < 8192 ? 512 : 1024;
   return kend > (a.Lq <= 8 ? 1024 : 2048) ? (kend + per - 1) / per : 1;
 }
+// Is a call of `units` units better left to the two-tile forward, one CTA per unit?  With heads of more than 64 features
+// that kernel streams K and V about as fast once every SM has a CTA, so what decides is how full its last wave is:
+// units / (148 waves).  This kernel's side of the scale grows with the queries (their fragments, 8 and 16 of them a
+// step longer, and their partial outputs) and falls with the keys.  Times of this kernel over the other's, d = 128, 4096
+// keys, at 96 / 128 / 148 | 192 / 256 / 288 units (65, 86, 100 | 65, 86, 97 %): 1 query 0.82 1.04 1.09 | 0.78 0.94 1.04,
+// 4 queries 0.85 1.08 1.13 | 0.82 0.98 1.09, 8 queries 0.90 1.15 1.20 | 0.88 1.04 1.16, 16 queries 1.06 1.35 1.41 |
+// 1.05 1.23 1.36; at 16384 keys 0.76 0.92 1.03 | 0.74 0.92 0.99, ..., 0.91 1.08 1.19 | 0.88 1.09 1.15.  The percentages
+// below are where the ratio passes 1, in one wave | in more (101: nowhere); heads padded to 128 are 6 % better off here.
+bool decode_leaves(const AttnArgs& a, long long units) {
+  if (a.d <= 64 && a.dv <= 64) return false;
+  constexpr int kFull[2][4][2] = {{{80, 101}, {80, 97}, {75, 86}, {56, 64}},       // fewer than 8192 keys in reach
+                                  {{93, 101}, {93, 101}, {85, 95}, {75, 80}}};
+  const long long waves = (units + 147) / 148;
+  const int q = a.Lq <= 2 ? 0 : (a.Lq <= 4 ? 1 : (a.Lq <= 8 ? 2 : 3));
+  const int full = kFull[dec_key_end(a) < 8192 ? 0 : 1][q][waves > 1 ? 1 : 0] + (a.d < 128 ? 6 : 0);
+  return units * 100 >= full * waves * 148;
+}
 size_t decode_workspace_bytes(const AttnArgs& a) {
   const int n = decode_split_count(a);
   return n > 1 ? (size_t)split_ws_floats(a, n) * sizeof(float) : 0;   // 0: not split

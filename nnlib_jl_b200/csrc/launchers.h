@@ -58,6 +58,7 @@ cudaError_t tile_split(const AttnArgs& a, int dtype, cudaStream_t st);   // a.ws
 // at most 16 queries, 16-bit arrays, no side input: keys streamed through warp-level products (attn_decode.cu)
 bool decode_supports(const AttnArgs& a, int dtype);
 int decode_split_count(const AttnArgs& a);
+bool decode_leaves(const AttnArgs& a, long long units);  // better left to the two-tile forward, in a call of so many units
 size_t decode_workspace_bytes(const AttnArgs& a);        // 0: too few keys to split
 cudaError_t decode_fwd(const AttnArgs& a, int dtype, int n_splits, cudaStream_t st);   // a.ws holds the workspace
 

@@ -1878,20 +1878,22 @@ def test_float32_split_log_sum_exp_is_rounded_once():
     assert (np.abs(got - (t.astype(np.float64) + log_n)) <= bound).all()
 
 
-@pytest.mark.parametrize("dtype,d,H,B,Lq,Lkv", [
-    (torch.bfloat16, 128, 4, 2, 1, 3000),
-    (torch.float16, 64, 3, 3, 12, 2500),
-    (torch.float32, 64, 4, 2, 5, 2100),
+@pytest.mark.parametrize("dtype,d,H,B,Lq,Lkv,split", [
+    (torch.bfloat16, 128, 4, 2, 1, 3000, True),
+    (torch.float16, 64, 3, 3, 12, 2500, True),
+    (torch.float32, 64, 4, 2, 5, 2100, True),
+    (torch.bfloat16, 72, 32, 3, 16, 2100, False),    # 96 units are left to the two-tile kernel, 32 alone would not be
 ])
 @pytest.mark.parametrize("pinned", [False, True])
-def test_shards_of_a_call_with_split_keys(dtype, d, H, B, Lq, Lkv, pinned):
-    """Shards (plain and, from pinned memory, pipelined) of a call whose keys are split give the bits of the call."""
+def test_shards_of_a_call_with_split_keys(dtype, d, H, B, Lq, Lkv, split, pinned):
+    """Shards (plain and, from pinned memory, pipelined) of a call of few queries go the way of the whole call, keys
+    split or not, and give its bits."""
     from nnlib_jl_b200.shard import ShardedAttention
     g = torch.Generator().manual_seed(Lkv)
     q, k, v = (torch.randn(B, L, d * H, generator=g).to(dtype).permute(2, 1, 0) for L in (Lq, Lkv, Lkv))
     mask = nb.CausalMask(Lkv - Lq)
     x, a = nb.dot_product_attention(*(_dev(nb.jl_to_numpy(t), dtype) for t in (q, k, v)), mask=mask, nheads=H)
-    assert _lib.load().nnlib_b200_attn_decode_workspace_bytes(ctypes.byref(a._problem.p)) > 0   # keys are split
+    assert (_lib.load().nnlib_b200_attn_decode_workspace_bytes(ctypes.byref(a._problem.p)) > 0) == split
     if pinned:
         q, k, v = (t.permute(2, 1, 0).contiguous().pin_memory().permute(2, 1, 0) for t in (q, k, v))
     for n in (1, 3):
