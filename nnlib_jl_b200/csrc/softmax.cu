@@ -15,6 +15,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <type_traits>
 #include "common.cuh"
 #include "launchers.h"
 
@@ -390,68 +391,92 @@ __global__ void __launch_bounds__((G > 256 ? G : 256)) softmax_cols_kernel(typen
   }
 }
 
-// ---- reduction dimension strided (inner > 1): TI neighbours along i by NT / TI rows of the reduction -----------
+// ---- reduction dimension strided (inner > 1): TI columns by NT / TI rows of the reduction ----------------------
 // A block owns TI consecutive columns; each of its NT / TI rows of threads takes every (NT / TI)-th element of them,
-// eight loads in flight per thread, and the partial statistics are merged through shared memory.  (One thread per
-// column left a few hundred threads walking the whole reduction one load at a time: Float32 logsoftmax of a
-// (428, 8704) array over dims = 2, 15 MB, took 8.3 ms with its pullback and takes 56 us so; (46, 192, 260) 183 -> 29 us.)  The second pass over a column
-// re-reads it from L2; a thread writes only what it has read itself, so the in-place forms are safe.
-template <typename T, int MODE, int TI, int NT, bool NA>
+// eight loads in flight per thread, and the partial statistics are merged through shared memory; with one row (TI = NT)
+// a column is a thread's own, without a barrier.  FLAT: the columns (i, o) are numbered through, so that narrow slices
+// leave no lane idle; else a block keeps to one slice o, whose columns then start on a sector.  The second pass over a
+// column re-reads it from L2; a thread writes only what it has read itself, so the in-place forms are safe.
+template <typename T, int MODE, int TI, int NT, bool FLAT, bool NA>
 __global__ void __launch_bounds__(NT) softmax_strided_kernel(typename Ptrs<T, NA>::In x, typename Ptrs<T, NA>::In dy,
                                                              typename Ptrs<T, NA>::Out out, long long inner, long long n,
                                                              long long outer) {
-  constexpr int TJ = NT / TI, U = 8;
+  constexpr int TJ = NT / TI;
   constexpr bool FWD = (MODE == SM_FWD || MODE == LSM_FWD);
-  __shared__ ColStat sh_stat[FWD ? TJ : 1][TI];
-  __shared__ float sh_sum[FWD ? 1 : TJ][TI];
+  __shared__ ColStat sh_stat[FWD && TJ > 1 ? TJ : 1][TI];
+  __shared__ float sh_sum[!FWD && TJ > 1 ? TJ : 1][TI];
   const int ti = threadIdx.x % TI, tj = threadIdx.x / TI;
-  const long long itiles = (inner + TI - 1) / TI, tiles = itiles * outer;
+  const long long itiles = (inner + TI - 1) / TI, tiles = FLAT ? (inner * outer + TI - 1) / TI : itiles * outer;
   for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    const long long i = (tile % itiles) * TI + ti, base = i + inner * n * (tile / itiles);
-    const long long nj = i < inner ? n : 0;        // columns beyond the edge have nothing to do
+    long long i, o;
+    if (FLAT) {
+      const long long p = tile * TI + ti;
+      o = (p | inner) >> 32 ? p / inner : (long long)((unsigned)p / (unsigned)inner);
+      i = p - o * inner;
+    } else {
+      o = tile / itiles;
+      i = (tile - o * itiles) * TI + ti;
+    }
+    const long long base = i + inner * n * o;
+    const long long nj = (FLAT ? o < outer : i < inner) ? n : 0;        // columns beyond the edge have nothing to do
+    // f(number of elements, the first one's j) over the thread's elements: eight at a time, what is left of a column
+    // that is a thread's own in fours and twos
+    auto over = [&](auto f) {
+      long long j = tj;
+      for (; j + 7 * TJ < nj; j += 8 * TJ) f(std::integral_constant<int, 8>(), j);
+      if constexpr (TJ == 1) {
+        if (j + 3 < nj) {
+          f(std::integral_constant<int, 4>(), j);
+          j += 4;
+        }
+        if (j + 1 < nj) {
+          f(std::integral_constant<int, 2>(), j);
+          j += 2;
+        }
+      }
+      for (; j < nj; j += TJ) f(std::integral_constant<int, 1>(), j);
+    };
     if constexpr (FWD) {
       ColStat c = stat_init();
-      long long j = tj;
-      for (; j + (U - 1) * TJ < nj; j += U * TJ) {
+      over([&](auto cnt, long long j) {
+        constexpr int U = decltype(cnt)::value;
         float f[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) f[u] = Elem<T>::to_f(load_elem<T, NA>(x + base + (j + u * TJ) * inner));
         stat_add_pack<U>(c, f);
-      }
-      for (; j < nj; j += TJ) {
-        const float f[1] = {Elem<T>::to_f(load_elem<T, NA>(x + base + j * inner))};
-        stat_add_pack<1>(c, f);
-      }
-      sh_stat[tj][ti] = c;
-      __syncthreads();
-#pragma unroll
-      for (int s = TJ / 2; s > 0; s >>= 1) {
-        if (tj < s) sh_stat[tj][ti] = stat_merge(sh_stat[tj][ti], sh_stat[tj + s][ti]);
+      });
+      if (TJ > 1) {
+        sh_stat[tj][ti] = c;
         __syncthreads();
+#pragma unroll
+        for (int s = TJ / 2; s > 0; s >>= 1) {
+          if (tj < s) sh_stat[tj][ti] = stat_merge(sh_stat[tj][ti], sh_stat[tj + s][ti]);
+          __syncthreads();
+        }
+        c = sh_stat[0][ti];
       }
-      c = sh_stat[0][ti];
       stat_finish(c);
       const float inv_s = 1.f / c.s;
       const float log_s = (MODE == LSM_FWD) ? __logf(c.m == f_inf() ? (float)c.n_inf : c.s) : 0.f;
-      j = tj;
-      for (; j + (U - 1) * TJ < nj; j += U * TJ) {
+      over([&](auto cnt, long long j) {
+        constexpr int U = decltype(cnt)::value;
         float f[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) f[u] = Elem<T>::to_f(load_elem<T, NA>(x + base + (j + u * TJ) * inner));
-        fwd_pack<MODE, U>(c, inv_s, log_s, f);
+        if constexpr (TJ == 1) {   // (short sums: the division's one rounding counts)
+#pragma unroll
+          for (int u = 0; u < U; ++u) f[u] = fwd_value<MODE>(c, f[u], log_s);
+        } else {
+          fwd_pack<MODE, U>(c, inv_s, log_s, f);
+        }
 #pragma unroll
         for (int u = 0; u < U; ++u) out[base + (j + u * TJ) * inner] = Elem<T>::from_f(f[u]);
-      }
-      for (; j < nj; j += TJ) {
-        float f[1] = {Elem<T>::to_f(load_elem<T, NA>(x + base + j * inner))};
-        fwd_pack<MODE, 1>(c, inv_s, log_s, f);
-        out[base + j * inner] = Elem<T>::from_f(f[0]);
-      }
+      });
     } else {
       // sum of dy * y (softmax) or of dy (logsoftmax), then y * (dy - sum) or dy - exp(y) * sum
       float acc = 0.f;
-      long long j = tj;
-      for (; j + (U - 1) * TJ < nj; j += U * TJ) {
+      over([&](auto cnt, long long j) {
+        constexpr int U = decltype(cnt)::value;
         float d[U], y[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -459,22 +484,20 @@ __global__ void __launch_bounds__(NT) softmax_strided_kernel(typename Ptrs<T, NA
           y[u] = (MODE == SM_BWD) ? Elem<T>::to_f(load_elem<T, NA>(x + base + (j + u * TJ) * inner)) : 1.f;
         }
 #pragma unroll
-        for (int u = 0; u < U; ++u) acc += d[u] * y[u];
-      }
-      for (; j < nj; j += TJ) {
-        const float d = Elem<T>::to_f(load_elem<T, NA>(dy + base + j * inner));
-        acc += (MODE == SM_BWD) ? d * Elem<T>::to_f(load_elem<T, NA>(x + base + j * inner)) : d;
-      }
-      sh_sum[tj][ti] = acc;
-      __syncthreads();
-#pragma unroll
-      for (int s = TJ / 2; s > 0; s >>= 1) {
-        if (tj < s) sh_sum[tj][ti] += sh_sum[tj + s][ti];
+        for (int u = 0; u < U; ++u) acc = (MODE == SM_BWD) ? fmaf(d[u], y[u], acc) : acc + d[u];
+      });
+      if (TJ > 1) {
+        sh_sum[tj][ti] = acc;
         __syncthreads();
+#pragma unroll
+        for (int s = TJ / 2; s > 0; s >>= 1) {
+          if (tj < s) sh_sum[tj][ti] += sh_sum[tj + s][ti];
+          __syncthreads();
+        }
+        acc = sh_sum[0][ti];
       }
-      acc = sh_sum[0][ti];
-      j = tj;
-      for (; j + (U - 1) * TJ < nj; j += U * TJ) {
+      over([&](auto cnt, long long j) {
+        constexpr int U = decltype(cnt)::value;
         float d[U], y[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -485,14 +508,9 @@ __global__ void __launch_bounds__(NT) softmax_strided_kernel(typename Ptrs<T, NA
         for (int u = 0; u < U; ++u)
           out[base + (j + u * TJ) * inner] =
               Elem<T>::from_f((MODE == SM_BWD) ? y[u] * (d[u] - acc) : d[u] - __expf(y[u]) * acc);
-      }
-      for (; j < nj; j += TJ) {
-        const float d = Elem<T>::to_f(load_elem<T, NA>(dy + base + j * inner));
-        const float y = Elem<T>::to_f(load_elem<T, NA>(x + base + j * inner));
-        out[base + j * inner] = Elem<T>::from_f((MODE == SM_BWD) ? y * (d - acc) : d - __expf(y) * acc);
-      }
+      });
     }
-    __syncthreads();                               // the shared statistics are used again
+    if (TJ > 1) __syncthreads();                   // the shared statistics are used again
   }
 }
 
@@ -552,19 +570,30 @@ cudaError_t launch_softmax(const void* x, const void* dy, void* out, long long i
     }
 #undef NB_SM_LAUNCH
   } else {
-    // 32 columns a block while that gives every SM four blocks; else the columns of one 32-byte sector (narrower ones
-    // would fetch sectors twice), with 1024 threads when the reduction is long enough for that many rows
     constexpr int kW = 32 / (int)sizeof(T);
-    const long long cap = 148ll * 32, wide = (inner + 31) / 32 * outer, narrow = (inner + kW - 1) / kW * outer;
-#define NB_SM_STRIDED(TI, NT, TILES)                                                                               \
+    const long long cols = inner * outer;
+    auto tiles_of = [&](long long ti, bool flat) { return flat ? (cols + ti - 1) / ti : (inner + ti - 1) / ti * outer; };
+#define NB_SM_STRIDED(TI, NT, FLAT)                                                                                \
   do {                                                                                                             \
-    const unsigned blocks = (unsigned)((TILES) < cap ? (TILES) : cap);                                             \
-    if (no_alias) softmax_strided_kernel<T, MODE, TI, NT, true><<<blocks, NT, 0, st>>>(xp, dp, op, inner, n, outer);   \
-    else softmax_strided_kernel<T, MODE, TI, NT, false><<<blocks, NT, 0, st>>>(xp, dp, op, inner, n, outer);       \
+    const long long tiles = tiles_of(TI, FLAT), cap = 148ll * 32 * ((NT) < 256 ? 256 / (NT) : 1);                  \
+    const unsigned blocks = (unsigned)(tiles < cap ? tiles : cap);                                                 \
+    if (no_alias) softmax_strided_kernel<T, MODE, TI, NT, FLAT, true><<<blocks, NT, 0, st>>>(xp, dp, op, inner, n, outer);   \
+    else softmax_strided_kernel<T, MODE, TI, NT, FLAT, false><<<blocks, NT, 0, st>>>(xp, dp, op, inner, n, outer); \
   } while (0)
-    if (wide >= 4 * 148) NB_SM_STRIDED(32, 256, wide);
-    else if (n >= 1024) NB_SM_STRIDED(kW, 1024, narrow);
-    else NB_SM_STRIDED(kW, 256, narrow);
+    // The shorter the reduction and the more the columns, the fewer threads share one: a column is a thread's own up to 8
+    // elements, or up to 24 / 48 once the columns alone fill the GPU (30000 / 100000), else four or eight share it, or
+    // the 32 / 16 that are left beside the columns of one 32-byte sector (narrower blocks would fetch sectors twice).
+    // Float32, forward, against one thread a column walking it one load at a time and against eight rows of 32 columns of
+    // a slice for everything: (2, 4, 1M) 26 and 2633 -> 26 us, (8, 10, 2.5M) 598 and 8662 -> 494, (16, 64, 50000) 199 and
+    // 285 -> 110, (46, 192, 260) 98 and 13 -> 8, (428, 8704, 1) 4163 and 25 -> 25; over 2816 shapes within 10 % of the
+    // better of the two but for 25, and 20 % below it on average.
+    if (n <= 8 || (n <= 24 && cols >= 30000) || (n <= 48 && cols >= 100000)) NB_SM_STRIDED(128, 128, true);
+    else if (n < 24) NB_SM_STRIDED(32, 128, true);
+    else if (n >= 1024 && cols < 148ll * kW) NB_SM_STRIDED(kW, 1024, false);
+    else if (n >= 512 ? (inner < 32 || cols < 25000) : (cols < 5000 || (inner < 8 && n >= 48 && n * 400 >= cols)))
+      NB_SM_STRIDED(kW, 256, true);
+    else if (n >= 200 || (n >= 48 && cols < 25000)) NB_SM_STRIDED(32, 256, true);
+    else NB_SM_STRIDED(32, 128, true);
 #undef NB_SM_STRIDED
   }
   count_launch();

@@ -152,7 +152,14 @@ def test_random_shapes_and_dims_match_the_oracle(seed):
     (7, 65, 3),           # fewer columns than a sector
     (33, 300, 2),         # one column past a block of 32; eight loads in flight and a remainder
     (40, 1500, 1),        # long reduction: 1024 threads
-    (70, 63, 400),        # enough columns for blocks of 32
+    (70, 63, 400),        # enough columns for four threads each
+    (2, 4, 700),          # a column a thread: blocks run across the slices
+    (3, 23, 10001),       # 8 + 8 + 4 + 2 + 1 elements, the last block not whole
+    (5, 33, 23000),       # ... of more than 100000 columns
+    (9, 19, 300),         # four threads a column, across slices
+    (33, 130, 600),       # eight threads a column, across slices
+    (11, 515, 900),       # the columns of a sector, across slices
+    (3, 1025, 90),        # 1024 threads, a slice narrower than a sector
 ])
 @pytest.mark.parametrize("log", [False, True])
 def test_strided_reduction_blocks(dtype, inner, n, outer, log):
@@ -181,3 +188,29 @@ def test_strided_reduction_blocks(dtype, inner, n, outer, log):
     wantd = d64 - torch.exp(y64) * s if log else y64 * (d64 - s)
     size = d64.abs() + (torch.exp(y64) if log else y64) * (d64 if log else d64 * y64).abs().sum(1, keepdim=True) + y64.abs() * d64.abs()
     assert ((dx.double() - wantd).abs() <= 2 * rel * size + 1e-12)[ok].all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("inner,n,outer", [(2, 2, 1000000), (2, 4, 1000000), (5, 5, 300000), (8, 10, 500000)])
+def test_short_reductions_of_many_columns_run_at_the_speed_of_memory(dtype, inner, n, outer):
+    """A handful of elements per column, few columns per slice: within 12 times of a copy of the array, forward and
+    back (two to five times is usual; one block per slice took 50 to 140)."""
+    x = torch.randn(outer, n, inner, device="cuda:0").to(dtype).permute(2, 1, 0)
+    y = nb.softmax.softmax(x, dims=2)
+    other = torch.empty(outer, n, inner, device="cuda:0", dtype=dtype)
+
+    def once(f):
+        best = float("inf")
+        for _ in range(5):
+            e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            e0.record()
+            for _ in range(4):
+                f()
+            e1.record()
+            torch.cuda.synchronize()
+            best = min(best, e0.elapsed_time(e1) / 4)
+        return best
+
+    copy = once(lambda: other.copy_(x.permute(2, 1, 0))) + 0.02     # and 20 us for a call from Python
+    assert once(lambda: nb.softmax.softmax(x, dims=2)) < 12 * copy
+    assert once(lambda: nb.softmax.softmax_pullback(x, y, dims=2)) < 12 * copy
