@@ -118,7 +118,7 @@ __device__ __forceinline__ bool softmax_threads_sync_any(bool flag) {
 // XM = side + 3*drop as in the fused forward (attn_umma.cu): side 0 = no side input (optionally causal),
 // 1 = Bool mask array, 2 = bias (and mask); drop: dropout code compiled in.  The passes are bound by
 // instruction issue, so what a call does not use must not be in its loop.
-template <int D, bool BF16, int XM>
+template <int D, bool BF16, int XM, bool SHIFT>
 __global__ void __launch_bounds__(kShThreads, 1)
 attn_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_a, const AttnArgs a,
@@ -410,7 +410,7 @@ attn_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         uint32_t s0[32], s1[32];
         auto prepare = [&](int g, uint32_t (&s)[32], const uint4 (&bq)[4], const uint4 (&mq)[2]) {
           if (XBIAS) {
-            side_apply<true>(rs, s, bq, mq, g * 32, a.Lkv, lim, row_ok, c2);
+            side_apply<true, false, SHIFT>(rs, s, bq, mq, g * 32, a.Lkv, lim, row_ok, c2);
           } else {
             // keep bits of the chunk: the row's range (the causal diagonal, the end of the keys), and the mask array
             unsigned int kb;
@@ -433,15 +433,15 @@ attn_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           tmem_st32(lane_base + g * 32, s);
         };
         const int g_end = t_end * 4;
-        if (XBIAS) side_issue<true>(rs, t_first * kBN, a.Lkv, bq0, mq0);
+        if (XBIAS) side_issue<true, SHIFT>(rs, t_first * kBN, a.Lkv, bq0, mq0);
         tmem_ld32(lane_base + t_first * kBN, s0);
 #pragma unroll 1
         for (int g = t_first * 4; g < g_end; g += 2) {
-          if (XBIAS) side_issue<true>(rs, (g + 1) * 32, a.Lkv, bq1, mq1);
+          if (XBIAS) side_issue<true, SHIFT>(rs, (g + 1) * 32, a.Lkv, bq1, mq1);
           tmem_wait_ld();
           tmem_ld32(lane_base + (g + 1) * 32, s1);
           prepare(g, s0, bq0, mq0);
-          if (XBIAS && g + 2 < g_end) side_issue<true>(rs, (g + 2) * 32, a.Lkv, bq0, mq0);
+          if (XBIAS && g + 2 < g_end) side_issue<true, SHIFT>(rs, (g + 2) * 32, a.Lkv, bq0, mq0);
           tmem_wait_ld();
           if (g + 2 < g_end) tmem_ld32(lane_base + (g + 2) * 32, s0);
           prepare(g + 1, s1, bq1, mq1);
@@ -672,10 +672,10 @@ int sm_count() {
   return n;
 }
 
-template <int D, bool BF16, int XM>
-cudaError_t launch_short(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& ma,
+template <int D, bool BF16, int XM, bool SHIFT>
+cudaError_t launch_short_impl(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& ma,
                          const AttnArgs& a, cudaStream_t st) {
-  auto kern = attn_short_kernel<D, BF16, XM>;
+  auto kern = attn_short_kernel<D, BF16, XM, SHIFT>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ShCfg<D>::kSmemBytes);
   if (e != cudaSuccess) return e;
   const int n_qtiles = (a.Lq + kBM - 1) / kBM;
@@ -695,6 +695,15 @@ cudaError_t launch_short(const CUtensorMap& mq, const CUtensorMap& mk, const CUt
   kern<<<(unsigned)blocks, kShThreads, ShCfg<D>::kSmemBytes, st>>>(mq, mk, mv, ma, a, n_qtiles, (int)n_work);
   count_launch();
   return cudaGetLastError();
+}
+
+template <int D, bool BF16, int XM>
+cudaError_t launch_short(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& ma,
+                         const AttnArgs& a, cudaStream_t st) {
+  if constexpr ((XM % 3) == 2) {
+    if (side_rows_shift(a)) return launch_short_impl<D, BF16, XM, true>(mq, mk, mv, ma, a, st);
+  }
+  return launch_short_impl<D, BF16, XM, false>(mq, mk, mv, ma, a, st);
 }
 
 }  // namespace

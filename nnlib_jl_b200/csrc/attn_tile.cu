@@ -91,10 +91,11 @@ template <> struct Fmt<__half> { static constexpr uint32_t v = 0; };
 template <> struct Fmt<__nv_bfloat16> { static constexpr uint32_t v = 1; };
 template <> struct Fmt<float> { static constexpr uint32_t v = 2; };
 
-// SIDE: bias / Bool mask arrays are handled (through the per-row helpers of extras.cuh, chosen at run time);
+// SIDE: bias / Bool mask arrays are handled (through the per-row helpers of extras.cuh, chosen at run time; 2: with the
+// form for rows of any alignment);
 // without it the loop holds no trace of them — the generic helpers cost 1.6 k of a tile's 3.7 k cycles even
 // when a call has neither.
-template <typename T, int DQ, int DV, int MODE, bool SIDE>
+template <typename T, int DQ, int DV, int MODE, int SIDE>
 __global__ void __launch_bounds__(kTThreads, TCfg<T, DQ, DV>::kCtasPerSm)
 attn_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const AttnArgs a, const int n_qtiles, const int n_splits,
@@ -299,7 +300,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       // (one set of bias / mask words: the second chunk's are fetched once the first chunk's have been used, so
       // that the forward modes fit two CTAs on an SM)
       uint4 bq[4], mq[2];
-      if (SIDE) side_issue<true>(rs, j0, a.Lkv, bq, mq);
+      if (SIDE) side_issue<true, SIDE == 2>(rs, j0, a.Lkv, bq, mq);
       unsigned int kb[2] = {0xffffffffu, 0xffffffffu};
       if (MODE != TM_STATS && drop) {
 #pragma unroll
@@ -320,9 +321,9 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       }
       // scaled base-2 logits with bias, masks, causal limit and the end of the keys applied
       if (SIDE) {
-        side_apply<true>(rs, sr[0], bq, mq, j0, a.Lkv, lim, row_ok, c2);
-        side_issue<true>(rs, j0 + 32, a.Lkv, bq, mq);
-        side_apply<true>(rs, sr[1], bq, mq, j0 + 32, a.Lkv, lim, row_ok, c2);
+        side_apply<true, false, SIDE == 2>(rs, sr[0], bq, mq, j0, a.Lkv, lim, row_ok, c2);
+        side_issue<true, SIDE == 2>(rs, j0 + 32, a.Lkv, bq, mq);
+        side_apply<true, false, SIDE == 2>(rs, sr[1], bq, mq, j0 + 32, a.Lkv, lim, row_ok, c2);
       } else if (__any_sync(0xffffffffu, j0 + kTBN - 1 > lim || !row_ok)) {
         // the causal diagonal, the end of the keys or the end of the queries runs through this tile
 #pragma unroll
@@ -567,7 +568,7 @@ bool make_head_map(CUtensorMap* m, const void* base, int dtype, long long dhead,
 
 bool tile_stride_ok(long long s, int esz) { return s > 0 && (s * esz) % 16 == 0 && s * esz < (1ll << 40); }
 
-template <typename T, int DQ, int DV, int MODE, bool SIDE>
+template <typename T, int DQ, int DV, int MODE, int SIDE>
 cudaError_t launch_tile_side(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnArgs& a,
                              cudaStream_t st, int n_splits) {
   using C = TCfg<T, DQ, DV>;
@@ -603,8 +604,9 @@ cudaError_t launch_tile_side(const CUtensorMap& mq, const CUtensorMap& mk, const
 template <typename T, int DQ, int DV, int MODE>
 cudaError_t launch_tile(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnArgs& a,
                         cudaStream_t st, int n_splits = 1) {
-  if (a.bias != nullptr || a.mask != nullptr) return launch_tile_side<T, DQ, DV, MODE, true>(mq, mk, mv, a, st, n_splits);
-  return launch_tile_side<T, DQ, DV, MODE, false>(mq, mk, mv, a, st, n_splits);
+  if (side_rows_shift(a)) return launch_tile_side<T, DQ, DV, MODE, 2>(mq, mk, mv, a, st, n_splits);
+  if (a.bias != nullptr || a.mask != nullptr) return launch_tile_side<T, DQ, DV, MODE, 1>(mq, mk, mv, a, st, n_splits);
+  return launch_tile_side<T, DQ, DV, MODE, 0>(mq, mk, mv, a, st, n_splits);
 }
 
 template <typename T, int MODE>

@@ -655,7 +655,7 @@ __device__ __forceinline__ void store_score_chunk(T* dst, const uint32_t (&pk)[1
   }
 }
 
-template <int D, bool BF16, int XM, bool TST>
+template <int D, bool BF16, int XM, bool TST, bool SHIFT>
 __global__ void __launch_bounds__(kScThreads, 2)
 attn_scores_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                         const __grid_constant__ CUtensorMap tm_a, const AttnArgs a, const int n_qtiles) {
@@ -821,8 +821,8 @@ attn_scores_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         const int sb = j & 1;
         uint4 bq[2][4], mq[2][2];
         if (EXTRAS) {   // bias / mask of the first 64 keys: in flight while the scores are awaited
-          side_issue<XBIAS>(rs, j0, a.Lkv, bq[0], mq[0]);
-          side_issue<XBIAS>(rs, j0 + 32, a.Lkv, bq[1], mq[1]);
+          side_issue<XBIAS, SHIFT>(rs, j0, a.Lkv, bq[0], mq[0]);
+          side_issue<XBIAS, SHIFT>(rs, j0 + 32, a.Lkv, bq[1], mq[1]);
         }
         bool ok = mbar_wait(&bars->s_full[sb], (j >> 1) & 1, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
@@ -846,8 +846,8 @@ attn_scores_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
             if (lane == 0) mbar_arrive(&bars->s_empty[sb]);
           }
           if (EXTRAS) {
-            side_apply<XBIAS>(rs, sr[c & 1], bq[c & 1], mq[c & 1], jc, a.Lkv, lim, row_ok, c2);
-            if (c + 2 < 4) side_issue<XBIAS>(rs, j0 + (c + 2) * 32, a.Lkv, bq[c & 1], mq[c & 1]);
+            side_apply<XBIAS, false, SHIFT>(rs, sr[c & 1], bq[c & 1], mq[c & 1], jc, a.Lkv, lim, row_ok, c2);
+            if (c + 2 < 4) side_issue<XBIAS, SHIFT>(rs, j0 + (c + 2) * 32, a.Lkv, bq[c & 1], mq[c & 1]);
           }
           uint32_t pk[16];
 #pragma unroll
@@ -1095,35 +1095,24 @@ cudaError_t launch_fwd_impl(const CUtensorMap& mq, const CUtensorMap& mk, const 
   return cudaGetLastError();
 }
 
-// every row of the mask (of the bias) starts on a 16-byte boundary and holds whole chunks of 32 keys
-bool mask_rows_aligned(const AttnArgs& a) {
-  return !a.mask || (a.mask_s[0] == 1 && aligned16(a.mask) && a.mask_s[1] % 16 == 0 && a.mask_s[2] % 16 == 0 &&
-                     a.mask_s[3] % 16 == 0 && a.Lkv % 32 == 0);
-}
-bool bias_rows_aligned(const AttnArgs& a) {
-  return !a.bias || (a.bias_dtype != NNLIB_B200_F32 && a.bias_s[0] == 1 && aligned16(a.bias) && a.bias_s[1] % 8 == 0 &&
-                     a.bias_s[2] % 8 == 0 && a.bias_s[3] % 8 == 0 && a.Lkv % 32 == 0);
-}
-
 // `mb` != nullptr: the bias can be staged through shared memory by TMA (d = 64 forward with bias)
 template <int D, bool BF16, int XM, bool STATS>
 cudaError_t launch_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap* mb,
                        const AttnArgs& a, cudaStream_t st) {
-  if constexpr ((XM % 3) != 0 && !STATS) {
-    const bool mask_al = mask_rows_aligned(a);
-    if constexpr (D == 64 && (XM % 3) == 2) {
-      if (mb && mask_al) return launch_fwd_impl<D, BF16, XM, STATS, true, false>(mq, mk, mv, *mb, a, st);
-      if (mb) return launch_fwd_impl<D, BF16, XM, STATS, true, true>(mq, mk, mv, *mb, a, st);
-    }
-    if (mask_al && bias_rows_aligned(a)) return launch_fwd_impl<D, BF16, XM, STATS, false, false>(mq, mk, mv, mq, a, st);
+  if constexpr (D == 64 && (XM % 3) == 2 && !STATS) {
+    if (mb && mask_rows_shift(a)) return launch_fwd_impl<D, BF16, XM, STATS, true, true>(mq, mk, mv, *mb, a, st);
+    if (mb) return launch_fwd_impl<D, BF16, XM, STATS, true, false>(mq, mk, mv, *mb, a, st);
   }
-  return launch_fwd_impl<D, BF16, XM, STATS, false, true>(mq, mk, mv, mq, a, st);
+  if constexpr ((XM % 3) != 0) {
+    if (side_rows_shift(a)) return launch_fwd_impl<D, BF16, XM, STATS, false, true>(mq, mk, mv, mq, a, st);
+  }
+  return launch_fwd_impl<D, BF16, XM, STATS, false, false>(mq, mk, mv, mq, a, st);
 }
 
-template <int D, bool BF16, int XM, bool TST>
-cudaError_t launch_scores(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& ma, const AttnArgs& a,
+template <int D, bool BF16, int XM, bool TST, bool SHIFT>
+cudaError_t launch_scores_impl(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& ma, const AttnArgs& a,
                           cudaStream_t st) {
-  auto kern = attn_scores_umma_kernel<D, BF16, XM, TST>;
+  auto kern = attn_scores_umma_kernel<D, BF16, XM, TST, SHIFT>;
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ScCfg<D, TST>::kSmemBytes);
   if (e != cudaSuccess) return e;
@@ -1133,6 +1122,15 @@ cudaError_t launch_scores(const CUtensorMap& mq, const CUtensorMap& mk, const CU
   kern<<<(unsigned)blocks, kScThreads, ScCfg<D, TST>::kSmemBytes, st>>>(mq, mk, ma, a, n_qtiles);
   count_launch();
   return cudaGetLastError();
+}
+
+template <int D, bool BF16, int XM, bool TST>
+cudaError_t launch_scores(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& ma, const AttnArgs& a,
+                          cudaStream_t st) {
+  if constexpr (XM != 0) {
+    if (side_rows_shift(a)) return launch_scores_impl<D, BF16, XM, TST, true>(mq, mk, ma, a, st);
+  }
+  return launch_scores_impl<D, BF16, XM, TST, false>(mq, mk, ma, a, st);
 }
 
 // Tensor map over the bias array as (Lkv, Lq, H or 1, B or 1) with 64-key x 128-query boxes, for the

@@ -46,6 +46,21 @@ __device__ __forceinline__ RowSide make_row_side(const AttnArgs& a, int i, int h
   return rs;
 }
 
+// Host: does a call have bias or mask rows that the shifted form below is for, key stride 1 but not all of them aligned
+// and made of whole chunks of 32 keys?  The kernels are compiled with and without that form: the registers and
+// instructions it takes cost calls with aligned rows, and those whose rows it cannot serve, 5 - 20 %.
+inline bool mask_rows_shift(const AttnArgs& a) {
+  return a.mask && a.mask_s[0] == 1 &&
+         ((reinterpret_cast<unsigned long long>(a.mask) & 15ull) != 0 || a.mask_s[1] % 16 != 0 || a.mask_s[2] % 16 != 0 ||
+          a.mask_s[3] % 16 != 0 || a.Lkv % 32 != 0);
+}
+inline bool bias_rows_shift(const AttnArgs& a) {
+  return a.bias && a.bias_dtype != NNLIB_B200_F32 && a.bias_s[0] == 1 &&
+         ((reinterpret_cast<unsigned long long>(a.bias) & 15ull) != 0 || a.bias_s[1] % 8 != 0 || a.bias_s[2] % 8 != 0 ||
+          a.bias_s[3] % 8 != 0 || a.Lkv % 32 != 0);
+}
+inline bool side_rows_shift(const AttnArgs& a) { return mask_rows_shift(a) || bias_rows_shift(a); }
+
 // 4 N bytes from p, at any alignment, as words; bytes at and beyond `end` are whatever shares a word with a byte in
 // front of it, else 0.  Aligned words are read and shifted into place, all loads under way together (a word that
 // holds a byte of the array lies within the array's allocation, whose granularity is far coarser).
@@ -65,9 +80,9 @@ __device__ __forceinline__ void load_shifted(const unsigned char* p, const unsig
 // words.  (Rows of an odd number of keys are aligned once in eight; read one element after the other, as other strides
 // still are in groups of eight, they cost 32 load latencies per chunk: x and alpha of 5356 keys with bias and mask
 // took 10.1 ms, 4.1 so.)
-// SHIFT = false: a kernel compiled for calls whose rows are all aligned and whole (the host decides); it holds no trace
-// of the other form, which costs the aligned calls 5 - 10 %.
-template <bool WITH_BIAS, bool SHIFT = true>
+// SHIFT = false: no trace of the shifted form (see side_rows_shift); rows that are not aligned, and the last chunk, are
+// then read element by element.
+template <bool WITH_BIAS, bool SHIFT>
 __device__ __forceinline__ void side_issue(const RowSide& rs, int jj0, int Lkv, uint4 (&bq)[4], uint4 (&mq)[2]) {
   const bool inside = jj0 + 32 <= Lkv;
   if (WITH_BIAS && (SHIFT ? rs.bias_s1 : rs.bias_vec && inside)) {
@@ -136,7 +151,7 @@ __device__ __forceinline__ unsigned int mask_keep_bits_bytes(const RowSide& rs, 
 // masked, beyond `lim` (causal / end of the keys) or the row is out of range.  Works in place.
 // BIAS_STAGED: bq was filled from a shared-memory copy of the bias tile (zero beyond the array), so the
 // vector form applies to every chunk.
-template <bool WITH_BIAS, bool BIAS_STAGED = false, bool SHIFT = true>
+template <bool WITH_BIAS, bool BIAS_STAGED, bool SHIFT>
 __device__ __forceinline__ void side_apply(const RowSide& rs, unsigned int (&s)[32], const uint4 (&bq)[4],
                                            const uint4 (&mq)[2], int jj0, int Lkv, int lim, bool row_ok, float c2) {
   constexpr float kLog2eF = 1.4426950408889634f;
