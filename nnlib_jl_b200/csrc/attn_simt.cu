@@ -5,8 +5,9 @@
 // reference (NNlib.jl src/softmax.jl:69-79): pass A finds the row's
 // log-sum-exp, pass B forms alpha = exp(logit - lse), applies dropout and
 // accumulates x = sum_j alpha'_j v_j (src/attention.jl:96-98,117-126).
-// Shapes the tensor-core kernels do not take (f32 inputs, head sizes other
-// than 64/128, unaligned rows) run here.
+// What runs here: head sizes above 128 that no tensor-core kernel takes (the
+// tiled kernels of attn_fma.cu serve the others), and everything under
+// NNLIB_B200_FORCE_SIMT=1.
 #include "common.cuh"
 #include "launchers.h"
 

@@ -23,8 +23,8 @@
 //   TM_SCORES  alpha (after dropout) from a given log-sum-exp, written straight to the (Lkv, Lq, H, B) array
 //   TM_SPLIT   few queries (Lq <= 128: one query tile) against many keys: the key tiles of a unit are dealt to
 //              `n_splits` CTAs, each leaving its running maximum, its sum and its unnormalised O in a
-//              workspace; attn_split_reduce_kernel merges them into x and the log-sum-exp.  This is what
-//              keeps every SM busy when H*B is small (one new token against a long key / value history).
+//              workspace; attn_split_reduce_kernel merges them into x and the log-sum-exp.  For calls of few
+//              units that attn_decode.cu does not take (side inputs, TF32, 17 to 128 queries).
 #include <cuda.h>
 
 #include <algorithm>
