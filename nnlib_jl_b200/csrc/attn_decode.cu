@@ -337,11 +337,12 @@ bool decode_supports(const AttnArgs& a, int dtype) {
 
 // Shares the keys of one unit are cut into.  A function of the number of keys alone, so that a (head, batch) unit gives
 // the same bits in whatever company it is computed (a shard of a larger call, a batch of another size): 512 keys each,
-// 1024 from 8192 keys on, where the set-up and merge of a share show and units or shares enough remain for every SM
-// (one query, d = 128, 8192 keys, 256 units, bf16: 192 us = 5.6 TB/s, 202 with shares of 512, 228 with one share
-// per CTA and three CTAs on an SM, 221 - 235 with one 256-row tile per unit).  Up to 1024 keys (2048 for more than 8
-// queries, whose fragments take twice the registers) the call is left to the other kernels, whose one launch takes
-// less than two (384 keys, 256 units, d = 64: 23.5 us against 28.9; 16 queries, 1408 keys, 192 units: 45.1 against 47.1).
+// 1024 from 8192 keys on, where many units pay for the set-up and merge of a share (one query, d = 128, 256 units, bf16,
+// in a graph: 8191 keys 198 us, 8192 keys 187 us = 5.7 TB/s; the two-tile kernel 200 and 209).  Few units pay for the
+// longer shares instead (8 units, with a slower merge than now: 8191 keys 17.8 us, 8192 keys 20.5, both 34.6 with their
+// keys split by the number of units on the one-tile kernels).  Up to 1024 keys (2048 for more than 8 queries, whose
+// fragments take twice the registers) the call is left to the other kernels, whose one launch takes less than two (384
+// keys, 256 units, d = 64: 23.5 us against 28.9; 16 queries, 1408 keys, 192 units: 45.1 against 47.1).
 int decode_split_count(const AttnArgs& a) {
   const int kend = dec_key_end(a), per = kend < 8192 ? 512 : 1024;
   return kend > (a.Lq <= 8 ? 1024 : 2048) ? (kend + per - 1) / per : 1;

@@ -14,7 +14,7 @@
 //                each leaving its maximum, sum and O in a workspace (split_reduce.cuh merges them)
 // A warp per query that walked the keys one lane per key (attn_simt.cu, still there for larger heads) re-read every
 // key row through L1 for each query, uncoalesced: 441 us for x and alpha at d = 64, 8 heads, 128 x 128, batch 4,
-// where one pass of the row kernel takes 32 us including 25 us of host time between calls.
+// where a call of the row kernel takes 26 us, nearly all of it host time.
 //
 //   attn_fma_row_kernel  x, alpha and the log-sum-exp in one pass for short key sequences: the logits of a
 //                        block's queries stay in shared memory, so each is computed and exponentiated once
