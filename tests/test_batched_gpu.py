@@ -197,6 +197,10 @@ def test_random_products_match_the_oracle(seed):
     (33, 31, 17, 2),          # 32 x 32 tiles, one K element past a stage
     (65, 130, 16, 50),        # 64 x 64 tiles, exactly one stage
     (257, 127, 33, 60),       # 128 x 128 tiles, ragged in every dimension
+    (8, 8, 9, 300),           # one thread per element, however many products
+    (33, 8, 40, 3),           # ... 8 columns (A transposed: 32 x 32 tiles)
+    (9, 9, 5, 200),           # 32 x 32 tiles, mostly padding
+    (40, 60, 20, 200),        # 64 x 64 tiles where there are enough for 128 x 128 ones
 ])
 def test_float32_product_tiles(ta, tb, M, N, K, nbatch):
     rng = np.random.default_rng(M + N + K)
@@ -234,3 +238,24 @@ def test_products_the_copy_engine_cannot_address(dtype, ta, tb, M, N, K, nbatch)
     _close(got, BO.batched_gemm(ta, tb, np.float32(1), An, Bn, np.float32(0), zero), dtype, f"{ta}{tb}")
     nb.batched_mul_(C, opA, opB, 0.5, 2.0)
     _close(nb.jl_to_numpy(C), BO.batched_gemm(ta, tb, np.float32(0.5), An, Bn, np.float32(2), Cn), dtype, f"{ta}{tb} with an addend")
+
+
+def test_tiny_products_in_large_numbers():
+    """A product of 8 x 8 matrices is not worth a 128 x 128 tile, however many there are: within 12 times of a copy of
+    the arrays (twice is usual, 40 times with such tiles)."""
+    A, B = (torch.randn(10000, 8, 8, device="cuda:0").permute(2, 1, 0) for _ in range(2))
+    src, dst = torch.empty(3 * 640000, device="cuda:0"), torch.empty(3 * 640000, device="cuda:0")
+
+    def once(f):
+        best = float("inf")
+        for _ in range(5):
+            e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            e0.record()
+            for _ in range(20):
+                f()
+            e1.record()
+            torch.cuda.synchronize()
+            best = min(best, e0.elapsed_time(e1) / 20)
+        return best
+
+    assert once(lambda: nb.batched_mul(A, B)) < 12 * once(lambda: dst.copy_(src)) + 0.05    # and 50 us for a call
