@@ -1745,22 +1745,38 @@ def test_float32_masked_keys_may_hold_anything():
         np.testing.assert_array_equal(got, want)
 
 
-@pytest.mark.parametrize("dtype,d,dv,H,B,Lq,Lkv,off", [
-    (torch.bfloat16, 128, 128, 2, 1, 1, 1, 0),          # one key
-    (torch.bfloat16, 64, 64, 3, 2, 8, 17, 9),           # one key past a step of 16; all 8 rows of the small form
-    (torch.float16, 128, 128, 4, 120, 9, 130, 121),     # 9 queries: the 16-row form; one CTA per unit
-    (torch.bfloat16, 80, 40, 2, 3, 16, 999, 983),       # heads narrower than the padded sizes, dv != d
-    (torch.float16, 8, 128, 2, 1, 1, 5000, 4999),       # split, d = 8
-    (torch.bfloat16, 128, 64, 1, 1, 16, 4097, 4000),    # split, the last keys out of every query's reach
-    (torch.bfloat16, 64, 64, 2, 2, 5, 700, -2),         # the first two queries see no key
-    (torch.float16, 64, 64, 2, 2, 7, 300, None),        # no mask
-    (torch.float32, 64, 64, 2, 1, 1, 3000, 2999),       # exact Float32, keys split over blocks of 8 queries
-    (torch.float32, 128, 96, 1, 2, 40, 1500, 1460),     # ... and of 32
-    (torch.float32, 32, 32, 2, 1, 4, 2000, -1),         # ... the first query sees no key
-    (torch.bfloat16, 128, 40, 1, 1, 2, 40000, 39998),   # 40 shares: more than the lanes of the warp that merges them
-    (torch.float32, 64, 64, 1, 1, 1, 8300, 8299),       # 33 shares
+def _key_shares(pr):
+    """Shares the library cuts the keys of a unit into for this call (0: not split), from the workspace it asks for:
+    a maximum, a sum (rounded up to 4 floats in all) and dv partial outputs per share and query."""
+    p = pr.p
+    need = _lib.load().nnlib_b200_attn_decode_workspace_bytes(ctypes.byref(p)) // 4
+    rows = p.H * p.B * p.Lq
+    n = round(need / (rows * (p.dv + 2)))
+    assert need == (((rows * n * 2 + 3) & ~3) + rows * n * p.dv if n else 0)
+    return n
+
+
+@pytest.mark.parametrize("dtype,d,dv,H,B,Lq,Lkv,off,shares", [
+    # streamed keys: shares of 512, 1024 from 8192 keys on, above 1024 keys (2048 for more than 8 queries)
+    (torch.bfloat16, 64, 64, 3, 2, 8, 1041, 1033, 3),        # one key past a step of 16; all 8 rows of the small form
+    (torch.float16, 128, 128, 4, 3, 9, 2050, 2041, 5),       # 9 queries: the 16-row form
+    (torch.bfloat16, 64, 64, 2, 2, 16, 2049, 2033, 5),       # ... with 64 features, all 16 rows
+    (torch.bfloat16, 80, 40, 2, 3, 16, 2999, 2983, 6),       # heads narrower than the padded sizes, dv != d
+    (torch.float16, 8, 128, 2, 1, 1, 5000, 4999, 10),        # d = 8
+    (torch.bfloat16, 128, 64, 1, 1, 16, 4097, 4000, 8),      # the last keys out of every query's reach
+    (torch.float16, 64, 64, 2, 2, 7, 1300, None, 3),         # no mask
+    (torch.bfloat16, 128, 40, 1, 1, 2, 40000, 39998, 40),    # more shares than the lanes of the warp that merges them
+    # exact Float32: shares of 256 above 1024 keys
+    (torch.float32, 64, 64, 2, 1, 1, 3000, 2999, 12),        # blocks of 8 queries
+    (torch.float32, 128, 96, 1, 2, 30, 1500, 1470, 6),       # ... and of 32
+    (torch.float32, 64, 64, 1, 1, 1, 8300, 8299, 33),
+    # not split: few keys, more queries, hardly a key in reach
+    (torch.bfloat16, 128, 128, 2, 1, 1, 1, 0, 0),
+    (torch.bfloat16, 64, 64, 2, 2, 5, 700, -2, 0),           # the first two queries see no key
+    (torch.float32, 128, 96, 1, 2, 40, 1500, 1460, 0),
+    (torch.float32, 32, 32, 2, 1, 4, 2000, -1, 0),           # the first query sees no key
 ])
-def test_decode_steps_match_the_oracle(dtype, d, dv, H, B, Lq, Lkv, off):
+def test_decode_steps_match_the_oracle(dtype, d, dv, H, B, Lq, Lkv, off, shares):
     """A handful of queries against a key / value history: x and (through the lazy alpha) the log-sum-exp."""
     rng = np.random.default_rng(500 + Lq + Lkv)
     qn = _round_to(rng.standard_normal((d * H, Lq, B)), dtype)
@@ -1769,6 +1785,7 @@ def test_decode_steps_match_the_oracle(dtype, d, dv, H, B, Lq, Lkv, off):
     mask = None if off is None else _offset_mask(Lkv, Lq, off)
     y, a = nb.dot_product_attention(_dev(qn, dtype), _dev(kn, dtype), _dev(vn, dtype),
                                     mask=None if off is None else nb.CausalMask(off), nheads=H)
+    assert _key_shares(a._problem) == shares
     with np.errstate(invalid="ignore"):
         yo, ao = O.dot_product_attention(qn, kn, vn, mask=mask, nheads=H)
     live = np.ones(Lq, bool) if mask is None else mask.any(axis=0)
@@ -1899,3 +1916,34 @@ def test_shards_of_a_call_with_split_keys(dtype, d, H, B, Lq, Lkv, split, pinned
     for n in (1, 3):
         y = ShardedAttention([f"cuda:{i % torch.cuda.device_count()}" for i in range(n)])(q, k, v, mask=mask, nheads=H)
         assert torch.equal(y.to(DEV), x)
+
+
+@pytest.mark.parametrize("d,H,B", [(128, 16, 32), (64, 32, 32)])
+def test_decode_of_many_units_gives_each_the_bits_it_has_alone(d, H, B):
+    """So many (unit, share) pairs that a CTA takes two shares of a unit in turn, the last one ragged: every unit has
+    the bits of a call of one batch element, where a CTA takes one."""
+    g = torch.Generator(device=DEV).manual_seed(d)
+    Lkv = 2900                                               # six shares; 512 (1024) units of them
+    q, k, v = (torch.randn(B, L, d * H, generator=g, device=DEV).to(torch.bfloat16).permute(2, 1, 0) for L in (1, Lkv, Lkv))
+    x, a = nb.dot_product_attention(q, k, v, mask=nb.CausalMask(Lkv - 1), nheads=H)
+    assert _key_shares(a._problem) == 6
+    for b in (0, B // 2, B - 1):
+        one, _ = nb.dot_product_attention(*(t[:, :, b:b + 1] for t in (q, k, v)), mask=nb.CausalMask(Lkv - 1), nheads=H)
+        assert torch.equal(one[:, :, 0], x[:, :, b])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_decode_with_nan_logits(dtype):
+    """A NaN among the keys: NaN for the queries that attend to it, nothing for those before it and the other heads."""
+    rng = np.random.default_rng(3)
+    d, H, Lq, Lkv = 64, 2, 4, 1300
+    qn, kn, vn = (_round_to(rng.standard_normal((d * H, L, 1)), dtype) for L in (Lq, Lkv, Lkv))
+    kn[5, -2, 0] = np.nan                                    # the last key but one, head 0
+    mask = nb.CausalMask(Lkv - Lq)
+    y, a = nb.dot_product_attention(_dev(qn, dtype), _dev(kn, dtype), _dev(vn, dtype), mask=mask, nheads=H)
+    assert _key_shares(a._problem) > 1
+    yn = nb.jl_to_numpy(y)
+    assert np.isnan(yn[:d, 2:]).all()
+    yo, _ = O.dot_product_attention(qn, np.nan_to_num(kn), vn, mask=_offset_mask(Lkv, Lq, Lkv - Lq), nheads=H)
+    _close(yn[:d, :2], yo[:d, :2], dtype, "x before the NaN")
+    _close(yn[d:], yo[d:], dtype, "x of the other head")
