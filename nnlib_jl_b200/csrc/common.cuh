@@ -69,7 +69,6 @@ struct GemmArgs {
   int a_bcast, b_bcast;                  // 1: one matrix for every batch
   float alpha, beta;
   int c_vec;                             // 16-byte stores into C are possible
-  int c_tma;                             // C is written through TMA stores
   int tiles_m, tiles_n;
   long long tiles;
   int* status;

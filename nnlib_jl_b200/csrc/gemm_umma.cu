@@ -46,15 +46,13 @@ constexpr int kGemmThreads = 320;
 constexpr int kBK = 64;                  // K elements per stage: one 128-byte swizzle row
 constexpr int kHalfBytes = 128 * 128;    // 128 rows x 64 K elements, either layout
 
-template <int NH, int MT>
+template <int NH, int MT, int OUT>
 struct GCfg {
   static constexpr int kNBytes = NH * kHalfBytes;
   static constexpr int kMBytes = (MT / 128) * kHalfBytes;
   static constexpr int kStage = kNBytes + kMBytes;
-  // epilogue staging: per warp one (NH = 2, whose ring needs the room) or two boxes of 32 columns x 128 bytes
-  static constexpr int kOutBufs = (NH == 2) ? 1 : 2;
-  static constexpr int kOutBytes = 8 * kOutBufs * 4096;
-  static constexpr int kStages = (226 * 1024 - kOutBytes) / kStage;   // 3 (64 KB), 3 (48 KB), 5 (32 KB)
+  static constexpr int kOutBytes = 8 * OUT * 4096;               // epilogue staging: OUT boxes of 32 columns x 128 bytes a warp
+  static constexpr int kStages = (226 * 1024 - kOutBytes) / kStage;   // OUT = 0: 3 (64 KB), 4 (48 KB), 7 (32 KB); 2: 3 and 5
   static constexpr int kAccCols = NH * MT;                       // fp32 columns of one tile
   static constexpr int kAccBufs = (kAccCols <= 256) ? 2 : 1;
   static constexpr int kTmemCols = (kAccCols * kAccBufs <= 256) ? 256 : 512;
@@ -62,9 +60,10 @@ struct GCfg {
   static constexpr int kBarOff = kOutOff + kOutBytes;
   static constexpr int kSmemBytes = kBarOff + 256 + 1024;
 };
-static_assert(GCfg<2, 256>::kStages == 3 && GCfg<1, 256>::kStages == 3 && GCfg<1, 128>::kStages == 5, "ring depth");
-static_assert(GCfg<2, 256>::kSmemBytes <= 232448 && GCfg<1, 256>::kSmemBytes <= 232448 && GCfg<1, 128>::kSmemBytes <= 232448,
-              "shared memory budget");
+static_assert(GCfg<2, 256, 0>::kStages == 3 && GCfg<2, 256, 1>::kStages == 3 && GCfg<1, 256, 0>::kStages == 4, "ring depth");
+static_assert(GCfg<1, 256, 2>::kStages == 3 && GCfg<1, 128, 2>::kStages == 5 && GCfg<1, 128, 0>::kStages == 7, "ring depth");
+static_assert(GCfg<2, 256, 1>::kSmemBytes <= 232448 && GCfg<1, 256, 0>::kSmemBytes <= 232448 && GCfg<1, 128, 0>::kSmemBytes <= 232448 &&
+              GCfg<1, 256, 2>::kSmemBytes <= 232448 && GCfg<1, 128, 2>::kSmemBytes <= 232448, "shared memory budget");
 
 struct GBarriers {
   uint64_t full[8], empty[8];
@@ -74,11 +73,11 @@ struct GBarriers {
 };
 static_assert(sizeof(GBarriers) <= 256, "barrier block");
 
-template <bool BF16, int NH, int MT, bool N_KMAJ, bool M_KMAJ>
+template <bool BF16, int NH, int MT, bool N_KMAJ, bool M_KMAJ, int OUT>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_umma_kernel(const __grid_constant__ CUtensorMap tm_n, const __grid_constant__ CUtensorMap tm_m,
                  const __grid_constant__ CUtensorMap tm_c, const GemmArgs g) {
-  using C = GCfg<NH, MT>;
+  using C = GCfg<NH, MT, OUT>;
   using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -202,7 +201,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tm_n, const __grid_constant
     constexpr int kCols = (NH == 2) ? MT : MT / 2;
     const int col0 = (NH == 2) ? 0 : part * kCols;
     const float alpha = g.alpha, beta = g.beta;
-    uint8_t* out = smem + C::kOutOff + (warp - 2) * (C::kOutBufs * 4096);
+    uint8_t* out = smem + C::kOutOff + (warp - 2) * (OUT * 4096);
     int n_out = 0;                           // boxes this warp has sent
     bool ok = true;
     int ti = 0;
@@ -216,7 +215,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tm_n, const __grid_constant
       tc_fence_after();
       const int n = n0 + half * 128 + wq * 32 + lane;
       const uint32_t taddr = tmem + (static_cast<uint32_t>(wq * 32) << 16) + ab * C::kAccCols + half * MT + col0;
-      if (g.c_tma) {
+      if constexpr (OUT > 0) {
 #pragma unroll 1
         for (int c = 0; c < kCols / 64; ++c, ++n_out) {
           uint32_t acc[2][32];
@@ -228,8 +227,8 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tm_n, const __grid_constant
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars->acc_empty[ab]);
           }
-          uint8_t* box = out + (n_out % C::kOutBufs) * 4096;
-          if (lane == 0 && n_out >= C::kOutBufs) tma_store_wait_read<C::kOutBufs - 1>();   // its last store has left
+          uint8_t* box = out + (n_out % OUT) * 4096;
+          if (lane == 0 && n_out >= OUT) tma_store_wait_read<OUT - 1>();   // its last store has left
           __syncwarp();
 #pragma unroll
           for (int p = 0; p < 8; ++p) {
@@ -249,56 +248,56 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tm_n, const __grid_constant
             tma_store_commit();
           }
         }
-        continue;
-      }
-      T* ccol = reinterpret_cast<T*>(g.C) + (long long)b * g.strideC + (long long)n * g.ldc;
+      } else {
+        T* ccol = reinterpret_cast<T*>(g.C) + (long long)b * g.strideC + (long long)n * g.ldc;
 #pragma unroll 1
-      for (int c = 0; c < kCols / 32; ++c) {
-        uint32_t acc[32];
-        tmem_ld32(taddr + c * 32, acc);
-        tmem_wait_ld();
-        if (c == kCols / 32 - 1) {
-          // this warp has read its share of the accumulator: the issuer may start the tile after next
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bars->acc_empty[ab]);
-        }
-        const int m = m0 + col0 + c * 32;
-        if (n < g.N && m < g.M) {
-          T* dst = ccol + m;
-          if (g.c_vec && m + 32 <= g.M) {
+        for (int c = 0; c < kCols / 32; ++c) {
+          uint32_t acc[32];
+          tmem_ld32(taddr + c * 32, acc);
+          tmem_wait_ld();
+          if (c == kCols / 32 - 1) {
+            // this warp has read its share of the accumulator: the issuer may start the tile after next
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->acc_empty[ab]);
+          }
+          const int m = m0 + col0 + c * 32;
+          if (n < g.N && m < g.M) {
+            T* dst = ccol + m;
+            if (g.c_vec && m + 32 <= g.M) {
 #pragma unroll
-            for (int e = 0; e < 32; e += 8) {
-              float f[8];
+              for (int e = 0; e < 32; e += 8) {
+                float f[8];
 #pragma unroll
-              for (int u = 0; u < 8; ++u) f[u] = alpha * __uint_as_float(acc[e + u]);
-              if (beta != 0.f) {
-                const uint4 old = *reinterpret_cast<const uint4*>(dst + e);
-                const T* o = reinterpret_cast<const T*>(&old);
+                for (int u = 0; u < 8; ++u) f[u] = alpha * __uint_as_float(acc[e + u]);
+                if (beta != 0.f) {
+                  const uint4 old = *reinterpret_cast<const uint4*>(dst + e);
+                  const T* o = reinterpret_cast<const T*>(&old);
 #pragma unroll
-                for (int u = 0; u < 8; ++u) f[u] = fmaf(beta, Elem<T>::to_f(o[u]), f[u]);
+                  for (int u = 0; u < 8; ++u) f[u] = fmaf(beta, Elem<T>::to_f(o[u]), f[u]);
+                }
+                uint4 v;
+                v.x = pack2<BF16>(f[0], f[1]);
+                v.y = pack2<BF16>(f[2], f[3]);
+                v.z = pack2<BF16>(f[4], f[5]);
+                v.w = pack2<BF16>(f[6], f[7]);
+                *reinterpret_cast<uint4*>(dst + e) = v;
               }
-              uint4 v;
-              v.x = pack2<BF16>(f[0], f[1]);
-              v.y = pack2<BF16>(f[2], f[3]);
-              v.z = pack2<BF16>(f[4], f[5]);
-              v.w = pack2<BF16>(f[6], f[7]);
-              *reinterpret_cast<uint4*>(dst + e) = v;
-            }
-          } else {
+            } else {
 #pragma unroll
-            for (int e = 0; e < 32; ++e) {
-              if (m + e < g.M) {
-                float f = alpha * __uint_as_float(acc[e]);
-                if (beta != 0.f) f = fmaf(beta, Elem<T>::to_f(dst[e]), f);
-                dst[e] = Elem<T>::from_f(f);
+              for (int e = 0; e < 32; ++e) {
+                if (m + e < g.M) {
+                  float f = alpha * __uint_as_float(acc[e]);
+                  if (beta != 0.f) f = fmaf(beta, Elem<T>::to_f(dst[e]), f);
+                  dst[e] = Elem<T>::from_f(f);
+                }
               }
             }
           }
         }
       }
     }
-    if (lane == 0) tma_store_wait_read<0>();   // shared memory stays until the last box has been read
+    if (OUT > 0 && lane == 0) tma_store_wait_read<0>();   // shared memory stays until the last box has been read
   }
 
   // ---------------------------------------------------------------- teardown
@@ -353,10 +352,10 @@ int sm_count() {
   return n;
 }
 
-template <bool BF16, int NH, int MT, bool N_KMAJ, bool M_KMAJ>
-cudaError_t launch_gemm(const CUtensorMap& mn, const CUtensorMap& mm, const CUtensorMap& mc, GemmArgs g, cudaStream_t st) {
-  using C = GCfg<NH, MT>;
-  auto kern = gemm_umma_kernel<BF16, NH, MT, N_KMAJ, M_KMAJ>;
+template <bool BF16, int NH, int MT, bool N_KMAJ, bool M_KMAJ, int OUT>
+cudaError_t launch_gemm_out(const CUtensorMap& mn, const CUtensorMap& mm, const CUtensorMap& mc, GemmArgs g, cudaStream_t st) {
+  using C = GCfg<NH, MT, OUT>;
+  auto kern = gemm_umma_kernel<BF16, NH, MT, N_KMAJ, M_KMAJ, OUT>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) return e;
   g.tiles_m = (g.M + MT - 1) / MT;
@@ -366,6 +365,21 @@ cudaError_t launch_gemm(const CUtensorMap& mn, const CUtensorMap& mm, const CUte
   kern<<<(unsigned)grid, kGemmThreads, C::kSmemBytes, st>>>(mn, mm, mc, g);
   count_launch();
   return cudaGetLastError();
+}
+
+template <bool BF16, int NH, int MT, bool N_KMAJ, bool M_KMAJ>
+cudaError_t launch_gemm(const CUtensorMap& mn, const CUtensorMap& mm, const CUtensorMap& mc, const GemmArgs& g, bool out_map,
+                        cudaStream_t st) {
+  // Staging pays where the product is little more than writing C.  A longer K keeps the narrow tiles' whole ring (direct
+  // stores: 4096 x 64 x 4096, batch 4: 31 us, 37 with the stage that two staging boxes cost), and so does beta != 0,
+  // which reads C (2048 x 2048 x 64, batch 64: 342 and 370); the 256 x 256 tile has the room either way.
+  const int out = !out_map ? 0 : (NH == 2 ? 1 : (g.K < 512 ? 2 : 0));
+  if constexpr (NH == 1) {
+    if (out == 2) return launch_gemm_out<BF16, NH, MT, N_KMAJ, M_KMAJ, 2>(mn, mm, mc, g, st);
+  } else {
+    if (out == 1) return launch_gemm_out<BF16, NH, MT, N_KMAJ, M_KMAJ, 1>(mn, mm, mc, g, st);
+  }
+  return launch_gemm_out<BF16, NH, MT, N_KMAJ, M_KMAJ, 0>(mn, mm, mc, g, st);
 }
 
 }  // namespace
@@ -397,7 +411,7 @@ cudaError_t gemm_umma(const GemmArgs& g0, int dtype, cudaStream_t st) {
   g.c_vec = (aligned16(g.C) && g.ldc % 8 == 0 && (g.batch == 1 || g.strideC % 8 == 0)) ? 1 : 0;
   // (a tensor map addresses strides below 2^40 bytes and extents below 2^32; the direct stores know no such limit)
   CUtensorMap mc = mn;
-  g.c_tma = (g.c_vec && g.beta == 0.f && make_out_map(&mc, g, dtype)) ? 1 : 0;
+  const bool out_map = g.c_vec && g.beta == 0.f && make_out_map(&mc, g, dtype);
   const bool bf16 = dtype == NNLIB_B200_BF16;
   // tile: 256 x 256 for large products, 128 n-rows for narrow ones, 128 m-columns for short ones
   // (a short K leaves the 256 x 256 tile, whose accumulator fills all of tensor memory, with nothing to overlap
@@ -407,11 +421,11 @@ cudaError_t gemm_umma(const GemmArgs& g0, int dtype, cudaStream_t st) {
 #define NB_G4(BF, NHH, MTT)                                                               \
   do {                                                                                    \
     if (n_kmaj) {                                                                         \
-      if (m_kmaj) return launch_gemm<BF, NHH, MTT, true, true>(mn, mm, mc, g, st);            \
-      return launch_gemm<BF, NHH, MTT, true, false>(mn, mm, mc, g, st);                       \
+      if (m_kmaj) return launch_gemm<BF, NHH, MTT, true, true>(mn, mm, mc, g, out_map, st);            \
+      return launch_gemm<BF, NHH, MTT, true, false>(mn, mm, mc, g, out_map, st);                       \
     }                                                                                     \
-    if (m_kmaj) return launch_gemm<BF, NHH, MTT, false, true>(mn, mm, mc, g, st);             \
-    return launch_gemm<BF, NHH, MTT, false, false>(mn, mm, mc, g, st);                        \
+    if (m_kmaj) return launch_gemm<BF, NHH, MTT, false, true>(mn, mm, mc, g, out_map, st);             \
+    return launch_gemm<BF, NHH, MTT, false, false>(mn, mm, mc, g, out_map, st);                        \
   } while (0)
 #define NB_G3(BF)                                            \
   do {                                                       \
