@@ -534,14 +534,15 @@ int nnlib_b200_batched_gemm(const nnlib_b200_gemm_params* p, void* stream) {
     if (check_all_pointers() && !on_current_device(g.B, dev)) return NNLIB_B200_INVALID_ARG;
   }
   const char* why = force_simt() ? "NNLIB_B200_FORCE_SIMT is set" : gemm_umma_reject_reason(g, p->dtype);
+  const bool mma = why && !force_simt() && gemm_mma_supports(g, p->dtype);
   if (log_calls()) {
     static const char* const names[] = {"f16", "bf16", "f32"};
     std::fprintf(stderr, "[nnlib_b200] batched_gemm %s %c%c M=%d N=%d K=%d batch=%d alpha=%g beta=%g -> %s%s%s\n",
                  names[p->dtype], g.transA ? 'T' : 'N', g.transB ? 'T' : 'N', g.M, g.N, g.K, g.batch, (double)g.alpha,
-                 (double)g.beta, why ? "cuda-core" : "tcgen05", why ? ": " : "", why ? why : "");
+                 (double)g.beta, !why ? "tcgen05" : (mma ? "warp-level products" : "cuda-core"), why ? ": " : "", why ? why : "");
   }
   if (!why) return finish(gemm_umma(g, p->dtype, (cudaStream_t)stream));
-  if (!force_simt() && gemm_mma_supports(g, p->dtype)) return finish(gemm_mma(g, p->dtype, (cudaStream_t)stream));
+  if (mma) return finish(gemm_mma(g, p->dtype, (cudaStream_t)stream));
   return finish(gemm_simt(g, p->dtype, (cudaStream_t)stream));
 }
 

@@ -259,3 +259,14 @@ def test_tiny_products_in_large_numbers():
         return best
 
     assert once(lambda: nb.batched_mul(A, B)) < 12 * once(lambda: dst.copy_(src)) + 0.05    # and 50 us for a call
+
+
+def test_log_names_the_kernel_of_a_product():
+    import os, subprocess, sys
+    code = ("import torch, nnlib_jl_b200 as nb\n"
+            "for m, dt in ((64, torch.float16), (33, torch.float16), (33, torch.float32)):\n"
+            "    a = torch.zeros(1, 64, m, device='cuda', dtype=dt).permute(2, 1, 0)\n"
+            "    nb.batched_mul(a, torch.zeros(1, 64, 64, device='cuda', dtype=dt).permute(2, 1, 0))\n")
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, NNLIB_B200_LOG="1"), capture_output=True, text=True)
+    lines = [l.split("->")[1].split(":")[0].strip() for l in r.stderr.splitlines() if "batched_gemm" in l]
+    assert lines == ["tcgen05", "warp-level products", "cuda-core"], r.stderr
