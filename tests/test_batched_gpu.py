@@ -261,6 +261,16 @@ def test_tiny_products_in_large_numbers():
     assert once(lambda: nb.batched_mul(A, B)) < 12 * once(lambda: dst.copy_(src)) + 0.05    # and 50 us for a call
 
 
+def test_long_sums_of_products_the_copy_engine_cannot_address():
+    """16385 positive terms: nearly every element is the exact sum rounded to f16.  A Float32 sum of them is off by some
+    sqrt(K) 2^-24 = 8e-6, against 5e-4 - 1e-3 between neighbouring f16 numbers."""
+    g = torch.Generator(device="cuda:0").manual_seed(5)
+    A, B = (torch.rand(1, n, m, generator=g, device="cuda:0").half().permute(2, 1, 0) for m, n in ((65, 16385), (16385, 65)))
+    C = nb.batched_mul(A, B)
+    want = torch.einsum("mkb,knb->mnb", A.double(), B.double()).half()
+    assert (C == want).double().mean() > 0.95
+
+
 def test_log_names_the_kernel_of_a_product():
     import os, subprocess, sys
     code = ("import torch, nnlib_jl_b200 as nb\n"
