@@ -164,6 +164,7 @@ cudaError_t launch_gemm_fma(const GemmArgs& g, cudaStream_t st) {
 
 cudaError_t gemm_simt(const GemmArgs& g, int dtype, cudaStream_t st) {
   if (g.M < 1 || g.N < 1 || g.batch < 1) return cudaSuccess;
+  // (the grid of gemm_element_kernel; the tiles' grids hold more)
   if ((g.N + 7LL) / 8 > 65535 || g.batch > 65535) return cudaErrorInvalidConfiguration;
   switch (dtype) {
     case NNLIB_B200_F16:  return launch_gemm_fma<__half>(g, st);

@@ -168,9 +168,10 @@ cudaError_t launch_gemm_mma(const GemmArgs& g, cudaStream_t st) {
 // 16-bit products worth a 128 x 128 tile; thinner ones are left to the CUDA-core tiles, and so are sums of more than 4096
 // terms: the products' accumulation does not round each step to nearest, which adds up (error against Float64, f16,
 // all terms positive: as with one fused multiply-add after the other up to K = 1000, + 0.7 % at 4095, + 11 % at 16385).
+// The columns are limited as for every product off the tcgen05 path (gemm_fma.cu).
 bool gemm_mma_supports(const GemmArgs& g, int dtype) {
   return (dtype == NNLIB_B200_F16 || dtype == NNLIB_B200_BF16) && g.M >= 32 && g.N >= 32 && g.K >= 16 && g.K <= 4096 &&
-         g.batch >= 1 && g.batch <= 65535 && (reinterpret_cast<uintptr_t>(g.A) & 1u) == 0 &&
+         (g.N + 7LL) / 8 <= 65535 && g.batch >= 1 && g.batch <= 65535 && (reinterpret_cast<uintptr_t>(g.A) & 1u) == 0 &&
          (reinterpret_cast<uintptr_t>(g.B) & 1u) == 0;
 }
 cudaError_t gemm_mma(const GemmArgs& g, int dtype, cudaStream_t st) {

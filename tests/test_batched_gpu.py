@@ -271,6 +271,14 @@ def test_long_sums_of_products_the_copy_engine_cannot_address():
     assert (C == want).double().mean() > 0.95
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_more_columns_than_the_grids_hold_are_refused(dtype):
+    A = torch.zeros(1, 17, 33, device="cuda:0", dtype=dtype).permute(2, 1, 0)
+    B = torch.zeros(1, 8 * 65535 + 1, 17, device="cuda:0", dtype=dtype).permute(2, 1, 0)
+    with pytest.raises(_lib.NNlibB200Error):
+        nb.batched_mul(A, B)
+
+
 def test_log_names_the_kernel_of_a_product():
     import os, subprocess, sys
     code = ("import torch, nnlib_jl_b200 as nb\n"
