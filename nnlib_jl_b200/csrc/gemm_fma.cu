@@ -148,10 +148,10 @@ cudaError_t launch_gemm_fma(const GemmArgs& g, cudaStream_t st) {
   auto tiles = [&](long long t) { return ((g.M + t - 1) / t) * ((g.N + t - 1) / t) * g.batch; };
   auto grid = [&](long long t) { return dim3((unsigned)((g.M + t - 1) / t), (unsigned)((g.N + t - 1) / t), (unsigned)g.batch); };
   // The largest tile that is not mostly padding and still gives every SM a block.  Results of at most 8 columns take one
-  // thread per element where the lanes of a warp read A along its columns (4096 x 8 x 512, batch 4: 27 us against 45 of
-  // 64-square tiles), tiny ones always (8 x 8 x 8, batch 10000: 14 us against 205 of the 128-square tiles that their
-  // number alone had chosen).
-  if (g.N <= 8 && (!g.transA || g.M <= 8))
+  // thread per element where the lanes of a warp read A along its columns and the sum is not long (4096 x 8 x 512, batch
+  // 4: 28 us against 45 of 64-square tiles; 4096 x 1 x 4096: 193 against 130 of 32-square ones), tiny ones always (8 x 8 x
+  // 8, batch 10000: 14 us against 205 of the 128-square tiles that their number alone had chosen).
+  if (g.N <= 8 && (g.M <= 8 || (!g.transA && g.K <= 1024)))
     gemm_element_kernel<T><<<dim3((unsigned)((g.M + 31) / 32), (unsigned)((g.N + 7) / 8), (unsigned)g.batch), 256, 0, st>>>(g);
   else if (g.M > 64 && g.N > 64 && tiles(128) >= 148) gemm_fma_kernel<T, 128><<<grid(128), 256, 0, st>>>(g);
   else if (g.M > 32 && g.N > 32 && tiles(64) >= 148) gemm_fma_kernel<T, 64><<<grid(64), 256, 0, st>>>(g);
