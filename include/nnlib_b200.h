@@ -271,6 +271,17 @@ typedef struct nnlib_b200_attn_grads {
 NNLIB_B200_API int nnlib_b200_attn_bwd(const nnlib_b200_attn_params* p, const nnlib_b200_attn_grads* g,
                                        void* stream);
 
+/* The same pullback in one pass over the scores instead of two (five products per block of scores instead of
+   seven), for the calls that run on the tensor cores: dq is gathered in Float32 in the caller's workspace by atomic
+   additions, whose order is not fixed, so that dq may differ in its last bit from one call to the next
+   (nnlib_b200_attn_bwd gives the same bits each time).  workspace: device memory, 16-byte aligned, at least
+   nnlib_b200_attn_bwd_workspace_bytes(p, g) bytes, which need not be cleared and is free again when the call's
+   kernels have run.  A result of 0 bytes: no workspace is used and the call is nnlib_b200_attn_bwd.  g->delta is
+   not used where a workspace is. */
+NNLIB_B200_API size_t nnlib_b200_attn_bwd_workspace_bytes(const nnlib_b200_attn_params* p, const nnlib_b200_attn_grads* g);
+NNLIB_B200_API int nnlib_b200_attn_bwd_ws(const nnlib_b200_attn_params* p, const nnlib_b200_attn_grads* g,
+                                          void* workspace, size_t workspace_bytes, void* stream);
+
 /* NNLIB_B200_PATH_* that attn_bwd would take for (p, g), or a negative error.  The tensor-core
    backward covers 16-bit element types with d = dv any multiple of 8 up to 128 and every option of the forward
    (causal flag, Bool mask arrays, dropout, bias with dbias); Float32 arrays and other head sizes

@@ -408,6 +408,7 @@ Base.@kwdef struct B200AttnGrads
     dbias_stride::NTuple{4,Int64} = (0, 0, 0, 0)
     delta::CuPtr{Float32} = CU_NULL
 end
+_with(g::B200AttnGrads; kw...) = B200AttnGrads(; (f => getfield(g, f) for f in fieldnames(B200AttnGrads))..., kw...)
 
 function ChainRulesCore.rrule(::typeof(dot_product_attention), q::DenseCuArray{T,3}, k::DenseCuArray{T,3},
                               v::DenseCuArray{T,3}, bias=nothing; fdrop=identity, mask=nothing,
@@ -419,16 +420,24 @@ function ChainRulesCore.rrule(::typeof(dot_product_attention), q::DenseCuArray{T
     function attention_pullback(Δ)
         dx = convert(CuArray{T,3}, unthunk(Δ[1]))   # the cotangent of α is not supported (α is lazy)
         dq, dk, dv = similar(q), similar(k), similar(v)
-        delta = CuArray{Float32}(undef, p.Lq * p.H * p.B)
         dbias32 = bias === nothing ? nothing : CUDA.zeros(Float32, size(bias))
         g = B200AttnGrads(; struct_size=sizeof(B200AttnGrads), dx=reinterpret(CuPtr{Cvoid}, pointer(dx)),
             dq=reinterpret(CuPtr{Cvoid}, pointer(dq)), dk=reinterpret(CuPtr{Cvoid}, pointer(dk)),
-            dv=reinterpret(CuPtr{Cvoid}, pointer(dv)), delta=pointer(delta),
+            dv=reinterpret(CuPtr{Cvoid}, pointer(dv)),
             dbias=dbias32 === nothing ? CuPtr{Float32}(0) : pointer(dbias32),
             dbias_stride=dbias32 === nothing ? (0, 0, 0, 0) : _bcast_strides("bias", dbias32, (p.Lkv, p.Lq, p.H, p.B)))
-        GC.@preserve q k v x α dx dq dk dv delta dbias32 bias mask begin
-            rc = ccall((:nnlib_b200_attn_bwd, libnnlib_b200[]), Cint,
-                       (Ref{B200AttnParams}, Ref{B200AttnGrads}, Ptr{Cvoid}), p, g, stream().handle)
+        # one pass over the scores where the library asks for a workspace (dq is then summed by atomic additions)
+        need = ccall((:nnlib_b200_attn_bwd_workspace_bytes, libnnlib_b200[]), Csize_t,
+                     (Ref{B200AttnParams}, Ref{B200AttnGrads}), p, g)
+        scratch = CuArray{Float32}(undef, need > 0 ? cld(Int(need), 4) : p.Lq * p.H * p.B)
+        g = _with(g; delta=pointer(scratch))
+        GC.@preserve q k v x α dx dq dk dv scratch dbias32 bias mask begin
+            rc = need > 0 ?
+                ccall((:nnlib_b200_attn_bwd_ws, libnnlib_b200[]), Cint,
+                      (Ref{B200AttnParams}, Ref{B200AttnGrads}, CuPtr{Cvoid}, Csize_t, Ptr{Cvoid}),
+                      p, g, reinterpret(CuPtr{Cvoid}, pointer(scratch)), need, stream().handle) :
+                ccall((:nnlib_b200_attn_bwd, libnnlib_b200[]), Cint,
+                      (Ref{B200AttnParams}, Ref{B200AttnGrads}, Ptr{Cvoid}), p, g, stream().handle)
             _b200_check(rc, "attn_bwd")
         end
         dbias = bias === nothing ? NoTangent() : convert(typeof(bias), dbias32)

@@ -46,6 +46,8 @@ EXPORTS = (
     "nnlib_b200_static_scratch",
     "nnlib_b200_attn_bwd",
     "nnlib_b200_attn_bwd_path",
+    "nnlib_b200_attn_bwd_ws",
+    "nnlib_b200_attn_bwd_workspace_bytes",
     "nnlib_b200_batched_gemm",
     "nnlib_b200_batched_gemm_path",
     "nnlib_b200_causal_fill",
@@ -190,6 +192,10 @@ def load() -> C.CDLL:
     lib.nnlib_b200_selftest_wait_runout.restype = C.c_int
     lib.nnlib_b200_attn_bwd.argtypes = [P, C.POINTER(AttnGrads), C.c_void_p]
     lib.nnlib_b200_attn_bwd.restype = C.c_int
+    lib.nnlib_b200_attn_bwd_ws.argtypes = [P, C.POINTER(AttnGrads), C.c_void_p, C.c_size_t, C.c_void_p]
+    lib.nnlib_b200_attn_bwd_ws.restype = C.c_int
+    lib.nnlib_b200_attn_bwd_workspace_bytes.argtypes = [P, C.POINTER(AttnGrads)]
+    lib.nnlib_b200_attn_bwd_workspace_bytes.restype = C.c_size_t
     lib.nnlib_b200_attn_bwd_path.argtypes = [P, C.POINTER(AttnGrads)]
     lib.nnlib_b200_attn_bwd_path.restype = C.c_int
     lib.nnlib_b200_workspace_bytes.argtypes = [P]

@@ -560,18 +560,24 @@ def dot_product_attention_pullback(q, k, v, bias=None, *, fdrop: Callable = iden
         dq = jl_empty(q.shape, q.dtype, pr.dev)
         dk = jl_empty(k.shape, k.dtype, pr.dev)
         dv = jl_empty(v.shape, v.dtype, pr.dev)
-        delta = torch.empty(pr.Lq * pr.H * pr.B, dtype=torch.float32, device=pr.dev)
         g = _lib.AttnGrads()
-        g.dx, g.dq, g.dk, g.dv, g.delta = dx.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), delta.data_ptr()
+        g.dx, g.dq, g.dk, g.dv = dx.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
         dbias32 = None
         if bias is not None:
             dbias32 = torch.zeros(tuple(bias.shape)[::-1], dtype=torch.float32, device=pr.dev)
             dbias32 = dbias32.permute(*range(bias.ndim - 1, -1, -1)) if bias.ndim else dbias32
             g.dbias = dbias32.data_ptr()
             g.dbias_stride = (C.c_int64 * 4)(*_bcast_strides("bias", dbias32, (pr.Lkv, pr.Lq, pr.H, pr.B)))
+        # the one-pass backward sums dq by atomic additions: a program that asks torch for deterministic algorithms
+        # gets the one that needs no workspace and adds in a fixed order
+        need = 0 if torch.are_deterministic_algorithms_enabled() else \
+            lib.nnlib_b200_attn_bwd_workspace_bytes(C.byref(pr.p), C.byref(g))
+        scratch = torch.empty(need or 4 * pr.Lq * pr.H * pr.B, dtype=torch.uint8, device=pr.dev)
+        g.delta = scratch.data_ptr()
         back.path = lib.nnlib_b200_attn_bwd_path(C.byref(pr.p), C.byref(g))   # PATH_UMMA / PATH_SIMT, for tests
         with torch.cuda.device(pr.dev):
-            _check(lib.nnlib_b200_attn_bwd(C.byref(pr.p), C.byref(g), _stream()), "attn_bwd")
+            _check(lib.nnlib_b200_attn_bwd_ws(C.byref(pr.p), C.byref(g), scratch.data_ptr(), need, _stream()) if need else
+                   lib.nnlib_b200_attn_bwd(C.byref(pr.p), C.byref(g), _stream()), "attn_bwd")
         return dq, dk, dv, (None if dbias32 is None else dbias32.to(bias.dtype))
 
     return x, alpha, back

@@ -392,12 +392,12 @@ int nnlib_b200_attn_apply(const nnlib_b200_attn_params* p, void* stream) {
 
 // shared front half of attn_bwd / attn_bwd_path: validates and resolves both argument blocks
 static int resolve_bwd(const nnlib_b200_attn_params* p, const nnlib_b200_attn_grads* g, AttnArgs* a, BwdArgs* b,
-                       bool launching = true) {
+                       bool launching = true, bool need_delta = true) {
   const int rc = resolve(p, NEED_QK | NEED_V | NEED_LSE_IN, a, false);   // the device check comes last
   if (rc) return rc;
   if (!g || g->struct_size != sizeof(nnlib_b200_attn_grads)) return NNLIB_B200_INVALID_ARG;
   const bool empty = (a->Lq == 0 || a->B == 0);
-  if (!empty && (!g->dx || !g->dq || !g->delta)) return NNLIB_B200_INVALID_ARG;
+  if (!empty && (!g->dx || !g->dq || (need_delta && !g->delta))) return NNLIB_B200_INVALID_ARG;
   // dk and dv are written (zeros) even when there are no queries, as long as there are keys
   if (a->B > 0 && a->Lkv > 0 && (!g->dk || !g->dv)) return NNLIB_B200_INVALID_ARG;
   std::memset(b, 0, sizeof(*b));
@@ -432,6 +432,39 @@ int nnlib_b200_attn_bwd(const nnlib_b200_attn_params* p, const nnlib_b200_attn_g
                                                        : "16-bit arrays with d = dv a multiple of 8 up to 128 and 16-byte aligned rows only");
   return finish(!force_simt() && fma_supports(a.d, a.dv) ? fma_bwd(a, b, p->dtype, (cudaStream_t)stream)
                                                          : simt_bwd(a, b, p->dtype, (cudaStream_t)stream));
+}
+
+// The one-pass backward: what the tensor-core backward takes, given a workspace, but for a handful of key tiles (a CTA
+// each) with long walks over the queries, which the dq half spreads over the GPU: 128 keys and 4096 queries of 4 units
+// 61 us in two halves, 71 in one pass; of 32 units 101 and 88; 300 keys and 8000 queries of 4 units 129 and 137;
+// 1024 keys and queries of 4 units 45 and 39.  Its arguments are those of the two halves but for delta, which it does
+// not use.
+static bool use_bwd_fused(const AttnArgs& a, BwdArgs b, int dtype) {
+  if (!b.delta) b.delta = a.lse;
+  if (a.Lq < 1 || a.B < 1 || force_simt() || !umma_bwd_supports(a, b, dtype)) return false;
+  const long long key_tiles = (a.Lkv + 127ll) / 128, query_tiles = (a.Lq + 127ll) / 128;
+  return key_tiles * a.H * a.B >= 16 || query_tiles <= 2 * key_tiles;
+}
+
+size_t nnlib_b200_attn_bwd_workspace_bytes(const nnlib_b200_attn_params* p, const nnlib_b200_attn_grads* g) {
+  AttnArgs a;
+  BwdArgs b;
+  if (resolve_bwd(p, g, &a, &b, false, false) != NNLIB_B200_OK || !use_bwd_fused(a, b, p->dtype)) return 0;
+  return umma_bwd_fused_workspace_bytes(a);
+}
+
+int nnlib_b200_attn_bwd_ws(const nnlib_b200_attn_params* p, const nnlib_b200_attn_grads* g, void* workspace,
+                           size_t workspace_bytes, void* stream) {
+  AttnArgs a;
+  BwdArgs b;
+  const int rc = resolve_bwd(p, g, &a, &b, true, false);
+  if (rc) return rc;
+  if (!use_bwd_fused(a, b, p->dtype)) return nnlib_b200_attn_bwd(p, g, stream);
+  if (!workspace || workspace_bytes < umma_bwd_fused_workspace_bytes(a) || (reinterpret_cast<uintptr_t>(workspace) & 15u) != 0)
+    return NNLIB_B200_WORKSPACE_TOO_SMALL;
+  a.ws = static_cast<float*>(workspace);
+  log_call("attn_bwd", p, a, "tcgen05 (one pass)", nullptr);
+  return finish(umma_bwd_fused(a, b, p->dtype, (cudaStream_t)stream));
 }
 
 int nnlib_b200_attn_bwd_path(const nnlib_b200_attn_params* p, const nnlib_b200_attn_grads* g) {
@@ -574,15 +607,16 @@ int nnlib_b200_attn_path(const nnlib_b200_attn_params* p) {
 }
 
 int nnlib_b200_device_health(void* stream) {
-  int v = 0, w = 0, u = 0, t = 0, s = 0;
+  int v = 0, w = 0, u = 0, t = 0, s = 0, f = 0;
   cudaError_t e = short_take_abort(&s, (cudaStream_t)stream);
   v = 0;
   if (e == cudaSuccess) e = umma_take_abort(&v, (cudaStream_t)stream);
   if (e == cudaSuccess) e = umma_bwd_take_abort(&w, (cudaStream_t)stream);
+  if (e == cudaSuccess) e = umma_bwd_fused_take_abort(&f, (cudaStream_t)stream);
   if (e == cudaSuccess) e = gemm_take_abort(&u, (cudaStream_t)stream);
   if (e == cudaSuccess) e = tile_take_abort(&t, (cudaStream_t)stream);
   if (e != cudaSuccess) return finish(e);
-  return (v || w || u || t || s) ? NNLIB_B200_TIMEOUT : NNLIB_B200_OK;
+  return (v || w || u || t || s || f) ? NNLIB_B200_TIMEOUT : NNLIB_B200_OK;
 }
 
 int nnlib_b200_selftest_wait_runout(uint64_t limit_ns, int32_t* status, void* stream) {

@@ -29,7 +29,8 @@ struct AttnArgs {
   void* alpha;
   long long alpha_sb;
   int* status;
-  float* ws;                 // split-key forward: per-split partial results (see attn_tile.cu)
+  float* ws;                 // the caller's workspace: partial results of the split-key forward (attn_tile.cu), dQ of the
+                             // one-pass backward (attn_bwd_fused.cu)
   long long rng_h0, rng_b0, rng_H;
   unsigned int key0, key1, off_lo, off_hi;
   unsigned int rkey[20];   // the ten round keys of Philox4x32-10 (key0 + r*W0, key1 + r*W1), bumped once on the host

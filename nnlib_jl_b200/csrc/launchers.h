@@ -72,6 +72,11 @@ bool umma_bwd_supports(const AttnArgs& a, const BwdArgs& g, int dtype);
 cudaError_t umma_bwd(const AttnArgs& a, const BwdArgs& g, int dtype, cudaStream_t st);
 cudaError_t umma_bwd_take_abort(int* out, cudaStream_t st);
 
+// one-pass tcgen05 backward, same calls, with a workspace in a.ws (attn_bwd_fused.cu)
+size_t umma_bwd_fused_workspace_bytes(const AttnArgs& a);
+cudaError_t umma_bwd_fused(const AttnArgs& a, const BwdArgs& g, int dtype, cudaStream_t st);
+cudaError_t umma_bwd_fused_take_abort(int* out, cudaStream_t st);
+
 // strided-batched matrix product: tcgen05 kernel for 16-bit arrays (gemm_umma.cu), CUDA-core kernel for the rest
 // (gemm_fma.cu)
 const char* gemm_umma_reject_reason(const GemmArgs& g, int dtype);

@@ -1501,6 +1501,56 @@ def test_pullback_with_bias_on_tensor_cores(dtype, bias_dtype, E, H, Lq, Lkv, B,
     _grad_close(nb.jl_to_numpy(db), gb, bias_dtype if bias_dtype != torch.float32 else dtype, "dbias")
 
 
+@pytest.mark.parametrize("dtype,d,H,Lq,Lkv,B,mask,bias,drop", [
+    (torch.bfloat16, 8, 1, 1, 1, 1, None, None, 0.0),               # one score
+    (torch.float16, 64, 2, 128, 128, 1, "causal", None, 0.0),       # exactly one tile
+    (torch.bfloat16, 128, 2, 129, 127, 2, None, None, 0.0),         # a row past a tile, a key short of one
+    (torch.bfloat16, 72, 2, 385, 513, 1, None, None, 0.2),          # CTAs start at different query tiles and wrap round
+    (torch.float16, 128, 1, 520, 520, 2, "causal", None, 0.1),      # walks of 5, 4 .. 1 tiles
+    (torch.bfloat16, 64, 2, 257, 416, 1, "rows16", None, 0.0),      # mask rows on 16-byte boundaries, whole groups of 32
+    (torch.bfloat16, 128, 2, 200, 301, 1, "rows", None, 0.0),       # rows of any alignment, a ragged last group of keys
+    (torch.float16, 40, 2, 300, 130, 2, "queries", None, 0.3),      # no dependence on the key
+    (torch.bfloat16, 128, 2, 150, 290, 1, "pad", "f32", 0.1),
+    (torch.float16, 64, 2, 290, 150, 2, None, "heads", 0.0),        # dbias summed over the batch
+])
+def test_both_tensor_core_backwards_match_the_gradient_oracle(dtype, d, H, Lq, Lkv, B, mask, bias, drop):
+    """The one-pass backward (dq gathered in the workspace) and, when torch is asked for deterministic algorithms, the
+    two half backwards, which need none: both against the oracle, the second with the same bits every time."""
+    rng = np.random.default_rng(70 + d + Lq)
+    E = d * H
+    qn, kn, vn, dyn = (_round_to(rng.standard_normal((E, n, B)), dtype) for n in (Lq, Lkv, Lkv, Lq))
+    mask_arg, mask_np, bn, bias_t = None, None, None, None
+    if mask == "causal":
+        mask_arg = nb.make_causal_mask(_dev(qn, dtype))
+        mask_np = np.arange(Lkv)[:, None] <= np.arange(Lq)[None, :]
+    elif mask is not None:
+        shape = {"pad": (Lkv, 1, 1, B), "queries": (1, Lq, 1, B)}.get(mask, (Lkv, Lq, H, B))
+        mask_np = rng.random(shape) > 0.4
+        mask_np[:1] = True
+        mask_arg = nb.jl_from_numpy(mask_np, device=DEV)
+    if bias is not None:
+        bias_t = torch.float32 if bias == "f32" else dtype
+        bn = _round_to(0.5 * rng.standard_normal((Lkv, Lq, H) if bias == "heads" else (Lkv, Lq, H, B)), bias_t)
+    fd = nb.PhiloxDropout(drop, seed=5, offset=2) if drop > 0 else nb.identity
+    keep = P.keep_mask((Lkv, Lq, H, B), drop, 5, 2) if drop > 0 else None
+    x, _, back = nb.dot_product_attention_pullback(_dev(qn, dtype), _dev(kn, dtype), _dev(vn, dtype),
+                                                   None if bn is None else _dev(bn, bias_t), mask=mask_arg, nheads=H, fdrop=fd)
+    want = O.dot_product_attention_grad(qn, kn, vn, dyn, bn, mask=mask_np, nheads=H, keep=keep, p=drop)
+    dy = _dev(dyn, dtype)
+    for deterministic in (False, True):
+        torch.use_deterministic_algorithms(deterministic, warn_only=True)
+        try:
+            got, again = back(dy), back(dy)
+        finally:
+            torch.use_deterministic_algorithms(False)
+        assert back.path == _lib.PATH_UMMA
+        nb.device_health()
+        for name, g, w in zip(("dq", "dk", "dv", "dbias"), got, want):
+            if g is not None:
+                _grad_close(nb.jl_to_numpy(g), w, dtype, f"{name}, deterministic={deterministic}")
+        assert not deterministic or all(torch.equal(a, b) for a, b in zip(got[:3], again[:3]))
+
+
 def test_pullback_fully_masked_query_gives_no_gradient():
     """A query that attends to nothing has NaN output (src/softmax.jl:71-76); the library lets no gradient
     flow through it (both backward paths), so the other queries' gradients stay finite."""
