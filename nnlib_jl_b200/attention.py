@@ -128,6 +128,9 @@ _status_lock = threading.Lock()
 
 def _status_word(dev: torch.device) -> torch.Tensor:
     idx = dev.index if dev.index is not None else torch.cuda.current_device()
+    w = _status_words.get(idx)       # words are never taken out again
+    if w is not None:
+        return w
     with _status_lock:
         w = _status_words.get(idx)
         if w is None:
@@ -160,15 +163,35 @@ def _check(rc: int, where: str):
     raise _lib.NNlibB200Error(rc, where)
 
 
+# The short ways to the current device and stream when torch offers them: a Stream object and a device guard cost
+# several microseconds per call, which a small problem notices.
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_raw_device = getattr(torch._C, "_cuda_getDevice", None)
 
 
 def _stream() -> int:
-    """The current stream of the current device as a raw handle (the short way when torch offers it: building
-    a Stream object costs several microseconds per call, which a small problem notices)."""
+    """The current stream of the current device as a raw handle."""
     if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+        return _raw_stream(torch.cuda.current_device() if _raw_device is None else _raw_device())
     return torch.cuda.current_stream().cuda_stream
+
+
+class _SameDevice:
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_same_device = _SameDevice()
+
+
+def _on_device(dev: torch.device):
+    """``torch.cuda.device(dev)``, or nothing to enter when ``dev``, the device of a CUDA tensor, is current already."""
+    if _raw_device is not None and dev.index == _raw_device():
+        return _same_device
+    return torch.cuda.device(dev)
 
 
 def _require_dense_cuda(name: str, t: torch.Tensor):
@@ -178,8 +201,17 @@ def _require_dense_cuda(name: str, t: torch.Tensor):
         raise TypeError(f"{name} lives on {t.device}: this method is defined for CUDA arrays only")
     if t.dtype not in _DTYPES:
         raise TypeError(f"{name} has eltype {t.dtype}; supported: Float16, BFloat16, Float32")
+    size = t.shape
+    if len(size) == 3 and t.stride() == (1, size[0], size[0] * size[1]):
+        return                       # the common case at a glance
     if not is_column_major(t):
         raise TypeError(f"{name} is not a dense column-major array (strides {t.stride()} for size {tuple(t.shape)})")
+
+
+def _empty3(n0: int, n1: int, n2: int, dtype, dev) -> torch.Tensor:
+    """``jl_empty`` of three dimensions."""
+    s1 = n0 or 1
+    return torch.empty_strided((n0, n1, n2), (1, s1, s1 * (n1 or 1)), dtype=dtype, device=dev)
 
 
 def _bcast_strides(name: str, t: torch.Tensor, full: tuple) -> list:
@@ -200,6 +232,10 @@ def _bcast_strides(name: str, t: torch.Tensor, full: tuple) -> list:
     return out
 
 
+# what a call starts from: every field 0 (the library's defaults) but the two that the structure's constructor sets
+_blank_params = bytes(_lib.AttnParams())
+
+
 class _Problem:
     """Everything one call of the library needs, kept alive together."""
 
@@ -215,7 +251,7 @@ class _Problem:
         self.q, self.k, self.v = q, k, v
         self.Ev = v.shape[0] if need_v else E
         self.dv = self.Ev // H
-        p = _lib.AttnParams()
+        p = _lib.AttnParams.from_buffer_copy(_blank_params)
         p.dtype = _DTYPES[q.dtype]
         p.d, p.dv, p.H, p.Lq, p.Lkv, p.B = self.d, self.dv, H, Lq, Lkv, B
         p.q, p.k = q.data_ptr(), k.data_ptr()
@@ -248,10 +284,10 @@ class _Problem:
                 p.mask = m8.data_ptr()
                 p.mask_stride = (C.c_int64 * 4)(*st)
                 self.keep.append(m8)
-        p.causal = 1 if causal else 0
-        p.nan_on_fully_masked = 1
-        p.allow_tf32 = 1 if (_fast_math and q.dtype == torch.float32) else 0
-        p.scale = 0.0
+        if causal:
+            p.causal = 1
+        if _fast_math and q.dtype == torch.float32:
+            p.allow_tf32 = 1
         if dropout is not None and dropout.p > 0.0:
             p.dropout_p = dropout.p
             p.philox_seed = dropout.seed & 0xFFFFFFFFFFFFFFFF
@@ -264,17 +300,19 @@ class _Problem:
         self.p = p
 
     def alloc_lse(self):
-        self.lse = jl_empty((self.Lq, self.H, self.B), torch.float32, self.dev)
+        self.lse = _empty3(self.Lq, self.H, self.B, torch.float32, self.dev)
         self.p.lse = self.lse.data_ptr()
         return self.lse
 
     def alloc_x(self):
-        self.x = jl_empty((self.Ev, self.Lq, self.B), self.dtype, self.dev)
+        self.x = _empty3(self.Ev, self.Lq, self.B, self.dtype, self.dev)
         self.p.x = self.x.data_ptr()
         return self.x
 
     def alloc_alpha(self):
-        a = jl_empty((self.Lkv, self.Lq, self.H, self.B), self.dtype, self.dev)
+        s1 = self.Lkv or 1
+        s2 = s1 * (self.Lq or 1)
+        a = torch.empty_strided((self.Lkv, self.Lq, self.H, self.B), (1, s1, s2, s2 * self.H), dtype=self.dtype, device=self.dev)
         self.p.alpha = a.data_ptr()
         return a
 
@@ -293,7 +331,7 @@ def _is_causal_matrix(mask: torch.Tensor, Lq: int, Lkv: int) -> bool:
         return True
     lib = _lib.load()
     flag = torch.empty(1, dtype=torch.int32, device=mask.device)
-    with torch.cuda.device(mask.device):
+    with _on_device(mask.device):
         _check(lib.nnlib_b200_causal_check(mask.view(torch.uint8).data_ptr(), Lq, flag.data_ptr(), _stream()),
                "causal_check")
     return bool(flag.item())
@@ -365,7 +403,7 @@ class LazyAttnScores:
             pr = self._problem
             alpha = pr.alloc_alpha()
             if pr.Lkv > 0 and pr.Lq > 0 and pr.B > 0:
-                with torch.cuda.device(pr.dev):
+                with _on_device(pr.dev):
                     _check(_lib.load().nnlib_b200_attn_scores(C.byref(pr.p), _stream()), "attn_scores")
             self._value = jl_reshape(alpha, self._shape)
         return self._value
@@ -394,20 +432,21 @@ class LazyAttnScores:
 
 def _validate_3d(q, k, v, nheads):
     """The four checks of ``src/attention.jl:55-78``, same order and wording."""
-    if any(t.shape[0] % nheads != 0 for t in (q, k, v)):
+    sq, sk, sv = q.shape, k.shape, v.shape
+    if sq[0] % nheads != 0 or sk[0] % nheads != 0 or sv[0] % nheads != 0:
         raise ArgumentError(
             "First dimension in query, key and value must be divisible by `nheads`.\n"
             f"Instead:\n- size(q): {tuple(q.shape)}\n- size(k): {tuple(k.shape)}\n"
             f"- size(v): {tuple(v.shape)}\n- nheads: {nheads}")
-    if not (q.shape[2] == k.shape[2] == v.shape[2]):
+    if not (sq[2] == sk[2] == sv[2]):
         raise ArgumentError(
             "Batch dimensions have to be the same. Instead:\n"
             f"- size(q): {tuple(q.shape)}\n- size(k): {tuple(k.shape)}\n- size(v): {tuple(v.shape)}")
-    if q.shape[0] != k.shape[0]:
+    if sq[0] != sk[0]:
         raise ArgumentError(
             "First dimension in query and key has to be the same. Instead:\n"
             f"- size(q): {tuple(q.shape)}\n- size(k): {tuple(k.shape)}")
-    if k.shape[1] != v.shape[1]:
+    if sk[1] != sv[1]:
         raise ArgumentError(
             "Second dimension in key and value has to be the same. Instead:\n"
             f"- size(k): {tuple(k.shape)}\n- size(v): {tuple(v.shape)}")
@@ -437,7 +476,7 @@ def dot_product_attention(q, k, v, bias=None, *, fdrop: Callable = identity, mas
     if not (q.dtype == k.dtype == v.dtype):
         raise TypeError("query, key and value must share one element type")
     batch_size = tuple(q.shape[2:])
-    if q.ndim != 3:
+    if len(batch_size) != 1:
         # N-d wrapper, src/attention.jl:40-50: flatten the batch dims, restore them on both outputs.
         if not (batch_size == tuple(k.shape[2:]) == tuple(v.shape[2:])):
             raise ArgumentError("Batch dimensions have to be the same.")
@@ -466,12 +505,12 @@ def _fused(q, k, v, bias, mask, nheads, dropout):
     if _eager_scores:
         alpha = pr.alloc_alpha()
         if pr.Lq > 0 and pr.B > 0 and pr.Lkv > 0:
-            with torch.cuda.device(pr.dev):
+            with _on_device(pr.dev):
                 _check(_lib.load().nnlib_b200_attention(C.byref(pr.p), None, 0, _stream()), "attention")
         return x, alpha
     if pr.Lq > 0 and pr.B > 0:
         lib = _lib.load()
-        with torch.cuda.device(pr.dev):
+        with _on_device(pr.dev):
             # few queries against many keys: the library splits the keys of a unit over several CTAs when that
             # pays and tells how much scratch memory the partial results need (0: the ordinary forward)
             need = lib.nnlib_b200_attn_decode_workspace_bytes(C.byref(pr.p)) if pr.Lq <= 128 else 0
@@ -491,7 +530,7 @@ def _launch_part(pr, units: int, piece: bool = False):
     if pr.Lq == 0 or pr.B == 0:
         return
     lib, p = _lib.load(), pr.p
-    with torch.cuda.device(pr.dev):
+    with _on_device(pr.dev):
         if piece:
             _check(lib.nnlib_b200_attn_fwd(C.byref(p), _stream()), "attn_fwd")
             return
@@ -549,7 +588,7 @@ def dot_product_attention_pullback(q, k, v, bias=None, *, fdrop: Callable = iden
     pr.alloc_lse()
     lib = _lib.load()
     if pr.Lq > 0 and pr.B > 0:
-        with torch.cuda.device(pr.dev):
+        with _on_device(pr.dev):
             _check(lib.nnlib_b200_attn_fwd(C.byref(pr.p), _stream()), "attn_fwd")
     alpha = LazyAttnScores(pr, (pr.Lkv, pr.Lq, pr.H, pr.B))
 
@@ -568,14 +607,14 @@ def dot_product_attention_pullback(q, k, v, bias=None, *, fdrop: Callable = iden
             dbias32 = dbias32.permute(*range(bias.ndim - 1, -1, -1)) if bias.ndim else dbias32
             g.dbias = dbias32.data_ptr()
             g.dbias_stride = (C.c_int64 * 4)(*_bcast_strides("bias", dbias32, (pr.Lkv, pr.Lq, pr.H, pr.B)))
-        # the one-pass backward sums dq by atomic additions: a program that asks torch for deterministic algorithms
-        # gets the one that needs no workspace and adds in a fixed order
+        # the one-pass backward of 16-bit arrays sums dq by atomic additions: a program that asks torch for deterministic
+        # algorithms gets the one that needs no workspace and adds in a fixed order
         need = 0 if torch.are_deterministic_algorithms_enabled() else \
             lib.nnlib_b200_attn_bwd_workspace_bytes(C.byref(pr.p), C.byref(g))
         scratch = torch.empty(need or 4 * pr.Lq * pr.H * pr.B, dtype=torch.uint8, device=pr.dev)
         g.delta = scratch.data_ptr()
         back.path = lib.nnlib_b200_attn_bwd_path(C.byref(pr.p), C.byref(g))   # PATH_UMMA / PATH_SIMT, for tests
-        with torch.cuda.device(pr.dev):
+        with _on_device(pr.dev):
             _check(lib.nnlib_b200_attn_bwd_ws(C.byref(pr.p), C.byref(g), scratch.data_ptr(), need, _stream()) if need else
                    lib.nnlib_b200_attn_bwd(C.byref(pr.p), C.byref(g), _stream()), "attn_bwd")
         return dq, dk, dv, (None if dbias32 is None else dbias32.to(bias.dtype))
@@ -591,7 +630,7 @@ def _unfused(q, k, v, bias, mask, nheads, fdrop):
     x = pr.alloc_x()
     pr.alloc_lse()
     alpha = pr.alloc_alpha()
-    with torch.cuda.device(pr.dev):
+    with _on_device(pr.dev):
         if pr.Lq > 0 and pr.B > 0:
             _check(lib.nnlib_b200_attn_stats(C.byref(pr.p), _stream()), "attn_stats")
             _check(lib.nnlib_b200_attn_scores(C.byref(pr.p), _stream()), "attn_scores")
@@ -629,7 +668,7 @@ def dot_product_attention_scores(q, k, bias=None, *, fdrop: Callable = identity,
     alpha = pr.alloc_alpha()
     if pr.Lq > 0 and pr.B > 0 and pr.Lkv > 0:
         lib = _lib.load()
-        with torch.cuda.device(pr.dev):
+        with _on_device(pr.dev):
             _check(lib.nnlib_b200_attn_stats(C.byref(pr.p), _stream()), "attn_stats")
             _check(lib.nnlib_b200_attn_scores(C.byref(pr.p), _stream()), "attn_scores")
     if dropout is None and fdrop is not None and fdrop is not identity:

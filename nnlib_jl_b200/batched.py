@@ -16,7 +16,7 @@ import math
 import torch
 
 from . import _lib
-from .attention import _DTYPES, ArgumentError, _check, _status_word, _stream
+from .attention import _DTYPES, ArgumentError, _check, _on_device, _status_word, _stream
 from .layout import jl_empty, jl_reshape
 
 __all__ = ["DimensionMismatch", "batched_mul", "batched_mul_", "batched_transpose", "batched_adjoint", "batched_mul_path"]
@@ -96,7 +96,7 @@ def batched_mul_(Cm: torch.Tensor, A: torch.Tensor, B: torch.Tensor, alpha=1.0, 
     if Cm.numel() and Cm.stride(0) != 1 and Cm.shape[0] > 1:
         raise ArgumentError("batched_mul!: C must have unit stride along its first dimension")
     p, keep = _params(Cm, A, B, alpha, beta)
-    with torch.cuda.device(Cm.device):
+    with _on_device(Cm.device):
         _check(_lib.load().nnlib_b200_batched_gemm(C.byref(p), _stream()), "batched_gemm")
     del keep
     return Cm

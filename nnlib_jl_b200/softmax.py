@@ -13,7 +13,7 @@ from typing import Optional
 import torch
 
 from . import _lib
-from .attention import _DTYPES, ArgumentError, _check, _require_dense_cuda, _stream
+from .attention import _DTYPES, ArgumentError, _check, _on_device, _require_dense_cuda, _stream
 from .layout import is_column_major, jl_empty
 
 __all__ = ["softmax", "logsoftmax", "softmax_pullback", "logsoftmax_pullback"]
@@ -63,7 +63,7 @@ def _run(x: torch.Tensor, dy: Optional[torch.Tensor], dims, log: bool, out: Opti
     p.dy = dy.data_ptr() if dy is not None else None
     p.out = out.data_ptr()
     lib = _lib.load()
-    with torch.cuda.device(x.device):
+    with _on_device(x.device):
         if dy is None:
             _check(lib.nnlib_b200_softmax_fwd(C.byref(p), _stream()), "softmax_fwd")
         else:
