@@ -348,11 +348,11 @@ __global__ void __launch_bounds__((G > 256 ? G : 256)) softmax_cols_kernel(typen
           unpack<T>(cx[k], f);
           if (FWD) {
             const bool special = c.nan || c.m == f_ninf() || c.m == f_inf();
-            if (MODE == SM_FWD && !special) {
-#pragma unroll
-              for (int u = 0; u < V; ++u) f[u] *= inv_s;      // f holds exp(x - max) from the second sweep
-            } else {
+            if (special) {
               fwd_pack<MODE, V>(c, inv_s, log_s, f);
+            } else {                                          // softmax: f holds exp(x - max) from the second sweep
+#pragma unroll
+              for (int u = 0; u < V; ++u) f[u] = MODE == SM_FWD ? f[u] * inv_s : f[u] - c.m - log_s;
             }
             store_pack<T>(oc + jp * V, f);
           } else {
@@ -514,6 +514,131 @@ __global__ void __launch_bounds__(NT) softmax_strided_kernel(typename Ptrs<T, NA
   }
 }
 
+// ---- forward over long contiguous columns: the next column on its way while one is worked on -------------------
+// A column that takes a whole block's registers leaves room for one block on an SM, and a block that loads, reduces
+// twice and stores keeps the memory system idle for most of that time: 32000 BFloat16 x 4096, logsoftmax, 121 us =
+// 4.3 TB/s with a column after the other loaded into the registers of 1024 threads.  Here the next S columns of a block
+// arrive in shared memory (cp.async; a thread reads back only the packets that it copied itself, so its own wait is all
+// that is needed, and refills their place at once), and blocks of G threads, 1024 / G on an SM, are in different phases:
+// 107 us = 4.9 TB/s there (one block of 1024 threads, two columns arriving: 127), softmax 163 -> 110; 50000 BFloat16 x
+// 2000 178 -> 96, 10000 Float32 x 4096 116 -> 64.
+// What a thread does with its at most KP packets, and so the result, is softmax_cols_kernel's.
+constexpr int kRingSmem = 226 * 1024;
+template <typename T, int MODE, int G, int KP, int S>
+__global__ void __launch_bounds__(G, 1024 / G) softmax_ring_kernel(const T* __restrict__ x, T* __restrict__ out, long long n,
+                                                                   long long cols) {
+  constexpr int V = Pack<T>::V;
+  constexpr int kWarps = G / 32;
+  extern __shared__ __align__(16) uint4 ring[];
+  const int np = (int)(n / V);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = threadIdx.x;
+  __shared__ float sh[2][kWarps];
+  auto fetch = [&](long long col, int st) {
+    if (col < cols) {
+#pragma unroll
+      for (int k = 0; k < KP; ++k) {
+        const int jp = t + k * G;
+        if (jp < np) {
+          const unsigned int d = (unsigned int)__cvta_generic_to_shared(ring + st * np + jp);
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(x + col * n + (long long)jp * V) : "memory");
+        }
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // over the block; `buf` alternates, so that one barrier a reduction is enough
+  auto block_reduce = [&](float v, int buf, auto op) -> float {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, off));
+    if (lane == 0) sh[buf][warp] = v;
+    __syncthreads();
+    v = sh[buf][lane % kWarps];
+#pragma unroll
+    for (int off = kWarps / 2; off > 0; off >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, off));
+    return v;
+  };
+  auto add = [](float a, float b) { return a + b; };
+#pragma unroll
+  for (int st = 0; st < S; ++st) fetch(blockIdx.x + (long long)st * gridDim.x, st);
+  int st = 0;
+  for (long long col = blockIdx.x; col < cols; col += gridDim.x, st = st + 1 == S ? 0 : st + 1) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(S - 1) : "memory");
+    uint4 cx[KP];
+    ColStat c = stat_init();
+#pragma unroll
+    for (int k = 0; k < KP; ++k) {
+      const int jp = t + k * G;
+      if (jp < np) {
+        cx[k] = ring[st * np + jp];
+        float f[V];
+        unpack<T>(cx[k], f);
+#pragma unroll
+        for (int u = 0; u < V; ++u) c.m = max_nan(c.m, f[u]);
+      }
+    }
+    fetch(col + (long long)S * gridDim.x, st);
+    c.m = block_reduce(c.m, 0, [](float a, float b) { return max_nan(a, b); });
+    if (c.m != c.m) {            // a NaN somewhere in the column
+      c.nan = 1;
+      c.m = 0.f;
+    }
+    // the sum of the exponentials; of a column whose maximum is +Inf the number of its +Inf entries, which share
+    // the weight (src/softmax.jl:71-76)
+    const bool special = c.nan || c.m == f_ninf() || c.m == f_inf();
+    float part = 0.f;
+#pragma unroll
+    for (int k = 0; k < KP; ++k) {
+      const int jp = t + k * G;
+      if (jp < np) {
+        float f[V];
+        unpack<T>(cx[k], f);
+        if (!special) {
+#pragma unroll
+          for (int u = 0; u < V; ++u) {
+            f[u] = __expf(f[u] - c.m);
+            part += f[u];
+          }
+          if (MODE == SM_FWD) cx[k] = repack<T>(f);
+        } else {
+#pragma unroll
+          for (int u = 0; u < V; ++u) part += (f[u] == f_inf()) ? 1.f : 0.f;
+        }
+      }
+    }
+    c.s = block_reduce(part, 1, add);
+    c.n_inf = special ? (int)c.s : 0;
+    const float log_s = (MODE == LSM_FWD) ? __logf(c.s) : 0.f;
+    const float inv_s = (MODE == SM_FWD) ? 1.f / c.s : 0.f;
+#pragma unroll
+    for (int k = 0; k < KP; ++k) {
+      const int jp = t + k * G;
+      if (jp < np) {
+        float f[V];
+        unpack<T>(cx[k], f);
+        if (special) {
+          fwd_pack<MODE, V>(c, inv_s, log_s, f);
+        } else {
+#pragma unroll
+          for (int u = 0; u < V; ++u) f[u] = MODE == SM_FWD ? f[u] * inv_s : f[u] - c.m - log_s;
+        }
+        store_pack<T>(out + col * n + (long long)jp * V, f);
+      }
+    }
+  }
+}
+
+template <typename T, int MODE, int G, int KP, int S>
+cudaError_t launch_ring(const T* x, T* out, long long n, long long cols, cudaStream_t st) {
+  auto kern = softmax_ring_kernel<T, MODE, G, KP, S>;
+  constexpr int per_sm = 1024 / G;
+  const int smem = (int)(n * sizeof(T)) * S;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRingSmem / per_sm);
+  if (e != cudaSuccess) return e;
+  kern<<<(unsigned)(cols < 148 * per_sm ? cols : 148 * per_sm), G, smem, st>>>(x, out, n, cols);
+  count_launch();
+  return cudaGetLastError();
+}
+
 template <typename T, int MODE>
 cudaError_t launch_softmax(const void* x, const void* dy, void* out, long long inner, long long n, long long outer,
                            cudaStream_t st) {
@@ -537,6 +662,15 @@ cudaError_t launch_softmax(const void* x, const void* dy, void* out, long long i
     // per thread: 8 raw packets for Float32 forward, 4 otherwise, 4 + 4 in the pullbacks)
     constexpr bool FWD = (MODE == SM_FWD || MODE == LSM_FWD);
     constexpr int kBig = (FWD && sizeof(T) == 4) ? 8 : 4;
+    // long columns, enough of them for every block to have a next one (20000 Float16 x 300: 15 us in the other kernel, 19
+    // here; x 700: 24 and 22).  Columns that 256 threads hold (2048 packets) leave enough blocks on an SM as it is: 16384
+    // BFloat16 x 4096 52 us, and 60 with the next column arriving.  In-place calls keep the other kernel, too.
+    if constexpr (FWD) {
+      if (vect && no_alias && outer >= 4 * 148) {
+        if (np > 256ll * 8 && np <= 512ll * 8) return launch_ring<T, MODE, 512, 8, 1>(xp, op, n, outer, st);
+        if (np > 512ll * 8 && np <= 1024ll * 7) return launch_ring<T, MODE, 1024, 7, 2>(xp, op, n, outer, st);
+      }
+    }
 #define NB_SM_LAUNCH(GG, VV, KK)                                                                       \
   do {                                                                                                 \
     constexpr int kBlock = (GG) > 256 ? (GG) : 256;                                                    \

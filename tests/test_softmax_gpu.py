@@ -54,6 +54,33 @@ def test_forward_and_pullbacks_match_the_oracle(dtype, shape, dims):
     np.testing.assert_allclose(nb.jl_to_numpy(dlx), want, atol=4 * tol * max(1.0, np.abs(want).max()), rtol=4 * tol)
 
 
+@pytest.mark.parametrize("dtype,n,cols", [
+    (torch.bfloat16, 16392, 593),     # one packet more than 256 threads hold
+    (torch.float16, 32768, 592),      # all eight packets of 512 threads
+    (torch.float32, 16388, 601),      # one packet beyond that: 1024 threads, two columns arriving
+    (torch.bfloat16, 57344, 593),     # all seven of those
+    (torch.bfloat16, 57352, 593),     # longer than that, the other kernel
+    (torch.bfloat16, 16392, 591),     # too few columns
+])
+def test_long_columns_arriving_ahead(dtype, n, cols):
+    """Long contiguous columns, among them ones with +Inf, -Inf and NaN entries, against the same columns in a batch too
+    small for them to be fetched ahead (torch's Float64 softmax for the ordinary ones)."""
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    t = torch.empty((cols, n), device=DEV).normal_(0, 3, generator=gen)
+    inf = float("inf")
+    t[5, 17], t[5, n - 1], t[300, 3], t[590, :], t[7, 0] = inf, inf, float("nan"), -inf, -inf
+    x = t.to(dtype).t()
+    few = [0, 5, 7, 148, 300, 295, 296, cols - 1, 590]
+    for f, ref in ((SM.softmax, torch.softmax), (SM.logsoftmax, torch.log_softmax)):
+        y = f(x)
+        sub = _as_cm(x[:, few], dtype)
+        assert torch.allclose(y[:, few].float(), f(sub).float(), rtol=2 * TOL[dtype], atol=1e-6 if f is SM.softmax else 2 * TOL[dtype],
+                              equal_nan=True)
+        want = ref(x[:, [0, 7, 148, 296]].double(), 0)
+        got = y[:, [0, 7, 148, 296]].double()
+        assert torch.allclose(got, want, rtol=TOL[dtype] if dtype != torch.float32 else 1e-5, atol=1e-9 if dtype != torch.float16 else 6e-8)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("shape,dims", [((300, 33), 1), ((70000, 3), 1), ((64, 50, 4), 2)])
 def test_in_place_forms(dtype, shape, dims):
