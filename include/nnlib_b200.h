@@ -272,9 +272,9 @@ NNLIB_B200_API int nnlib_b200_attn_bwd(const nnlib_b200_attn_params* p, const nn
                                        void* stream);
 
 /* The same pullback in one pass over the scores instead of two (five products per block of scores instead of
-   seven), for the calls that run on the tensor cores: dq is gathered in Float32 in the caller's workspace by atomic
-   additions, whose order is not fixed, so that dq may differ in its last bit from one call to the next
-   (nnlib_b200_attn_bwd gives the same bits each time).  workspace: device memory, 16-byte aligned, at least
+   seven).  On the tensor cores dq is gathered in Float32 in the caller's workspace by atomic additions, whose order is
+   not fixed, so that dq may differ in its last bit from one call to the next (nnlib_b200_attn_bwd gives the same bits
+   each time); Float32 arrays leave partial results there, which are added in a fixed order.  workspace: device memory, 16-byte aligned, at least
    nnlib_b200_attn_bwd_workspace_bytes(p, g) bytes, which need not be cleared and is free again when the call's
    kernels have run.  A result of 0 bytes: no workspace is used and the call is nnlib_b200_attn_bwd.  g->delta is
    not used where a workspace is. */

@@ -1,6 +1,7 @@
 // The C ABI of libnnlib_b200.so (include/nnlib_b200.h): argument checking,
 // defaults, kernel selection.  No exceptions leave this file, no device memory
 // is allocated, nothing synchronises except nnlib_b200_device_health.
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -446,11 +447,25 @@ static bool use_bwd_fused(const AttnArgs& a, BwdArgs b, int dtype) {
   return key_tiles * a.H * a.B >= 16 || query_tiles <= 2 * key_tiles;
 }
 
+// Float32 in one pass on the CUDA cores: five products instead of seven.  By the number of tiles, whichever form needs
+// fewer products one after the other: the longest walk of a block or the whole of the work over the blocks that fit at
+// once (the launch that merges the parts counts as one).  64 keys and queries of 4 units 26 us in two halves and 24 in
+// one pass, 100 of 8 units 32 and 25, the larger ones in attn_bwd_fma.cu.  The workspace, a Float32 per score for d = 64,
+// ends at 1 GiB.  (With a gradient of the bias the half that owns queries stays: its lanes add to neighbouring elements of it.)
+static bool use_bwd_fma_all(const AttnArgs& a, const BwdArgs& b, int dtype) {
+  if (a.Lq < 1 || a.B < 1 || a.Lkv < 1 || dtype != NNLIB_B200_F32 || b.dbias || force_simt() || !fma_supports(a.d, a.dv)) return false;
+  const double kt = (a.Lkv + 63ll) / 64, qt = (a.Lq + 63ll) / 64, tiles = kt * qt * a.H * a.B * (a.causal ? 0.5 : 1.0);
+  const double at_once = 148 * (a.d <= 64 && a.dv <= 64 ? 2 : 1), len = fma_bwd_chunk(a);
+  if (kt * qt * a.H * a.B * 64 * (a.d + 4) * 4 > (double)(1 << 30)) return false;
+  return std::max(5 * len, 5 * tiles / at_once) + 1 < std::max(std::max(4 * qt, 3 * kt), 7 * tiles / at_once);
+}
+
 size_t nnlib_b200_attn_bwd_workspace_bytes(const nnlib_b200_attn_params* p, const nnlib_b200_attn_grads* g) {
   AttnArgs a;
   BwdArgs b;
-  if (resolve_bwd(p, g, &a, &b, false, false) != NNLIB_B200_OK || !use_bwd_fused(a, b, p->dtype)) return 0;
-  return umma_bwd_fused_workspace_bytes(a);
+  if (resolve_bwd(p, g, &a, &b, false, false) != NNLIB_B200_OK) return 0;
+  if (use_bwd_fused(a, b, p->dtype)) return umma_bwd_fused_workspace_bytes(a);
+  return use_bwd_fma_all(a, b, p->dtype) ? fma_bwd_workspace_bytes(a) : 0;
 }
 
 int nnlib_b200_attn_bwd_ws(const nnlib_b200_attn_params* p, const nnlib_b200_attn_grads* g, void* workspace,
@@ -459,10 +474,17 @@ int nnlib_b200_attn_bwd_ws(const nnlib_b200_attn_params* p, const nnlib_b200_att
   BwdArgs b;
   const int rc = resolve_bwd(p, g, &a, &b, true, false);
   if (rc) return rc;
-  if (!use_bwd_fused(a, b, p->dtype)) return nnlib_b200_attn_bwd(p, g, stream);
-  if (!workspace || workspace_bytes < umma_bwd_fused_workspace_bytes(a) || (reinterpret_cast<uintptr_t>(workspace) & 15u) != 0)
+  const bool fused = use_bwd_fused(a, b, p->dtype);
+  if (!fused && !use_bwd_fma_all(a, b, p->dtype)) return nnlib_b200_attn_bwd(p, g, stream);
+  const size_t need = fused ? umma_bwd_fused_workspace_bytes(a) : fma_bwd_workspace_bytes(a);
+  if (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 15u) != 0)
     return NNLIB_B200_WORKSPACE_TOO_SMALL;
   a.ws = static_cast<float*>(workspace);
+  if (!fused) {
+    b.delta = a.ws;
+    log_call("attn_bwd", p, a, "cuda-core (one pass)", simt_reason(a, p->dtype, true));
+    return finish(fma_bwd(a, b, p->dtype, (cudaStream_t)stream));
+  }
   log_call("attn_bwd", p, a, "tcgen05 (one pass)", nullptr);
   return finish(umma_bwd_fused(a, b, p->dtype, (cudaStream_t)stream));
 }

@@ -8,8 +8,16 @@
 // the two arrays of their own rows in shared memory and stream the two of the other side, so one code serves
 // both; they share a launch because neither alone fills the GPU at the sizes Float32 is used for.  No atomics
 // except for dbias: the gradients of a call are the same bits every time.
-// One training step (forward and backward) at d = 64, 8 heads, 512 x 512 causal, batch 8: 23.06 ms with the warp-per-row
-// kernels, 0.46 ms with these (16 TFLOP/s counting seven products over the causal half).
+//
+// With a workspace there is another form, of one pass: every block owns 64 keys and computes a tile of scores once, with
+// five products instead of the two kinds' seven, and leaves its share of the queries' dq in the workspace, 16 KB a tile at
+// d = 64; a third launch adds the shares up, in the same order every time.  Where the keys alone make too few blocks, the
+// walks over the queries are cut as well and dk and dv are put together in the same way.  What bounds a tile is shared
+// memory: 4 x 4 scores a thread read 8 floats for 16 multiply-adds.
+// Backward at d = 64, 8 heads, 512 x 512 causal, batch 8: 306 us in two halves, 234 in one pass (222 with atomic
+// additions of dq, whose bits change from call to call); 16 heads, 2048 x 2048 causal 1025 and 736; 2 units of 1815 x 1815
+// 385 and 187; 4 units of 128 keys and 2000 queries 424 and 41, of 4000 keys and 40 queries 653 and 43.  One training step
+// (forward and backward) of the first: 23.06 ms with the warp-per-row kernels, 0.44 ms in two halves, 0.36 in one pass.
 #include <algorithm>
 
 #include "common.cuh"
@@ -42,10 +50,52 @@ __global__ void __launch_bounds__(128) attn_bwd_delta_kernel(const AttnArgs a, c
 template <int DP>
 __host__ __device__ constexpr int bwd_smem() { return 4 * (4 * kBM * (DP + 4) + 2 * kBM * kLDP) + kBM * 8; }
 
-// KEYS: the block owns keys (dk, dv); else queries (dq, dbias)
-template <typename T, int DP, int NTHR, bool KEYS>
+// Workspace of the one-pass form, in floats: D of all queries, then per unit and tile of 64 queries one partial dq from
+// every tile of keys, then, where the walks are cut into chunks, per unit and tile of keys one partial dk and dv from
+// every chunk.  Rows are dd = d (dv) rounded up to 4.
+struct Parts {
+  int kt, qt, chunks, len, dd, dvd;   // tiles, chunks of a walk, query tiles of a chunk
+  long long dq_off, dk_off, floats;
+};
+inline Parts make_parts(const AttnArgs& a) {
+  Parts p;
+  p.kt = (a.Lkv + kBM - 1) / kBM;
+  p.qt = (a.Lq + kBN - 1) / kBN;
+  p.len = fma_bwd_chunk(a);
+  p.chunks = (p.qt + p.len - 1) / p.len;
+  p.dd = (a.d + 3) & ~3;
+  p.dvd = (a.dv + 3) & ~3;
+  const long long units = (long long)a.H * a.B;
+  p.dq_off = ((long long)a.Lq * units + 3) & ~3ll;
+  p.dk_off = p.dq_off + units * p.qt * p.kt * (kBN * p.dd);
+  p.floats = p.dk_off + (p.chunks > 1 ? units * p.kt * p.chunks * (kBM * (p.dd + p.dvd)) : 0);
+  return p;
+}
+// first query that the keys of tile `t` are seen by, rounded down to a tile
+__device__ __forceinline__ int first_query(const AttnArgs& a, int t) {
+  const long long first = (long long)t * kBM - a.coff;
+  return !a.causal || first <= 0 ? 0 : (first < a.Lq ? (int)first / kBN * kBN : a.Lq);
+}
+
+// a thread's columns of a row of a partial result
+template <int DP>
+__device__ __forceinline__ void put_part(float* row, const float (&v)[DP / 16], float mul, int tx, int dd) {
+#pragma unroll
+  for (int c = 0; c < DP / 16; c += 2) {
+    const int e = colmap<DP>(tx, c);
+    if ((c & 3) == 0 && c + 3 < DP / 16) {
+      if (e < dd) *reinterpret_cast<float4*>(row + e) = make_float4(v[c] * mul, v[c + 1] * mul, v[c + 2] * mul, v[c + 3] * mul);
+    } else if ((c & 3) == 0) {
+      if (e < dd) *reinterpret_cast<float2*>(row + e) = make_float2(v[c] * mul, v[c + 1] * mul);   // (dd is even)
+    }
+  }
+}
+
+// KEYS: the block owns keys (dk, dv); else queries (dq, dbias).  ALL (with KEYS, Float32): it walks over chunk `chunk` of
+// the query tiles and leaves its part of their dq, and of dk and dv if there are several chunks, in the workspace.
+template <typename T, int DP, int NTHR, bool KEYS, bool ALL>
 __device__ __forceinline__ void bwd_block(const AttnArgs& a, const BwdArgs& g, const int tile, const int unit, const int vec,
-                                          float* sm) {
+                                          float* sm, const Parts& ws, const int chunk) {
   constexpr int MI = kBM * 16 / NTHR, LD = DP + 4, CN = DP / 16;
   float* a1 = sm;                    // own rows: K, V  or  Q, dX
   float* a2 = a1 + kBM * LD;
@@ -98,7 +148,23 @@ __device__ __forceinline__ void bwd_block(const AttnArgs& a, const BwdArgs& g, c
       c_end = last < 0 ? 0 : (last + 1 < n_cols ? (int)last + 1 : n_cols);
     }
   }
+  const bool part = ALL && ws.chunks > 1;
+  if (ALL) {
+    c_begin = max(c_begin, chunk * ws.len * kBN);
+    c_end = min(c_end, (int)min((long long)n_cols, (long long)(chunk + 1) * ws.len * kBN));
+    if (part && c_begin >= c_end) {    // the merge knows
+      cp_async_commit();
+      cp_async_wait<0>();
+      return;
+    }
+  }
   const int d4 = (a.d + 3) >> 2, dv4 = (a.dv + 3) >> 2;
+  bool a1_bad = false;
+  if (ALL) {                         // a key that takes no part may hold anything (accumulate_t)
+    cp_async_commit();
+    cp_async_wait<0>();
+    a1_bad = __syncthreads_or(tile_not_finite<T, kBM, DP, LD, NTHR>(a1, (vec & kVecK) != 0)) != 0;
+  }
   for (int c0 = c_begin; c0 < c_end; c0 += kBN) {
     const bool v1 = (vec & (KEYS ? kVecQ : kVecK)) != 0, v2 = (vec & (KEYS ? kVecD : kVecV)) != 0;
     if (KEYS) {
@@ -120,6 +186,9 @@ __device__ __forceinline__ void bwd_block(const AttnArgs& a, const BwdArgs& g, c
       col_lse[j] = (KEYS && gc < a.Lq) ? lse[gc] : ninf();
       col_delta[j] = (KEYS && gc < a.Lq) ? delta[gc] : 0.f;
     }
+    // nothing but the scale is to be applied to the tile's logits
+    const bool plain = !a.bias && !a.mask && !drop && r0 + kBM <= n_rows && c0 + kBN <= n_cols &&
+                       (!a.causal || j0 + kBN - 1 <= i0 + a.coff);
     cp_async_wait<1>();
     __syncthreads();
     float p[MI][4];
@@ -135,7 +204,9 @@ __device__ __forceinline__ void bwd_block(const AttnArgs& a, const BwdArgs& g, c
         const float L = KEYS ? col_lse[j] : row_lse[i];
         const int ql = qi - i0, kl = kj - j0;
         float pv = ninf();                                 // marks a score without any part in the result
-        if (gr < n_rows && gc < n_cols && L != ninf()) {
+        if (plain) {
+          if (L != ninf()) pv = expf(p[i][j] * a.scale - L);
+        } else if (gr < n_rows && gc < n_cols && L != ninf()) {
           const float t = finish_logit(a, p[i][j], kj, qi, h, b);
           if (t != ninf()) pv = expf(t - L);
         }
@@ -172,12 +243,36 @@ __device__ __forceinline__ void bwd_block(const AttnArgs& a, const BwdArgs& g, c
     const int nk = min(kBN, c_end - c0);
     if constexpr (KEYS) accumulate<MI, DP, LD>(ps, kLDP, b2, nk, ty, tx, skip, acc2);
     accumulate<MI, DP, LD>(ds, kLDP, b1, nk, ty, tx, skip, acc1);
+    if constexpr (ALL) {
+      float o[MI][CN];
+#pragma unroll
+      for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int c = 0; c < CN; ++c) o[i][c] = 0.f;
+      accumulate_t<MI, DP, LD>(ds, kLDP, a1, ty, tx, a1_bad, o);
+#pragma unroll
+      for (int i = 0; i < MI; ++i)
+        put_part<DP>(a.ws + ws.dq_off + (((long long)unit * ws.qt + c0 / kBN) * ws.kt + tile) * (kBN * ws.dd) +
+                     (ty * MI + i) * ws.dd, o[i], a.scale, tx, ws.dd);
+    }
     __syncthreads();
   }
   cp_async_wait<0>();
 
   T* o1 = reinterpret_cast<T*>(KEYS ? g.dk : g.dq) + (long long)n_rows * b * ((long long)a.H * a.d) + (long long)h * a.d;
   T* o2 = reinterpret_cast<T*>(g.dv) + (long long)n_rows * b * ((long long)a.H * a.dv) + (long long)h * a.dv;
+  if constexpr (ALL) {
+    if (part) {
+      float* w = a.ws + ws.dk_off + (((long long)unit * ws.kt + tile) * ws.chunks + chunk) * (kBM * (ws.dd + ws.dvd)) + ty * MI * ws.dd;
+      float* wv = w + kBM * ws.dd + ty * MI * (ws.dvd - ws.dd);
+#pragma unroll
+      for (int i = 0; i < MI; ++i) {
+        put_part<DP>(w + i * ws.dd, acc1[i], a.scale, tx, ws.dd);
+        put_part<DP>(wv + i * ws.dvd, acc2[i], 1.f, tx, ws.dvd);
+      }
+      return;
+    }
+  }
 #pragma unroll
   for (int i = 0; i < MI; ++i) {
     const int gr = r0 + ty * MI + i;
@@ -191,35 +286,107 @@ __device__ __forceinline__ void bwd_block(const AttnArgs& a, const BwdArgs& g, c
   }
 }
 
-template <typename T, int DP, int NTHR>
+template <typename T, int DP, int NTHR, bool ALL>
 __global__ void __launch_bounds__(NTHR, DP <= 64 ? 2 : 1)
-attn_bwd_fma_kernel(const AttnArgs a, const BwdArgs g, const int nkt, const int nqt, const int vec) {
+attn_bwd_fma_kernel(const AttnArgs a, const BwdArgs g, const int nkt, const int nqt, const int vec, const Parts ws) {
   extern __shared__ __align__(16) float sm[];
   const int units = a.H * a.B;
   const int t = blockIdx.x / units, unit = blockIdx.x % units;
   // causal: the first keys are seen by the most queries, the last queries see the most keys
-  if (t < nkt) bwd_block<T, DP, NTHR, true>(a, g, t, unit, vec, sm);
-  else bwd_block<T, DP, NTHR, false>(a, g, nkt + nqt - 1 - t, unit, vec, sm);
+  if (ALL) bwd_block<T, DP, NTHR, true, ALL>(a, g, t / ws.chunks, unit, vec, sm, ws, t % ws.chunks);
+  else if (t < nkt) bwd_block<T, DP, NTHR, true, false>(a, g, t, unit, vec, sm, ws, 0);
+  else bwd_block<T, DP, NTHR, false, false>(a, g, nkt + nqt - 1 - t, unit, vec, sm, ws, 0);
 }
 
-template <typename T, int DP, int NTHR>
-cudaError_t launch_bwd(const AttnArgs& a, const BwdArgs& g, int vec, cudaStream_t st) {
+// The parts of the one-pass form added up, always in the same order.  A block sums 1024 elements (a thread four) of the
+// 64 rows of one tile of queries (dq) or, behind those, of keys (dk and dv).
+__global__ void __launch_bounds__(256) attn_bwd_fma_merge_kernel(const AttnArgs a, const BwdArgs g, const Parts ws) {
+  const int units = a.H * a.B;
+  const int e = (blockIdx.y * 256 + threadIdx.x) * 4;
+  int t = blockIdx.x / units;
+  const int unit = blockIdx.x % units, h = unit % a.H, b = unit / a.H;
+  const bool keys = t >= ws.qt;
+  if (keys) t -= ws.qt;
+  const float* w;
+  long long stride;
+  int n, first = 0, row, col, width, d = a.d;
+  float* out;
+  long long rows;
+  if (!keys) {
+    width = ws.dd;
+    row = e / width; col = e % width;
+    out = reinterpret_cast<float*>(g.dq);
+    rows = a.Lq;
+    stride = kBN * ws.dd;
+    w = a.ws + ws.dq_off + ((long long)unit * ws.qt + t) * ws.kt * stride + e;
+    // tiles of keys that the queries see any of: the first so many
+    n = ws.kt;
+    if (a.causal)
+      for (n = 0; n < ws.kt && first_query(a, n) <= t * kBN;) ++n;
+  } else {
+    const bool v = e >= kBM * ws.dd;
+    const int f = v ? e - kBM * ws.dd : e;
+    width = v ? ws.dvd : ws.dd;
+    row = f / width; col = f % width;
+    out = reinterpret_cast<float*>(v ? g.dv : g.dk);
+    rows = a.Lkv;
+    stride = kBM * (ws.dd + ws.dvd);
+    w = a.ws + ws.dk_off + ((long long)unit * ws.kt + t) * ws.chunks * stride + e;
+    const int q = first_query(a, t);
+    first = q / (ws.len * kBN);
+    n = q < a.Lq ? ws.chunks : 0;
+    d = v ? a.dv : a.d;
+  }
+  if (row >= kBM || (long long)t * kBM + row >= rows) return;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int k = first; k < n; ++k) {
+    const float4 f = *reinterpret_cast<const float4*>(w + k * stride);
+    s.x += f.x; s.y += f.y; s.z += f.z; s.w += f.w;
+  }
+  float* o = out + ((long long)t * kBM + row + rows * b) * ((long long)a.H * d) + (long long)h * d + col;
+  const float r[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+    if (col + u < d) o[u] = r[u];
+}
+
+template <typename T, int DP, int NTHR, bool ALL>
+cudaError_t launch_bwd_form(const AttnArgs& a, const BwdArgs& g, int vec, cudaStream_t st) {
   const long long rows = (long long)a.Lq * a.H * a.B, db = (rows + 3) / 4;
   const int nkt = (a.Lkv + kBM - 1) / kBM, nqt = (a.Lq + kBM - 1) / kBM;
-  const long long blocks = ((long long)nkt + nqt) * a.H * a.B;
+  Parts ws = {};
+  if (ALL) ws = make_parts(a);
+  const long long blocks = (ALL ? (long long)nkt * ws.chunks : (long long)nkt + nqt) * a.H * a.B;
   if (db > 0x7fffffffLL || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   if (db > 0) {
     attn_bwd_delta_kernel<T><<<(unsigned)db, 128, 0, st>>>(a, g);
     count_launch();
   }
   if (blocks > 0) {
-    auto kern = attn_bwd_fma_kernel<T, DP, NTHR>;
+    auto kern = attn_bwd_fma_kernel<T, DP, NTHR, ALL>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd_smem<DP>());
     if (e != cudaSuccess) return e;
-    kern<<<(unsigned)blocks, NTHR, bwd_smem<DP>(), st>>>(a, g, nkt, nqt, vec);
+    kern<<<(unsigned)blocks, NTHR, bwd_smem<DP>(), st>>>(a, g, nkt, nqt, vec, ws);
     count_launch();
+    if (ALL) {
+      e = cudaGetLastError();
+      if (e != cudaSuccess) return e;
+      const int keys = ws.chunks > 1, floats = kBM * (keys ? ws.dd + ws.dvd : ws.dd);
+      attn_bwd_fma_merge_kernel<<<dim3((unsigned)((ws.qt + (keys ? ws.kt : 0)) * a.H * a.B), (unsigned)((floats + 1023) / 1024)), 256, 0,
+                                  st>>>(a, g, ws);
+      count_launch();
+    }
   }
   return cudaGetLastError();
+}
+
+template <typename T, int DP, int NTHR>
+cudaError_t launch_bwd(const AttnArgs& a, const BwdArgs& g, int vec, cudaStream_t st) {
+  if constexpr (sizeof(T) == 4) {
+    if (a.ws) return launch_bwd_form<T, DP, NTHR, true>(a, g, vec, st);
+  }
+  return launch_bwd_form<T, DP, NTHR, false>(a, g, vec, st);
 }
 
 template <typename T>
@@ -239,6 +406,18 @@ cudaError_t launch_bwd_dims(const AttnArgs& a, const BwdArgs& g, int dtype, cuda
 }
 
 }  // namespace
+
+// One pass: how many query tiles a block walks over.  All of them where the blocks of keys alone fill the GPU; otherwise
+// so few that there are one and a half times as many blocks as fit on it at once.
+int fma_bwd_chunk(const AttnArgs& a) {
+  const long long kt = (a.Lkv + kBM - 1) / kBM, qt = (a.Lq + kBN - 1) / kBN, blocks = kt * a.H * a.B;
+  const long long at_once = 148 * (a.d <= 64 && a.dv <= 64 ? 2 : 1);
+  if (blocks >= at_once) return (int)std::max(qt, 1ll);
+  const long long chunks = std::max(1ll, std::min(qt, (3 * at_once / 2 + blocks - 1) / std::max(blocks, 1ll)));
+  return (int)((qt + chunks - 1) / chunks);
+}
+
+size_t fma_bwd_workspace_bytes(const AttnArgs& a) { return (size_t)make_parts(a).floats * sizeof(float); }
 
 cudaError_t fma_bwd(const AttnArgs& a, const BwdArgs& g, int dtype, cudaStream_t st) {
   if (a.H == 0 || a.B == 0) return cudaSuccess;

@@ -160,6 +160,36 @@ __device__ __forceinline__ void accumulate(const float* P, int pitch, const floa
   else accumulate_impl<MI, DP, LD, false>(P, pitch, V, nk, ty, tx, o);
 }
 
+// o[i][c] += sum_k P[k][ty*MI + i] V[k][colmap(tx, c)] over the tile's 64 rows k: the same with the transpose of a tile
+template <int MI, int DP, int LD, bool SKIP>
+__device__ __forceinline__ void accumulate_t_impl(const float* P, int pitch, const float* V, int ty, int tx, float (&o)[MI][DP / 16]) {
+  static_assert(MI == 4 || MI == 8, "rows of a thread");
+  constexpr int CN = DP / 16;
+  const float* pp = P + ty * MI;
+#pragma unroll 4
+  for (int k = 0; k < kBN; ++k) {
+    float p[MI], v[CN];
+#pragma unroll
+    for (int i = 0; i < MI; i += 4) {
+      const float4 f = *reinterpret_cast<const float4*>(pp + k * pitch + i);
+      p[i] = f.x; p[i + 1] = f.y; p[i + 2] = f.z; p[i + 3] = f.w;
+    }
+    load_cols<DP>(V + k * LD, tx, v);
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+      if (!SKIP || p[i] != 0.f) {
+#pragma unroll
+        for (int c = 0; c < CN; ++c) o[i][c] = fmaf(p[i], v[c], o[i][c]);
+      }
+  }
+}
+template <int MI, int DP, int LD>
+__device__ __forceinline__ void accumulate_t(const float* P, int pitch, const float* V, int ty, int tx, bool skip_zero,
+                                             float (&o)[MI][DP / 16]) {
+  if (skip_zero) accumulate_t_impl<MI, DP, LD, true>(P, pitch, V, ty, tx, o);
+  else accumulate_t_impl<MI, DP, LD, false>(P, pitch, V, ty, tx, o);
+}
+
 // Keep bits of dropout for a tile of `rows` score rows x 64 keys (keys k0 .., k0 a multiple of 8): byte g of
 // row r covers keys k0 + 8g .. +7.  One Philox call serves eight scores.
 // row_of(r): the global score-row number of tile row r.

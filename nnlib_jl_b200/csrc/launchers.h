@@ -30,6 +30,9 @@ size_t fma_split_workspace_bytes(const AttnArgs& a, int dtype);
 cudaError_t fma_split(const AttnArgs& a, int dtype, cudaStream_t st);   // a.ws holds the workspace
 bool fma_row_supports(const AttnArgs& a, int dtype);     // x, alpha and lse in one pass (short key sequences)
 cudaError_t fma_row(const AttnArgs& a, int dtype, cudaStream_t st);
+size_t fma_bwd_workspace_bytes(const AttnArgs& a);
+int fma_bwd_chunk(const AttnArgs& a);                     // query tiles of a block of the one-pass form
+// a.ws set: one pass, partial results in the workspace (Float32)
 cudaError_t fma_bwd(const AttnArgs& a, const BwdArgs& g, int dtype, cudaStream_t st);
 
 // backward on CUDA cores (attn_bwd_simt.cu)

@@ -1767,6 +1767,46 @@ def test_float32_tiles_match_the_oracle(d, dv, H, Lq, Lkv, B, kind, drop):
                 _grad_close(nb.jl_to_numpy(got), w, dtype, name)
 
 
+@pytest.mark.parametrize("d,dv,H,Lq,Lkv,B,kind,drop", [
+    (64, 64, 1, 129, 64, 1, "none", 0.0),        # one tile of keys: the walk over three of queries is cut
+    (40, 24, 2, 130, 200, 1, "pad", 0.0),        # dv != d, rows of 40 and 24
+    (30, 30, 2, 200, 333, 1, "none", 0.2),       # rows padded to 32 in the workspace, dropout
+    (128, 128, 2, 70, 300, 1, "offset", 0.0),    # causal against a longer history
+    (96, 96, 1, 700, 65, 2, "none", 0.0),        # many queries, few keys; two columns of a thread stand apart
+    (64, 64, 8, 320, 320, 8, "causal", 0.0),     # keys enough: the walks stay whole
+    (32, 32, 3, 1, 4000, 1, "none", 0.0),        # one query, 63 tiles of keys
+])
+def test_float32_backward_in_one_pass(d, dv, H, Lq, Lkv, B, kind, drop):
+    """Partial dq (and dk, dv where walks are cut) merged in a fixed order: against the gradient oracle, the same bits
+    every time, and within rounding of the form that needs no workspace."""
+    rng = np.random.default_rng(80 + d + Lq)
+    f32 = torch.float32
+    qn, kn = (rng.standard_normal((d * H, n, B), dtype=np.float32) for n in (Lq, Lkv))
+    vn, dyn = (rng.standard_normal((dv * H, n, B), dtype=np.float32) for n in (Lkv, Lq))
+    mask_arg, mask_np = None, None
+    if kind == "pad":
+        mask_np = np.arange(Lkv)[:, None, None, None] < rng.integers(Lkv // 2, Lkv + 1, size=B)[None, None, None, :]
+        mask_arg = nb.jl_from_numpy(mask_np, device=DEV)
+    elif kind in ("causal", "offset"):
+        mask_np, mask_arg = _offset_mask(Lkv, Lq, Lkv - Lq), nb.CausalMask(Lkv - Lq)
+    fd = nb.PhiloxDropout(drop, seed=9, offset=4) if drop > 0 else nb.identity
+    keep = P.keep_mask((Lkv, Lq, H, B), drop, 9, 4) if drop > 0 else None
+    x, _, back = nb.dot_product_attention_pullback(_dev(qn, f32), _dev(kn, f32), _dev(vn, f32), mask=mask_arg, nheads=H, fdrop=fd)
+    dy = _dev(dyn, f32)
+    got, again = back(dy), back(dy)
+    torch.use_deterministic_algorithms(True, warn_only=True)
+    try:
+        other = back(dy)
+    finally:
+        torch.use_deterministic_algorithms(False)
+    want = O.dot_product_attention_grad(qn, kn, vn, dyn, None, mask=mask_np, nheads=H, keep=keep, p=drop)
+    for name, g, a, o, w in zip(("dq", "dk", "dv"), got, again, other, want):
+        _grad_close(nb.jl_to_numpy(g), w, f32, name)
+        assert torch.equal(g, a), name
+        # sums of at most 4000 products in another order: 4000 half ulps of the largest at the very most
+        assert (g - o).abs().max() <= 4000 * 6e-8 * o.abs().max(), name
+
+
 def test_float32_masked_keys_may_hold_anything():
     """A key that the mask takes out contributes nothing, whatever its rows of k and v hold: x, alpha and the
     gradients of the kept ones are those of the same arrays with zeros there (the tiled kernels leave a zero
