@@ -12,7 +12,7 @@
 //                    cost 16 8-byte shared-memory reads a step and thread instead of 32 16-byte ones (1 KB a warp
 //                    instead of 4, on the pipe that feeds the products)
 //   warps 8-11       dQ: tensor memory -> registers -> shared memory -> additions to global memory
-//   warp 12          TMA: K, V, ring of Q with the queries' lse and D;   warp 15: ring of dX
+//   warp 12          TMA: the first loads of all, then the ring of Q with the queries' lse and D;   warp 15: ring of dX
 //   warp 13          issues S and dV;   warp 14: issues dP, dQ and dK
 // Tensor memory columns, D = 128: S [0,128) | dP [128,256) | dV | dK; D = 64: S | dP | dV [256,320) | dK | dQ [384,448).
 // P^T (16 bits) is written over S, each thread over columns that it alone has read.  With D = 128 there is no room left
@@ -63,7 +63,7 @@ struct FuCfg {
 static_assert(FuCfg<128>::kSmemBytes <= 232448, "shared memory budget");
 
 struct FuBarriers {
-  uint64_t fix_full, q_full[2], q_empty[2], x_full[2], x_empty[2];
+  uint64_t k_full, v_full, q_full[2], q_empty[2], x_full[2], x_empty[2];
   uint64_t s_full, p_ready, dp_full, dp_read, ds_ready, dq_full, dq_read, acc_full;
   uint32_t tmem_base;
   int abort_flag;
@@ -78,7 +78,7 @@ template <int D, bool BF16, int FEAT>
 __global__ void __launch_bounds__(kFuThreads, 1)
 attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                       const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_dx,
-                      const AttnArgs a, const BwdArgs g, const int n_tiles, const int tail_units) {
+                      const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv, const AttnArgs a, const BwdArgs g, const int n_tiles, const int tail_units) {
   using C = FuCfg<D>;
   constexpr bool MASKED = (FEAT & 1) != 0, DROP = (FEAT & 2) != 0, BIAS = (FEAT & 4) != 0;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -122,8 +122,25 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
   const float* cols_u = a.ws + (long long)unit * n_q * (kColBytes / 4);
   float* dq_u = a.ws + tiles_all * (kColBytes / 4) + (long long)unit * n_q * (128 * D);
 
-  if (threadIdx.x == 0) {
-    mbar_init(&bars->fix_full, 1);
+  auto load_tile = [&](int off, const CUtensorMap* m, uint64_t* bar, int first) {
+    for (int c = 0; c < D / 64; ++c) tma_load_4d(smem + off + c * kChunkBytes, m, bar, c * 64, h, first, b);
+  };
+  auto load_q = [&](int it) {
+    const int s = it & 1;
+    mbar_arrive_expect_tx(&bars->q_full[s], C::kTile + kColBytes);
+    load_tile(C::kQOff + s * C::kTile, &tm_q, &bars->q_full[s], tile_of(it) * 128);
+    bulk_load(smem + C::kColOff + s * kColBytes, cols_u + (long long)tile_of(it) * (kColBytes / 4), &bars->q_full[s], kColBytes);
+  };
+  auto load_x = [&](int it) {
+    const int s = it % C::kXStages;
+    mbar_arrive_expect_tx(&bars->x_full[s], C::kTile);
+    load_tile(C::kXOff + s * C::kTile, &tm_dx, &bars->x_full[s], tile_of(it) * 128);
+  };
+  if (threadIdx.x == 12 * 32) {
+    prefetch_tensormap(&tm_k);
+    prefetch_tensormap(&tm_q);
+    mbar_init(&bars->k_full, 1);
+    mbar_init(&bars->v_full, 1);
     for (int s = 0; s < 2; ++s) {
       mbar_init(&bars->q_full[s], 1);
       mbar_init(&bars->q_empty[s], 1);
@@ -138,10 +155,18 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     mbar_init(&bars->dq_full, 1);
     mbar_init(&bars->dq_read, 4);
     mbar_init(&bars->acc_full, 2);
-    bars->abort_flag = *reinterpret_cast<volatile int*>(&g_bwd_fused_abort);
     fence_mbar_init();
+    // the first loads at once, while tensor memory is allocated and the block comes together (3 of a CTA's 48 us went
+    // by before its first scores were there)
+    mbar_arrive_expect_tx(&bars->k_full, C::kTile);
+    load_tile(C::kFixOff, &tm_k, &bars->k_full, t0);
+    load_q(0);
+    mbar_arrive_expect_tx(&bars->v_full, C::kTile);
+    load_tile(C::kFixOff + C::kTile, &tm_v, &bars->v_full, t0);
+    load_x(0);
+    bars->abort_flag = *reinterpret_cast<volatile int*>(&g_bwd_fused_abort);
   }
-  if (warp == 12) {
+  if (warp == 13) {
     tmem_alloc(&bars->tmem_base, 512);
     tmem_relinquish();
   }
@@ -156,50 +181,31 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
   constexpr int kRegOut = D == 64 ? 96 : (FEAT == 0 ? 144 : 128), kRegCompute = (512 * 128 - 128 * 64 - 128 * kRegOut) / 256;
   if (warp >= 12) {
     setmaxnreg_dec<64>();
-    if (start_ok && warp == 12) {
-      // ------------------------------------------------ TMA: K, V, ring of Q with its column values
+    if (warp == 12) {
+      // ------------------------------------------------ TMA: ring of Q with its column values
       if (lane == 0) {
-        prefetch_tensormap(&tm_k);
-        prefetch_tensormap(&tm_v);
-        prefetch_tensormap(&tm_q);
-        mbar_arrive_expect_tx(&bars->fix_full, 2 * C::kTile);
-        for (int c = 0; c < D / 64; ++c)
-          tma_load_4d(smem + C::kFixOff + c * kChunkBytes, &tm_k, &bars->fix_full, c * 64, h, t0, b);
         bool ok = true;
-        int it = 0;
-        for (; it < n; ++it) {
-          const int s = it & 1;
-          if (it >= 2) ok = mbar_wait(&bars->q_empty[s], ((it >> 1) - 1) & 1, abort_flag);
+        int it = 1;
+        for (; it < n && start_ok; ++it) {
+          if (it >= 2) ok = mbar_wait(&bars->q_empty[it & 1], ((it >> 1) - 1) & 1, abort_flag);
           if (!ok) break;
-          mbar_arrive_expect_tx(&bars->q_full[s], C::kTile + kColBytes);
-          for (int c = 0; c < D / 64; ++c)
-            tma_load_4d(smem + C::kQOff + s * C::kTile + c * kChunkBytes, &tm_q, &bars->q_full[s], c * 64, h,
-                        tile_of(it) * 128, b);
-          bulk_load(smem + C::kColOff + s * kColBytes, cols_u + (long long)tile_of(it) * (kColBytes / 4), &bars->q_full[s],
-                    kColBytes);
-          if (it == 0)
-            for (int c = 0; c < D / 64; ++c)
-              tma_load_4d(smem + C::kFixOff + C::kTile + c * kChunkBytes, &tm_v, &bars->fix_full, c * 64, h, t0, b);
+          load_q(it);
         }
         if (*abort_flag) {
-          mbar_wait_drain(&bars->fix_full, 0, kDrainNs);
+          mbar_wait_drain(&bars->k_full, 0, kDrainNs);
+          mbar_wait_drain(&bars->v_full, 0, kDrainNs);
           for (int jj = max(0, it - 2); jj < it; ++jj) mbar_wait_drain(&bars->q_full[jj & 1], (jj >> 1) & 1, kDrainNs);
         }
       }
-    } else if (start_ok && warp == 15) {
+    } else if (warp == 15) {
       // ------------------------------------------------ TMA: ring of dX
       if (lane == 0) {
-        prefetch_tensormap(&tm_dx);
         bool ok = true;
-        int it = 0;
-        for (; it < n; ++it) {
-          const int s = it % C::kXStages;
-          if (it >= C::kXStages) ok = mbar_wait(&bars->x_empty[s], (it / C::kXStages - 1) & 1, abort_flag);
+        int it = 1;
+        for (; it < n && start_ok; ++it) {
+          if (it >= C::kXStages) ok = mbar_wait(&bars->x_empty[it % C::kXStages], (it / C::kXStages - 1) & 1, abort_flag);
           if (!ok) break;
-          mbar_arrive_expect_tx(&bars->x_full[s], C::kTile);
-          for (int c = 0; c < D / 64; ++c)
-            tma_load_4d(smem + C::kXOff + s * C::kTile + c * kChunkBytes, &tm_dx, &bars->x_full[s], c * 64, h,
-                        tile_of(it) * 128, b);
+          load_x(it);
         }
         if (*abort_flag)
           for (int jj = max(0, it - C::kXStages); jj < it; ++jj)
@@ -235,7 +241,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                          idesc_acc, (first && kk == 0) ? 0u : 1u);
         };
 
-        bool ok = mbar_wait(&bars->fix_full, 0, abort_flag);
+        bool ok = mbar_wait(&bars->k_full, 0, abort_flag);
         if (warp == 13) {
           if (ok) ok = mbar_wait(&bars->q_full[0], 0, abort_flag);
           if (ok) {
@@ -259,6 +265,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
           }
           if (ok) umma_commit(&bars->acc_full);
         } else {
+          if (ok) ok = mbar_wait(&bars->v_full, 0, abort_flag);
           if (ok) ok = mbar_wait(&bars->x_full[0], 0, abort_flag);
           if (ok) {
             issue_nt(C::kColDP, v16, x16);
@@ -350,7 +357,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
           }
         }
       }
-      if (lane == 0) tma_store_wait<0>();
+      if (lane == 0) tma_store_wait_read<0>();
     }
   } else {
     setmaxnreg_inc<kRegCompute>();
@@ -671,29 +678,35 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
       }
       if (ok) {
         tc_fence_after();
-        const int row = t0 + wq * 32 + lane;
-        const long long dense = 2ll * (((long long)row + (long long)a.Lkv * b) * ((long long)a.H * a.d) + (long long)h * a.d);
-        uint8_t* out = reinterpret_cast<uint8_t*>(half == 0 ? g.dv : g.dk) + dense;
+        // through K's place (dV through V's: every product has read them) in the layout of the copy engine, which leaves
+        // out keys past the end and padding; stored from here, 16 bytes a row and thread, they took 3 us
+        const int r = wq * 32 + lane;
+        uint8_t* stage = smem + C::kFixOff + (half == 0 ? C::kTile : 0);
         const float mul = half == 0 ? 1.f : a.scale;
         const uint32_t col = lane_base + (half == 0 ? C::kColDV : C::kColDK);
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
           uint32_t o[32];
-          __syncwarp();   // the stores of the previous chunk are per-row branches
           tmem_ld32(col + c * 32, o);
           tmem_wait_ld();
-          if (row < a.Lkv) {
 #pragma unroll
-            for (int e = 0; e < 32; e += 8) {
-              if (c * 32 + e >= a.d) continue;   // a head narrower than the padded size: the rest is padding
-              uint4 v;
-              v.x = pack2<BF16>(__uint_as_float(o[e]) * mul, __uint_as_float(o[e + 1]) * mul);
-              v.y = pack2<BF16>(__uint_as_float(o[e + 2]) * mul, __uint_as_float(o[e + 3]) * mul);
-              v.z = pack2<BF16>(__uint_as_float(o[e + 4]) * mul, __uint_as_float(o[e + 5]) * mul);
-              v.w = pack2<BF16>(__uint_as_float(o[e + 6]) * mul, __uint_as_float(o[e + 7]) * mul);
-              *reinterpret_cast<uint4*>(out + (c * 32 + e) * 2) = v;
-            }
+          for (int e = 0; e < 32; e += 8) {
+            uint4 v;
+            v.x = pack2<BF16>(__uint_as_float(o[e]) * mul, __uint_as_float(o[e + 1]) * mul);
+            v.y = pack2<BF16>(__uint_as_float(o[e + 2]) * mul, __uint_as_float(o[e + 3]) * mul);
+            v.z = pack2<BF16>(__uint_as_float(o[e + 4]) * mul, __uint_as_float(o[e + 5]) * mul);
+            v.w = pack2<BF16>(__uint_as_float(o[e + 6]) * mul, __uint_as_float(o[e + 7]) * mul);
+            const int piece = (c & 1) * 4 + e / 8;
+            *reinterpret_cast<uint4*>(stage + (c >> 1) * kChunkBytes + r * 128 + ((piece ^ (r & 7)) << 4)) = v;
           }
+        }
+        fence_proxy_async_smem();
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+        if (wq == 0 && lane == 0) {
+          for (int c = 0; c < D / 64; ++c)
+            if (c * 64 < a.d) tma_store_4d(half == 0 ? &tm_dv : &tm_dk, stage + c * kChunkBytes, c * 64, h, t0, b);
+          tma_store_commit();
+          tma_store_wait_read<0>();
         }
       }
     }
@@ -701,7 +714,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 12) {
+  if (warp == 13) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
   }
@@ -800,7 +813,7 @@ __global__ void __launch_bounds__(256) attn_bwd_fused_post_kernel(const AttnArgs
 
 template <int D, bool BF16, int FEAT>
 cudaError_t launch_fused(const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mq, const CUtensorMap& mdx,
-                         const AttnArgs& a, const BwdArgs& g, cudaStream_t st) {
+                         const CUtensorMap& mdk, const CUtensorMap& mdv, const AttnArgs& a, const BwdArgs& g, cudaStream_t st) {
   auto kern = attn_bwd_fused_kernel<D, BF16, FEAT>;
   constexpr int smem = FuCfg<D>::kSmemBytes;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -823,7 +836,7 @@ cudaError_t launch_fused(const CUtensorMap& mk, const CUtensorMap& mv, const CUt
   attn_bwd_fused_pre_kernel<D, BF16><<<(unsigned)q_blocks, 256, 0, st>>>(a, g, n_q);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  kern<<<(unsigned)blocks, kFuThreads, smem, st>>>(mk, mv, mq, mdx, a, g, n_tiles, (int)tail_units);
+  kern<<<(unsigned)blocks, kFuThreads, smem, st>>>(mk, mv, mq, mdx, mdk, mdv, a, g, n_tiles, (int)tail_units);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   attn_bwd_fused_post_kernel<D, BF16><<<(unsigned)q_blocks, 256, 0, st>>>(a, g, n_q);
@@ -839,23 +852,26 @@ size_t umma_bwd_fused_workspace_bytes(const AttnArgs& a) {
 }
 
 cudaError_t umma_bwd_fused(const AttnArgs& a, const BwdArgs& g, int dtype, cudaStream_t st) {
-  CUtensorMap mq, mk, mv, mdx;
+  CUtensorMap mq, mk, mv, mdx, mdk, mdv;
   if (!make_head_map(&mq, a.q, dtype, a.d, a.H, a.Lq, a.B, a.q_sl, a.q_sb)) return cudaErrorInvalidValue;
   if (!make_head_map(&mk, a.k, dtype, a.d, a.H, a.Lkv, a.B, a.k_sl, a.k_sb)) return cudaErrorInvalidValue;
   if (!make_head_map(&mv, a.v, dtype, a.d, a.H, a.Lkv, a.B, a.v_sl, a.v_sb)) return cudaErrorInvalidValue;
   if (!make_head_map(&mdx, g.dx, dtype, a.d, a.H, a.Lq, a.B, g.dx_sl, g.dx_sb)) return cudaErrorInvalidValue;
+  const long long E = (long long)a.H * a.d;
+  if (!make_head_map(&mdk, g.dk, dtype, a.d, a.H, a.Lkv, a.B, E, E * a.Lkv)) return cudaErrorInvalidValue;
+  if (!make_head_map(&mdv, g.dv, dtype, a.d, a.H, a.Lkv, a.B, E, E * a.Lkv)) return cudaErrorInvalidValue;
   const bool bf16 = dtype == NNLIB_B200_BF16;
   const int feat = (a.mask ? 1 : 0) | (a.dropout_p > 0.f ? 2 : 0) | (a.bias ? 4 : 0);
 #define NB_FU(DD, BF)                                                  \
   switch (feat) {                                                      \
-    case 0: return launch_fused<DD, BF, 0>(mk, mv, mq, mdx, a, g, st); \
-    case 1: return launch_fused<DD, BF, 1>(mk, mv, mq, mdx, a, g, st); \
-    case 2: return launch_fused<DD, BF, 2>(mk, mv, mq, mdx, a, g, st); \
-    case 3: return launch_fused<DD, BF, 3>(mk, mv, mq, mdx, a, g, st); \
-    case 4: return launch_fused<DD, BF, 4>(mk, mv, mq, mdx, a, g, st); \
-    case 5: return launch_fused<DD, BF, 5>(mk, mv, mq, mdx, a, g, st); \
-    case 6: return launch_fused<DD, BF, 6>(mk, mv, mq, mdx, a, g, st); \
-    default: return launch_fused<DD, BF, 7>(mk, mv, mq, mdx, a, g, st); \
+    case 0: return launch_fused<DD, BF, 0>(mk, mv, mq, mdx, mdk, mdv, a, g, st); \
+    case 1: return launch_fused<DD, BF, 1>(mk, mv, mq, mdx, mdk, mdv, a, g, st); \
+    case 2: return launch_fused<DD, BF, 2>(mk, mv, mq, mdx, mdk, mdv, a, g, st); \
+    case 3: return launch_fused<DD, BF, 3>(mk, mv, mq, mdx, mdk, mdv, a, g, st); \
+    case 4: return launch_fused<DD, BF, 4>(mk, mv, mq, mdx, mdk, mdv, a, g, st); \
+    case 5: return launch_fused<DD, BF, 5>(mk, mv, mq, mdx, mdk, mdv, a, g, st); \
+    case 6: return launch_fused<DD, BF, 6>(mk, mv, mq, mdx, mdk, mdv, a, g, st); \
+    default: return launch_fused<DD, BF, 7>(mk, mv, mq, mdx, mdk, mdv, a, g, st); \
   }
   if (a.d > 64) {
     if (bf16) { NB_FU(128, true) } else { NB_FU(128, false) }
