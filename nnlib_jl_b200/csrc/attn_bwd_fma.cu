@@ -32,19 +32,32 @@ using namespace fma_tile;
 constexpr int kBM = 64;                                    // rows a block owns
 constexpr int kVecQ = 1, kVecK = 2, kVecV = 4, kVecD = 8;  // 16-byte copies of that array's rows are possible
 
-template <typename T>
+// D_i = dx_i . x_i, sixteen lanes a query; rows of 16-byte pieces (VEC) are read as such
+template <typename T, bool VEC>
 __global__ void __launch_bounds__(128) attn_bwd_delta_kernel(const AttnArgs a, const BwdArgs g) {
-  const int lane = threadIdx.x & 31;
-  const long long row = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (row >= (long long)a.Lq * a.H * a.B) return;
-  const int i = (int)(row % a.Lq), h = (int)((row / a.Lq) % a.H), b = (int)(row / ((long long)a.Lq * a.H));
-  const T* xrow = reinterpret_cast<const T*>(a.x) + (long long)i * a.x_sl + (long long)b * a.x_sb + (long long)h * a.dv;
-  const T* dxrow = reinterpret_cast<const T*>(g.dx) + (long long)i * g.dx_sl + (long long)b * g.dx_sb + (long long)h * a.dv;
+  const int lane = threadIdx.x & 15;
+  const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 4);
+  const bool row_ok = row < (long long)a.Lq * a.H * a.B;
   float dl = 0.f;
-  for (int e = lane; e < a.dv; e += 32) dl = fmaf(Elem<T>::to_f(dxrow[e]), Elem<T>::to_f(xrow[e]), dl);
+  if (row_ok) {
+    const int i = (int)(row % a.Lq), h = (int)((row / a.Lq) % a.H), b = (int)(row / ((long long)a.Lq * a.H));
+    const T* xrow = reinterpret_cast<const T*>(a.x) + (long long)i * a.x_sl + (long long)b * a.x_sb + (long long)h * a.dv;
+    const T* dxrow = reinterpret_cast<const T*>(g.dx) + (long long)i * g.dx_sl + (long long)b * g.dx_sb + (long long)h * a.dv;
+    if constexpr (VEC) {
+      for (int e = lane * 4; e < a.dv; e += 64) {
+        const float4 x = *reinterpret_cast<const float4*>(xrow + e), y = *reinterpret_cast<const float4*>(dxrow + e);
+        dl = fmaf(y.x, x.x, dl);
+        dl = fmaf(y.y, x.y, dl);
+        dl = fmaf(y.z, x.z, dl);
+        dl = fmaf(y.w, x.w, dl);
+      }
+    } else {
+      for (int e = lane; e < a.dv; e += 16) dl = fmaf(Elem<T>::to_f(dxrow[e]), Elem<T>::to_f(xrow[e]), dl);
+    }
+  }
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) dl += __shfl_xor_sync(0xffffffffu, dl, off);
-  if (lane == 0) g.delta[row] = dl;
+  for (int off = 8; off > 0; off >>= 1) dl += __shfl_xor_sync(0xffffffffu, dl, off);
+  if (row_ok && lane == 0) g.delta[row] = dl;
 }
 
 template <int DP>
@@ -353,14 +366,19 @@ __global__ void __launch_bounds__(256) attn_bwd_fma_merge_kernel(const AttnArgs 
 
 template <typename T, int DP, int NTHR, bool ALL>
 cudaError_t launch_bwd_form(const AttnArgs& a, const BwdArgs& g, int vec, cudaStream_t st) {
-  const long long rows = (long long)a.Lq * a.H * a.B, db = (rows + 3) / 4;
+  const long long rows = (long long)a.Lq * a.H * a.B, db = (rows + 7) / 8;
   const int nkt = (a.Lkv + kBM - 1) / kBM, nqt = (a.Lq + kBM - 1) / kBM;
   Parts ws = {};
   if (ALL) ws = make_parts(a);
   const long long blocks = (ALL ? (long long)nkt * ws.chunks : (long long)nkt + nqt) * a.H * a.B;
   if (db > 0x7fffffffLL || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   if (db > 0) {
-    attn_bwd_delta_kernel<T><<<(unsigned)db, 128, 0, st>>>(a, g);
+    bool dvec = false;
+    if constexpr (sizeof(T) == 4) {
+      dvec = (vec & kVecD) != 0 && rows_vec(a.x, a.x_sl, a.x_sb, a.dv, NNLIB_B200_F32);
+      if (dvec) attn_bwd_delta_kernel<T, true><<<(unsigned)db, 128, 0, st>>>(a, g);
+    }
+    if (!dvec) attn_bwd_delta_kernel<T, false><<<(unsigned)db, 128, 0, st>>>(a, g);
     count_launch();
   }
   if (blocks > 0) {

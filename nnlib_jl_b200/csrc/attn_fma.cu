@@ -73,27 +73,25 @@ __device__ __forceinline__ float make_lse(float m, float l) {
 
 template <int DP, int BM>
 __host__ __device__ constexpr int kp_floats() { return kBN * (DP + 4) > BM * kLDP ? kBN * (DP + 4) : BM * kLDP; }
-// x in one pass, heads up to 96: the P tile has a place of its own, and the next K and V tiles are copied while the
-// block works on this one (with larger heads it would cost the second block on an SM); with the tiles that need nothing
-// but the scale told apart, 512 x 512, d = 64, 64 units 267 -> 217 us, causal 134 -> 122, 2048 x 2048 causal, 16 units
-// 504 -> 432
-__host__ __device__ constexpr bool fm_ahead(int mode, int dp) { return mode == FM_FWD && dp <= 96; }
-template <int DP, int BM, int MODE>
+// AHEAD (x in one pass, heads up to 96): the P tile has a place of its own, and the next K and V tiles are copied while
+// the block works on this one (with larger heads it would cost the second block on an SM); tiles that need nothing but
+// the scale are told apart.  512 x 512, d = 64, 64 units 267 -> 217 us, causal 134 -> 122, 2048 x 2048 causal, 16 units
+// 504 -> 432.
+template <int DP, int BM, int MODE, bool AHEAD>
 __host__ __device__ constexpr int fma_smem() {
   return 4 * ((MODE != FM_APPLY ? BM * (DP + 4) : 0) +
-              (fm_ahead(MODE, DP) ? kBN * (DP + 4) + BM * kLDP : kp_floats<DP, BM>()) +
+              (AHEAD ? kBN * (DP + 4) + BM * kLDP : kp_floats<DP, BM>()) +
               (MODE != FM_STATS && MODE != FM_SCORES ? kBN * (DP + 4) : 0)) + BM * 8;
 }
 
 __host__ __device__ constexpr bool fm_with_v(int mode) { return mode == FM_FWD || mode == FM_APPLY || mode == FM_SPLIT; }
 
 // (d = 64, 8 rows a thread: three blocks on an SM with a few spilled words are faster than two without)
-template <typename T, int DP, int MI, int NTHR, int MODE>
+template <typename T, int DP, int MI, int NTHR, int MODE, bool AHEAD>
 __global__ void __launch_bounds__(NTHR, MODE == FM_FWD && MI == 8 && DP == 64 ? 3 : 1) attn_fma_kernel(const AttnArgs a, const int n_tiles, const int vec) {
   constexpr int BM = NTHR / 16 * MI, LD = DP + 4, CN = DP / 16;
   extern __shared__ __align__(16) float sm[];
   float* qs = sm;
-  constexpr bool AHEAD = fm_ahead(MODE, DP);
   float* kp = qs + (MODE != FM_APPLY ? BM * LD : 0);       // the K tile, then the P tile
   float* ps = AHEAD ? kp + kBN * LD : kp;
   float* vs = AHEAD ? ps + BM * kLDP : kp + kp_floats<DP, BM>();
@@ -429,11 +427,15 @@ __global__ void __launch_bounds__(NTHR) attn_fma_row_kernel(const AttnArgs a, co
 // Rows of a block: 64 (8 per thread) reads shared memory least per FMA and is the choice once the blocks fill
 // the GPU twice over; 32 when they do not, 8 for a handful of queries (a decode step), where most of a larger
 // block would be padding.
-template <typename T, int DP, int MI, int MODE>
+template <typename T, int DP, int MI, int MODE, bool AHEAD = false>
 cudaError_t launch_fma_mi(const AttnArgs& a, int vec, cudaStream_t st, int n_splits = 1) {
+  // walks of one or two tiles with a ragged end have nothing to gain: 102 x 102 causal, 320 units 61.5 us, 64.0 ahead
+  if constexpr (MODE == FM_FWD && DP <= 96 && !AHEAD) {
+    if (a.Lkv > 2 * kBN || a.Lkv % kBN == 0) return launch_fma_mi<T, DP, MI, MODE, true>(a, vec, st, n_splits);
+  }
   constexpr int NTHR = 128, BM = NTHR / 16 * MI;
-  constexpr int smem = fma_smem<DP, BM, MODE>();
-  auto kern = attn_fma_kernel<T, DP, MI, NTHR, MODE>;
+  constexpr int smem = fma_smem<DP, BM, MODE, AHEAD>();
+  auto kern = attn_fma_kernel<T, DP, MI, NTHR, MODE, AHEAD>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   const long long n_tiles = ((long long)a.Lq + BM - 1) / BM, blocks = n_tiles * a.H * a.B;
