@@ -14,6 +14,7 @@
 //   warp 2      allocates / frees the 512 TMEM columns
 //   warps 4-7   softmax of query tile 0 (thread r owns query row r: no shuffles)
 //   warps 8-11  softmax of query tile 1
+//   warps 12-15 with dropout and a mask array or bias: the random numbers, as keep bits in shared memory up to two rounds ahead
 //
 // TMEM columns: S_0 [0,128) S_1 [128,256) O_0 [256,384) O_1 [384,512); the
 // half-precision probabilities P_t overwrite the first 64 columns of S_t.
@@ -46,21 +47,24 @@ __device__ int g_umma_abort = 0;  // sticky: a bounded wait ran out somewhere
 namespace {
 
 constexpr int kQT = 2;                 // query tiles per CTA
-constexpr int kThreads = 384;
+constexpr int kThreads = 384, kRngThreads = 512;
 constexpr float kRescaleGap = 8.0f;    // raise the running max only when it grew by > 2^8
 
-template <int D>
+// RNG (warps of its own for the random numbers): keep bits of two rounds, [round & 1][query tile][query], 128 bits each,
+// in the place of one V tile
+template <int D, bool RNG = false>
 struct Cfg {
   static constexpr int kChunks = D / 64;
   static constexpr int kTileBytes = kChunks * kChunkBytes;
   // A K tile is released early in the round after its last use, a V tile only at the end of its
   // round, so V needs the deeper ring to keep a full round of copy latency hidden.
   static constexpr int kStagesK = (D == 128) ? 2 : 4;
-  static constexpr int kStagesV = (D == 128) ? 3 : 4;
+  static constexpr int kStagesV = ((D == 128) ? 3 : 4) - (RNG ? 1 : 0);
   static constexpr int kQOff = 0;
   static constexpr int kKOff = kQOff + kQT * kTileBytes;
   static constexpr int kVOff = kKOff + kStagesK * kTileBytes;
-  static constexpr int kBarOff = kVOff + kStagesV * kTileBytes;
+  static constexpr int kKeepOff = kVOff + kStagesV * kTileBytes;
+  static constexpr int kBarOff = kKeepOff + (RNG ? 2 * kQT * kBM * 16 : 0);
   static constexpr int kSmemBytes = kBarOff + 512 + 1024;  // barrier block + alignment slack
   // staged-bias variant (d = 64): per query tile two half tiles (64 keys x 128 queries) of the bias
   static constexpr int kBiasOff = kBarOff;
@@ -69,13 +73,15 @@ struct Cfg {
   static constexpr int kSmemBytesStaged = kBarOffStaged + 512 + 1024;
 };
 static_assert(Cfg<128>::kSmemBytes <= 232448 && Cfg<64>::kSmemBytes <= 232448, "shared memory budget");
-static_assert(Cfg<64>::kSmemBytesStaged <= 232448, "shared memory budget (staged bias)");
+static_assert(Cfg<64>::kSmemBytesStaged <= 232448 && Cfg<64, true>::kSmemBytesStaged <= Cfg<64>::kSmemBytesStaged &&
+              Cfg<128, true>::kSmemBytes <= Cfg<128>::kSmemBytes, "shared memory budget (staged bias, dropout)");
 
 struct Barriers {
   uint64_t q_full[kQT];
   uint64_t k_full[4], k_empty[4], v_full[4], v_empty[4];
   uint64_t s_full[kQT], p_half[kQT][2], o_full[kQT];
   uint64_t bias_full[kQT][2], bias_empty[kQT][2];   // staged bias half tiles
+  uint64_t keep_full[kQT][2], keep_free[kQT][2];    // keep bits of a round, by its parity
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -88,15 +94,23 @@ static_assert(sizeof(Barriers) <= 512, "barrier block");
 // idle warp 2) instead of through per-thread loads; needs a 16-bit bias with key stride 1 whose rows
 // the tensor map can address (the host decides).
 // SHIFT: bias / mask rows of any alignment (extras.cuh); without it they are all aligned and whole.
+//
+// Random numbers: sixteen calls of Philox a thread and round.  Where the softmax warps have side inputs to work in, the
+// numbers come from four warps of their own; without side inputs the softmax warps wait for their scores anyway and draw
+// them meanwhile.  f16, bias, d = 64, 256 x 2048, 256 units 210 -> 190 us; padding, d = 80, 1000 x 777, 48 units 105 -> 97;
+// window mask and bias, d = 64, 1024 x 1024, 32 units 66 -> 63; without side inputs, d = 64, 2048 x 2048, 128 units 444
+// and, with the four warps, 530.
+__host__ __device__ constexpr bool rng_warps(int xm, bool stats) { return xm > 3 && !stats; }
 template <int D, bool BF16, int XM, bool STATS, bool BSM, bool SHIFT>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(rng_warps(XM, STATS) ? kRngThreads : kThreads, 1)
 attn_fwd_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_b,
                      const AttnArgs a, const int n_qblocks, const int tail_units) {
-  using C = Cfg<D>;
+  constexpr bool DROP = XM >= 3 && !STATS;   // dropout code compiled in
+  constexpr bool RNG = rng_warps(XM, STATS);
+  using C = Cfg<D, RNG>;
   constexpr bool EXTRAS = (XM % 3) != 0;
   constexpr bool XBIAS = (XM % 3) == 2;   // bias code compiled in
-  constexpr bool DROP = XM >= 3;          // dropout code compiled in
   static_assert(!BSM || (XBIAS && D == 64 && !STATS), "staged bias: d = 64 forward with bias only");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -150,6 +164,8 @@ attn_fwd_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       for (int hf = 0; hf < 2; ++hf) {
         mbar_init(&bars->bias_full[t][hf], 1);
         mbar_init(&bars->bias_empty[t][hf], 4);
+        mbar_init(&bars->keep_full[t][hf], 4);
+        mbar_init(&bars->keep_free[t][hf], 4);
       }
     }
     for (int s = 0; s < 4; ++s) {
@@ -172,9 +188,9 @@ attn_fwd_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   const bool start_ok = (*abort_flag == 0);
 
   // The softmax threads hold a whole 128-wide score row in registers: move the
-  // register budget from the copy / issue warps to them.
+  // register budget from the copy / issue warps to them (with RNG 256 x 208 + 128 x 56 + 128 x 40 = the 512 x 128 launched).
   if (warp < 4) {
-    setmaxnreg_dec<72>();
+    setmaxnreg_dec<RNG ? 56 : 72>();
     if (start_ok && warp == 0 && lane == 0) {
       // ------------------------------------------------- producer of Q and K
       prefetch_tensormap(&tm_q);
@@ -331,8 +347,31 @@ attn_fwd_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 #undef NB_ISSUE_QK
 #undef NB_ISSUE_PV
     }
+  } else if (RNG && warp >= 12) {
+    // ------------------------------------------------------- random numbers
+    setmaxnreg_dec<40>();
+    if (start_ok) {
+      const int r = (warp - 12) * 32 + lane;
+      bool ok = true;
+      for (int j = 0; j < n_kv && ok; ++j) {
+#pragma unroll 1
+        for (int t = 0; t < kQT && ok; ++t) {
+          if (j >= (t == 0 ? n_t0 : n_t1)) continue;
+          if (j >= 2) ok = mbar_wait(&bars->keep_free[t][j & 1], ((j >> 1) - 1) & 1, abort_flag);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          const int i = q0 + t * kBM + r;
+          const unsigned long long srow = score_row(a, i < a.Lq ? i : 0, h, b);
+          uint32_t* kb = reinterpret_cast<uint32_t*>(smem + C::kKeepOff + (((j & 1) * kQT + t) * kBM + r) * 16);
+#pragma unroll 1
+          for (int c = 0; c < 4; ++c) kb[c] = dropout_keep32x4(a, srow, (unsigned int)(j * kBN >> 5) + c);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->keep_full[t][j & 1]);
+        }
+      }
+    }
   } else {
-    setmaxnreg_inc<216>();
+    setmaxnreg_inc<RNG ? 208 : 216>();
     const int t = (warp - 4) >> 2;        // query tile of this warpgroup
     const int nt = (t == 0) ? n_t0 : n_t1;
     if (start_ok && nt > 0) {
@@ -364,7 +403,7 @@ attn_fwd_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         // which of this tile's 128 scores survive dropout depends on their position only: drawn while
         // the tensor core still works on the scores
         unsigned int kb[4] = {0u, 0u, 0u, 0u};
-        if (DROP) {
+        if (DROP && !RNG) {
 #pragma unroll
           for (int c = 0; c < 4; ++c) kb[c] = dropout_keep32(a, srow, (unsigned int)(j * kBN >> 5) + c);
         }
@@ -516,6 +555,16 @@ attn_fwd_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             if (hf == 1) NB_EXP_HALF_W(1, m_sub);
             if (DROP) {
               // the row sum keeps the dropped scores (dropout follows the softmax)
+              if (RNG) {
+                if (hf == 0) {
+                  ok = mbar_wait(&bars->keep_full[t][j & 1], (j >> 1) & 1, abort_flag);
+                  ok = __all_sync(0xffffffffu, ok);
+                  if (!ok) break;
+                }
+                const uint2 k2 = *reinterpret_cast<const uint2*>(smem + C::kKeepOff + (((j & 1) * kQT + t) * kBM + r) * 16 + hf * 8);
+                kb[hf * 2] = k2.x;
+                kb[hf * 2 + 1] = k2.y;
+              }
 #pragma unroll
               for (int cc = 0; cc < 2; ++cc) {
                 const unsigned int kbc = kb[hf * 2 + cc];
@@ -530,8 +579,12 @@ attn_fwd_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&bars->p_half[t][hf]);
+            if (lane == 0) {
+              mbar_arrive(&bars->p_half[t][hf]);
+              if (RNG && hf == 1) mbar_arrive(&bars->keep_free[t][j & 1]);
+            }
           }
+          if (RNG && !ok) break;
         } else {
           // statistics only: running maximum and sum
           if (raise) {
@@ -1080,7 +1133,8 @@ template <int D, bool BF16, int XM, bool STATS, bool BSM, bool SHIFT>
 cudaError_t launch_fwd_impl(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mb,
                             const AttnArgs& a, cudaStream_t st) {
   auto kern = attn_fwd_umma_kernel<D, BF16, XM, STATS, BSM, SHIFT>;
-  constexpr int smem = BSM ? Cfg<D>::kSmemBytesStaged : Cfg<D>::kSmemBytes;
+  constexpr bool RNG = rng_warps(XM, STATS);
+  constexpr int smem = BSM ? Cfg<D, RNG>::kSmemBytesStaged : Cfg<D, RNG>::kSmemBytes;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   const int n_qblocks = (a.Lq + kQT * kBM - 1) / (kQT * kBM);
@@ -1090,7 +1144,7 @@ cudaError_t launch_fwd_impl(const CUtensorMap& mq, const CUtensorMap& mk, const 
   const long long n_units = (long long)a.H * a.B;
   long long tail_units = a.causal ? 2 * ((fwd_sm_count() + n_qblocks - 1) / n_qblocks) : 0;
   if (tail_units > n_units) tail_units = n_units;
-  kern<<<(unsigned)blocks, kThreads, smem, st>>>(mq, mk, mv, mb, a, n_qblocks, (int)tail_units);
+  kern<<<(unsigned)blocks, RNG ? kRngThreads : kThreads, smem, st>>>(mq, mk, mv, mb, a, n_qblocks, (int)tail_units);
   count_launch();
   return cudaGetLastError();
 }

@@ -173,6 +173,38 @@ __device__ __forceinline__ unsigned int dropout_keep32(const AttnArgs& a, unsign
   }
   return bits;
 }
+// Four calls of the generator at once, in lockstep: for warps that do little else, whose time is the latency of a call's
+// chain of ten rounds.  Call g: words w[g][..] of row r + g * dr, keys 8 (j8 + g * dj) .. + 7.
+__device__ __forceinline__ void dropout_words4(const AttnArgs& a, unsigned long long r, unsigned int dr, unsigned int j8,
+                                               unsigned int dj, unsigned int (&w)[4][4]) {
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    const unsigned long long rg = r + (unsigned long long)(g * dr);
+    w[g][0] = j8 + g * dj;
+    w[g][1] = (unsigned int)rg;
+    w[g][2] = (unsigned int)(rg >> 32) + a.off_hi;
+    w[g][3] = a.off_lo;
+  }
+#pragma unroll
+  for (int i = 0; i < 10; ++i) {
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const unsigned long long p0 = 0xD2511F53ull * w[g][0], p1 = 0xCD9E8D57ull * w[g][2];
+      w[g][0] = (unsigned int)(p1 >> 32) ^ w[g][1] ^ a.rkey[2 * i];
+      w[g][1] = (unsigned int)p1;
+      w[g][2] = (unsigned int)(p0 >> 32) ^ w[g][3] ^ a.rkey[2 * i + 1];
+      w[g][3] = (unsigned int)p0;
+    }
+  }
+}
+// dropout_keep32 with them
+__device__ __forceinline__ unsigned int dropout_keep32x4(const AttnArgs& a, unsigned long long r, unsigned int c32) {
+  unsigned int w[4][4], bits = 0;
+  dropout_words4(a, r, 0u, c32 * 4, 1u, w);
+#pragma unroll
+  for (int n = 0; n < 16; ++n) bits |= keep_lanes(a, w[n >> 2][n & 3]) >> (15 - n);
+  return bits;
+}
 // all-ones halves for the surviving keys of pair e (keys 2e and 2e+1 of the 32)
 __device__ __forceinline__ unsigned int keep_pair_mask(unsigned int bits, int e) {
   unsigned int m;
