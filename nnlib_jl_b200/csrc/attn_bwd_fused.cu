@@ -11,7 +11,7 @@
 //                    in the fragment layout (tmem_ld_frag): 16 queries per thread, so that the per-query lse and D
 //                    cost 16 8-byte shared-memory reads a step and thread instead of 32 16-byte ones (1 KB a warp
 //                    instead of 4, on the pipe that feeds the products)
-//   warps 8-11       dQ: tensor memory -> registers -> shared memory -> additions to global memory
+//   warps 8-11       dQ: tensor memory -> registers -> shared memory -> additions to global memory; dropout's keep bits
 //   warp 12          TMA: the first loads of all, then the ring of Q with the queries' lse and D;   warp 15: ring of dX
 //   warp 13          issues S and dV;   warp 14: issues dP, dQ and dK
 // Tensor memory columns, D = 128: S [0,128) | dP [128,256) | dV | dK; D = 64: S | dP | dV [256,320) | dK | dQ [384,448).
@@ -43,28 +43,30 @@ __device__ int g_bwd_fused_abort = 0;  // sticky: a bounded wait of the kernel r
 namespace {
 
 constexpr int kFuThreads = 512;
-constexpr int kPieceBytes = 4096;
 constexpr int kColBytes = 1024;        // per tile of queries: -lse (base 2) of 128 queries, then -D
 
-template <int D>
+template <int D, bool DROP>
 struct FuCfg {
+  // features of a piece of dQ on its way out (with dropout at D = 128 half as many, for the room of the keep bits)
+  static constexpr int kPieceFeat = DROP && D == 128 ? 16 : 32, kPieceBytes = 32 * kPieceFeat * 4;
   static constexpr int kTile = (D / 64) * kChunkBytes;     // 128 rows x D halves
   static constexpr int kFixOff = 0;                        // K, V
   static constexpr int kQOff = 2 * kTile;
   static constexpr int kXStages = D == 128 ? 1 : 2;        // with D = 128 there is no room for more
   static constexpr int kXOff = kQOff + 2 * kTile;          // dX
   static constexpr int kDsOff = kXOff + kXStages * kTile;  // dS^T: 128 keys x 128 queries, halves
-  static constexpr int kOutOff = kDsOff + 2 * kChunkBytes; // dQ on its way out: per warp two pieces of 32 queries x 32
-  static constexpr int kColOff = kOutOff + 8 * kPieceBytes;
+  static constexpr int kOutOff = kDsOff + 2 * kChunkBytes; // dQ on its way out: per warp two pieces of 32 queries
+  static constexpr int kKeepOff = kOutOff + 8 * kPieceBytes;   // keep bits of two steps: [step & 1][32 keys][query]
+  static constexpr int kColOff = kKeepOff + (DROP ? 4096 : 0);
   static constexpr int kBarOff = kColOff + 2 * kColBytes;
   static constexpr int kSmemBytes = kBarOff + 256;         // no slack: the kernel checks its 1 KB alignment
   static constexpr uint32_t kColS = 0, kColDP = 128, kColDV = 256, kColDK = 256 + D, kColDQ = D == 128 ? 128 : 384;
 };
-static_assert(FuCfg<128>::kSmemBytes <= 232448, "shared memory budget");
+static_assert(FuCfg<128, false>::kSmemBytes <= 232448 && FuCfg<128, true>::kSmemBytes <= 232448, "shared memory budget");
 
 struct FuBarriers {
   uint64_t k_full, v_full, q_full[2], q_empty[2], x_full[2], x_empty[2];
-  uint64_t s_full, p_ready, dp_full, dp_read, ds_ready, dq_full, dq_read, acc_full;
+  uint64_t keep_full[2], keep_free[2], s_full, p_ready, dp_full, dp_read, ds_ready, dq_full, dq_read, acc_full;
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -73,14 +75,26 @@ static_assert(sizeof(FuBarriers) <= 256, "barrier block");
 // floats of workspace per tile of 128 queries of a unit: the column values of all tiles come first, then dQ
 __host__ __device__ constexpr long long fused_tile_floats(int dpad) { return kColBytes / 4 + 128ll * dpad; }
 
+// all ones where the sign of byte k of w is set, and the same of two words in the halves of a word
+__device__ __forceinline__ unsigned int byte_sign(unsigned int w, int k) {
+  unsigned int m;
+  asm("prmt.b32 %0, %1, 0, %2;" : "=r"(m) : "r"(w), "r"(0x8888u + 0x1111u * k));
+  return m;
+}
+__device__ __forceinline__ unsigned int byte_sign_pair(unsigned int w0, unsigned int w1, int k) {
+  unsigned int m;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(m) : "r"(w0), "r"(w1), "r"(0xcc88u + 0x1111u * k));
+  return m;
+}
+
 // FEAT: 1 = Bool mask array, 2 = dropout, 4 = bias (as in attn_bwd_umma.cu)
 template <int D, bool BF16, int FEAT>
 __global__ void __launch_bounds__(kFuThreads, 1)
 attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                       const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_dx,
                       const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv, const AttnArgs a, const BwdArgs g, const int n_tiles, const int tail_units) {
-  using C = FuCfg<D>;
   constexpr bool MASKED = (FEAT & 1) != 0, DROP = (FEAT & 2) != 0, BIAS = (FEAT & 4) != 0;
+  using C = FuCfg<D, DROP>;
   extern __shared__ __align__(1024) uint8_t smem[];
   if ((smem_u32(smem) & 1023u) != 0) {
     // the swizzled tiles need 1 KB alignment and the budget leaves no room to round up: refuse cleanly
@@ -146,6 +160,8 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
       mbar_init(&bars->q_empty[s], 1);
       mbar_init(&bars->x_full[s], 1);
       mbar_init(&bars->x_empty[s], 2);   // dV and dP
+      mbar_init(&bars->keep_full[s], 4);
+      mbar_init(&bars->keep_free[s], 8);
     }
     mbar_init(&bars->s_full, 1);
     mbar_init(&bars->p_ready, 8);
@@ -316,7 +332,43 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
       // A warp's 32 queries x 32 features at a time, staged as [feature / 4][query][4] (the workspace's order, a warp's
       // queries together) and added by the copy engine.  Additions from registers keep the load / store queue busy
       // at the rate L2 takes them (22 bytes a cycle and SM), and everything else behind them in it waits.
-      uint8_t* out_s = smem + C::kOutOff + wq * 2 * kPieceBytes;
+      uint8_t* out_s = smem + C::kOutOff + wq * 2 * C::kPieceBytes;
+      // Which scores of the warp's 32 keys survived the forward's dropout, a word per query: drawn here, two steps ahead,
+      // because these warps have the time: d = 64, 2048 x 2048, 128 units 882 us with the compute warps drawing and trading
+      // by votes, 765 so; d = 80, 1000 x 777, padding 139 and 126.  Lane L draws the call of (query L % 8 of eight, keys
+      // 8 (L / 8) ..), and the bytes of a query's four calls are put together by exchanges.  Four calls in lockstep hide
+      // each other's latency; beside a bias, with its stores, two in turn are quicker (256 x 2048, 256 units 906 and 978).
+      auto draw_keep = [&](int it) {
+        const unsigned int j8 = (unsigned int)(t0 + wq * 32) / 8u + (unsigned int)(lane >> 3);
+        unsigned int* words = reinterpret_cast<unsigned int*>(smem + C::kKeepOff) + ((it & 1) * 4 + wq) * 128;
+        const unsigned long long row0 = score_row(a, tile_of(it) * 128 + (lane & 7), h, b);
+#pragma unroll 1
+        for (int q32 = 0; q32 < 4; ++q32) {
+          unsigned int word = 0u, w[4][4];
+          if (!BIAS) dropout_words4(a, row0 + (unsigned int)(q32 * 32), 8u, j8, 0u, w);
+#pragma unroll(BIAS ? 2 : 4)
+          for (int q8 = 0; q8 < 4; ++q8) {
+            unsigned int (&wq8)[4] = w[BIAS ? 0 : q8];
+            if (BIAS) dropout_words(a, row0 + (unsigned int)(q32 * 32 + q8 * 8), j8, wq8);
+            // bits 15 / 31 of a word's test belong to keys 2 e / 2 e + 1
+            unsigned int k = keep_lanes(a, wq8[0]) >> 15;
+            k |= keep_lanes(a, wq8[1]) >> 13;
+            k |= keep_lanes(a, wq8[2]) >> 11;
+            k |= keep_lanes(a, wq8[3]) >> 9;
+            unsigned int v = ((k & 0x55u) | ((k >> 15) & 0xaau)) << (8 * (lane >> 3));
+            v |= __shfl_xor_sync(0xffffffffu, v, 8);
+            v |= __shfl_xor_sync(0xffffffffu, v, 16);
+            if ((lane >> 3) == q8) word = v;
+          }
+          words[q32 * 32 + lane] = word;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->keep_full[it & 1]);
+      };
+      if (DROP) {
+        draw_keep(0);
+        if (n > 1) draw_keep(1);
+      }
       for (int it = 0; it < n; ++it) {
         ok = mbar_wait(&bars->dq_full, it & 1, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
@@ -337,24 +389,35 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
           uint32_t (&vc)[32] = v[c % kHeld];
-          uint8_t* piece = out_s + (c & 1) * kPieceBytes;
-          if (lane == 0) tma_store_wait_read<1>();          // the piece before the last has been read
-          __syncwarp();
+          constexpr int PF = C::kPieceFeat;
 #pragma unroll
-          for (int e = 0; e < 32; e += 4)
-            *reinterpret_cast<uint4*>(piece + (e >> 2) * 512 + lane * 16) = make_uint4(vc[e], vc[e + 1], vc[e + 2], vc[e + 3]);
-          if (kHeld < D / 32 && c == 0) {
+          for (int f = 0; f < 32; f += PF) {
+            uint8_t* piece = out_s + ((c * 32 + f) / PF & 1) * C::kPieceBytes;
+            if (lane == 0) tma_store_wait_read<1>();          // the piece before the last has been read
             __syncwarp();
-            tmem_ld32(tDQ + 32 * kHeld, v[0]);
-            tmem_wait_ld();
-            release();
+#pragma unroll
+            for (int e = 0; e < PF; e += 4)
+              *reinterpret_cast<uint4*>(piece + (e >> 2) * 512 + lane * 16) =
+                  make_uint4(vc[f + e], vc[f + e + 1], vc[f + e + 2], vc[f + e + 3]);
+            if (kHeld < D / 32 && c == 0 && f + PF == 32) {
+              __syncwarp();
+              tmem_ld32(tDQ + 32 * kHeld, v[0]);
+              tmem_wait_ld();
+              release();
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              bulk_add_f32(p + c * 1024 + f * 32, piece, C::kPieceBytes);
+              tma_store_commit();
+            }
           }
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            bulk_add_f32(p + c * 1024, piece, kPieceBytes);
-            tma_store_commit();
-          }
+        }
+        if (DROP && it + 2 < n) {
+          ok = mbar_wait(&bars->keep_free[it & 1], (it >> 1) & 1, abort_flag);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          draw_keep(it + 2);
         }
       }
       if (lane == 0) tma_store_wait_read<0>();
@@ -413,7 +476,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         const float* cols = col_s + st * (kColBytes / 4);
 
         // mask bytes of the warp's 32 keys x 64 queries, a word of 32 bits per query: the threads need those of their 16
-        // queries, shifted so that key 8 k + lane / 4 is bit 8 k.  Where a query's keys lie side by side a lane reads
+        // queries, shifted so that key 8 k + lane / 4 is the sign of byte k.  Where a query's keys lie side by side a lane reads
         // the 32 bytes of two queries and the words change hands; otherwise a query's keys are read by the 32 lanes
         // and voted into a word.
         unsigned int mv[16];
@@ -458,31 +521,23 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
             }
           }
 #pragma unroll
-          for (int k = 0; k < 16; ++k) mv[k] >>= lane >> 2;
+          for (int k = 0; k < 16; ++k) mv[k] <<= 7 - (lane >> 2);
         }
-        // survivors of the forward's dropout: lane L draws the call of (query L % 8 of block j, keys 8 (L / 8) ..) and
-        // the lanes trade by votes; vote e has bit 8 g + i for (query i, key 8 g + e), kept by the lanes of key e
-        // (shifted so that bit 8 g + e' is the thread's query e' of group g)
-        unsigned int kv[8];
+        // survivors of the forward's dropout, in the same form
+        unsigned int kw[16];
         if (DROP) {
-          const unsigned int j8 = (unsigned int)(t0 + wq * 32) / 8u + (unsigned int)(lane >> 3);
-#pragma unroll 2
+          ok = mbar_wait(&bars->keep_full[st], (it >> 1) & 1, abort_flag);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          const unsigned int* words = reinterpret_cast<const unsigned int*>(smem + C::kKeepOff) + (st * 4 + wq) * 128 + cb;
+#pragma unroll
           for (int j = 0; j < 8; ++j) {
-            unsigned int w[4];
-            dropout_words(a, score_row(a, c0 + half * 64 + 8 * j + (lane & 7), h, b), j8, w);
-            unsigned int vote = 0u;
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const unsigned int k = keep_lanes(a, w[e]);
-              const unsigned int v0 = __ballot_sync(0xffffffffu, (k & 0x8000u) != 0u);
-              const unsigned int v1 = __ballot_sync(0xffffffffu, (int)k < 0);
-              if ((lane >> 2) == 2 * e) vote = v0;
-              if ((lane >> 2) == 2 * e + 1) vote = v1;
-            }
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-              if (k == j) kv[k] = vote >> (2 * (lane & 3));
+            const uint2 w = *reinterpret_cast<const uint2*>(words + 8 * j);
+            kw[2 * j] = w.x << (7 - (lane >> 2));
+            kw[2 * j + 1] = w.y << (7 - (lane >> 2));
           }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->keep_free[st]);
         }
         // 16-bit bias: element pairs (one key, two queries) packed to a word
         unsigned int bw[2][16];
@@ -570,9 +625,9 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
             for (int j = 0; j < 8; ++j)
 #pragma unroll
               for (int e = 0; e < 2; ++e)
-                if (((mv[2 * j + e] >> (8 * k)) & 1u) == 0u) su[k >> 1][4 * j + 2 * (k & 1) + e] = 0u;
+                su[k >> 1][4 * j + 2 * (k & 1) + e] &= byte_sign(mv[2 * j + e], k);
         }
-        // P^T rounded to the element type over S: what dV takes (with dropout alpha' = P keep / (1 - p))
+        // P^T rounded to the element type over S: what dV takes, with dropout alpha' (1 - p) = P keep
         uint32_t pk[16];
         __syncwarp();
 #pragma unroll
@@ -581,12 +636,8 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
           for (int j = 0; j < 8; ++j)
 #pragma unroll
             for (int s = 0; s < 2; ++s) {
-              float p0 = __uint_as_float(su[hh][4 * j + 2 * s]), p1 = __uint_as_float(su[hh][4 * j + 2 * s + 1]);
-              if (DROP) {
-                p0 = ((kv[j] >> (8 * (2 * hh + s))) & 1u) ? p0 * a.inv_keep : 0.f;
-                p1 = ((kv[j] >> (8 * (2 * hh + s) + 1)) & 1u) ? p1 * a.inv_keep : 0.f;
-              }
-              pk[2 * j + s] = pack2<BF16>(p0, p1);
+              pk[2 * j + s] = pack2<BF16>(__uint_as_float(su[hh][4 * j + 2 * s]), __uint_as_float(su[hh][4 * j + 2 * s + 1]));
+              if (DROP) pk[2 * j + s] &= byte_sign_pair(kw[2 * j], kw[2 * j + 1], 2 * hh + s);
             }
           tmem_st_frag16(tS + (static_cast<uint32_t>(16 * hh) << 16), pk);
         }
@@ -595,8 +646,8 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->p_ready);
 
-        // dS = P (dP - D), rounded to the element type: over dP and, transposed for dQ, in shared memory, once the
-        // previous step's dQ product has read it
+        // dS = P (dP - D), rounded to the element type, in shared memory, once the previous step's products have read it;
+        // with dropout dS (1 - p) = P (dP keep - D (1 - p)): the pre-kernel's D has that factor, dq and dk get it back
         ok = mbar_wait(&bars->dp_full, st, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
@@ -625,11 +676,11 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
 #pragma unroll
               for (int s = 0; s < 2; ++s) {
                 const int e0 = 4 * (j + jj) + 2 * s;
-                float g0 = __uint_as_float(dp[hh][e0]), g1 = __uint_as_float(dp[hh][e0 + 1]);
                 if (DROP) {
-                  g0 = ((kv[j + jj] >> (8 * (2 * hh + s))) & 1u) ? g0 * a.inv_keep : 0.f;
-                  g1 = ((kv[j + jj] >> (8 * (2 * hh + s) + 1)) & 1u) ? g1 * a.inv_keep : 0.f;
+                  dp[hh][e0] &= byte_sign(kw[2 * (j + jj)], 2 * hh + s);
+                  dp[hh][e0 + 1] &= byte_sign(kw[2 * (j + jj) + 1], 2 * hh + s);
                 }
+                const float g0 = __uint_as_float(dp[hh][e0]), g1 = __uint_as_float(dp[hh][e0 + 1]);
                 float d0, d1;
                 pair_unpack(pair_mul(pair_add(pair_pack(g0, g1), ndp),
                                      pair_pack(__uint_as_float(su[hh][e0]), __uint_as_float(su[hh][e0 + 1]))), d0, d1);
@@ -662,7 +713,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
               for (int e = 0; e < 2; ++e) {
                 const int col = c0 + cb + 8 * j + e;
                 if (col >= a.Lq) continue;
-                const float v = __uint_as_float(su[k >> 1][4 * j + 2 * (k & 1) + e]);
+                const float v = __uint_as_float(su[k >> 1][4 * j + 2 * (k & 1) + e]) * (DROP ? a.inv_keep : 1.f);
                 float* oc = o + (long long)col * g.dbias_s[1];
                 if (dbias_exclusive) *oc = v; else atomicAdd(oc, v);
               }
@@ -682,7 +733,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         // out keys past the end and padding; stored from here, 16 bytes a row and thread, they took 3 us
         const int r = wq * 32 + lane;
         uint8_t* stage = smem + C::kFixOff + (half == 0 ? C::kTile : 0);
-        const float mul = half == 0 ? 1.f : a.scale;
+        const float mul = (half == 0 ? 1.f : a.scale) * (DROP ? a.inv_keep : 1.f);
         const uint32_t col = lane_base + (half == 0 ? C::kColDV : C::kColDK);
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
@@ -771,7 +822,7 @@ __global__ void __launch_bounds__(256) attn_bwd_fused_pre_kernel(const AttnArgs 
         const float l = __ldg(a.lse + (long long)a.Lq * h + a.lse_sb * b + q);
         if (l != neg_inf()) {
           nl = -(l * kLog2e);
-          nd = -acc;
+          nd = -acc * (1.f / a.inv_keep);           // (no dropout: 1)
         }
       }
       cols[r] = nl;
@@ -788,6 +839,7 @@ __global__ void __launch_bounds__(256) attn_bwd_fused_post_kernel(const AttnArgs
   const long long tiles_all = gridDim.x;
   const int r = threadIdx.x & 127, q = t * 128 + r;
   if (q >= a.Lq) return;
+  const float mul = a.scale * a.inv_keep;        // (no dropout: 1)
   const float4* w = reinterpret_cast<const float4*>(a.ws + tiles_all * (kColBytes / 4) + tile * (128 * DPAD)) + (r >> 5) * (8 * DPAD) + (r & 31);
   uint8_t* out = reinterpret_cast<uint8_t*>(g.dq) +
                  2ll * (((long long)q + (long long)a.Lq * b) * ((long long)a.H * a.d) + (long long)h * a.d);
@@ -802,10 +854,10 @@ __global__ void __launch_bounds__(256) attn_bwd_fused_post_kernel(const AttnArgs
     for (int u = 0; u < 2; ++u) {
       if (f + 8 * u >= a.d) break;
       uint4 o;
-      o.x = pack2<BF16>(v[2 * u].x * a.scale, v[2 * u].y * a.scale);
-      o.y = pack2<BF16>(v[2 * u].z * a.scale, v[2 * u].w * a.scale);
-      o.z = pack2<BF16>(v[2 * u + 1].x * a.scale, v[2 * u + 1].y * a.scale);
-      o.w = pack2<BF16>(v[2 * u + 1].z * a.scale, v[2 * u + 1].w * a.scale);
+      o.x = pack2<BF16>(v[2 * u].x * mul, v[2 * u].y * mul);
+      o.y = pack2<BF16>(v[2 * u].z * mul, v[2 * u].w * mul);
+      o.z = pack2<BF16>(v[2 * u + 1].x * mul, v[2 * u + 1].y * mul);
+      o.w = pack2<BF16>(v[2 * u + 1].z * mul, v[2 * u + 1].w * mul);
       *reinterpret_cast<uint4*>(out + (f + 8 * u) * 2) = o;
     }
   }
@@ -815,7 +867,7 @@ template <int D, bool BF16, int FEAT>
 cudaError_t launch_fused(const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mq, const CUtensorMap& mdx,
                          const CUtensorMap& mdk, const CUtensorMap& mdv, const AttnArgs& a, const BwdArgs& g, cudaStream_t st) {
   auto kern = attn_bwd_fused_kernel<D, BF16, FEAT>;
-  constexpr int smem = FuCfg<D>::kSmemBytes;
+  constexpr int smem = FuCfg<D, (FEAT & 2) != 0>::kSmemBytes;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   const int n_tiles = (a.Lkv + 127) / 128, n_q = (a.Lq + 127) / 128;
