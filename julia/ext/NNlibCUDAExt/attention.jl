@@ -429,7 +429,13 @@ function ChainRulesCore.rrule(::typeof(dot_product_attention), q::DenseCuArray{T
         # one pass over the scores where the library asks for a workspace (dq is then summed by atomic additions)
         need = ccall((:nnlib_b200_attn_bwd_workspace_bytes, libnnlib_b200[]), Csize_t,
                      (Ref{B200AttnParams}, Ref{B200AttnGrads}), p, g)
-        scratch = CuArray{Float32}(undef, need > 0 ? cld(Int(need), 4) : p.Lq * p.H * p.B)
+        scratch = try
+            CuArray{Float32}(undef, need > 0 ? cld(Int(need), 4) : p.Lq * p.H * p.B)
+        catch err
+            (need > 0 && err isa CUDA.OutOfGPUMemoryError) || rethrow()
+            need = Csize_t(0)                # the other one gets by with D
+            CuArray{Float32}(undef, p.Lq * p.H * p.B)
+        end
         g = _with(g; delta=pointer(scratch))
         GC.@preserve q k v x α dx dq dk dv scratch dbias32 bias mask begin
             rc = need > 0 ?

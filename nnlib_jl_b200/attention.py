@@ -611,7 +611,14 @@ def dot_product_attention_pullback(q, k, v, bias=None, *, fdrop: Callable = iden
         # algorithms gets the one that needs no workspace and adds in a fixed order
         need = 0 if torch.are_deterministic_algorithms_enabled() else \
             lib.nnlib_b200_attn_bwd_workspace_bytes(C.byref(pr.p), C.byref(g))
-        scratch = torch.empty(need or 4 * pr.Lq * pr.H * pr.B, dtype=torch.uint8, device=pr.dev)
+        scratch = None
+        if need:
+            try:
+                scratch = torch.empty(need, dtype=torch.uint8, device=pr.dev)
+            except torch.OutOfMemoryError:
+                need = 0                     # the other one gets by with D
+        if scratch is None:
+            scratch = torch.empty(4 * pr.Lq * pr.H * pr.B, dtype=torch.uint8, device=pr.dev)
         g.delta = scratch.data_ptr()
         back.path = lib.nnlib_b200_attn_bwd_path(C.byref(pr.p), C.byref(g))   # PATH_UMMA / PATH_SIMT, for tests
         with _on_device(pr.dev):

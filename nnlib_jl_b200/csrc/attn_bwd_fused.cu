@@ -26,8 +26,9 @@
 // Added from registers instead (red.v4.f32) they go at the same rate but keep the load / store queue, and the compute
 // warps' tensor memory stores behind them in it, waiting: 5600 a step.  Polynomials in place of a quarter to half of
 // the exponentials shorten that phase (1345 -> 1080) and nothing else.  One backward (pre and post included) went
-// 4140 -> 3060 us there, 3560 -> 2570 for one sequence of 16384 and 16 heads, 470 -> 341 for 16 heads of d = 64,
-// L = 2048, 8 sequences, 1604 -> 900 for the same not causal with dropout.
+// 4140 -> 2940 us there, 3560 -> 2670 for one sequence of 16384 and 16 heads, 473 -> 325 for 16 heads of d = 64,
+// L = 2048, 8 sequences, 1604 -> 769 for the same not causal with dropout.  Of a CTA's 46 us there 2.3 pass before its
+// first scores and 3.9 behind its last dS.
 #include <cuda.h>
 
 #include "common.cuh"

@@ -90,6 +90,24 @@ def _grads(**kw):
     return g
 
 
+def test_backward_workspace_query_without_a_gpu(lib):
+    """Float32: the one-pass form is chosen by the number of tiles alone, so the query can be asked here."""
+    def need(H=64, L=512, Lq=None, **kw):
+        g = _grads(delta=None, **{k: kw.pop(k) for k in ("dbias",) if k in kw})     # delta is not used with a workspace
+        p = _params(lse=0x2000, dtype=_lib.F32, H=H, Lq=Lq or L, Lkv=L, **kw)
+        return lib.nnlib_b200_attn_bwd_workspace_bytes(C.byref(p), C.byref(g))
+    # D and a partial dq of 64 x 64 floats per tile; the keys fill the GPU, so no parts of dk and dv
+    assert need() == 4 * (64 * 512 + 64 * 8 * 8 * 64 * 64)
+    # two tiles of keys of four units: the 32 tiles of queries are dealt to as many blocks, each with a part of dk and dv
+    assert need(H=4, L=128, Lq=2000) == 4 * (4 * 2000 + 4 * 32 * 2 * 64 * 64 + 4 * 2 * 32 * 64 * 128)
+    assert need(H=2, L=16) == 0                                          # five products in a row, and a launch: not four
+    assert need(dbias=0x4000, bias=0x5000, bias_dtype=_lib.F32) == 0      # the half that owns queries adds to dbias
+    assert need(L=16384) == 0                                            # more than 1 GiB of parts
+    assert need(d=200, dv=200) == 0 and need(B=0) == 0
+    assert lib.nnlib_b200_attn_bwd_workspace_bytes(None, C.byref(_grads())) == 0
+    assert lib.nnlib_b200_attn_bwd_ws(C.byref(_params()), C.byref(_grads()), None, 0, None) == _lib.INVALID_ARG
+
+
 def test_backward_argument_checks_and_path_without_a_gpu(lib):
     p = _params(lse=0x2000)
     # the forward's lse is required, so are dx / dq / dk / dv / delta, and the struct size is checked
