@@ -14,7 +14,7 @@
 //   warp 2      allocates / frees the 512 TMEM columns
 //   warps 4-7   softmax of query tile 0 (thread r owns query row r: no shuffles)
 //   warps 8-11  softmax of query tile 1
-//   warps 12-15 with dropout and a mask array or bias: the random numbers, as keep bits in shared memory up to two rounds ahead
+//   warps 12-15 with dropout and side inputs (rng_warps): the random numbers, as keep bits in shared memory up to two rounds ahead
 //
 // TMEM columns: S_0 [0,128) S_1 [128,256) O_0 [256,384) O_1 [384,512); the
 // half-precision probabilities P_t overwrite the first 64 columns of S_t.
@@ -95,19 +95,19 @@ static_assert(sizeof(Barriers) <= 512, "barrier block");
 // the tensor map can address (the host decides).
 // SHIFT: bias / mask rows of any alignment (extras.cuh); without it they are all aligned and whole.
 //
-// Random numbers: sixteen calls of Philox a thread and round.  Where the softmax warps have side inputs to work in, the
-// numbers come from four warps of their own; without side inputs the softmax warps wait for their scores anyway and draw
-// them meanwhile.  f16, bias, d = 64, 256 x 2048, 256 units 210 -> 190 us; padding, d = 80, 1000 x 777, 48 units 105 -> 97;
-// window mask and bias, d = 64, 1024 x 1024, 32 units 66 -> 63; without side inputs, d = 64, 2048 x 2048, 128 units 444
-// and, with the four warps, 530.
-__host__ __device__ constexpr bool rng_warps(int xm, bool stats) { return xm > 3 && !stats; }
+// Random numbers: sixteen calls of Philox a thread and round.  Where the softmax warps have a bias to work in, or a mask
+// array in the longer rounds of D = 128, the numbers come from four warps of their own; otherwise the softmax warps wait
+// for their scores anyway and draw them meanwhile.  f16, bias, d = 64, 256 x 2048, 256 units 209 -> 191 us; window mask and
+// bias, d = 64, 1024 x 1024, 32 units 66 -> 63; padding, d = 80, 1000 x 777, 48 units 105 -> 97, but d = 64, 256 x 2048, 128
+// units 90.7 and, with the four warps, 92.6; without side inputs, d = 64, 2048 x 2048, 128 units 444 and 530.
+__host__ __device__ constexpr bool rng_warps(int d, int xm, bool stats) { return (xm == 5 || (xm == 4 && d == 128)) && !stats; }
 template <int D, bool BF16, int XM, bool STATS, bool BSM, bool SHIFT>
-__global__ void __launch_bounds__(rng_warps(XM, STATS) ? kRngThreads : kThreads, 1)
+__global__ void __launch_bounds__(rng_warps(D, XM, STATS) ? kRngThreads : kThreads, 1)
 attn_fwd_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_b,
                      const AttnArgs a, const int n_qblocks, const int tail_units) {
   constexpr bool DROP = XM >= 3 && !STATS;   // dropout code compiled in
-  constexpr bool RNG = rng_warps(XM, STATS);
+  constexpr bool RNG = rng_warps(D, XM, STATS);
   using C = Cfg<D, RNG>;
   constexpr bool EXTRAS = (XM % 3) != 0;
   constexpr bool XBIAS = (XM % 3) == 2;   // bias code compiled in
@@ -1133,7 +1133,7 @@ template <int D, bool BF16, int XM, bool STATS, bool BSM, bool SHIFT>
 cudaError_t launch_fwd_impl(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mb,
                             const AttnArgs& a, cudaStream_t st) {
   auto kern = attn_fwd_umma_kernel<D, BF16, XM, STATS, BSM, SHIFT>;
-  constexpr bool RNG = rng_warps(XM, STATS);
+  constexpr bool RNG = rng_warps(D, XM, STATS);
   constexpr int smem = BSM ? Cfg<D, RNG>::kSmemBytesStaged : Cfg<D, RNG>::kSmemBytes;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
