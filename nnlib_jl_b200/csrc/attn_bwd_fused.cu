@@ -130,7 +130,17 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
   // query tiles: the causal walk goes from the key tile's own to the last; otherwise the CTAs of a unit start at
   // different ones, so that they do not all add to the same tile of dQ at once
   const int n_q = (a.Lq + 127) / 128;
-  const int r0 = tix % n_q;             // causal: Lq = Lkv, so tix itself
+  if (a.causal && tix >= n_q) {         // keys behind the last query: no query sees them, dk = dv = 0
+    const int pieces = a.d / 8, rows = min(128, a.Lkv - t0);
+    for (int i = threadIdx.x; i < rows * pieces; i += kFuThreads) {
+      const long long o = ((long long)(t0 + i / pieces) + (long long)a.Lkv * b) * ((long long)a.H * a.d) + (long long)h * a.d +
+                          (i % pieces) * 8;
+      *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(g.dk) + 2 * o) = make_uint4(0u, 0u, 0u, 0u);
+      *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(g.dv) + 2 * o) = make_uint4(0u, 0u, 0u, 0u);
+    }
+    return;
+  }
+  const int r0 = tix % n_q;             // (causal: tix itself)
   const int n = a.causal ? n_q - r0 : n_q;
   auto tile_of = [&](int it) { const int t = r0 + it; return t < n_q ? t : t - n_q; };
   const long long tiles_all = (long long)n_q * a.H * a.B;

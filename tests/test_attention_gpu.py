@@ -1633,6 +1633,91 @@ def test_abi_backward_causal_flag_on_a_head_slice(Lq, Lkv):
     np.testing.assert_allclose(delta.cpu().numpy(), want_delta, rtol=1e-3, atol=1e-3)
 
 
+@pytest.mark.parametrize("Lq,Lkv,B,drop,pad", [
+    (100, 300, 2, 0.0, 0),      # two tiles of keys behind the only tile of queries
+    (100, 300, 1, 0.2, 24),     # the same with dropout; lse of the shard inside a larger array, padded dx
+    (515, 130, 4, 0.0, 8),      # more queries than keys
+    (260, 700, 1, 0.0, 0),      # six tiles of keys, three of queries
+])
+def test_abi_one_pass_backward_on_a_head_slice(Lq, Lkv, B, drop, pad):
+    """The causal flag with kv_len != q_len on heads 1..2 of 4 (pointer offsets, the parent's strides, lse with a batch
+    stride of its own, dx with padded rows) through the one-pass backward: keys past the last query get zero gradient."""
+    lib = _lib.load()
+    rng = np.random.default_rng(64)
+    dtype, H, d, h0, Hs = torch.float16, 4, 72, 1, 2
+    E, Ed = H * d, H * d + pad
+    qn, kn, vn, dyn = (_round_to(rng.standard_normal((E, n, B)), dtype) for n in (Lq, Lkv, Lkv, Lq))
+    q, k, v = _dev(qn, dtype), _dev(kn, dtype), _dev(vn, dtype)
+    dx = nb.jl_zeros((Ed, Lq, B), dtype, DEV)
+    dx[:E] = _dev(dyn, dtype)
+    x = nb.jl_zeros((E, Lq, B), dtype, DEV)
+    lse = torch.empty((B, H, Lq), dtype=torch.float32, device=DEV)
+    dq, dk, dv = (nb.jl_zeros((Hs * d, n, B), dtype, DEV) for n in (Lq, Lkv, Lkv))
+    for t in (dq, dk, dv):
+        t.fill_(7)                                   # every element is to be written
+    p = _lib.AttnParams()
+    p.dtype = _lib.F16
+    p.d, p.dv, p.H, p.Lq, p.Lkv, p.B = d, d, Hs, Lq, Lkv, B
+    off = h0 * d * 2
+    p.q, p.k, p.v, p.x = q.data_ptr() + off, k.data_ptr() + off, v.data_ptr() + off, x.data_ptr() + off
+    p.q_stride_l = p.k_stride_l = p.v_stride_l = p.x_stride_l = E
+    p.q_stride_b, p.x_stride_b = E * Lq, E * Lq
+    p.k_stride_b = p.v_stride_b = E * Lkv
+    p.lse, p.lse_stride_b = lse.data_ptr() + 4 * h0 * Lq, H * Lq
+    p.causal = 1
+    p.dropout_p, p.philox_seed = drop, 3
+    p.rng_h0, p.rng_H = h0, H
+    g = _lib.AttnGrads()
+    g.dx = dx.data_ptr() + off
+    g.dx_stride_l, g.dx_stride_b = Ed, Ed * Lq
+    g.dq, g.dk, g.dv = dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
+    st = torch.cuda.current_stream().cuda_stream
+    assert lib.nnlib_b200_attn_fwd(ctypes.byref(p), st) == 0
+    need = lib.nnlib_b200_attn_bwd_workspace_bytes(ctypes.byref(p), ctypes.byref(g))
+    assert need > 0
+    ws = torch.empty(need, dtype=torch.uint8, device=DEV)
+    assert lib.nnlib_b200_attn_bwd_ws(ctypes.byref(p), ctypes.byref(g), ws.data_ptr(), need, st) == 0
+    nb.device_health()
+    mask_np = np.arange(Lkv)[:, None] <= np.arange(Lq)[None, :]
+    sl = slice(h0 * d, (h0 + Hs) * d)
+    keep = P.keep_mask((Lkv, Lq, H, B), drop, 3, 0)[:, :, h0:h0 + Hs] if drop > 0 else None
+    want = O.dot_product_attention_grad(qn[sl], kn[sl], vn[sl], dyn[sl], None, mask=mask_np, nheads=Hs, keep=keep, p=drop)
+    for name, got, w in zip(("dq", "dk", "dv"), (dq, dk, dv), want):
+        _grad_close(nb.jl_to_numpy(got), w, dtype, name)
+    assert (nb.jl_to_numpy(dk)[:, Lq:] == 0).all() and (nb.jl_to_numpy(dv)[:, Lq:] == 0).all()
+
+
+@pytest.mark.parametrize("Lq,Lkv", [(96, 640), (100, 200), (300, 150)])
+@pytest.mark.parametrize("dtype,d,bias,drop", [
+    (torch.bfloat16, 128, None, 0.0), (torch.float16, 64, None, 0.2), (torch.bfloat16, 64, "full", 0.0), (torch.float16, 128, "heads", 0.1),
+])
+def test_pullback_causal_with_other_lengths(Lq, Lkv, dtype, d, bias, drop):
+    """``CausalMask()`` (key j is seen by the queries from j on) where keys and queries differ in number, both 16-bit
+    backwards: keys behind the last query take no part, in the gradient of the bias neither."""
+    rng = np.random.default_rng(65 + Lq)
+    H, B = 2, 2
+    qn, kn, vn, dyn = (_round_to(rng.standard_normal((d * H, n, B)), dtype) for n in (Lq, Lkv, Lkv, Lq))
+    bn = None if bias is None else _round_to(0.5 * rng.standard_normal((Lkv, Lq, H, B) if bias == "full" else (Lkv, Lq, H)), dtype)
+    mask_np = np.arange(Lkv)[:, None] <= np.arange(Lq)[None, :]
+    fd = nb.PhiloxDropout(drop, seed=5, offset=1) if drop > 0 else nb.identity
+    keep = P.keep_mask((Lkv, Lq, H, B), drop, 5, 1) if drop > 0 else None
+    x, _, back = nb.dot_product_attention_pullback(_dev(qn, dtype), _dev(kn, dtype), _dev(vn, dtype),
+                                                   None if bn is None else _dev(bn, dtype), mask=nb.CausalMask(), nheads=H, fdrop=fd)
+    want = O.dot_product_attention_grad(qn, kn, vn, dyn, bn, mask=mask_np, nheads=H, keep=keep, p=drop)
+    dy = _dev(dyn, dtype)
+    for deterministic in (False, True):
+        torch.use_deterministic_algorithms(deterministic, warn_only=True)
+        try:
+            got = back(dy)
+        finally:
+            torch.use_deterministic_algorithms(False)
+        nb.device_health()
+        for name, g, w in zip(("dq", "dk", "dv", "dbias"), got, want):
+            if g is not None:
+                _grad_close(nb.jl_to_numpy(g), w, dtype, f"{name}, deterministic={deterministic}")
+        assert not bool(got[1][:, Lq:].any()) and not bool(got[2][:, Lq:].any())
+
+
 @pytest.mark.parametrize("dtype,E,H,Lq,Lkv,B", [(torch.bfloat16, 256, 2, 200, 264, 2), (torch.float16, 128, 2, 129, 520, 1)])
 def test_opaque_fdrop_on_tensor_cores(dtype, E, H, Lq, Lkv, B):
     """fdrop is an arbitrary callable: stats -> scores -> fdrop -> x = V·α′ (src/attention.jl:91-98), with the
