@@ -638,7 +638,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
               for (int e = 0; e < 2; ++e)
                 su[k >> 1][4 * j + 2 * (k & 1) + e] &= byte_sign(mv[2 * j + e], k);
         }
-        // P^T rounded to the element type over S: what dV takes, with dropout alpha' (1 - p) = P keep
+        // P^T rounded to the element type over S: what dV takes, with dropout alpha' = P keep / (1 - p)
         uint32_t pk[16];
         __syncwarp();
 #pragma unroll
@@ -647,7 +647,9 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
           for (int j = 0; j < 8; ++j)
 #pragma unroll
             for (int s = 0; s < 2; ++s) {
-              pk[2 * j + s] = pack2<BF16>(__uint_as_float(su[hh][4 * j + 2 * s]), __uint_as_float(su[hh][4 * j + 2 * s + 1]));
+              float p0 = __uint_as_float(su[hh][4 * j + 2 * s]), p1 = __uint_as_float(su[hh][4 * j + 2 * s + 1]);
+              if (DROP) pair_unpack(pair_mul(pair_pack(p0, p1), pair_of(a.inv_keep)), p0, p1);
+              pk[2 * j + s] = pack2<BF16>(p0, p1);
               if (DROP) pk[2 * j + s] &= byte_sign_pair(kw[2 * j], kw[2 * j + 1], 2 * hh + s);
             }
           tmem_st_frag16(tS + (static_cast<uint32_t>(16 * hh) << 16), pk);
@@ -657,8 +659,9 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->p_ready);
 
-        // dS = P (dP - D), rounded to the element type, in shared memory, once the previous step's products have read it;
-        // with dropout dS (1 - p) = P (dP keep - D (1 - p)): the pre-kernel's D has that factor, dq and dk get it back
+        // dS = P (dP - D), with dropout P (dP keep / (1 - p) - D), rounded to the element type, in shared memory, once the
+        // previous step's products have read it.  (1 / (1 - p) belongs in front of the roundings: left to the results, dS of
+        // a p near 1 falls among Float16's subnormal numbers.)
         ok = mbar_wait(&bars->dp_full, st, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
@@ -693,7 +696,8 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                 }
                 const float g0 = __uint_as_float(dp[hh][e0]), g1 = __uint_as_float(dp[hh][e0 + 1]);
                 float d0, d1;
-                pair_unpack(pair_mul(pair_add(pair_pack(g0, g1), ndp),
+                const unsigned long long gp = pair_pack(g0, g1);
+                pair_unpack(pair_mul(DROP ? pair_fma(gp, pair_of(a.inv_keep), ndp) : pair_add(gp, ndp),
                                      pair_pack(__uint_as_float(su[hh][e0]), __uint_as_float(su[hh][e0 + 1]))), d0, d1);
                 pk4[2 * jj + s] = pack2<BF16>(d0, d1);
                 if (BIAS) {
@@ -724,7 +728,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
               for (int e = 0; e < 2; ++e) {
                 const int col = c0 + cb + 8 * j + e;
                 if (col >= a.Lq) continue;
-                const float v = __uint_as_float(su[k >> 1][4 * j + 2 * (k & 1) + e]) * (DROP ? a.inv_keep : 1.f);
+                const float v = __uint_as_float(su[k >> 1][4 * j + 2 * (k & 1) + e]);
                 float* oc = o + (long long)col * g.dbias_s[1];
                 if (dbias_exclusive) *oc = v; else atomicAdd(oc, v);
               }
@@ -744,7 +748,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         // out keys past the end and padding; stored from here, 16 bytes a row and thread, they took 3 us
         const int r = wq * 32 + lane;
         uint8_t* stage = smem + C::kFixOff + (half == 0 ? C::kTile : 0);
-        const float mul = (half == 0 ? 1.f : a.scale) * (DROP ? a.inv_keep : 1.f);
+        const float mul = half == 0 ? 1.f : a.scale;
         const uint32_t col = lane_base + (half == 0 ? C::kColDV : C::kColDK);
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
@@ -833,7 +837,7 @@ __global__ void __launch_bounds__(256) attn_bwd_fused_pre_kernel(const AttnArgs 
         const float l = __ldg(a.lse + (long long)a.Lq * h + a.lse_sb * b + q);
         if (l != neg_inf()) {
           nl = -(l * kLog2e);
-          nd = -acc * (1.f / a.inv_keep);           // (no dropout: 1)
+          nd = -acc;
         }
       }
       cols[r] = nl;
@@ -850,7 +854,7 @@ __global__ void __launch_bounds__(256) attn_bwd_fused_post_kernel(const AttnArgs
   const long long tiles_all = gridDim.x;
   const int r = threadIdx.x & 127, q = t * 128 + r;
   if (q >= a.Lq) return;
-  const float mul = a.scale * a.inv_keep;        // (no dropout: 1)
+  const float mul = a.scale;
   const float4* w = reinterpret_cast<const float4*>(a.ws + tiles_all * (kColBytes / 4) + tile * (128 * DPAD)) + (r >> 5) * (8 * DPAD) + (r & 31);
   uint8_t* out = reinterpret_cast<uint8_t*>(g.dq) +
                  2ll * (((long long)q + (long long)a.Lq * b) * ((long long)a.H * a.d) + (long long)h * a.d);

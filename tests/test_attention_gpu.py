@@ -1551,6 +1551,37 @@ def test_both_tensor_core_backwards_match_the_gradient_oracle(dtype, d, H, Lq, L
         assert not deterministic or all(torch.equal(a, b) for a, b in zip(got[:3], again[:3]))
 
 
+@pytest.mark.parametrize("d", [64, 128])
+def test_dropout_of_most_scores_keeps_small_float16_gradients(d):
+    """dS = P (dP keep / (1 - p) - D) of both 16-bit backwards with p = 15/16 and dS of 2^-24 to 2^-18, among Float16's
+    subnormal numbers: each is off by half of 2^-24 at most, and so are the results."""
+    rng = np.random.default_rng(66)
+    dtype, H, Lq, Lkv, B, p = torch.float16, 2, 32, 64, 8, 15 / 16
+    qn, kn = (_round_to(0.25 * rng.standard_normal((d * H, n, B)), dtype) for n in (Lq, Lkv))
+    vn = _round_to(2.0 ** -10 * rng.standard_normal((d * H, Lkv, B)), dtype)
+    dyn = _round_to(2.0 ** -10 * rng.standard_normal((d * H, Lq, B)), dtype)
+    keep = P.keep_mask((Lkv, Lq, H, B), p, 5, 2)
+    x, _, back = nb.dot_product_attention_pullback(_dev(qn, dtype), _dev(kn, dtype), _dev(vn, dtype), nheads=H,
+                                                   fdrop=nb.PhiloxDropout(p, seed=5, offset=2))
+    gq, gk, _, _ = O.dot_product_attention_grad(qn, kn, vn, dyn, None, nheads=H, keep=keep, p=p)
+    scale, half = 1 / math.sqrt(d), 2.0 ** -25
+    # sums of |k| (|q|) over the keys (queries) times the rounding of dS, the result's own rounding, and 1 % of the
+    # result for what comes from x, which is rounded too
+    tol_q = scale * half * np.abs(kn).sum(1, keepdims=True) + half
+    tol_k = scale * half * np.abs(qn).sum(1, keepdims=True) + half
+    dy = _dev(dyn, dtype)
+    for deterministic in (False, True):
+        torch.use_deterministic_algorithms(deterministic, warn_only=True)
+        try:
+            dq, dk, _, _ = back(dy)
+        finally:
+            torch.use_deterministic_algorithms(False)
+        nb.device_health()
+        for name, g, w, tol in (("dq", dq, gq, tol_q), ("dk", dk, gk, tol_k)):
+            off = np.abs(nb.jl_to_numpy(g).astype(np.float64) - w)
+            assert (off <= tol + 0.01 * np.abs(w)).all(), (name, deterministic, float((off / tol).max()))
+
+
 def test_pullback_fully_masked_query_gives_no_gradient():
     """A query that attends to nothing has NaN output (src/softmax.jl:71-76); the library lets no gradient
     flow through it (both backward paths), so the other queries' gradients stay finite."""
