@@ -521,10 +521,13 @@ __global__ void __launch_bounds__(NT) softmax_strided_kernel(typename Ptrs<T, NA
 // arrive in shared memory (cp.async; a thread reads back only the packets that it copied itself, so its own wait is all
 // that is needed, and refills their place at once), and blocks of G threads, 1024 / G on an SM, are in different phases:
 // 107 us = 4.9 TB/s there (one block of 1024 threads, two columns arriving: 127), softmax 163 -> 110; 50000 BFloat16 x
-// 2000 178 -> 96, 10000 Float32 x 4096 116 -> 64.
-// What a thread does with its at most KP packets, and so the result, is softmax_cols_kernel's.
+// 2000 195 -> 112, softmax 211 -> 126 (113 with the exponentials kept as 16-bit values, see ONCE), 10000 Float32 x 4096 116 -> 64.
+// The statistics are softmax_cols_kernel's with their sums in another order, so a column's last bit may depend on whether
+// there are enough of them for this kernel.  ONCE: the 16-bit x stays in the registers and its exponentials are taken
+// again for the result, which is rounded once; without it they are kept there as 16-bit values, as in the other kernel
+// for columns of the same length (up to 4096 packets).
 constexpr int kRingSmem = 226 * 1024;
-template <typename T, int MODE, int G, int KP, int S>
+template <typename T, int MODE, int G, int KP, int S, bool ONCE>
 __global__ void __launch_bounds__(G, 1024 / G) softmax_ring_kernel(const T* __restrict__ x, T* __restrict__ out, long long n,
                                                                    long long cols) {
   constexpr int V = Pack<T>::V;
@@ -598,7 +601,7 @@ __global__ void __launch_bounds__(G, 1024 / G) softmax_ring_kernel(const T* __re
             f[u] = __expf(f[u] - c.m);
             part += f[u];
           }
-          if (MODE == SM_FWD) cx[k] = repack<T>(f);
+          if (MODE == SM_FWD && !ONCE) cx[k] = repack<T>(f);
         } else {
 #pragma unroll
           for (int u = 0; u < V; ++u) part += (f[u] == f_inf()) ? 1.f : 0.f;
@@ -619,7 +622,7 @@ __global__ void __launch_bounds__(G, 1024 / G) softmax_ring_kernel(const T* __re
           fwd_pack<MODE, V>(c, inv_s, log_s, f);
         } else {
 #pragma unroll
-          for (int u = 0; u < V; ++u) f[u] = MODE == SM_FWD ? f[u] * inv_s : f[u] - c.m - log_s;
+          for (int u = 0; u < V; ++u) f[u] = MODE == SM_FWD ? (ONCE ? __expf(f[u] - c.m) : f[u]) * inv_s : f[u] - c.m - log_s;
         }
         store_pack<T>(out + col * n + (long long)jp * V, f);
       }
@@ -627,9 +630,9 @@ __global__ void __launch_bounds__(G, 1024 / G) softmax_ring_kernel(const T* __re
   }
 }
 
-template <typename T, int MODE, int G, int KP, int S>
+template <typename T, int MODE, int G, int KP, int S, bool ONCE>
 cudaError_t launch_ring(const T* x, T* out, long long n, long long cols, cudaStream_t st) {
-  auto kern = softmax_ring_kernel<T, MODE, G, KP, S>;
+  auto kern = softmax_ring_kernel<T, MODE, G, KP, S, ONCE>;
   constexpr int per_sm = 1024 / G;
   const int smem = (int)(n * sizeof(T)) * S;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRingSmem / per_sm);
@@ -667,8 +670,9 @@ cudaError_t launch_softmax(const void* x, const void* dy, void* out, long long i
     // BFloat16 x 4096 52 us, and 60 with the next column arriving.  In-place calls keep the other kernel, too.
     if constexpr (FWD) {
       if (vect && no_alias && outer >= 4 * 148) {
-        if (np > 256ll * 8 && np <= 512ll * 8) return launch_ring<T, MODE, 512, 8, 1>(xp, op, n, outer, st);
-        if (np > 512ll * 8 && np <= 1024ll * 7) return launch_ring<T, MODE, 1024, 7, 2>(xp, op, n, outer, st);
+        if (np > 256ll * 8 && np <= 512ll * 8) return launch_ring<T, MODE, 512, 8, 1, false>(xp, op, n, outer, st);
+        if (np > 512ll * 8 && np <= 1024ll * 7)
+          return launch_ring<T, MODE, 1024, 7, 2, MODE == SM_FWD && sizeof(T) == 2>(xp, op, n, outer, st);
       }
     }
 #define NB_SM_LAUNCH(GG, VV, KK)                                                                       \

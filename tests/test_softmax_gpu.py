@@ -81,6 +81,20 @@ def test_long_columns_arriving_ahead(dtype, n, cols):
         assert torch.allclose(got, want, rtol=TOL[dtype] if dtype != torch.float32 else 1e-5, atol=1e-9 if dtype != torch.float16 else 6e-8)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("n,cols", [(32776, 592), (50000, 700), (57344, 592), (57352, 592), (50000, 300)])
+def test_softmax_of_very_long_16_bit_columns_is_rounded_once(dtype, n, cols):
+    """Columns that no kernel keeps the exponentials of, fetched ahead or not: half a unit of the element type, and 2^-16
+    for the exponentials and their Float32 sum."""
+    gen = torch.Generator(device="cuda").manual_seed(n + cols)
+    x = torch.empty((cols, n), device=DEV).normal_(0, 3, generator=gen).to(dtype).t()
+    y = SM.softmax(x).t().double()
+    want = torch.softmax(x.t().double(), 1)
+    digits, sub = (8, 0.0) if dtype == torch.bfloat16 else (11, 2.0 ** -25)
+    half = torch.clamp(torch.ldexp(torch.ones_like(want), torch.frexp(want).exponent - 1 - digits), min=sub)
+    assert bool(((y - want).abs() <= half + 2.0 ** -16 * want).all())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("shape,dims", [((300, 33), 1), ((70000, 3), 1), ((64, 50, 4), 2)])
 def test_in_place_forms(dtype, shape, dims):
