@@ -218,7 +218,8 @@ __device__ __forceinline__ void bwd_block(const AttnArgs& a, const BwdArgs& g, c
         const int ql = qi - i0, kl = kj - j0;
         float pv = ninf();                                 // marks a score without any part in the result
         if (plain) {
-          if (L != ninf()) pv = expf(p[i][j] * a.scale - L);
+          const float t = p[i][j] * a.scale;
+          if (L != ninf() && t != ninf()) pv = expf(t - L);
         } else if (gr < n_rows && gc < n_cols && L != ninf()) {
           const float t = finish_logit(a, p[i][j], kj, qi, h, b);
           if (t != ninf()) pv = expf(t - L);

@@ -1951,6 +1951,33 @@ def test_float32_masked_keys_may_hold_anything():
         np.testing.assert_array_equal(got, want)
 
 
+@pytest.mark.parametrize("L", [128, 100])
+def test_float32_keys_with_logits_of_minus_infinity_may_hold_anything(L):
+    """The same without a mask: a key whose logits are all -Inf takes no part, and whatever v holds there the gradients
+    of the others are those of the call without it, on whole tiles as on ragged ones and in both forms."""
+    rng = np.random.default_rng(28)
+    f32, d, H, B, dead = torch.float32, 64, 4, 2, 37
+    qn = np.abs(rng.standard_normal((d * H, L, B), dtype=np.float32)) + np.float32(0.01)
+    kn, vn, dyn = (rng.standard_normal((d * H, L, B), dtype=np.float32) for _ in range(3))
+    live = np.arange(L) != dead
+    want = O.dot_product_attention_grad(qn, kn[:, live], vn[:, live], dyn, None, nheads=H)
+    kn[:, dead] = -np.inf
+    for value in (0.0, np.inf, np.nan):
+        vn[:, dead] = value
+        x, _, back = nb.dot_product_attention_pullback(_dev(qn, f32), _dev(kn, f32), _dev(vn, f32), nheads=H)
+        for deterministic in (False, True):
+            torch.use_deterministic_algorithms(deterministic, warn_only=True)
+            try:
+                dq, dk, dv, _ = (None if t is None else nb.jl_to_numpy(t) for t in back(_dev(dyn, f32)))
+            finally:
+                torch.use_deterministic_algorithms(False)
+            what = f"v = {value}, deterministic={deterministic}"
+            _grad_close(dq, want[0], f32, "dq, " + what)
+            _grad_close(dk[:, live], want[1], f32, "dk, " + what)
+            _grad_close(dv[:, live], want[2], f32, "dv, " + what)
+            assert not dk[:, dead].any() and not dv[:, dead].any(), what
+
+
 def _key_shares(pr):
     """Shares the library cuts the keys of a unit into for this call (0: not split), from the workspace it asks for:
     a maximum, a sum (rounded up to 4 floats in all) and dv partial outputs per share and query."""
