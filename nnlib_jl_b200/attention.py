@@ -620,7 +620,8 @@ def dot_product_attention_pullback(q, k, v, bias=None, *, fdrop: Callable = iden
         if scratch is None:
             scratch = torch.empty(4 * pr.Lq * pr.H * pr.B, dtype=torch.uint8, device=pr.dev)
         g.delta = scratch.data_ptr()
-        back.path = lib.nnlib_b200_attn_bwd_path(C.byref(pr.p), C.byref(g))   # PATH_UMMA / PATH_SIMT, for tests
+        # for tests: PATH_UMMA / PATH_SIMT, and whether that was the form of one pass with a workspace
+        back.path, back.one_pass = lib.nnlib_b200_attn_bwd_path(C.byref(pr.p), C.byref(g)), need > 0
         with _on_device(pr.dev):
             _check(lib.nnlib_b200_attn_bwd_ws(C.byref(pr.p), C.byref(g), scratch.data_ptr(), need, _stream()) if need else
                    lib.nnlib_b200_attn_bwd(C.byref(pr.p), C.byref(g), _stream()), "attn_bwd")

@@ -1817,6 +1817,82 @@ def test_query_gradient_of_a_ragged_tile_is_the_same_every_time():
     assert all(torch.equal(back(dy)[0], first) for _ in range(400))
 
 
+def test_query_gradient_of_the_two_halves_is_the_same_every_time():
+    """The case above through the two half backwards, whose dq half is the one in which a warp without rows runs ahead
+    (the one-pass backward is told apart by its workspace, and sums dq in any order)."""
+    rng = np.random.default_rng(24)
+    d, H, Lq, Lkv, B = 48, 3, 333, 295, 2
+    q, k, v, dy = (_dev(_round_to(rng.standard_normal((d * H, n, B)), torch.bfloat16), torch.bfloat16)
+                   for n in (Lq, Lkv, Lkv, Lq))
+    bias = _dev(_round_to(0.5 * rng.standard_normal((Lkv, 1, 1, B)), torch.bfloat16), torch.bfloat16)
+    for lens in ([226, 168], [295, 290]):
+        mask = nb.jl_from_numpy(np.arange(Lkv)[:, None, None, None] < np.array(lens)[None, None, None, :], device=DEV)
+        x, _, back = nb.dot_product_attention_pullback(q, k, v, bias, mask=mask, nheads=H, fdrop=nb.PhiloxDropout(0.25, seed=7))
+        torch.use_deterministic_algorithms(True, warn_only=True)
+        try:
+            first = back(dy)[0].clone()
+            assert back.path == nb._lib.PATH_UMMA and not back.one_pass
+            assert all(torch.equal(back(dy)[0], first) for _ in range(400))
+        finally:
+            torch.use_deterministic_algorithms(False)
+        back(dy)
+        assert back.one_pass
+
+
+@pytest.mark.parametrize("seed", range(24))
+def test_random_configurations_of_both_backwards_match_the_gradient_oracle(seed):
+    """Seeded draws of the calls that the one-pass backwards take (16-bit: every mask form, bias, dropout; Float32 without
+    a bias), each through them and through the two halves."""
+    rng = np.random.default_rng(9500 + seed)
+    dtype = [torch.bfloat16, torch.float16, torch.float32][seed % 3]
+    half = dtype != torch.float32
+    d = int(rng.choice([64, 128, 32, 48, 80, 8, 96]))
+    H, B = int(rng.integers(2, 5)), int(rng.integers(1, 4))
+    Lkv = int(rng.integers(129, 600)) if half else int(rng.integers(65, 300))
+    Lq = int(rng.integers(1, 450)) if half else int(rng.integers(65, 300))
+    qn, kn, vn, dyn = (_round_to(rng.standard_normal((d * H, n, B)), dtype) for n in (Lq, Lkv, Lkv, Lq))
+    kind = ["none", "causal", "offset", "keypad", "random", "matrix"][int(rng.integers(0, 6))]
+    if half and kind == "offset":
+        kind = "causal"                                    # (an offset goes to the CUDA-core kernels)
+    mask_np = mask_arg = None
+    if kind in ("causal", "offset"):
+        off = 0 if kind == "causal" else int(rng.integers(0, Lkv))
+        mask_np, mask_arg = _offset_mask(Lkv, Lq, off), nb.CausalMask(off)
+    elif kind != "none":
+        if kind == "keypad":
+            mask_np = np.arange(Lkv)[:, None, None, None] < rng.integers(1, Lkv + 1, size=B)[None, None, None, :]
+        else:
+            mask_np = rng.random({"random": (Lkv, Lq, H, B), "matrix": (Lkv, Lq)}[kind]) > 0.3
+            mask_np[0] = True
+        mask_arg = nb.jl_from_numpy(mask_np, device=DEV)
+    bn = None
+    if half and rng.random() < 0.4:
+        bn = _round_to(0.5 * rng.standard_normal([(Lkv, Lq, H, B), (Lkv, Lq), (Lkv, 1, 1, B)][int(rng.integers(0, 3))]), dtype)
+    p = float(rng.choice([0.0, 0.0, 0.1, 0.4]))
+    fdrop = nb.PhiloxDropout(p, seed=seed, offset=7) if p > 0 else nb.identity
+    keep = P.keep_mask((Lkv, Lq, H, B), p, seed, 7) if p > 0 else None
+    what = f"seed {seed}: {dtype} d={d} H={H} {Lq} x {Lkv} B={B} {kind} bias={None if bn is None else bn.shape} p={p}"
+    x, _, back = nb.dot_product_attention_pullback(_dev(qn, dtype), _dev(kn, dtype), _dev(vn, dtype),
+                                                   None if bn is None else _dev(bn, dtype), mask=mask_arg, nheads=H, fdrop=fdrop)
+    want = O.dot_product_attention_grad(qn, kn, vn, dyn, bn, mask=mask_np, nheads=H, keep=keep, p=p)
+    dy, forms = _dev(dyn, dtype), set()
+    for deterministic in (False, True):
+        torch.use_deterministic_algorithms(deterministic, warn_only=True)
+        try:
+            got = back(dy)
+        finally:
+            torch.use_deterministic_algorithms(False)
+        forms.add(back.one_pass)
+        for name, g, w in zip(("dq", "dk", "dv", "dbias"), got, want):
+            if g is not None:
+                _grad_close(nb.jl_to_numpy(g), w, dtype, f"{name}, one_pass={back.one_pass}, {what}")
+    nb.device_health()
+    key_tiles, query_tiles = -(-Lkv // 128), -(-Lq // 128)
+    if half and (key_tiles * H * B >= 16 or query_tiles <= 2 * key_tiles):
+        assert forms == {True, False}, what
+    assert False in forms
+
+
 # --------------------------------------------------------------------------
 # tiled CUDA-core kernels (exact Float32)
 # --------------------------------------------------------------------------
@@ -1921,6 +1997,37 @@ def test_float32_backward_in_one_pass(d, dv, H, Lq, Lkv, B, kind, drop):
         assert torch.equal(g, a), name
         # sums of at most 4000 products in another order: 4000 half ulps of the largest at the very most
         assert (g - o).abs().max() <= 4000 * 6e-8 * o.abs().max(), name
+
+
+@pytest.mark.parametrize("d,H,L,B,causal,drop,chunks", [
+    (64, 8, 512, 8, True, 0.0, 1),      # keys enough: whole walks of 8 .. 1 tiles, dk and dv stored at once
+    (64, 8, 512, 2, True, 0.0, 4),      # walks of two tiles; the later keys' merge begins at a later part
+    (128, 2, 640, 1, True, 0.1, 10),    # walks of one tile
+    (40, 4, 500, 4, False, 0.2, 4),     # walks of two tiles, ragged at the end
+])
+def test_float32_backward_in_one_pass_with_longer_walks(d, H, L, B, causal, drop, chunks):
+    """Walks over several tiles of queries, whole and cut: the form is asserted by its workspace (D, a partial dq of every
+    tile of scores and, where the walks are cut, a partial dk and dv of every part)."""
+    rng = np.random.default_rng(81 + d + B)
+    f32 = torch.float32
+    qn, kn, vn, dyn = (rng.standard_normal((d * H, L, B), dtype=np.float32) for _ in range(4))
+    fd = nb.PhiloxDropout(drop, seed=9, offset=4) if drop > 0 else nb.identity
+    keep = P.keep_mask((L, L, H, B), drop, 9, 4) if drop > 0 else None
+    x, alpha, back = nb.dot_product_attention_pullback(_dev(qn, f32), _dev(kn, f32), _dev(vn, f32), nheads=H, fdrop=fd,
+                                                       mask=nb.CausalMask() if causal else None)
+    dy = _dev(dyn, f32)
+    got, again = back(dy), back(dy)
+    assert back.one_pass
+    p, g = alpha._problem.p, _lib.AttnGrads()
+    g.dx, g.dq, g.dk, g.dv = dy.data_ptr(), got[0].data_ptr(), got[1].data_ptr(), got[2].data_ptr()
+    t, units = -(-L // 64), H * B
+    assert _lib.load().nnlib_b200_attn_bwd_workspace_bytes(ctypes.byref(p), ctypes.byref(g)) == \
+        4 * (L * units + units * t * t * 64 * d + (units * t * chunks * 64 * 2 * d if chunks > 1 else 0))
+    want = O.dot_product_attention_grad(qn, kn, vn, dyn, None, mask=_offset_mask(L, L, 0) if causal else None, nheads=H,
+                                        keep=keep, p=drop)
+    for name, o, a, w in zip(("dq", "dk", "dv"), got, again, want):
+        _grad_close(nb.jl_to_numpy(o), w, f32, name)
+        assert torch.equal(o, a), name
 
 
 def test_float32_masked_keys_may_hold_anything():
