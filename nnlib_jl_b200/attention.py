@@ -522,6 +522,28 @@ def _fused(q, k, v, bias, mask, nheads, dropout):
     return x, LazyAttnScores(pr, (pr.Lkv, pr.Lq, pr.H, pr.B))
 
 
+_SMALL_WORKSPACE = 32 << 20
+
+
+def _workspace(nbytes: int, dev: torch.device) -> Optional[torch.Tensor]:
+    """Device memory that a call is faster with but can do without, or None where there is none.  torch gives its whole
+    cache back to the driver before it reports that memory is short, and a program at its limit would pay for that on
+    every call: a large workspace is only asked for where torch's cache or the device has that much left."""
+    if nbytes >= _SMALL_WORKSPACE and not torch.cuda.is_current_stream_capturing():
+        try:
+            st = torch.cuda.memory_stats_as_nested_dict(dev)      # 8 us, the device's own count 70
+        except RuntimeError:                                      # an allocator of the program's own, without a count
+            st = None
+        if st:
+            cached = st["reserved_bytes"]["all"]["current"] - st["allocated_bytes"]["all"]["current"]
+            if cached < nbytes and torch.cuda.mem_get_info(dev)[0] < nbytes:
+                return None
+    try:
+        return torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    except torch.OutOfMemoryError:
+        return None
+
+
 def _launch_part(pr, units: int, piece: bool = False):
     """x of a part of a larger call of ``units`` (head, batch) units: a shard's heads and batches, a chunk of the
     batch.  The library takes the way it takes for the whole call wherever that way cuts a unit by its number of keys
@@ -611,13 +633,9 @@ def dot_product_attention_pullback(q, k, v, bias=None, *, fdrop: Callable = iden
         # algorithms gets the one that needs no workspace and adds in a fixed order
         need = 0 if torch.are_deterministic_algorithms_enabled() else \
             lib.nnlib_b200_attn_bwd_workspace_bytes(C.byref(pr.p), C.byref(g))
-        scratch = None
-        if need:
-            try:
-                scratch = torch.empty(need, dtype=torch.uint8, device=pr.dev)
-            except torch.OutOfMemoryError:
-                need = 0                     # the other one gets by with D
+        scratch = _workspace(need, pr.dev) if need else None
         if scratch is None:
+            need = 0                         # the other one gets by with D
             scratch = torch.empty(4 * pr.Lq * pr.H * pr.B, dtype=torch.uint8, device=pr.dev)
         g.delta = scratch.data_ptr()
         # for tests: PATH_UMMA / PATH_SIMT, and whether that was the form of one pass with a workspace

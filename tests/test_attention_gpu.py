@@ -1582,6 +1582,37 @@ def test_dropout_of_most_scores_keeps_small_float16_gradients(d):
             assert (off <= tol + 0.01 * np.abs(w)).all(), (name, deterministic, float((off / tol).max()))
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_backward_without_room_for_its_workspace(monkeypatch, dtype):
+    """The one-pass backward needs memory that a program near its limit may not have: the two halves then, and the next
+    call with room goes back to one pass."""
+    from nnlib_jl_b200 import attention as A
+    rng = np.random.default_rng(67)
+    qn, kn, vn, dyn = (_round_to(rng.standard_normal((128, n, 2)), dtype) for n in (300, 260, 260, 300))
+    x, _, back = nb.dot_product_attention_pullback(*(_dev(t, dtype) for t in (qn, kn, vn)), nheads=2)
+    dy = _dev(dyn, dtype)
+    want = O.dot_product_attention_grad(qn, kn, vn, dyn, None, nheads=2)
+    empty, tries = torch.empty, []
+
+    def short(n, *a, **kw):
+        if isinstance(n, int) and n > 4 * 300 * 2 * 2:
+            tries.append(n)
+            raise torch.OutOfMemoryError("none left")
+        return empty(n, *a, **kw)
+    monkeypatch.setattr(A.torch, "empty", short)
+    got = back(dy)
+    monkeypatch.undo()
+    assert len(tries) == 1 and not back.one_pass
+    for name, g, w in zip(("dq", "dk", "dv"), got, want):
+        _grad_close(nb.jl_to_numpy(g), w, dtype, name)
+    # more than the device has: not even tried
+    with torch.cuda.device(0):
+        assert A._workspace(1 << 45, torch.device("cuda", 0)) is None
+        assert A._workspace(64 << 20, torch.device("cuda", 0)).numel() == 64 << 20
+    back(dy)
+    assert back.one_pass
+
+
 def test_pullback_fully_masked_query_gives_no_gradient():
     """A query that attends to nothing has NaN output (src/softmax.jl:71-76); the library lets no gradient
     flow through it (both backward paths), so the other queries' gradients stay finite."""

@@ -189,3 +189,24 @@ def test_sharded_driver_rejects_opaque_fdrop():
     drv = S.ShardedAttention(["cpu:0"], compute=_cpu_compute)
     with pytest.raises(nb.ArgumentError):
         drv(q, q, q, fdrop=lambda a: a)
+
+
+@pytest.mark.parametrize("nbytes,cached,free,asked", [
+    (1 << 20, 0, 0, True),                   # small: simply asked for
+    (1 << 30, 1 << 30, 0, True),             # torch's cache has it
+    (1 << 30, 0, 1 << 30, True),             # the device has it
+    (1 << 30, 1 << 29, 1 << 29, False),      # neither: asking would cost the cache
+])
+def test_workspace_is_not_asked_for_at_the_memory_limit(monkeypatch, nbytes, cached, free, asked):
+    from nnlib_jl_b200 import attention as A
+    dev, asks = torch.device("cuda", 0), []
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(torch.cuda, "memory_stats_as_nested_dict", lambda d: {
+        "reserved_bytes": {"all": {"current": (1 << 33) + cached}}, "allocated_bytes": {"all": {"current": 1 << 33}}})
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda d: (free, 1 << 37))
+
+    def empty(n, dtype, device):
+        asks.append(n)
+        raise torch.OutOfMemoryError("none left")
+    monkeypatch.setattr(torch, "empty", empty)
+    assert A._workspace(nbytes, dev) is None and asks == ([nbytes] if asked else [])
