@@ -629,6 +629,17 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                 if (8 * j + e < first) su[k >> 1][4 * j + 2 * (k & 1) + e] = 0u;
           }
         }
+        // padded queries have lse = +inf, which the last query's bias (read in their place) may be as well, or NaN
+        if (BIAS && c0 + 128 > a.Lq) {
+          const int last = a.Lq - c0 - cb;
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+#pragma unroll
+              for (int e = 0; e < 2; ++e)
+                if (8 * j + e >= last) su[k >> 1][4 * j + 2 * (k & 1) + e] = 0u;
+        }
         if (MASKED && mask_per_step) {
 #pragma unroll
           for (int k = 0; k < 4; ++k)

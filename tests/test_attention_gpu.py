@@ -1551,6 +1551,35 @@ def test_both_tensor_core_backwards_match_the_gradient_oracle(dtype, d, H, Lq, L
         assert not deterministic or all(torch.equal(a, b) for a, b in zip(got[:3], again[:3]))
 
 
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("dtype,bias_dtype,d,drop", [
+    (torch.bfloat16, torch.bfloat16, 128, 0.0), (torch.float16, torch.float32, 64, 0.0), (torch.float16, torch.float16, 64, 0.2),
+])
+def test_pullback_takes_nothing_from_the_bias_where_the_mask_is_false(dtype, bias_dtype, d, drop, value):
+    """Keys that a query does not see may have any bias (the reference replaces the logit), in the last query's row, which
+    is read in the place of the rows past the end, too."""
+    rng = np.random.default_rng(68)
+    H, Lq, Lkv, B = 2, 100, 127, 2
+    qn, kn, vn, dyn = (_round_to(rng.standard_normal((d * H, n, B)), dtype) for n in (Lq, Lkv, Lkv, Lq))
+    bn = _round_to(0.5 * rng.standard_normal((Lkv, Lq, H, B)), bias_dtype)
+    mask_np = np.arange(Lkv)[:, None] <= np.arange(Lq)[None, :]
+    fd = nb.PhiloxDropout(drop, seed=5, offset=1) if drop > 0 else nb.identity
+    keep = P.keep_mask((Lkv, Lq, H, B), drop, 5, 1) if drop > 0 else None
+    want = O.dot_product_attention_grad(qn, kn, vn, dyn, bn, mask=mask_np, nheads=H, keep=keep, p=drop)
+    bn[~mask_np] = value
+    x, _, back = nb.dot_product_attention_pullback(_dev(qn, dtype), _dev(kn, dtype), _dev(vn, dtype), _dev(bn, bias_dtype),
+                                                   mask=nb.CausalMask(), nheads=H, fdrop=fd)
+    for deterministic in (False, True):
+        torch.use_deterministic_algorithms(deterministic, warn_only=True)
+        try:
+            got = back(_dev(dyn, dtype))
+        finally:
+            torch.use_deterministic_algorithms(False)
+        assert back.one_pass != deterministic
+        for name, g, w in zip(("dq", "dk", "dv", "dbias"), got, want):
+            _grad_close(nb.jl_to_numpy(g), w, dtype, f"{name}, deterministic={deterministic}")
+
+
 @pytest.mark.parametrize("d", [64, 128])
 def test_dropout_of_most_scores_keeps_small_float16_gradients(d):
     """dS = P (dP keep / (1 - p) - D) of both 16-bit backwards with p = 15/16 and dS of 2^-24 to 2^-18, among Float16's
