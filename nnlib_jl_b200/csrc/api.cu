@@ -450,13 +450,22 @@ static bool use_bwd_fused(const AttnArgs& a, BwdArgs b, int dtype) {
 // Float32 in one pass on the CUDA cores: five products instead of seven.  By the number of tiles, whichever form needs
 // fewer products one after the other: the longest walk of a block or the whole of the work over the blocks that fit at
 // once (the launch that merges the parts counts as one).  64 keys and queries of 4 units 26 us in two halves and 24 in
-// one pass, 100 of 8 units 32 and 25, the larger ones in attn_bwd_fma.cu.  The workspace, a Float32 per score for d = 64,
+// one pass, 100 of 8 units 32 and 25, the larger ones in attn_bwd_fma.cu.  Keys that the causal flag hides from all
+// queries give blocks without work; few of them (up to one and a half times what fits at once) cost nothing and do not
+// count: 58 queries and 740 keys of 8 units 19.5 us in two halves and 24.9 in one pass, while 87 and 1103 of 64 units,
+// d = 96, take 97 and 78.  The workspace, a Float32 per score for d = 64,
 // ends at 1 GiB.  (With a gradient of the bias the half that owns queries stays: its lanes add to neighbouring elements of it.)
 static bool use_bwd_fma_all(const AttnArgs& a, const BwdArgs& b, int dtype) {
   if (a.Lq < 1 || a.B < 1 || a.Lkv < 1 || dtype != NNLIB_B200_F32 || b.dbias || force_simt() || !fma_supports(a.d, a.dv)) return false;
-  const double kt = (a.Lkv + 63ll) / 64, qt = (a.Lq + 63ll) / 64, tiles = kt * qt * a.H * a.B * (a.causal ? 0.5 : 1.0);
+  const double units = (double)a.H * a.B, all_kt = (a.Lkv + 63ll) / 64, qt = (a.Lq + 63ll) / 64;
   const double at_once = 148 * (a.d <= 64 && a.dv <= 64 ? 2 : 1), len = fma_bwd_chunk(a);
-  if (kt * qt * a.H * a.B * 64 * (a.d + 4) * 4 > (double)(1 << 30)) return false;
+  if (all_kt * qt * units * 64 * (a.d + 4) * 4 > (double)(1 << 30)) return false;
+  double kt = all_kt;
+  if (a.causal && all_kt * units <= 1.5 * at_once) {
+    const long long seen = std::min((long long)a.Lkv, std::max(1ll, (long long)a.Lq + a.coff));
+    kt = (seen + 63) / 64;
+  }
+  const double tiles = kt * qt * units * (a.causal ? 0.5 : 1.0);
   return std::max(5 * len, 5 * tiles / at_once) + 1 < std::max(std::max(4 * qt, 3 * kt), 7 * tiles / at_once);
 }
 

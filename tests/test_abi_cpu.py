@@ -108,6 +108,17 @@ def test_backward_workspace_query_without_a_gpu(lib):
     assert lib.nnlib_b200_attn_bwd_ws(C.byref(_params()), C.byref(_grads()), None, 0, None) == _lib.INVALID_ARG
 
 
+def test_float32_backward_in_one_pass_only_where_it_is_quicker(lib):
+    """Causal calls with more keys than queries: blocks of keys that no query sees count where they fill the GPU."""
+    def need(d, H, Lq, Lkv, off=0, causal=1):
+        p = _params(lse=0x2000, dtype=_lib.F32, d=d, dv=d, H=H, Lq=Lq, Lkv=Lkv, B=1, causal=causal, causal_offset=off)
+        return lib.nnlib_b200_attn_bwd_workspace_bytes(C.byref(p), C.byref(_grads()))
+    assert need(64, 8, 58, 740) == 0 and need(64, 16, 83, 1323) == 0 and need(96, 16, 369, 731) == 0
+    assert need(64, 8, 58, 740, off=682) > 0 and need(64, 8, 58, 740, causal=0) > 0     # every key is seen
+    assert need(96, 64, 87, 1103) > 0                                                   # 1152 blocks
+    assert need(64, 8, 740, 58) > 0 and need(64, 8, 512, 512) > 0
+
+
 def test_backward_argument_checks_and_path_without_a_gpu(lib):
     p = _params(lse=0x2000)
     # the forward's lse is required, so are dx / dq / dk / dv / delta, and the struct size is checked
