@@ -435,16 +435,24 @@ int nnlib_b200_attn_bwd(const nnlib_b200_attn_params* p, const nnlib_b200_attn_g
                                                          : simt_bwd(a, b, p->dtype, (cudaStream_t)stream));
 }
 
-// The one-pass backward: what the tensor-core backward takes, given a workspace, but for a handful of key tiles (a CTA
-// each) with long walks over the queries, which the dq half spreads over the GPU: 128 keys and 4096 queries of 4 units
-// 61 us in two halves, 71 in one pass; of 32 units 101 and 88; 300 keys and 8000 queries of 4 units 129 and 137;
-// 1024 keys and queries of 4 units 45 and 39.  Its arguments are those of the two halves but for delta, which it does
-// not use.
+// The one-pass backward: what the tensor-core backward takes, given a workspace, but for calls in which the launch that it
+// takes more or its few long walks (a CTA for 128 keys) cost more than the second pass, which the dq half spreads over the
+// GPU.  A single tile of scores with nothing but the causal flag: 116 x 116 of 4 units, d = 80, 16.9 us in two halves and
+// 18.6 in one pass, 113 x 113 of 16 units, d = 32, 12.9 and 13.6.  Many tiles of queries for few of keys: 128 keys and 4096
+// queries of 4 units 61 and 71, of 32 units 101 and 88; 138 keys and 3207 queries of 8 units under a mask, d = 96, 195 and
+// 246.  What the halves do twice moves the line: with dropout (or a mask where d = 64) 16 tiles of keys are enough
+// (1565 x 92 of 16 units, d = 64, 76 and 56; 652 x 107 of 16 units under a mask, d = 32, 46 and 41), and so do their strided
+// reads of a bias (2380 x 948 of 2 units 209 and 166; 741 x 92 of 16 units 54 and 69).  Of 2230 random calls 87
+// are more than 3 % slower than in two halves (251 with 16 tiles of keys, or at most two tiles of queries per one of keys, for all).
+// Its arguments are those of the two halves but for delta, which it does not use.
 static bool use_bwd_fused(const AttnArgs& a, BwdArgs b, int dtype) {
   if (!b.delta) b.delta = a.lse;
   if (a.Lq < 1 || a.B < 1 || force_simt() || !umma_bwd_supports(a, b, dtype)) return false;
-  const long long key_tiles = (a.Lkv + 127ll) / 128, query_tiles = (a.Lq + 127ll) / 128;
-  return key_tiles * a.H * a.B >= 16 || query_tiles <= 2 * key_tiles;
+  const bool drop = a.dropout_p > 0.f;
+  const long long kt = (a.Lkv + 127ll) / 128, qt = (a.Lq + 127ll) / 128, all_kt = kt * a.H * a.B;
+  if (kt == 1 && qt == 1) return drop || a.mask || a.bias;
+  const bool twice = drop || (a.mask && !a.bias && a.d <= 64);
+  return all_kt >= (twice ? 16 : 32) || qt <= (a.bias && !drop && kt > 1 ? 3 : twice || all_kt >= 16 ? 2 : 1) * kt;
 }
 
 // Float32 in one pass on the CUDA cores: five products instead of seven.  By the number of tiles, whichever form needs

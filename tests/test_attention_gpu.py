@@ -1727,7 +1727,7 @@ def test_abi_backward_causal_flag_on_a_head_slice(Lq, Lkv):
 @pytest.mark.parametrize("Lq,Lkv,B,drop,pad", [
     (100, 300, 2, 0.0, 0),      # two tiles of keys behind the only tile of queries
     (100, 300, 1, 0.2, 24),     # the same with dropout; lse of the shard inside a larger array, padded dx
-    (515, 130, 4, 0.0, 8),      # more queries than keys
+    (515, 130, 8, 0.0, 8),      # more queries than keys
     (260, 700, 1, 0.0, 0),      # six tiles of keys, three of queries
 ])
 def test_abi_one_pass_backward_on_a_head_slice(Lq, Lkv, B, drop, pad):
@@ -1877,6 +1877,29 @@ def test_query_gradient_of_a_ragged_tile_is_the_same_every_time():
     assert all(torch.equal(back(dy)[0], first) for _ in range(400))
 
 
+@pytest.mark.parametrize("one_pass,units,Lq,Lkv,d,extra", [
+    (False, 4, 116, 116, 80, "causal"), (True, 4, 116, 116, 80, "drop"), (True, 4, 116, 130, 80, ""),
+    (False, 8, 3207, 138, 96, "mask"), (True, 16, 3207, 138, 96, "mask"), (True, 8, 3207, 138, 64, "mask"),
+    (False, 16, 741, 92, 128, "bias"), (True, 2, 2380, 948, 64, "bias"), (True, 16, 1565, 92, 64, "drop"),
+    (False, 8, 2855, 250, 80, ""), (True, 32, 4096, 4096, 128, "causal"), (True, 4, 300, 290, 128, "mask"),
+])
+def test_one_pass_backward_is_taken_where_it_is_quicker(one_pass, units, Lq, Lkv, d, extra):
+    """Both sides of the rule (queries of the workspace: nothing runs, the pointers are made up)."""
+    p, g = _lib.AttnParams(), _lib.AttnGrads()
+    p.dtype, p.d, p.dv, p.H, p.B, p.Lq, p.Lkv = _lib.BF16, d, d, units, 1, Lq, Lkv
+    p.q = p.k = p.v = p.x = p.lse = g.dx = g.dq = g.dk = g.dv = 0x10000
+    if extra == "causal":
+        p.causal = 1
+    elif extra == "drop":
+        p.dropout_p = 0.1
+    elif extra == "mask":
+        p.mask, p.mask_stride = 0x10000, (ctypes.c_int64 * 4)(1, Lkv, 0, 0)
+    elif extra == "bias":
+        p.bias, p.bias_dtype, p.bias_stride = 0x10000, _lib.BF16, (ctypes.c_int64 * 4)(1, Lkv, 0, 0)
+    need = _lib.load().nnlib_b200_attn_bwd_workspace_bytes(ctypes.byref(p), ctypes.byref(g))
+    assert (need > 0) == one_pass
+
+
 def test_query_gradient_of_the_two_halves_is_the_same_every_time():
     """The case above through the two half backwards, whose dq half is the one in which a warp without rows runs ahead
     (the one-pass backward is told apart by its workspace, and sums dq in any order)."""
@@ -1948,7 +1971,7 @@ def test_random_configurations_of_both_backwards_match_the_gradient_oracle(seed)
                 _grad_close(nb.jl_to_numpy(g), w, dtype, f"{name}, one_pass={back.one_pass}, {what}")
     nb.device_health()
     key_tiles, query_tiles = -(-Lkv // 128), -(-Lq // 128)
-    if half and (key_tiles * H * B >= 16 or query_tiles <= 2 * key_tiles):
+    if half and (key_tiles * H * B >= 32 or query_tiles <= key_tiles):
         assert forms == {True, False}, what
     assert False in forms
 
