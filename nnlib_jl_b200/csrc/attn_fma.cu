@@ -73,7 +73,7 @@ __device__ __forceinline__ float make_lse(float m, float l) {
 
 template <int DP, int BM>
 __host__ __device__ constexpr int kp_floats() { return kBN * (DP + 4) > BM * kLDP ? kBN * (DP + 4) : BM * kLDP; }
-// AHEAD (x in one pass, heads up to 96): the P tile has a place of its own, and the next K and V tiles are copied while
+// AHEAD (x in one pass, heads up to 96, see launch_fma_mi): the P tile has a place of its own, and the next K and V tiles are copied while
 // the block works on this one (with larger heads it would cost the second block on an SM); tiles that need nothing but
 // the scale are told apart.  512 x 512, d = 64, 64 units 267 -> 217 us, causal 134 -> 122, 2048 x 2048 causal, 16 units
 // 504 -> 432.
@@ -432,9 +432,15 @@ __global__ void __launch_bounds__(NTHR) attn_fma_row_kernel(const AttnArgs a, co
 // block would be padding.
 template <typename T, int DP, int MI, int MODE, bool AHEAD = false>
 cudaError_t launch_fma_mi(const AttnArgs& a, int vec, cudaStream_t st, int n_splits = 1) {
-  // walks of one or two tiles with a ragged end have nothing to gain: 102 x 102 causal, 320 units 61.5 us, 64.0 ahead
+  // Ahead where most tiles can be plain and enough blocks share an SM for their number (two or three instead of three or
+  // four) not to matter, by the tiles of 64 x 64 scores: 4 an SM, of causal calls, whose walks differ, 12.  Gains there
+  // are 2 to 16 % (742 x 742 of 32 units, d = 64: 5), below them and with a bias or a mask array the same kernels lose as
+  // much: 586 x 144 of 32 units, padding 60.0 us, 63.9 ahead; 126 x 343 of 8 units, d = 32, 33.8 and 36.2; 345 x 345 of 64
+  // units, causal 95 and 98.  Walks of one or two tiles have nothing to gain: 102 x 102 causal, 320 units 61.5, 64.0 ahead.
   if constexpr (MODE == FM_FWD && DP <= 96 && !AHEAD) {
-    if (a.Lkv > 2 * kBN || a.Lkv % kBN == 0) return launch_fma_mi<T, DP, MI, MODE, true>(a, vec, st, n_splits);
+    const long long tiles = ((a.Lq + 63ll) / 64) * ((a.Lkv + kBN - 1ll) / kBN) * a.H * a.B;
+    if (!a.bias && !a.mask && a.Lq >= 128 && a.Lkv > 2 * kBN && tiles >= (a.causal ? 2 * 12 : 4) * 148)
+      return launch_fma_mi<T, DP, MI, MODE, true>(a, vec, st, n_splits);
   }
   constexpr int NTHR = 128, BM = NTHR / 16 * MI;
   constexpr int smem = fma_smem<DP, BM, MODE, AHEAD>();
