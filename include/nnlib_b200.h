@@ -272,12 +272,14 @@ NNLIB_B200_API int nnlib_b200_attn_bwd(const nnlib_b200_attn_params* p, const nn
                                        void* stream);
 
 /* The same pullback in one pass over the scores instead of two (five products per block of scores instead of
-   seven).  On the tensor cores dq is gathered in Float32 in the caller's workspace by atomic additions, whose order is
-   not fixed, so that dq may differ in its last bit from one call to the next (nnlib_b200_attn_bwd gives the same bits
-   each time); Float32 arrays leave partial results there, which are added in a fixed order.  workspace: device memory, 16-byte aligned, at least
-   nnlib_b200_attn_bwd_workspace_bytes(p, g) bytes, which need not be cleared and is free again when the call's
-   kernels have run.  A result of 0 bytes: no workspace is used and the call is nnlib_b200_attn_bwd.  g->delta is
-   not used where a workspace is. */
+   seven).  On the tensor cores dq is gathered in Float32 in the caller's workspace by atomic additions, one for every 128
+   keys, whose order is not fixed: an element of dq may differ from one call to the next by about
+   (Lkv / 128) * 2^-24 * the sum of the additions' absolute values, and by the rounding of that to the element type.
+   Where the additions nearly cancel that is more than its last bit.  nnlib_b200_attn_bwd gives the same bits each
+   time, and so do Float32 arrays here, which leave partial results in the workspace that are added in a fixed order.
+   workspace: device memory, 16-byte aligned, at least nnlib_b200_attn_bwd_workspace_bytes(p, g) bytes, which need not
+   be cleared and is free again when the call's kernels have run.  A result of 0 bytes: no workspace is used and the
+   call is nnlib_b200_attn_bwd.  g->delta is not used where a workspace is. */
 NNLIB_B200_API size_t nnlib_b200_attn_bwd_workspace_bytes(const nnlib_b200_attn_params* p, const nnlib_b200_attn_grads* g);
 NNLIB_B200_API int nnlib_b200_attn_bwd_ws(const nnlib_b200_attn_params* p, const nnlib_b200_attn_grads* g,
                                           void* workspace, size_t workspace_bytes, void* stream);

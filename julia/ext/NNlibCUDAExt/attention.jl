@@ -426,9 +426,12 @@ function ChainRulesCore.rrule(::typeof(dot_product_attention), q::DenseCuArray{T
             dv=reinterpret(CuPtr{Cvoid}, pointer(dv)),
             dbias=dbias32 === nothing ? CuPtr{Float32}(0) : pointer(dbias32),
             dbias_stride=dbias32 === nothing ? (0, 0, 0, 0) : _bcast_strides("bias", dbias32, (p.Lkv, p.Lq, p.H, p.B)))
-        # one pass over the scores where the library asks for a workspace (dq is then summed by atomic additions)
-        need = ccall((:nnlib_b200_attn_bwd_workspace_bytes, libnnlib_b200[]), Csize_t,
-                     (Ref{B200AttnParams}, Ref{B200AttnGrads}), p, g)
+        # one pass over the scores where the library asks for a workspace.  dq of 16-bit arrays is then summed by atomic
+        # additions in no fixed order: a task that sets CUDA.math_mode!(CUDA.PEDANTIC_MATH) gets the two passes, which
+        # give the same bits each time (Python: torch.use_deterministic_algorithms)
+        need = CUDA.math_mode() == CUDA.PEDANTIC_MATH ? Csize_t(0) :
+            ccall((:nnlib_b200_attn_bwd_workspace_bytes, libnnlib_b200[]), Csize_t,
+                  (Ref{B200AttnParams}, Ref{B200AttnGrads}), p, g)
         scratch = try
             CuArray{Float32}(undef, need > 0 ? cld(Int(need), 4) : p.Lq * p.H * p.B)
         catch err

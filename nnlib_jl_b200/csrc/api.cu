@@ -441,8 +441,8 @@ int nnlib_b200_attn_bwd(const nnlib_b200_attn_params* p, const nnlib_b200_attn_g
 // 18.6 in one pass, 113 x 113 of 16 units, d = 32, 12.9 and 13.6.  Many tiles of queries for few of keys: 128 keys and 4096
 // queries of 4 units 61 and 71, of 32 units 101 and 88; 138 keys and 3207 queries of 8 units under a mask, d = 96, 195 and
 // 246.  What the halves do twice moves the line: with dropout (or a mask where d = 64) 16 tiles of keys are enough
-// (1565 x 92 of 16 units, d = 64, 76 and 56; 652 x 107 of 16 units under a mask, d = 32, 46 and 41), and so do their strided
-// reads of a bias (2380 x 948 of 2 units 209 and 166; 741 x 92 of 16 units 54 and 69).  Of 2230 random calls 87
+// (1565 x 92 of 16 units, d = 64, 76 and 56; 652 x 107 of 16 units under a mask, d = 32, 46 and 41); their strided reads
+// of a bias move it, too (2380 x 948 of 2 units 209 and 166; 741 x 92 of 16 units 54 and 69).  Of 2230 random calls 87
 // are more than 3 % slower than in two halves (251 with 16 tiles of keys, or at most two tiles of queries per one of keys, for all).
 // Its arguments are those of the two halves but for delta, which it does not use.
 static bool use_bwd_fused(const AttnArgs& a, BwdArgs b, int dtype) {
@@ -461,8 +461,7 @@ static bool use_bwd_fused(const AttnArgs& a, BwdArgs b, int dtype) {
 // one pass, 100 of 8 units 32 and 25, the larger ones in attn_bwd_fma.cu.  Keys that the causal flag hides from all
 // queries give blocks without work; few of them (up to one and a half times what fits at once) cost nothing and do not
 // count: 58 queries and 740 keys of 8 units 19.5 us in two halves and 24.9 in one pass, while 87 and 1103 of 64 units,
-// d = 96, take 97 and 78.  The workspace, a Float32 per score for d = 64,
-// ends at 1 GiB.  (With a gradient of the bias the half that owns queries stays: its lanes add to neighbouring elements of it.)
+// d = 96, take 97 and 78.  The workspace, a Float32 per score for d = 64, ends at 1 GiB.  (With a gradient of the bias the half that owns queries stays: its lanes add to neighbouring elements of it.)
 static bool use_bwd_fma_all(const AttnArgs& a, const BwdArgs& b, int dtype) {
   if (a.Lq < 1 || a.B < 1 || a.Lkv < 1 || dtype != NNLIB_B200_F32 || b.dbias || force_simt() || !fma_supports(a.d, a.dv)) return false;
   const double units = (double)a.H * a.B, all_kt = (a.Lkv + 63ll) / 64, qt = (a.Lq + 63ll) / 64;

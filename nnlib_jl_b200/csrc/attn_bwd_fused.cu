@@ -15,9 +15,10 @@
 //   warp 12          TMA: the first loads of all, then the ring of Q with the queries' lse and D;   warp 15: ring of dX
 //   warp 13          issues S and dV;   warp 14: issues dP, dQ and dK
 // Tensor memory columns, D = 128: S [0,128) | dP [128,256) | dV | dK; D = 64: S | dP | dV [256,320) | dK | dQ [384,448).
-// P^T (16 bits) is written over S, each thread over columns that it alone has read.  With D = 128 there is no room left
-// and dQ is written over dP, which makes a chain of a step: dP, the compute warps' dS, dQ, its way into registers, the
-// next dP.  So dQ is issued before dK, and a warp that takes dQ out holds a whole row of it in registers.
+// P^T (16 bits) is written over S, each warp over lanes and columns that it alone reads, once all its lanes have read
+// them.  With D = 128 there is no room left and dQ is written over dP, which makes a chain of a step: dP, the compute
+// warps' dS, dQ, its way into registers, the next dP.  So dQ is issued before dK, and a warp that takes dQ out holds a
+// whole row of it in registers.
 //
 // What bounds it, at config "bf16 causal, L = 4096, d = 128, 32 heads, 8 sequences" (cycles of a step, from clock reads
 // in a copy of the kernel): 3970 a step of 2560 cycles of tensor work.  The chain above takes about all of it: dP 770,
@@ -27,7 +28,7 @@
 // warps' tensor memory stores behind them in it, waiting: 5600 a step.  Polynomials in place of a quarter to half of
 // the exponentials shorten that phase (1345 -> 1080) and nothing else.  One backward (pre and post included) went
 // 4140 -> 2940 us there, 3560 -> 2670 for one sequence of 16384 and 16 heads, 473 -> 325 for 16 heads of d = 64,
-// L = 2048, 8 sequences, 1604 -> 769 for the same not causal with dropout.  Of a CTA's 46 us there 2.3 pass before its
+// L = 2048, 8 sequences, 1604 -> 773 for the same not causal with dropout.  Of a CTA's 46 us there 2.3 pass before its
 // first scores and 3.9 behind its last dS.
 #include <cuda.h>
 
@@ -346,7 +347,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
       uint8_t* out_s = smem + C::kOutOff + wq * 2 * C::kPieceBytes;
       // Which scores of the warp's 32 keys survived the forward's dropout, a word per query: drawn here, two steps ahead,
       // because these warps have the time: d = 64, 2048 x 2048, 128 units 882 us with the compute warps drawing and trading
-      // by votes, 765 so; d = 80, 1000 x 777, padding 139 and 126.  Lane L draws the call of (query L % 8 of eight, keys
+      // by votes, 773 so; d = 80, 1000 x 777, padding 139 and 128.  Lane L draws the call of (query L % 8 of eight, keys
       // 8 (L / 8) ..), and the bytes of a query's four calls are put together by exchanges.  Four calls in lockstep hide
       // each other's latency; beside a bias, with its stores, two in turn are quicker (256 x 2048, 256 units 906 and 978).
       auto draw_keep = [&](int it) {

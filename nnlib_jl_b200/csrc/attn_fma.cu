@@ -73,9 +73,9 @@ __device__ __forceinline__ float make_lse(float m, float l) {
 
 template <int DP, int BM>
 __host__ __device__ constexpr int kp_floats() { return kBN * (DP + 4) > BM * kLDP ? kBN * (DP + 4) : BM * kLDP; }
-// AHEAD (x in one pass, heads up to 96, see launch_fma_mi): the P tile has a place of its own, and the next K and V tiles are copied while
-// the block works on this one (with larger heads it would cost the second block on an SM); tiles that need nothing but
-// the scale are told apart.  512 x 512, d = 64, 64 units 267 -> 217 us, causal 134 -> 122, 2048 x 2048 causal, 16 units
+// AHEAD (x in one pass, heads up to 96; launch_fma_mi says when): the P tile has a place of its own, and the next K and V
+// tiles are copied while the block works on this one (with larger heads it would cost the second block on an SM); tiles
+// that need nothing but the scale are told apart.  512 x 512, d = 64, 64 units 267 -> 217 us, causal 134 -> 122, 2048 x 2048 causal, 16 units
 // 504 -> 432.
 template <int DP, int BM, int MODE, bool AHEAD>
 __host__ __device__ constexpr int fma_smem() {
