@@ -278,8 +278,9 @@ NNLIB_B200_API int nnlib_b200_attn_bwd(const nnlib_b200_attn_params* p, const nn
    Where the additions nearly cancel that is more than its last bit.  nnlib_b200_attn_bwd gives the same bits each
    time, and so do Float32 arrays here, which leave partial results in the workspace that are added in a fixed order.
    workspace: device memory, 16-byte aligned, at least nnlib_b200_attn_bwd_workspace_bytes(p, g) bytes, which need not
-   be cleared and is free again when the call's kernels have run.  A result of 0 bytes: no workspace is used and the
-   call is nnlib_b200_attn_bwd.  g->delta is not used where a workspace is. */
+   be cleared and is free again when the call's kernels have run.  A result of 0 bytes: the call is nnlib_b200_attn_bwd
+   (with g->delta, or where that is NULL with its Lq*H*B floats in the workspace, if one is given).  g->delta is not used
+   where a workspace is. */
 NNLIB_B200_API size_t nnlib_b200_attn_bwd_workspace_bytes(const nnlib_b200_attn_params* p, const nnlib_b200_attn_grads* g);
 NNLIB_B200_API int nnlib_b200_attn_bwd_ws(const nnlib_b200_attn_params* p, const nnlib_b200_attn_grads* g,
                                           void* workspace, size_t workspace_bytes, void* stream);

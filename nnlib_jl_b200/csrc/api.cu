@@ -491,7 +491,14 @@ int nnlib_b200_attn_bwd_ws(const nnlib_b200_attn_params* p, const nnlib_b200_att
   const int rc = resolve_bwd(p, g, &a, &b, true, false);
   if (rc) return rc;
   const bool fused = use_bwd_fused(a, b, p->dtype);
-  if (!fused && !use_bwd_fma_all(a, b, p->dtype)) return nnlib_b200_attn_bwd(p, g, stream);
+  if (!fused && !use_bwd_fma_all(a, b, p->dtype)) {
+    // (which calls use a workspace is a matter of speed: a caller that brings one need not bring delta, too)
+    nnlib_b200_attn_grads two = *g;
+    if (!two.delta && workspace && workspace_bytes >= sizeof(float) * (size_t)a.Lq * a.H * a.B &&
+        (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0)
+      two.delta = static_cast<float*>(workspace);
+    return nnlib_b200_attn_bwd(p, &two, stream);
+  }
   const size_t need = fused ? umma_bwd_fused_workspace_bytes(a) : fma_bwd_workspace_bytes(a);
   if (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 15u) != 0)
     return NNLIB_B200_WORKSPACE_TOO_SMALL;

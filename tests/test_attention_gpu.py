@@ -1900,6 +1900,37 @@ def test_one_pass_backward_is_taken_where_it_is_quicker(one_pass, units, Lq, Lkv
     assert (need > 0) == one_pass
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_abi_backward_with_a_workspace_that_the_call_does_not_need(dtype):
+    """A call for the two halves (a workspace of 0 bytes): D goes to the caller's workspace where delta is NULL."""
+    lib = _lib.load()
+    rng = np.random.default_rng(69)
+    H, d, L, B = 2, 64, 40, 2
+    qn, kn, vn, dyn = (_round_to(rng.standard_normal((H * d, L, B)), dtype) for _ in range(4))
+    q, k, v, dx = (_dev(a, dtype) for a in (qn, kn, vn, dyn))
+    x, dq, dk, dv = (nb.jl_zeros((H * d, L, B), dtype, DEV) for _ in range(4))
+    lse = torch.empty(L * H * B, dtype=torch.float32, device=DEV)
+    p, g = _lib.AttnParams(), _lib.AttnGrads()
+    p.dtype = _lib.BF16 if dtype == torch.bfloat16 else _lib.F32
+    p.d, p.dv, p.H, p.Lq, p.Lkv, p.B = d, d, H, L, L, B
+    p.q, p.k, p.v, p.x, p.lse = (t.data_ptr() for t in (q, k, v, x, lse))
+    g.dx, g.dq, g.dk, g.dv = (t.data_ptr() for t in (dx, dq, dk, dv))
+    st = torch.cuda.current_stream().cuda_stream
+    assert lib.nnlib_b200_attn_fwd(ctypes.byref(p), st) == 0
+    assert lib.nnlib_b200_attn_bwd_workspace_bytes(ctypes.byref(p), ctypes.byref(g)) == 0
+    n = 4 * L * H * B
+    ws = torch.empty(n + 16, dtype=torch.uint8, device=DEV)
+    ws[n:] = 7
+    run = lambda ptr, size: lib.nnlib_b200_attn_bwd_ws(ctypes.byref(p), ctypes.byref(g), ptr, size, st)
+    assert run(None, 0) == _lib.INVALID_ARG and run(ws.data_ptr(), n - 1) == _lib.INVALID_ARG
+    assert run(ws.data_ptr(), n) == 0
+    nb.device_health()
+    want = O.dot_product_attention_grad(qn, kn, vn, dyn, None, nheads=H)
+    for name, got, w in zip(("dq", "dk", "dv"), (dq, dk, dv), want):
+        _grad_close(nb.jl_to_numpy(got), w, dtype, name)
+    assert bool((ws[n:] == 7).all())
+
+
 def test_query_gradient_of_the_two_halves_is_the_same_every_time():
     """The case above through the two half backwards, whose dq half is the one in which a warp without rows runs ahead
     (the one-pass backward is told apart by its workspace, and sums dq in any order)."""
